@@ -9,6 +9,7 @@
 // with the logistic rate and the exact-time Poisson generator (LGN_nonlinear + get_spike,
 // src/discrete_input_convol.cu:1587-1821).
 #include "pv1_internal.cuh"
+#include "pv1_rng.cuh"
 
 namespace pv1 {
 
@@ -378,7 +379,7 @@ __global__ void lgn_rng_init_kernel(curandStateMRG32k3a *state, float *lnl, floa
     int id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= n) return;
     curandStateMRG32k3a s;
-    curand_init(seed, id, 0, &s);
+    mrg_seed(seed, id, &s);
     (void)curand_uniform(&s);
     lnl[id] = -logf(curand_uniform(&s));
     ltr[id] = 0.0f;

@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "pv1_internal.cuh"
+#include "pv1_rng.cuh"
 
 using pv1::kErrBarrier;
 
@@ -403,7 +404,7 @@ __global__ void lgn_tc_rng_init_kernel(curandStateMRG32k3a *state, float *lnl, f
     const int id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= n) return;
     curandStateMRG32k3a s;
-    curand_init(seed, id, 0, &s);
+    pv1::mrg_seed(seed, id, &s);
     lnl[id] = -logf(curand_uniform(&s));
     ltr[id] = 0.f;
     state[id] = s;

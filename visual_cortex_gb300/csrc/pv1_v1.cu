@@ -26,6 +26,7 @@
 // they stay in registers.
 #include <algorithm>
 #include "pv1_internal.cuh"
+#include "pv1_rng.cuh"
 
 namespace pv1 {
 
@@ -1656,8 +1657,8 @@ __global__ void v1_rng_init_kernel(curandStateMRG32k3a *cond, curandStateMRG32k3
     int id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= nV1) return;
     curandStateMRG32k3a a, b;
-    curand_init(seed, id, 0, &a);
-    curand_init(seed, (unsigned long long)nV1 + id, 0, &b);
+    mrg_seed(seed, id, &a);
+    mrg_seed(seed, (unsigned long long)nV1 + id, &b);
     (void)curand_uniform(&a);
     for (int q = trainDepth - 1; q > 0; q--) (void)curand_uniform(&a);
     cond[id] = a;
@@ -1687,8 +1688,8 @@ __global__ void __launch_bounds__(1024) v1_sp_init_kernel(V1Params P, unsigned l
     float sInfo = -1.f;
     if (active) {
         curandStateMRG32k3a a, nz;
-        curand_init(seed, id, 0, &a);
-        curand_init(seed, (unsigned long long)nV1 + id, 0, &nz);
+        mrg_seed(seed, id, &a);
+        mrg_seed(seed, (unsigned long long)nV1 + id, &nz);
         float *ru = recU ? recU + (size_t)id * 2 * depth : nullptr;
         int nu = 0;
         auto draw = [&]() {
