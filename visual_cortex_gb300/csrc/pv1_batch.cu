@@ -38,11 +38,11 @@ struct pv1_batch {
     int *dNTiles = nullptr;
     int *dActive = nullptr, *dNActive = nullptr;   // active trial list (persistent variant)
     unsigned *dBar = nullptr;                      // per-trial barrier counters
-    int slotCtas = 0, nSlots = 0;                  // persistent variant: CTAs per slot, slots
+    int slotCtas = 0, nSlots = 0, csize = 1;       // persistent variant: CTAs per slot, slots, CTAs per cluster
     int totalTiles = 0;
     int maxCellCtas = 0;
     bool allClass = true;
-    bool rng = false;
+    bool rng = false, general = false;       // which kernel the trials need
     unsigned *dCounts = nullptr;
     long long *dCountOff = nullptr;
     std::vector<long long> countOff;
@@ -137,7 +137,7 @@ int issue(pv1_batch *b, int k, int minB, long long *launches) {
     }
     if (minB == 0) {
         e = launch_v1_batch_persistent(b->dT, b->dActive, b->dNActive, b->slotCtas, b->nSlots, k, b->dBar, b->n,
-                                       b->rng, b->stream);
+                                       b->rng, b->general, b->csize, b->stream);
         if (e != cudaSuccess) return bfail(b, PV1_E_CUDA, std::string("v1 batch persistent: ") + cudaGetErrorString(e));
         n += 1;
     } else {
@@ -249,6 +249,7 @@ int pv1_batch_create(pv1_plan *const *plans, uint32_t nTrials, const uint64_t *t
         b->maxCellCtas = std::max(b->maxCellCtas, (v.lp.nMagno + 127) / 128);
         if (!v.lp.classCtw) b->allClass = false;
         if (v.vp.condRng || v.vp.noiseRng) b->rng = true;
+        if (v1_batch_general(v.vp)) b->general = true;
         if (v.lgnSlots < 64) b->allClass = false;
         PV1_BCUDA(b, cudaMemcpyAsync(v.d_stepBase, &b->step[q], sizeof(long long), cudaMemcpyHostToDevice,
                                      b->stream));
@@ -267,7 +268,15 @@ int pv1_batch_create(pv1_plan *const *plans, uint32_t nTrials, const uint64_t *t
     if (r) return r;
     // persistent variant: slots as large as the largest trial, as many as stay co-resident
     for (int q = 0; q < b->n; q++) b->slotCtas = std::max(b->slotCtas, b->hT[q].nCta);
-    const int cap = v1_batch_persistent_capacity(b->rng, b->device);
+    // in clusters of a block's CTAs when every trial's blocks have as many
+    b->csize = (b->hT[0].v.blockSize + 255) / 256;
+    for (int q = 1; q < b->n; q++)
+        if ((b->hT[q].v.blockSize + 255) / 256 != b->csize) b->csize = 1;
+    int cap = v1_batch_persistent_capacity(b->rng, b->general, b->device, b->csize);
+    if (b->csize > 1 && cap < b->slotCtas) {
+        b->csize = 1;
+        cap = v1_batch_persistent_capacity(b->rng, b->general, b->device, 1);
+    }
     b->nSlots = b->slotCtas > 0 ? std::min(cap / b->slotCtas, b->n) : 0;
     if (b->nSlots > 0) b->minB = 0;
     PV1_BCUDA(b, cudaStreamSynchronize(b->stream));
@@ -490,7 +499,7 @@ int pv1_batch_sweep(pv1_batch *b, float *ms) {
         cudaError_t e1 = launch_lgn_class_batch(dLs, b->n, b->maxCellCtas, (int)maxLeft, b->stream);
         if (e1 == cudaSuccess)
             e1 = launch_v1_batch_persistent(dTs, dList, dNList, b->slotCtas, b->nSlots, (int)maxLeft, b->dBar, b->n,
-                                            b->rng, b->stream);
+                                            b->rng, b->general, b->csize, b->stream);
         if (e1 == cudaSuccess) e1 = launch_batch_advance(dTs, b->n, (int)maxLeft, b->dSimTime, b->stream);
         cudaError_t e2 = cudaStreamEndCapture(b->stream, &g);
         e = e1 != cudaSuccess ? e1 : e2;

@@ -171,7 +171,7 @@ struct V1Params {
     int condRng;        // rGenCond draws can change results (some failure rate > 0)
     int noiseRng;       // some noisyDep > 0
     long long waitSpins;   // polls of a barrier wait before it gives up and raises kErrBarrier
-    int pushCta;           // far-push CTAs appended to the persistent grid (0: the neuron CTAs push)
+    int cluster, threads;  // the persistent launch: CTAs per cluster, threads per CTA (past 256: push warps)
     // LGN->V1 plasticity (the reference's learning 1-4): triplet rule on the LGN->E synapses
     // (type 0) and, with learning 2, on the LGN->I synapses (type 1)
     int ffMode;            // the reference's `learning` (0: off)
@@ -201,6 +201,7 @@ struct V1Params {
     int nnbMax;
     const int *nNearNB;        // [nblock]
     const int *nbId;           // [nblock][nnbMax]
+    int nearSelf;              // every block's near list is the block itself
     const float *conMat;       // [nblock][nnbMax][bs][bs]
     const int *nearRevOff;     // [nblock+1] near tiles that read block b's rows: nearRev[off[b]..off[b+1])
     const int *nearRev;        //            tile index (post block * nnbMax + position in its list)
@@ -352,9 +353,9 @@ cudaError_t launch_frames(const float *recSpk, int recSlots, int nV1, const floa
                           cudaStream_t st);
 // Adds farPull to the E/I conductances (the far part of the delivery before the first step).
 cudaError_t launch_far_pull_apply(const V1Params &p, cudaStream_t st);
-// Neuron CTAs of the persistent kernel; *fits: all can be resident at once; *pushCtas: the
-// far-push CTAs that fit beside them on the device (0 without far synapses).
-int v1_persistent_ctas(const V1Params &p, int device, bool *fits, int *pushCtas);
+// Cluster size and threads per CTA of the persistent kernel; false if its CTAs cannot all be
+// resident at once.
+bool v1_persistent_shape(const V1Params &p, int device, int *cluster, int *threads);
 // Evaluates the full-step decay factors of the three conductance kernels on the device and
 // stores them into p (synchronous).
 cudaError_t compute_step_decay(V1Params &p, cudaStream_t st);
@@ -405,11 +406,13 @@ cudaError_t launch_batch_rates(const BatchTrial *trials, const unsigned *counts,
                                const double *simTime, int trial, int nV1, double *rates,
                                double *meanRate, cudaStream_t st);
 int v1_batch_regs(int minB, bool rng);
-// Batched trials in one cooperative launch per chunk (slots of slotCtas CTAs, per-trial barriers).
-int v1_batch_persistent_capacity(bool rng, int device);
+// Batched trials in one cooperative launch per chunk (slots of slotCtas CTAs in clusters of csize,
+// per-trial barriers).
+bool v1_batch_general(const V1Params &p);
+int v1_batch_persistent_capacity(bool rng, bool general, int device, int csize);
 cudaError_t launch_v1_batch_persistent(const BatchTrial *trials, const int *activeList, const int *nActive,
                                        int slotCtas, int nSlots, int K, unsigned *barriers, int nTrials, bool rng,
-                                       cudaStream_t st);
+                                       bool general, int csize, cudaStream_t st);
 
 // Fixed-point scale for far-delivery accumulation: integer adds are associative, so the
 // sum of events does not depend on their order and runs are reproducible.

@@ -1215,6 +1215,9 @@ int pv1_v1_set_near(pv1_plan *p, uint32_t nnb, const uint32_t *nNearNB, const ui
     p->vp.conMat = d_c;
     p->vp.nearRevOff = d_ro;
     p->vp.nearRev = d_rev;
+    bool self = true;
+    for (int b = 0; b < nblock; b++) self = self && nNearNB[b] == 1 && nbId[(size_t)b * nnb] == (uint32_t)b;
+    p->vp.nearSelf = self;
     p->haveNear = true;
     drop_graph(p);
     return PV1_OK;
@@ -1804,12 +1807,10 @@ int64_t pv1_raw_record_floats(const pv1_plan *p) {
 // synapse lists fit in registers.
 static int choose_mode(pv1_plan *p) {
     if (p->modeChosen) return PV1_OK;
-    bool fits = false;
-    int push = 0;
-    v1_persistent_ctas(p->vp, p->device, &fits, &push);
-    p->persistent = fits && p->allowPersistent && !p->vp.multiSpike && !p->vp.farPullOn && !p->vp.nearPullOn &&
-                    !p->vp.ffMode;
-    p->vp.pushCta = p->persistent ? push : 0;
+    p->vp.cluster = 1;
+    p->vp.threads = 256;
+    p->persistent = p->allowPersistent && !p->vp.multiSpike && !p->vp.farPullOn && !p->vp.nearPullOn && !p->vp.ffMode &&
+                    v1_persistent_shape(p->vp, p->device, &p->vp.cluster, &p->vp.threads);
     if (p->persistent && !p->d_barrier) {
         int r = dev_alloc(p, &p->d_barrier, 2);
         if (r) return r;

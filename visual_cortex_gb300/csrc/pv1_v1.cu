@@ -67,14 +67,6 @@ __device__ __forceinline__ RecOff rec_off(const V1Params &P) {
     return o;
 }
 
-// Per-neuron dynamic state (registers).
-// LGN input of the next step fetched ahead by the persistent kernel: the synapses that
-// received spikes (bit mask, synapse order) and the spike word and weight of the first one.
-struct LgnPre {
-    unsigned mask;
-    float s0, f0;
-};
-
 // Starts the copies of one step's LGN spike words of a neuron's m synapses into shared memory
 // (ids and destinations [synapse][kCta] from this thread's column); lgn_words_wait completes
 // them.  Each thread reads back only what it copied, so no CTA barrier is needed.
@@ -88,41 +80,21 @@ __device__ __forceinline__ void lgn_words_async(const float *__restrict__ ring, 
 }
 __device__ __forceinline__ void lgn_words_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// Fetches the spike words of a neuron's (at most kMaxLgnReg) LGN synapses for one step: ids
-// at ids[q * Stride] (registers: Stride 1; shared memory: Stride kCta).
-template <int Stride>
-__device__ __forceinline__ LgnPre lgn_prefetch(const V1Params &P, const float *__restrict__ ring, const int *ids,
-                                               int m, int i) {
-    LgnPre pre{0u, 0.f, 0.f};
-    float sp[kMaxLgnReg];
-#pragma unroll
-    for (int q = 0; q < kMaxLgnReg; q++) sp[q] = q < m ? __ldcg(ring + ids[q * Stride]) : 0.f;
-#pragma unroll
-    for (int q = kMaxLgnReg - 1; q >= 0; q--) {
-        const bool hit = sp[q] >= 1.0f;
-        pre.mask |= (hit ? 1u : 0u) << q;
-        if (hit) pre.s0 = sp[q];
-    }
-    if (pre.mask) pre.f0 = __ldg(P.sLGN + (size_t)(__ffs(pre.mask) - 1) * P.nV1 + i);
-    return pre;
-}
-
+// Per-neuron dynamic state (registers).
 struct NState {
     float v, w, tBack, lastNoise;
     float gE[kMaxNG], hE[kMaxNG], gI[kMaxNG], hI[kMaxNG], gFF[kMaxNG], hFF[kMaxNG];
 };
 
+// Barrier among the CTA's kCta neuron threads (a persistent CTA can hold push warps beside them).
+__device__ __forceinline__ void neuron_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kCta) : "memory"); }
+
+// Staging of the general near delivery: the spikers of one neighbour block.
 struct Smem {
     int pre[kMaxBS];
-    float val[kMaxBS];
     float og[kMaxNG][kMaxBS];
     float oh[kMaxNG][kMaxBS];
     unsigned ball[kMaxBS / 32];
-    int pref[kMaxBS / 32];
-    int total, below;
-    unsigned fball[kWarps];
-    int fpre[kCta], fe0[kCta], fdeg[kCta], fpref[kCta + 1];
-    float fsi[kCta];
 };
 
 __device__ __forceinline__ void load_state(const V1Params &P, int i, NState &s) {
@@ -180,7 +152,7 @@ __device__ __forceinline__ int compact_spikers(const V1Params &P, const float *_
         const unsigned bal = __ballot_sync(0xffffffffu, f);
         if (k * kCta < bs && lane == 0) sm.ball[k * kWarps + warp] = bal;
     }
-    __syncthreads();
+    neuron_sync();
     // every warp scans the block's ballot words itself (no second barrier): lane l holds word l
     const unsigned wb = lane < nw ? sm.ball[lane] : 0u;
     const int c = __popc(wb);
@@ -224,7 +196,7 @@ __device__ __forceinline__ int compact_spikers(const V1Params &P, const float *_
             }
         }
     }
-    __syncthreads();
+    neuron_sync();
     return total;
 }
 
@@ -264,17 +236,127 @@ __device__ __forceinline__ void learn_avg_delivery(const V1Params &P, float post
     vAvg[0] = lAvgE;
 }
 
-__device__ __forceinline__ int far_ring_slot(const V1Params &P, long long t);
+// Ring slot of step t in the far/near event rings.
+__device__ __forceinline__ int far_ring_slot(const V1Params &P, long long t) {
+    const long long r = t % P.farDepth;
+    return (int)(r < 0 ? r + P.farDepth : r);
+}
 
-// Phase A: delivery of step tp's spikes to this thread's neuron (all threads of the CTA
-// must call it; `active` masks the neuron work).
+// Far events of one ring slot for one neuron, and whether a far presynaptic neuron spiked in
+// that step (the reference delivers far input only then).
+struct FarIn {
+    unsigned long long g[2 * kMaxNG], h[2 * kMaxNG];
+    bool spiked;
+};
+
+__device__ __forceinline__ void far_fetch(const V1Params &P, int farSlot, int flagSlot, int i, FarIn &f) {
+    const int ns = P.ngE + P.ngI, nV1 = P.nV1;
+    const unsigned long long *acc = P.farAcc + (size_t)farSlot * ns * 2 * nV1;
+    f.spiked = __ldcg(P.farFlag + flagSlot) != 0;
+#pragma unroll
+    for (int q = 0; q < 2 * kMaxNG; q++) {
+        f.g[q] = q < ns ? __ldcg(acc + (size_t)(2 * q) * nV1 + i) : 0ull;
+        f.h[q] = q < ns ? __ldcg(acc + (size_t)(2 * q + 1) * nV1 + i) : 0ull;
+    }
+}
+
+// Adds fetched far events to the conductances and clears the ring entries they came from.
+__device__ __forceinline__ void far_apply(const V1Params &P, int farSlot, int i, const FarIn &f, NState &st) {
+    const int ns = P.ngE + P.ngI, nV1 = P.nV1;
+    unsigned long long *acc = P.farAcc + (size_t)farSlot * ns * 2 * nV1;
+#pragma unroll
+    for (int q = 0; q < 2 * kMaxNG; q++) {
+        if (q < ns) {
+            if (f.g[q] | f.h[q]) {
+                acc[(size_t)(2 * q) * nV1 + i] = 0ull;
+                acc[(size_t)(2 * q + 1) * nV1 + i] = 0ull;
+            }
+            if (f.spiked) {
+                const float fg = far_from_fixed(f.g[q]);
+                const float fh = far_from_fixed(f.h[q]);
+#pragma unroll
+                for (int ig = 0; ig < kMaxNG; ig++) {
+                    if (q < P.ngE && ig == q) { st.gE[ig] += fg; st.hE[ig] += fh; }
+                    if (q >= P.ngE && ig == q - P.ngE) { st.gI[ig] += fg; st.hI[ig] += fh; }
+                }
+            }
+        }
+    }
+}
+
+// Delayed near events (noDelay = 0) of one ring slot: taken into lg/lh, entries cleared.
+__device__ __forceinline__ void near_ring_take(const V1Params &P, int farSlot, int i, float *lgE, float *lhE,
+                                               float *lgI, float *lhI) {
+    const int ns = P.ngE + P.ngI, nV1 = P.nV1, ngE = P.ngE;
+    unsigned long long *nacc = P.nearAcc + (size_t)farSlot * ns * 2 * nV1;
+#pragma unroll
+    for (int q = 0; q < 2 * kMaxNG; q++) {
+        if (q < ns) {
+            unsigned long long *pg = nacc + (size_t)(2 * q) * nV1 + i;
+            unsigned long long *ph = nacc + (size_t)(2 * q + 1) * nV1 + i;
+            const unsigned long long ug = __ldcg(pg), uh = __ldcg(ph);
+            if (ug | uh) {
+                *pg = 0ull;
+                *ph = 0ull;
+                const float fg = far_from_fixed(ug), fh = far_from_fixed(uh);
+#pragma unroll
+                for (int ig = 0; ig < kMaxNG; ig++) {
+                    if (q < ngE && ig == q) { lgE[ig] = fg; lhE[ig] = fh; }
+                    if (q >= ngE && ig == q - ngE) { lgI[ig] = fg; lhI[ig] = fh; }
+                }
+            }
+        }
+    }
+}
+
+// The conductances of step tp's record, complete once its spikes are delivered.
+__device__ __forceinline__ void record_conductances(const V1Params &P, long long tp, int i, const NState &st) {
+    const int nV1 = P.nV1;
+    float *r = P.rec + (tp % P.recSlots) * P.recStride;
+    const RecOff o = rec_off(P);
+#pragma unroll
+    for (int ig = 0; ig < kMaxNG; ig++) {
+        if (ig < P.ngE) r[o.gE + ig * nV1 + i] = st.gE[ig];
+        if (ig < P.ngI) r[o.gI + ig * nV1 + i] = st.gI[ig];
+        if (P.hWrite) {
+            if (ig < P.ngE) r[o.hE + ig * nV1 + i] = st.hE[ig];
+            if (ig < P.ngI) r[o.hI + ig * nV1 + i] = st.hI[ig];
+        }
+    }
+}
+
+// Failure draw of one near synapse from the spiker of rank `rank` among its block's E or I
+// spikers: the pre type comes from that rank, as the reference takes it
+// (src/coredynamics.cu:2760-2766, 2815-2821).
+__device__ __forceinline__ float near_failure(const V1Params &P, float strength, bool isE, int rank, int itype,
+                                              curandStateMRG32k3a &condState, float *recNear, int &nDraw) {
+    const int ja = isE ? 0 : P.nTypeE, jb = isE ? P.nTypeE : P.nType;
+    int jtype = ja;
+    for (int jj = ja; jj < jb; jj++) {
+        if (rank < P.typeAcc[jj]) { jtype = jj; break; }
+    }
+    const int idx = jtype * P.nType + itype;
+    const float lp = P.synFail[idx];
+    const float normed_std = sqrtf(lp * (1 - lp) / P.synPerCon[idx]);
+    const float rnd = curand_normal(&condState);
+    if (recNear) {
+        if (nDraw < P.recCap) recNear[nDraw] = rnd;
+        else atomicOr(P.err, kErrRecordOverflow);
+    }
+    nDraw++;
+    return strength * (1 - lp + normed_std * rnd);
+}
+
+// Phase A: delivery of step tp's spikes to this thread's neuron (all kCta neuron threads of the
+// CTA must call it; `active` masks the neuron work): any list of neighbour blocks, the spike
+// words read from global memory.
 template <bool Rng>
 __device__ __forceinline__ void deliver_prev(const V1Params &P, long long tp, int b, int local, int i,
                                              bool active, int itype, NState &st,
                                              curandStateMRG32k3a &condState, Smem &sm, int farSlot = -1) {
     const int bs = P.blockSize, nV1 = P.nV1;
     // the far ring slot of step tp (tp mod farDepth; passed in by the persistent kernel)
-    if (farSlot < 0) farSlot = far_ring_slot(P, tp);
+    if (farSlot < 0 && P.farOn) farSlot = far_ring_slot(P, tp);
     const int ngE = P.ngE, ngI = P.ngI;
     const float *sPrev = P.sInfo + (size_t)(tp & 1) * nV1;
     float lgE[kMaxNG], lhE[kMaxNG], lgI[kMaxNG], lhI[kMaxNG], ipE[kMaxNG], ipI[kMaxNG];
@@ -286,18 +368,9 @@ __device__ __forceinline__ void deliver_prev(const V1Params &P, long long tp, in
     }
     // far events arriving in step tp, fetched early so that the loads overlap the compaction
     const int ns = ngE + ngI;
-    unsigned long long farG[2 * kMaxNG], farH[2 * kMaxNG];
-    unsigned long long *acc = nullptr;
-    bool farSpiked = false;
-    if (P.farClass && active) {
-        acc = P.farAcc + (size_t)farSlot * ns * 2 * nV1;
-        farSpiked = __ldcg(P.farFlag + tp % 3) != 0;
-#pragma unroll
-        for (int q = 0; q < 2 * kMaxNG; q++) {
-            farG[q] = q < ns ? __ldcg(acc + (size_t)(2 * q) * nV1 + i) : 0ull;
-            farH[q] = q < ns ? __ldcg(acc + (size_t)(2 * q + 1) * nV1 + i) : 0ull;
-        }
-    }
+    const bool far = P.farClass && active;
+    FarIn fin;
+    if (far) far_fetch(P, farSlot, (int)((tp + 3) % 3), i, fin);
     float *recNear = nullptr;
     int nNearDraw = 0;
     if (Rng && P.recNear && active) {
@@ -354,29 +427,7 @@ __device__ __forceinline__ void deliver_prev(const V1Params &P, long long tp, in
     }
     // delayed near events (noDelay = 0): recal_G_mat sums them into the same step's
     // conductance update; here they were pushed into their own ring
-    if (!P.noDelay) {
-        if (P.nearOn && active) {
-            unsigned long long *nacc = P.nearAcc + (size_t)farSlot * ns * 2 * nV1;
-#pragma unroll
-            for (int q = 0; q < 2 * kMaxNG; q++) {
-                if (q < ns) {
-                    unsigned long long *pg = nacc + (size_t)(2 * q) * nV1 + i;
-                    unsigned long long *ph = nacc + (size_t)(2 * q + 1) * nV1 + i;
-                    const unsigned long long ug = __ldcg(pg), uh = __ldcg(ph);
-                    if (ug | uh) {
-                        *pg = 0ull;
-                        *ph = 0ull;
-                        const float fg = far_from_fixed(ug), fh = far_from_fixed(uh);
-#pragma unroll
-                        for (int ig = 0; ig < kMaxNG; ig++) {
-                            if (q < ngE && ig == q) { lgE[ig] = fg; lhE[ig] = fh; }
-                            if (q >= ngE && ig == q - ngE) { lgI[ig] = fg; lhI[ig] = fh; }
-                        }
-                    }
-                }
-            }
-        }
-    }
+    if (!P.noDelay && P.nearOn && active) near_ring_take(P, farSlot, i, lgE, lhE, lgI, lhI);
     const int nnb = P.noDelay ? P.nNearNB[b] : 0;
     for (int ib = 0; ib < nnb; ib++) {
         const int nb = P.nbId[b * P.nnbMax + ib];
@@ -397,26 +448,9 @@ __device__ __forceinline__ void deliver_prev(const V1Params &P, long long tp, in
                     if (r < cnt && strength > 0) {
                         const bool isE = r < cntE;
                         if constexpr (Rng) {
-                            if (P.condRng) {
-                                // pre type from the spiker's rank, as the reference does
-                                // (src/coredynamics.cu:2760-2766, 2815-2821)
-                                const int rank = isE ? r : r - cntE;
-                                const int ja = isE ? 0 : P.nTypeE, jb = isE ? P.nTypeE : P.nType;
-                                int jtype = ja;
-                                for (int jj = ja; jj < jb; jj++) {
-                                    if (rank < P.typeAcc[jj]) { jtype = jj; break; }
-                                }
-                                const int idx = jtype * P.nType + itype;
-                                const float lp = P.synFail[idx];
-                                const float normed_std = sqrtf(lp * (1 - lp) / P.synPerCon[idx]);
-                                const float rnd = curand_normal(&condState);
-                                if (recNear) {
-                                    if (nNearDraw < P.recCap) recNear[nNearDraw] = rnd;
-                                    else atomicOr(P.err, kErrRecordOverflow);
-                                }
-                                nNearDraw++;
-                                strength *= 1 - lp + normed_std * rnd;
-                            }
+                            if (P.condRng)
+                                strength = near_failure(P, strength, isE, isE ? r : r - cntE, itype, condState, recNear,
+                                                        nNearDraw);
                         }
                         if (strength > 0) {
                             if (isE) {
@@ -443,7 +477,7 @@ __device__ __forceinline__ void deliver_prev(const V1Params &P, long long tp, in
                 }
             }
         }
-        __syncthreads();
+        neuron_sync();
     }
     if (recNear) P.recNearCount[(size_t)(tp - P.recStep0) * nV1 + i] = nNearDraw;
     if (P.ffMode && P.ffMode != 3 && active && local < P.nE) learn_avg_delivery(P, __ldcg(sPrev + i), b, local);
@@ -468,40 +502,8 @@ __device__ __forceinline__ void deliver_prev(const V1Params &P, long long tp, in
         }
     }
     // far events (sum_G adds them after the near delivery); the ring slot is cleared
-    if (acc) {
-#pragma unroll
-        for (int q = 0; q < 2 * kMaxNG; q++) {
-            if (q < ns) {
-                if (farG[q] | farH[q]) {
-                    acc[(size_t)(2 * q) * nV1 + i] = 0ull;
-                    acc[(size_t)(2 * q + 1) * nV1 + i] = 0ull;
-                }
-                if (farSpiked) {
-                    const float fg = far_from_fixed(farG[q]);
-                    const float fh = far_from_fixed(farH[q]);
-#pragma unroll
-                    for (int ig = 0; ig < kMaxNG; ig++) {
-                        if (q < ngE && ig == q) { st.gE[ig] += fg; st.hE[ig] += fh; }
-                        if (q >= ngE && ig == q - ngE) { st.gI[ig] += fg; st.hI[ig] += fh; }
-                    }
-                }
-            }
-        }
-    }
-    if (P.rec && active) {
-        const long long slot = tp % P.recSlots;
-        float *r = P.rec + slot * P.recStride;
-        const RecOff o = rec_off(P);
-#pragma unroll
-        for (int ig = 0; ig < kMaxNG; ig++) {
-            if (ig < ngE) r[o.gE + ig * nV1 + i] = st.gE[ig];
-            if (ig < ngI) r[o.gI + ig * nV1 + i] = st.gI[ig];
-            if (P.hWrite) {
-                if (ig < ngE) r[o.hE + ig * nV1 + i] = st.hE[ig];
-                if (ig < ngI) r[o.hI + ig * nV1 + i] = st.hI[ig];
-            }
-        }
-    }
+    if (far) far_apply(P, farSlot, i, fin, st);
+    if (P.rec && active) record_conductances(P, tp, i, st);
 }
 
 // The tonic drive of the AdEx constructor (src/coredynamics.cuh:41-49).
@@ -547,60 +549,30 @@ __device__ __forceinline__ void lgn_input(const V1Params &P, int itype, float sF
     }
 }
 
-// Phase B: one membrane step of neuron i.  With SmemSyn the spike words and weights of the
-// neuron's synapses are in shared memory (smS, smW: [synapse][kCta] from the thread's column);
-// with RegSyn the synapse ids are the register array lgnIds (up to kMaxLgnReg of them) and
-// the weights are read only for synapses that received a spike; otherwise ids and weights are
-// loaded batch by batch.  Returns the spike word.
-template <bool Rng, bool RegSyn, bool SmemSyn = false>
-__device__ __forceinline__ float step_neuron(const V1Params &P, long long t, int i, int itype,
-                                             float tonic, float depC, int m, const int *lgnIds,
-                                             const float *__restrict__ lgnSInfo,
-                                             NState &st, curandStateMRG32k3a &condState,
-                                             curandStateMRG32k3a &noisyState,
-                                             const LgnPre *pre = nullptr, const float *smW = nullptr,
-                                             const float *smS = nullptr) {
+// What the feed-forward half of a membrane step hands to the integration half.
+struct FFStep {
+    float g0[kMaxNG];          // feed-forward conductances at the start of the integrated interval
+    float noise0, noise1, depOut;
+};
+
+// Phase B, first half: noise and the feed-forward conductances of step t (decay over the step and
+// the LGN input, src/coredynamics.cu:1422-1502); st.gFF/hFF leave at their end-of-step values.
+// Nothing here depends on what other neurons do in step t - 1, so the persistent kernels run it
+// while they wait for them.  With SmemSyn the spike words and weights of the neuron's synapses
+// are in shared memory (smS, smW: [synapse][kCta] from the thread's column); otherwise ids and
+// words are loaded batch by batch and weights only for synapses that received a spike.
+template <bool Rng, bool SmemSyn>
+__device__ __forceinline__ void step_feedforward(const V1Params &P, long long t, int i, int itype, float tonic,
+                                                 float depC, int m, const float *__restrict__ lgnSInfo, NState &st,
+                                                 curandStateMRG32k3a &condState, curandStateMRG32k3a &noisyState,
+                                                 FFStep &ff, const float *smW = nullptr, const float *smS = nullptr) {
     const int nV1 = P.nV1;
     const float dt = P.dt;
-    const int ngE = P.ngE, ngI = P.ngI, ngFF = P.ngFF;
-    // spike words of this neuron's LGN inputs, gathered first so that they overlap the decay
-    // (unless the caller fetched them already: pre)
-    float spReg[RegSyn ? kMaxLgnReg : 1];
-    if constexpr (RegSyn) {
-        if (!pre) {
-#pragma unroll
-            for (int q = 0; q < kMaxLgnReg; q++) spReg[q] = q < m ? __ldcg(lgnSInfo + lgnIds[q]) : 0.f;
-        }
-    }
-    const float vR = P.vR[itype], vThres = P.vThres[itype], gL = P.gL[itype];
-    const float Cm = P.C[itype], tRef = P.tRef[itype], vT = P.vT[itype];
-    const float deltaT = P.deltaT[itype], tau_w = P.tau_w[itype], aa = P.a[itype];
-    const float bb = P.b[itype];
-    const float v0 = st.v;
-    float w0 = st.w;
-    float tBack = st.tBack;
-    const float noise0 = st.lastNoise;
-
-    // cortical conductances: keep the start-of-step value, decay to the end
-    float ge[kMaxNG], he[kMaxNG], gi[kMaxNG], hi[kMaxNG];
-    float gE_t1 = 0.0f, gI_t1 = 0.0f;
-#pragma unroll
-    for (int ig = 0; ig < kMaxNG; ig++) {
-        ge[ig] = st.gE[ig]; he[ig] = st.hE[ig];
-        if (ig < ngE) {
-            cond_decay_step(P.condE, P.decE, st.gE[ig], st.hE[ig], ig);
-            gE_t1 += st.gE[ig];
-        }
-    }
-#pragma unroll
-    for (int ig = 0; ig < kMaxNG; ig++) {
-        gi[ig] = st.gI[ig]; hi[ig] = st.hI[ig];
-        if (ig < ngI) {
-            cond_decay_step(P.condI, P.decI, st.gI[ig], st.hI[ig], ig);
-            gI_t1 += st.gI[ig];
-        }
-    }
-    float g0[kMaxNG], h0[kMaxNG], g1[kMaxNG], h1[kMaxNG];
+    const int ngFF = P.ngFF;
+    const float tBack = st.tBack;
+    ff.noise0 = st.lastNoise;
+    float h0[kMaxNG], g1[kMaxNG], h1[kMaxNG];
+    float *g0 = ff.g0;
 #pragma unroll
     for (int ig = 0; ig < kMaxNG; ig++) {
         g1[ig] = st.gFF[ig];
@@ -613,7 +585,7 @@ __device__ __forceinline__ float step_neuron(const V1Params &P, long long t, int
     float noise1 = 0.f;
     if constexpr (Rng) {
         const float noiseRatio = P.noiseOnTonic ? tonic : 1.0f;
-        noise1 = sqrtf(2 * P.noisyDep[itype] * (vT - vR) * noiseRatio * dt);
+        noise1 = sqrtf(2 * P.noisyDep[itype] * (P.vT[itype] - P.vR[itype]) * noiseRatio * dt);
         if (noise1 > 0) {
             const float rnd = curand_normal(&noisyState);
             if (P.recNoise) {
@@ -623,18 +595,18 @@ __device__ __forceinline__ float step_neuron(const V1Params &P, long long t, int
             noise1 *= rnd;
             if (P.tau_noise > 0) {
                 noise1 /= P.tau_noise;
-                const float hk1 = -noise0 / P.tau_noise;
-                const float hk2 = -(noise0 + dt * hk1 + noise1) / P.tau_noise;
-                noise1 += noise0 + dt * (hk1 + hk2) / 2;
+                const float hk1 = -ff.noise0 / P.tau_noise;
+                const float hk2 = -(ff.noise0 + dt * hk1 + noise1) / P.tau_noise;
+                noise1 += ff.noise0 + dt * (hk1 + hk2) / 2;
                 st.lastNoise = noise1;
             }
         }
     }
+    ff.noise1 = noise1;
     const float pf = Rng ? P.synFailFF[itype] : 0.f;
     const float nSynFF = P.synPerConFF[itype];
     const bool backingUp = tBack < dt && tBack > 0;
-    const float depOut = depC + noise1;
-    P.dep[i] = depOut;
+    ff.depOut = depC + noise1;
     if (backingUp) {
 #pragma unroll
         for (int ig = 0; ig < kMaxNG; ig++)
@@ -659,29 +631,6 @@ __device__ __forceinline__ float step_neuron(const V1Params &P, long long t, int
             mask &= mask - 1;
             lgn_input<Rng>(P, itype, smS[q * kCta], smW[q * kCta], backingUp, tBack, pf, nSynFF, g0, h0, g1, h1,
                            condState, recFF, nFF);
-        }
-    } else if constexpr (RegSyn) {
-        // synapses that received a spike, as a bit mask; they are visited in synapse order
-        unsigned mask = 0u;
-        if (pre) {
-            mask = pre->mask;
-            if (mask) {  // the first spiking synapse comes with its spike word and weight
-                lgn_input<Rng>(P, itype, pre->s0, pre->f0, backingUp, tBack, pf, nSynFF, g0, h0, g1, h1, condState,
-                               recFF, nFF);
-                mask &= mask - 1;
-            }
-        } else {
-#pragma unroll
-            for (int q = 0; q < kMaxLgnReg; q++) mask |= (spReg[q] >= 1.0f ? 1u : 0u) << q;
-        }
-        while (mask) {
-            const int q = __ffs(mask) - 1;
-            mask &= mask - 1;
-            const size_t lid = (size_t)q * nV1 + i;
-            const float sFF = __ldcg(lgnSInfo + __ldg(P.lgnId + lid));
-            const float f = __ldg(P.sLGN + lid);
-            lgn_input<Rng>(P, itype, sFF, f, backingUp, tBack, pf, nSynFF, g0, h0, g1, h1, condState, recFF,
-                           nFF);
         }
     } else if (m <= kMaxLgnReg) {
         // ids and spike words in chunks of 16 (all loads of a chunk in flight together); the
@@ -728,15 +677,55 @@ __device__ __forceinline__ float step_neuron(const V1Params &P, long long t, int
         }
     }
     if (recFF) P.recFFCount[(size_t)(t - P.recStep0) * nV1 + i] = nFF;
+#pragma unroll
+    for (int ig = 0; ig < kMaxNG; ig++) {
+        st.gFF[ig] = g1[ig];
+        st.hFF[ig] = h1[ig];
+    }
+}
+
+// Phase B, second half: cortical conductances, integration and threshold of step t
+// (src/coredynamics.cu:1380-1590).  Returns the spike word.
+__device__ __forceinline__ float step_membrane(const V1Params &P, int itype, float depC, const FFStep &ff, NState &st) {
+    const float dt = P.dt;
+    const int ngE = P.ngE, ngI = P.ngI, ngFF = P.ngFF;
+    const float vR = P.vR[itype], vThres = P.vThres[itype], gL = P.gL[itype];
+    const float Cm = P.C[itype], tRef = P.tRef[itype], vT = P.vT[itype];
+    const float deltaT = P.deltaT[itype], tau_w = P.tau_w[itype], aa = P.a[itype];
+    const float bb = P.b[itype];
+    const float v0 = st.v;
+    float w0 = st.w;
+    float tBack = st.tBack;
+    const float noise0 = ff.noise0;
+    float noise1 = ff.noise1;
+    const bool backingUp = tBack < dt && tBack > 0;
+
+    // cortical conductances: keep the start-of-step value, decay to the end
+    float ge[kMaxNG], he[kMaxNG], gi[kMaxNG], hi[kMaxNG];
+    float gE_t1 = 0.0f, gI_t1 = 0.0f;
+#pragma unroll
+    for (int ig = 0; ig < kMaxNG; ig++) {
+        ge[ig] = st.gE[ig]; he[ig] = st.hE[ig];
+        if (ig < ngE) {
+            cond_decay_step(P.condE, P.decE, st.gE[ig], st.hE[ig], ig);
+            gE_t1 += st.gE[ig];
+        }
+    }
+#pragma unroll
+    for (int ig = 0; ig < kMaxNG; ig++) {
+        gi[ig] = st.gI[ig]; hi[ig] = st.hI[ig];
+        if (ig < ngI) {
+            cond_decay_step(P.condI, P.decI, st.gI[ig], st.hI[ig], ig);
+            gI_t1 += st.gI[ig];
+        }
+    }
     float gE_t0 = 0.0f;
 #pragma unroll
     for (int ig = 0; ig < kMaxNG; ig++) {
         if (ig < ngFF) {
-            gE_t0 += g0[ig];
-            gE_t1 += g1[ig];
+            gE_t0 += ff.g0[ig];
+            gE_t1 += st.gFF[ig];
         }
-        st.gFF[ig] = g1[ig];
-        st.hFF[ig] = h1[ig];
     }
 #pragma unroll
     for (int ig = 0; ig < kMaxNG; ig++) {
@@ -798,26 +787,43 @@ __device__ __forceinline__ float step_neuron(const V1Params &P, long long t, int
         w = (w0 - A) * expf(-(dt - tsp) / tau_w) + A;
         tBack -= dt;
     }
-    const float sInfo = spikeCount > 0 ? 1.0f + tsp / dt : v;
     st.v = v;
     if (P.iModel == 1) st.w = w;
     st.tBack = tBack;
+    return spikeCount > 0 ? 1.0f + tsp / dt : v;
+}
+
+// The step's spike word to global memory and to the records.
+__device__ __forceinline__ void store_step(const V1Params &P, long long t, int i, float sInfo, float depOut,
+                                           const NState &st) {
+    const int nV1 = P.nV1;
     __stcg(P.sInfo + (size_t)(t & 1) * nV1 + i, sInfo);
     if (P.recSpk) P.recSpk[(size_t)(t % P.recSlots) * nV1 + i] = sInfo;
     if (P.rec) {
-        const long long slot = t % P.recSlots;
-        float *r = P.rec + slot * P.recStride;
+        float *r = P.rec + (t % P.recSlots) * P.recStride;
         const RecOff o = rec_off(P);
         r[o.sinfo + i] = sInfo;
         r[o.dep + i] = depOut;
-        if (P.iModel == 1) r[o.w + i] = w;
-        r[o.v + i] = v;
+        if (P.iModel == 1) r[o.w + i] = st.w;
+        r[o.v + i] = st.v;
 #pragma unroll
         for (int ig = 0; ig < kMaxNG; ig++) {
-            if (ig < ngFF) r[o.gFF + ig * nV1 + i] = g1[ig];
-            if (P.hWrite && ig < ngFF) r[o.hFF + ig * nV1 + i] = h1[ig];
+            if (ig < P.ngFF) r[o.gFF + ig * nV1 + i] = st.gFF[ig];
+            if (P.hWrite && ig < P.ngFF) r[o.hFF + ig * nV1 + i] = st.hFF[ig];
         }
     }
+}
+
+// Phase B: one membrane step of neuron i with its LGN synapses in global memory.
+template <bool Rng>
+__device__ __forceinline__ float step_neuron(const V1Params &P, long long t, int i, int itype, float tonic, float depC,
+                                             int m, const float *__restrict__ lgnSInfo, NState &st,
+                                             curandStateMRG32k3a &condState, curandStateMRG32k3a &noisyState) {
+    FFStep ff;
+    step_feedforward<Rng, false>(P, t, i, itype, tonic, depC, m, lgnSInfo, st, condState, noisyState, ff);
+    const float sInfo = step_membrane(P, itype, depC, ff, st);
+    P.dep[i] = ff.depOut;
+    store_step(P, t, i, sInfo, ff.depOut, st);
     return sInfo;
 }
 
@@ -1186,36 +1192,58 @@ __device__ __noinline__ float step_neuron_multi(const V1Params &P, long long t, 
     return sInfo;
 }
 
-// One delayed event: the spike of `pre` at step t (spike word sI) through delayed synapse e,
-// in its k-th arrival slot; arrival step and offset as recal_G_vec (src/coredynamics.cu:282-333)
-// and recal_G_mat (2163-2200) compute them, with explicitly rounded operations.  `code` is the
-// synapse's packed word: post type in bits 16-23, class in bit 24 (1: near block, delivered
-// through nearAcc; 0: far, through farAcc).
-__device__ __forceinline__ void far_event(const V1Params &P, long long t, int tSlot, int pre, float sI, int post,
-                                          float f, int steps, int code, float frac, int kk) {
+// step_neuron_multi on copies of the state: passing the caller's own by reference to a function
+// that is not inlined would keep them in local memory for the whole kernel.
+template <bool Rng>
+__device__ __forceinline__ float step_multi(const V1Params &P, long long t, int i, int itype, float tonic, float depC, int m,
+                                            const float *__restrict__ lgnSInfo, NState &st,
+                                            curandStateMRG32k3a &condState, curandStateMRG32k3a &noisyState) {
+    NState s = st;
+    curandStateMRG32k3a a, b;
+    if (Rng) {
+        a = condState;
+        b = noisyState;
+    }
+    const float sInfo = step_neuron_multi<Rng>(P, t, i, itype, tonic, depC, m, lgnSInfo, s, a, b);
+    st = s;
+    if (Rng) {
+        condState = a;
+        noisyState = b;
+    }
+    return sInfo;
+}
+
+// One delayed event: the spike of a neuron at step t (spike word sI, excitatory: preE) through
+// a delayed synapse, in its k-th arrival slot; arrival step and offset as recal_G_vec
+// (src/coredynamics.cu:282-333) and recal_G_mat (2163-2200) compute them, with explicitly
+// rounded operations.  `code` is the synapse's packed word: whole-step delay in bits 0-15, post
+// type in bits 16-23, class in bit 24 (1: near block, delivered through nearAcc; 0: far, through
+// farAcc).  Offset of the event in its arrival step; the event exists if 0 <= offset < dt.
+__device__ __forceinline__ float far_offset(const V1Params &P, float sI, float frac, int kk) {
+    // dtsp = (sInfo - nsp + k)*dt - time2post, rounded step by step
+    const float x = __fadd_rn(__fsub_rn(sI, (float)(unsigned)floorf(sI)), (float)kk);
+    return __fsub_rn(__fmul_rn(x, P.dt), frac);
+}
+
+__device__ __forceinline__ void far_add(const V1Params &P, long long t, int tSlot, bool preE, float sI, int post,
+                                        float f, int code, float dtsp, int kk) {
     const int ptype = (code >> 16) & 0xff;
     const bool nearClass = (code >> 24) & 1;
-    const float dt = P.dt;
+    const int ahead = (code & 0xffff) - kk;   // arrival step - t
     const unsigned nsp = (unsigned)floorf(sI);
-    // dtsp = (sInfo - nsp + k)*dt - time2post, rounded step by step
-    const float x = __fadd_rn(__fsub_rn(sI, (float)nsp), (float)kk);
-    const float dtsp = __fsub_rn(__fmul_rn(x, dt), frac);
-    if (!(dtsp < dt && dtsp >= 0 && f > 0)) return;
-    const long long tArr = t + steps - kk;
-    if (tArr < t || tArr - t >= P.farDepth - 1) {
+    if (ahead < 0 || ahead >= P.farDepth - 1) {
         atomicOr(P.err, kErrFarOverflow);
         return;
     }
     const int nV1 = P.nV1;
     const int ns = P.ngE + P.ngI;
-    const bool preE = (pre % P.blockSize) < P.nE;
     const int ng = preE ? P.ngE : P.ngI;
     const int qoff = preE ? 0 : P.ngE;
-    const float delta = __fsub_rn(dt, dtsp);
-    // ring slot of tArr: tSlot is step t's (t mod farDepth, in [0, farDepth)) and 0 <= tArr - t
-    // < farDepth - 1 (the only arrival before step 0 is the delivery that precedes the first
+    const float delta = __fsub_rn(P.dt, dtsp);
+    // ring slot of the arrival step: tSlot is step t's (t mod farDepth, in [0, farDepth)) and 0 <=
+    // ahead < farDepth - 1 (the only arrival before step 0 is the delivery that precedes the first
     // step when there are initial spikes: step -1, slot farDepth - 1)
-    int aSlot = tSlot + (int)(tArr - t);
+    int aSlot = tSlot + ahead;
     if (aSlot >= P.farDepth) aSlot -= P.farDepth;
     unsigned long long *acc = (nearClass ? P.nearAcc : P.farAcc) + (size_t)aSlot * ns * 2 * nV1;
 #pragma unroll
@@ -1240,43 +1268,67 @@ __device__ __forceinline__ void far_event(const V1Params &P, long long t, int tS
     }
 }
 
-// Exclusive prefix of sm.fdeg[0..cnt) into sm.fpref (warp 0), total in sm.fpref[cnt].
-__device__ __forceinline__ void scan_degrees(Smem &sm, int cnt) {
+__device__ __forceinline__ void far_event(const V1Params &P, long long t, int tSlot, int pre, float sI, int post,
+                                          float f, int code, float frac, int kk) {
+    const float dtsp = far_offset(P, sI, frac, kk);
+    if (dtsp < P.dt && dtsp >= 0 && f > 0)
+        far_add(P, t, tSlot, (pre % P.blockSize) < P.nE, sI, post, f, code, dtsp, kk);
+}
+
+// Pushes the delayed events of up to 32 spikers of step t, one per lane (e0: first synapse, deg:
+// synapses, sI: spike word, preE; lanes without one: deg 0), with all lanes of the warps that
+// share them: warp `part` of `parts`.  sameStep: the events arriving in step t itself (whole-step
+// delay 0 or 1 with as many whole steps of the window, deg then counts only such synapses);
+// otherwise those arriving later.  A lane's items are 32 * parts apart; U of them are fetched
+// together.  The fixed-point ring makes the sums independent of who pushes what, and in which
+// order.
+template <int U>
+__device__ __forceinline__ void push_spikers(const V1Params &P, long long t, int tSlot, int e0, int deg, float sI,
+                                             bool preE, bool sameStep, int part, int parts) {
     const int lane = threadIdx.x & 31;
-    if ((threadIdx.x >> 5) == 0) {
-        int run = 0;
-        for (int base = 0; base < cnt; base += 32) {
-            const int r = base + lane;
-            const int d = r < cnt ? sm.fdeg[r] : 0;
-            int incl = d;
+    int incl = deg;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += y;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    // synapse of item w of the owning lane r: e0[r] + w - (incl[r] - deg[r])
+    const int shift = e0 - (incl - deg);
+    const unsigned packed = __ballot_sync(0xffffffffu, preE);
+    const float dt = P.dt;
+    for (int base = part * 32; base < total; base += U * parts * 32) {
+        int4 rc[U];
+        int own[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int w = base + u * parts * 32 + lane;
+            // first lane whose inclusive count exceeds w
+            int lo = 0;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const int y = __shfl_sync(0xffffffffu, incl, lo + o - 1);
+                if (y <= w) lo += o;
             }
-            if (r < cnt) sm.fpref[r] = run + incl - d;
-            run += __shfl_sync(0xffffffffu, incl, 31);
+            const int e = __shfl_sync(0xffffffffu, shift, lo & 31) + w;
+            own[u] = w < total ? lo : -1;
+            if (w < total) rc[u] = __ldg(P.farRec + e);
         }
-        if (lane == 0) sm.fpref[cnt] = run;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const float s = __shfl_sync(0xffffffffu, sI, own[u] & 31);
+            if (own[u] < 0) continue;
+            const bool pe = (packed >> own[u]) & 1;
+            const float f = __int_as_float(rc[u].y), frac = __int_as_float(rc[u].w);
+            const int code = rc[u].z, steps = code & 0xffff;
+            // the two arrival slots of the spike; at most one holds the event, up to rounding
+            const float d0 = far_offset(P, s, frac, 0), d1 = far_offset(P, s, frac, 1);
+            const bool k0 = d0 < dt && d0 >= 0 && f > 0 && (steps == 0) == sameStep;
+            const bool k1 = d1 < dt && d1 >= 0 && f > 0 && (steps == 1) == sameStep;
+            if (k0 || k1) far_add(P, t, tSlot, pe, s, rc[u].x, f, code, k0 ? d0 : d1, k0 ? 0 : 1);
+            if (k0 && k1) far_add(P, t, tSlot, pe, s, rc[u].x, f, code, d1, 1);
+        }
     }
-}
-
-// Entry r of the chunk in shared memory that owns flattened work item w: the last r with
-// fpref[r] <= w.
-__device__ __forceinline__ int owner_of(const Smem &sm, int cnt, int w) {
-    int lo = 0, hi = cnt - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (sm.fpref[mid] <= w) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
-// Ring slot of step t in the far/near event rings.
-__device__ __forceinline__ int far_ring_slot(const V1Params &P, long long t) {
-    const long long r = t % P.farDepth;
-    return (int)(r < 0 ? r + P.farDepth : r);
 }
 
 // Spiker count (high 32 bits) and synapse work (low 32 bits) of step tl's far list.
@@ -1284,97 +1336,43 @@ __device__ __forceinline__ unsigned long long far_list_size(const V1Params &P, l
     return __ldcg(P.farCount + (int)((tl + 3) % 3));
 }
 
-// Phase C, part 1 (runs in step tl + 1): the far events of step tl's spikes that arrive after
-// step tl, from the step's global spiker list.  The (spiker, synapse) work items are numbered
-// in list order; the items [lo, hi) are shared by the nCta CTAs given, thread gt of them
-// taking lo + gt, lo + gt + G, ... (G their threads), U items per pass with their synapse
-// loads issued together.  The fixed-point ring makes the sums independent of which thread
-// appends which event, and in which order.
-template <int U = 1>
-__device__ __forceinline__ void far_push_range(const V1Params &P, long long tl, Smem &sm, int cta, int nCta,
-                                               unsigned long long size, int lo, int hi, int tSlot = -1) {
-    const int n = (int)(size >> 32);
-    if (n == 0 || lo >= hi) return;
-    const int slot = (int)((tl + 3) % 3);  // tl >= -1
-    const int4 *list = P.farList + (size_t)slot * P.nV1;
-    if (tSlot < 0) tSlot = far_ring_slot(P, tl);
-    const int G = nCta * kCta;
-    const int gt = cta * kCta + threadIdx.x;
-    int base = 0;  // items of the earlier chunks
-    for (int c0 = 0; c0 < n && base < hi; c0 += kCta) {
-        const int cnt = min(kCta, n - c0);
-        __syncthreads();
-        if (threadIdx.x < cnt) {
-            const int4 e = __ldcg(list + c0 + threadIdx.x);
-            sm.fpre[threadIdx.x] = e.x;
-            sm.fe0[threadIdx.x] = e.y;
-            sm.fdeg[threadIdx.x] = e.z;
-            sm.fsi[threadIdx.x] = __int_as_float(e.w);
-        }
-        __syncthreads();
-        scan_degrees(sm, cnt);
-        __syncthreads();
-        const int work = sm.fpref[cnt];
-        // this chunk's items [base, base + work) within [lo, hi): the first of this thread's
-        // items at or after max(base, lo)
-        const int a = max(base, lo), z = min(base + work, hi);
-        int w = lo + gt;
-        if (w < a) w += (a - w + G - 1) / G * G;
-        for (; w < z; w += U * G) {
-            int rr[U], post[U], sp[U];
-            float f[U], frac[U];
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                const int wu = w + u * G - base;
-                rr[u] = -1;
-                if (w + u * G < z) {
-                    const int r = owner_of(sm, cnt, wu);
-                    const int e = sm.fe0[r] + (wu - sm.fpref[r]);
-                    rr[u] = r;
-                    const int4 rc = __ldg(P.farRec + e);
-                    post[u] = rc.x;
-                    f[u] = __int_as_float(rc.y);
-                    sp[u] = rc.z;
-                    frac[u] = __int_as_float(rc.w);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                if (rr[u] < 0) continue;
-                const int steps = sp[u] & 0xffff;
-                const int pre = sm.fpre[rr[u]];
-                const float sI = sm.fsi[rr[u]];
-                // the slot arriving in step tl itself (steps == k) was pushed in step tl
-                if (steps != 0) far_event(P, tl, tSlot, pre, sI, post[u], f[u], steps, sp[u], frac[u], 0);
-                if (steps != 1) far_event(P, tl, tSlot, pre, sI, post[u], f[u], steps, sp[u], frac[u], 1);
-            }
-        }
-        base += work;
+// The far events of step tl's spikes that arrive after step tl, from the step's global spiker list
+// (the per-step kernels push them in step tl + 1), shared by the kCta-thread groups of nCta CTAs.
+__device__ __forceinline__ void far_push_list(const V1Params &P, long long tl, int cta, int nCta) {
+    const int n = (int)(far_list_size(P, tl) >> 32);
+    if (n == 0) return;
+    const int4 *list = P.farList + (size_t)((tl + 3) % 3) * P.nV1;  // tl >= -1
+    const int tSlot = far_ring_slot(P, tl);
+    const int lane = threadIdx.x & 31;
+    for (int c0 = 0; c0 < n; c0 += 32) {
+        int4 e = make_int4(0, 0, 0, 0);
+        if (c0 + lane < n) e = __ldcg(list + c0 + lane);
+        push_spikers<2>(P, tl, tSlot, e.y, e.z, __int_as_float(e.w), (e.x % P.blockSize) < P.nE, false,
+                        cta * kWarps + (threadIdx.x >> 5), nCta * kWarps);
     }
 }
 
-// All of step tl's far push, shared by nCta CTAs.
-template <int U = 1>
-__device__ __forceinline__ void far_push_list(const V1Params &P, long long tl, Smem &sm, int cta, int nCta,
-                                              int tSlot = -1) {
-    const unsigned long long size = far_list_size(P, tl);
-    far_push_range<U>(P, tl, sm, cta, nCta, size, 0, (int)(size & 0xffffffffu), tSlot);
+// The far events of step t that arrive within step t itself (whole-step delay 0 or 1: the first n1
+// synapses of each list), which must be in the ring before the next step delivers it: each
+// warp pushes its own spikers'.  Also raises step t's flag of far presynaptic spikes and
+// clears the next step's (its last readers are two steps back).
+__device__ __forceinline__ void far_same_step(const V1Params &P, long long t, int t3, int tSlot, bool spk, float sInfo,
+                                              bool isFarPre, bool preE, int e0, int n1, bool first) {
+    if (first) P.farFlag[t3 == 2 ? 0 : t3 + 1] = 0;
+    if (spk && sInfo > 1.0f && isFarPre) P.farFlag[t3] = 1;
+    if (__any_sync(0xffffffffu, spk && n1 > 0))
+        push_spikers<1>(P, t, tSlot, e0, spk ? n1 : 0, sInfo, preE, true, 0, 1);
 }
 
-// Phase C, part 2 (runs in step t): appends this CTA's far presynaptic spikers to step t's
-// global list (one atomic per warp), and pushes the events that arrive within step t itself
-// (whole-step delay 0 or 1: the first n1 synapses of each list), which must be in the ring
-// before the next step delivers it.  All threads of the CTA call it.
+// Phase C of the per-step kernels (runs in step t): appends this CTA's far presynaptic spikers to
+// step t's global list (one atomic per warp) and pushes their same-step events.
 __device__ __forceinline__ void far_phase(const V1Params &P, long long t, int i, bool active, float sInfo,
-                                          bool isFarPre, int e0, int deg, int n1, Smem &sm, int cta,
-                                          int tSlot = -1) {
-    if (cta == 0 && threadIdx.x == 0) {
-        P.farFlag[(t + 1) % 3] = 0;
-        P.farCount[(t + 1) % 3] = 0ull;
-    }
-    if (active && sInfo > 1.0f && isFarPre) P.farFlag[t % 3] = 1;
+                                          bool isFarPre, bool preE, int e0, int deg, int n1, int cta) {
+    const int t3 = (int)(t % 3);
+    const bool first = cta == 0 && threadIdx.x == 0;
+    if (first) P.farCount[(t + 1) % 3] = 0ull;
     const bool spk = active && sInfo >= 1.0f;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
     const bool app = spk && deg > 0;
     const unsigned ab = __ballot_sync(0xffffffffu, app);
     if (ab) {
@@ -1383,49 +1381,13 @@ __device__ __forceinline__ void far_phase(const V1Params &P, long long t, int i,
         const unsigned wsum = __reduce_add_sync(0xffffffffu, app ? (unsigned)deg : 0u);
         int base = 0;
         if (lane == leader)
-            base = (int)(atomicAdd(P.farCount + t % 3, ((unsigned long long)__popc(ab) << 32) | wsum) >> 32);
+            base = (int)(atomicAdd(P.farCount + t3, ((unsigned long long)__popc(ab) << 32) | wsum) >> 32);
         base = __shfl_sync(0xffffffffu, base, leader);
         if (app)
-            P.farList[(size_t)(t % 3) * P.nV1 + base + __popc(ab & ((1u << lane) - 1u))] =
+            P.farList[(size_t)t3 * P.nV1 + base + __popc(ab & ((1u << lane) - 1u))] =
                 make_int4(i, e0, deg, __float_as_int(sInfo));
     }
-    const bool push = spk && n1 > 0;
-    const unsigned bal = __ballot_sync(0xffffffffu, push);
-    if (lane == 0) sm.fball[warp] = bal;
-    __syncthreads();
-    // list of this CTA's neurons with same-step events (ascending) and their counts
-    int cnt = 0, pos = 0;
-#pragma unroll
-    for (int w = 0; w < kWarps; w++) {
-        const int c = __popc(sm.fball[w]);
-        if (w < warp) pos += c;
-        cnt += c;
-    }
-    if (cnt == 0) return;
-    if (push) {
-        pos += __popc(bal & ((1u << lane) - 1u));
-        sm.fpre[pos] = i;
-        sm.fsi[pos] = sInfo;
-        sm.fe0[pos] = e0;
-        sm.fdeg[pos] = n1;
-    }
-    __syncthreads();
-    scan_degrees(sm, cnt);
-    __syncthreads();
-    const int work = sm.fpref[cnt];
-    if (tSlot < 0) tSlot = far_ring_slot(P, t);
-    for (int w = threadIdx.x; w < work; w += kCta) {
-        const int r = owner_of(sm, cnt, w);
-        const int e = sm.fe0[r] + (w - sm.fpref[r]);
-        const int4 rc = __ldg(P.farRec + e);
-        const int post = rc.x;
-        const float f = __int_as_float(rc.y);
-        const int sp = rc.z;
-        const float frac = __int_as_float(rc.w);
-        const int steps = sp & 0xffff;
-        // steps is 0 or 1 here: the slot with tArr == t
-        far_event(P, t, tSlot, sm.fpre[r], sm.fsi[r], post, f, steps, sp, frac, steps);
-    }
+    far_same_step(P, t, t3, far_ring_slot(P, t), spk, sInfo, isFarPre, preE, e0, n1, first);
 }
 
 // One V1 step (with the delivery of the previous step first) for CTA `cta` of the nCta CTAs
@@ -1462,11 +1424,9 @@ __device__ __forceinline__ void v1_step_body(const V1Params &P, long long t, int
         const float depC = tonic_current(P, itype, tonic);
         const float *lgnSInfo = lgnRing + (size_t)(t % lgnSlots) * P.lgnN;
         if (P.multiSpike)
-            sInfo = step_neuron_multi<Rng>(P, t, i, itype, tonic, depC, P.nLGNperV1[i], lgnSInfo, st, condState,
-                                           noisyState);
+            sInfo = step_multi<Rng>(P, t, i, itype, tonic, depC, P.nLGNperV1[i], lgnSInfo, st, condState, noisyState);
         else
-            sInfo = step_neuron<Rng, false>(P, t, i, itype, tonic, depC, P.nLGNperV1[i], nullptr, lgnSInfo, st,
-                                        condState, noisyState);
+            sInfo = step_neuron<Rng>(P, t, i, itype, tonic, depC, P.nLGNperV1[i], lgnSInfo, st, condState, noisyState);
         store_state(P, i, st);
         if (Rng && P.condRng) P.rGenCond[i] = condState;
         if (Rng && P.noiseRng) P.rNoisy[i] = noisyState;
@@ -1481,8 +1441,8 @@ __device__ __forceinline__ void v1_step_body(const V1Params &P, long long t, int
         const int deg = active ? P.farOff[i + 1] - e0 : 0;
         const int n1 = active ? P.farN1[i] : 0;
         const bool isFarPre = active && P.farPre[i];
-        far_push_list(P, t - 1, sm, cta, nCta);
-        far_phase(P, t, i, active, sInfo, isFarPre, e0, deg, n1, sm, cta);
+        far_push_list(P, t - 1, cta, nCta);
+        far_phase(P, t, i, active, sInfo, isFarPre, local < P.nE, e0, deg, n1, cta);
     }
 }
 
@@ -1497,29 +1457,65 @@ __global__ void __launch_bounds__(kCta) v1_step_kernel(V1Params P, const long lo
     v1_step_body<Rng>(P, t, blockIdx.x, gridDim.x, lgnRing, lgnSlots, deliverPrev, doStep, sm);
 }
 
-// Split grid barrier of the persistent kernel on a monotonic arrival counter (zeroed before
-// each launch): the barrier after step s completes when the counter reaches nCTA * (s + 1).
-// arrive() publishes this CTA's writes and counts it in; wait() polls the counter with a
-// bounded number of attempts.  A CTA that gives up sets kErrBarrier and the abort bit of the
-// counter, which releases and fails every other waiter.  Work placed between the two calls
-// must not read what other CTAs write in the step (the next step's LGN spike words are
-// written before the launch).
+// ---- K steps in one launch (persistent kernels) ----
+// What a step of a patch waits for, and how the kernels below keep it short:
+//   * the spikes of its own block (near delivery).  The CTAs of a block form a cluster: each
+//     thread that spikes writes its spike word into the shared memory of every CTA of the block
+//     and each warp its ballot word, and a cluster barrier (split into arrive and wait) hands
+//     them over.  Every warp then walks the block's ballot words itself: no global round trip, no
+//     CTA barrier.  Two buffers (parity of the step): a CTA writes step t + 1's only after the
+//     cluster barrier of step t, which its peers reach after they have read step t - 1's.
+//   * the far events arriving in the step, in the global ring.  A grid barrier per step orders the
+//     same-step pushes before their delivery; a block without far synapses or foreign
+//     neighbours needs none (one barrier per launch, after its first step, still bounds the
+//     start of the grid).  Between its arrival and its wait a CTA does everything of the next step
+//     that does not depend on other blocks: the near delivery, the feed-forward conductances, the
+//     copies of the next LGN words.
+//   * the later far events of a spike only have to be in the ring one barrier later: the CTA's
+//     spikers are listed in shared memory and pushed by kCta further threads of the CTA (push
+//     warps) during the next step, or by the neuron threads themselves between arrival and
+//     wait where the registers do not allow the extra warps.
+// Bound by the latency of one warp's instruction stream (two warps per scheduler).  Measured per
+// 800-step call: one block 5,740 -> 4,440 us, 4 blocks with noise and failures (301 steps) 3,179 ->
+// 2,339, 8 blocks with far synapses (203 steps) 2,282 -> 2,155, the 32-block patch with its
+// movie 13,577 -> 12,933; 12 trials of 4 blocks in one sweep 30,285 -> 29,291.
 constexpr unsigned kBarrierAbort = 0x80000000u;
-constexpr int kPushBatch = 8;   // far-push items per thread and pass of a far-push CTA
+constexpr int kPushU = 2;       // far items a lane fetches together
 
-__device__ __forceinline__ void barrier_arrive(unsigned *count, unsigned *s_arrived) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        *s_arrived = atomicAdd(count, 1u) + 1u;
-    }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ void store_at_rank(void *smem, int rank, unsigned v) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile(
+        "{ .reg .b32 r; mapa.shared::cluster.u32 r, %0, %1; st.shared::cluster.u32 [r], %2; }" ::"r"(a), "r"(rank),
+        "r"(v)
+        : "memory");
 }
 
-__device__ __forceinline__ bool barrier_wait(unsigned *count, unsigned target, const unsigned *s_arrived,
-                                             int *err, long long limit) {
-    __shared__ int s_ok;
+// Shared memory of a persistent CTA.
+struct PShared {
+    union {
+        struct {
+            float sp[2][kMaxBS];            // spike words of the block's spikers, by parity of the step
+            unsigned ball[2][kMaxBS / 32];  // who spiked
+        } list;
+        Smem near;                          // general neighbour lists
+    };
+    // this CTA's far spikers, by parity of the step
+    int cnt[2];
+    int e0[2][kCta], deg[2][kCta];
+    float si[2][kCta];
+    unsigned char preE[2][kCta];
+    unsigned arrived, peerFail;
+    int ok, abortStep;
+};
+
+// Grid (or trial) barrier on a monotonic arrival counter, zeroed before each launch.  wait()
+// polls with a bounded number of attempts; a CTA that gives up sets kErrBarrier and the abort bit
+// of the counter, which releases and fails every other waiter.
+__device__ __forceinline__ bool barrier_wait(unsigned *count, unsigned target, PShared &sm, int *err, long long limit) {
     if (threadIdx.x == 0) {
-        unsigned c = *s_arrived;
+        unsigned c = sm.arrived;   // the counter as this CTA's arrival left it
         long long spins = 0;
         while ((c & ~kBarrierAbort) < target && !(c & kBarrierAbort)) {
             if (++spins > limit) {
@@ -1532,52 +1528,191 @@ __device__ __forceinline__ bool barrier_wait(unsigned *count, unsigned target, c
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
         }
         __threadfence();
-        s_ok = (c & kBarrierAbort) ? 0 : 1;
+        sm.ok = (c & kBarrierAbort) ? 0 : 1;
     }
-    __syncthreads();
-    return s_ok != 0;
+    neuron_sync();
+    return sm.ok != 0;
 }
 
-// K steps in one cooperative launch.  Neuron state and generators stay in registers, the LGN
-// synapses of each thread's neuron (up to kMaxLgnReg: ids, weights, the step's spike words) in
-// shared memory; one grid barrier separates consecutive steps, and while a CTA waits at it the
-// spike words of its neurons' LGN synapses for the next step are copied in.
+// This step's spikes of the CTA (rank `rank` of the block's csize CTAs) to every CTA of the block.
+__device__ __forceinline__ void publish_spikes(PShared &sm, int par, int csize, int rank, bool spk, float sInfo) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned bal = __ballot_sync(0xffffffffu, spk);
+    if (lane < csize) store_at_rank(&sm.list.ball[par][rank * kWarps + warp], lane, bal);
+    if (spk)
+        for (int r = 0; r < csize; r++)
+            store_at_rank(&sm.list.sp[par][rank * kCta + threadIdx.x], r, __float_as_uint(sInfo));
+}
+
+// Near delivery of step tp from the block's published spikes (near list: the own block alone): up
+// to 32 spikers at a time, one lane each evaluating its unit conductance (output_g/h of compute_V,
+// src/coredynamics.cu:2008-2041), the others' conMat rows read eight together.  Ascending
+// neuron order and the arithmetic of deliver_prev.
 template <bool Rng>
-__global__ void __launch_bounds__(kCta, 1) v1_persistent_kernel(V1Params P, const long long *stepBase,
-                                                                 int K, const float *__restrict__ lgnRing,
-                                                                 int lgnSlots, int deliverFirst,
-                                                                 unsigned *barrier) {
-    __shared__ Smem sm;
-    __shared__ unsigned s_arrived;
-    const long long t0 = *stepBase;
+__device__ __forceinline__ void deliver_list(const V1Params &P, long long tp, int b, int local, int i, bool active,
+                                             int itype, NState &st, curandStateMRG32k3a &condState, const float *sp,
+                                             const unsigned *ball) {
+    const int lane = threadIdx.x & 31;
+    const int bs = P.blockSize, nE = P.nE, ngE = P.ngE, ngI = P.ngI;
+    const unsigned wb = ball[lane];
+    unsigned nz = __ballot_sync(0xffffffffu, wb != 0);
+    float *recNear = nullptr;
+    int nDraw = 0, cntE = 0;
+    if constexpr (Rng) {
+        if (P.recNear && active) {
+            const long long rs = tp - P.recStep0;
+            if (rs >= 0 && rs < P.recSteps) recNear = P.recNear + ((size_t)rs * P.nV1 + i) * P.recCap;
+        }
+        const unsigned inE = (lane + 1) * 32 <= nE ? 0xffffffffu : (lane * 32 < nE ? (1u << (nE - lane * 32)) - 1u : 0u);
+        cntE = __reduce_add_sync(0xffffffffu, __popc(wb & inE));
+    }
+    if (nz) {
+        float lgE[kMaxNG], lhE[kMaxNG], lgI[kMaxNG], lhI[kMaxNG];
+#pragma unroll
+        for (int ig = 0; ig < kMaxNG; ig++) lgE[ig] = lhE[ig] = lgI[ig] = lhI[ig] = 0.f;
+        const float *col = P.conMat + (size_t)b * P.nnbMax * bs * bs + local;
+        unsigned cur = 0u;
+        int w = 0, done = 0;
+        while (nz || cur) {
+            int j = 0, n = 0;
+            while (n < 32) {
+                if (!cur) {
+                    if (!nz) break;
+                    w = __ffs(nz) - 1;
+                    nz &= nz - 1;
+                    cur = __shfl_sync(0xffffffffu, wb, w);
+                }
+                const int bit = __ffs(cur) - 1;
+                cur &= cur - 1;
+                if (lane == n) j = w * 32 + bit;
+                n++;
+            }
+            float og[kMaxNG], oh[kMaxNG];
+            for (int r0 = 0; r0 < n; r0 += kConBatch) {
+                float sv[kConBatch];
+#pragma unroll
+                for (int k = 0; k < kConBatch; k++) {
+                    const int jr = __shfl_sync(0xffffffffu, j, (r0 + k) & 31);
+                    sv[k] = (r0 + k < n && active) ? __ldg(col + (size_t)jr * bs) : 0.f;
+                }
+                if (r0 == 0) {
+                    const float sI = sp[j];
+                    const float nsp = floorf(sI);
+                    const float tsp = (sI - nsp) * P.dt;
+                    const bool isE = j < nE;
+#pragma unroll
+                    for (int ig = 0; ig < kMaxNG; ig++) {
+                        og[ig] = oh[ig] = 0.f;
+                        if (lane < n && ig < (isE ? ngE : ngI))
+                            cond_input_v(isE ? P.condE.rise[ig] : P.condI.rise[ig],
+                                         isE ? P.condE.decay[ig] : P.condI.decay[ig],
+                                         isE ? P.condE.dod[ig] : P.condI.dod[ig], og[ig], oh[ig], nsp, P.dt - tsp);
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < kConBatch; k++) {
+                    if (r0 + k >= n) break;
+                    const int r = r0 + k;
+                    const bool isE = __shfl_sync(0xffffffffu, j, r) < nE;
+                    float strength = sv[k];
+                    if constexpr (Rng) {
+                        if (strength > 0 && P.condRng)
+                            strength = near_failure(P, strength, isE, isE ? done + r : done + r - cntE, itype, condState,
+                                                    recNear, nDraw);
+                    }
+#pragma unroll
+                    for (int ig = 0; ig < kMaxNG; ig++) {
+                        const float g = __shfl_sync(0xffffffffu, og[ig], r), h = __shfl_sync(0xffffffffu, oh[ig], r);
+                        if (strength > 0) {
+                            if (isE && ig < ngE) {
+                                const float str = strength * P.pE[itype * ngE + ig];
+                                lgE[ig] += str * g;
+                                lhE[ig] += str * h;
+                            }
+                            if (!isE && ig < ngI) {
+                                const float str = strength * P.pI[itype * ngI + ig];
+                                lgI[ig] += str * g;
+                                lhI[ig] += str * h;
+                            }
+                        }
+                    }
+                }
+            }
+            done += n;
+        }
+#pragma unroll
+        for (int ig = 0; ig < kMaxNG; ig++) {
+            st.gE[ig] += lgE[ig]; st.hE[ig] += lhE[ig];
+            st.gI[ig] += lgI[ig]; st.hI[ig] += lhI[ig];
+        }
+    }
+    if (Rng && recNear) P.recNearCount[(size_t)(tp - P.recStep0) * P.nV1 + i] = nDraw;
+}
+
+// The later far events of the CTA's spikers of step t (list of its parity), by nWarps warps.
+__device__ __forceinline__ void push_own(const V1Params &P, long long t, int tSlot, const PShared &sm, int par, int part,
+                                         int nWarps) {
+    const int n = sm.cnt[par], lane = threadIdx.x & 31;
+    for (int c0 = 0; c0 < n; c0 += 32) {
+        const int q = c0 + lane;
+        const bool in = q < n;
+        push_spikers<kPushU>(P, t, tSlot, in ? sm.e0[par][q] : 0, in ? sm.deg[par][q] : 0, in ? sm.si[par][q] : 1.f,
+                             in && sm.preE[par][q], false, part, nWarps);
+    }
+}
+
+// `steps` steps of the patch P from step t0 for CTA `cta` of its nCta CTAs (csize of them to a
+// cluster), with the neuron state, the generators and (up to mCap) the LGN synapses of its neurons
+// held on the SM.  Threads past kCta are push warps.  dyn: LGN weights, spike words and ids
+// [mRows][kCta] each.  General: patches with more than mRows LGN synapses or with several spikes per
+// step are accepted too.  False if a barrier gave up.
+template <bool Rng, bool General>
+__device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0, int steps, int cta, int nCta,
+                                                 const float *__restrict__ lgnRing, int lgnSlots, bool deliverFirst,
+                                                 unsigned *barrier, PShared &sm, float *dyn,
+                                                 int mRows) {
     const int bs = P.blockSize;
     const int nq = (bs + kCta - 1) / kCta;
-    const int nNeuron = (int)gridDim.x - P.pushCta;
-    // the far-push CTAs take the first items of each step's push (one batch per thread), the
-    // neuron CTAs the rest after their own step work
-    const int pushShare = P.pushCta * kCta * kPushBatch;
-    if ((int)blockIdx.x >= nNeuron) {
-        // far-push CTA: in step t it pushes the far events of step t - 1's spikers (those that
-        // arrive after step t - 1) while the neuron CTAs deliver and step; the grid barrier
-        // that ends step t orders them before the delivery that reads them
-        int fsPrev = far_ring_slot(P, t0 - 1);  // far ring slot of step t0 + s - 1
-        for (int s = 0; s < K; s++) {
-            if (P.farOn) {
-                const unsigned long long size = far_list_size(P, t0 + s - 1);
-                far_push_range<kPushBatch>(P, t0 + s - 1, sm, (int)blockIdx.x - nNeuron, P.pushCta, size, 0,
-                                           min((int)(size & 0xffffffffu), pushShare), fsPrev);
-            }
-            if (++fsPrev == P.farDepth) fsPrev = 0;
-            if (s + 1 < K) {
-                barrier_arrive(barrier, &s_arrived);
-                if (!barrier_wait(barrier, (unsigned)gridDim.x * (unsigned)(s + 1), &s_arrived, P.err, P.waitSpins))
-                    break;
+    const int b = cta / nq, rank = cta % nq;
+    const bool pushWarps = blockDim.x > kCta;
+    // as launched: a tool that relaunches the kernel without clusters gets the general path
+    int csize;
+    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(csize));
+    const bool list = P.noDelay && P.nearSelf && csize == nq;
+    const bool coupled = P.farOn || (P.noDelay && !list);
+    auto cta_sync = [&]() {
+        if (pushWarps) asm volatile("bar.sync 0, %0;" ::"n"(2 * kCta) : "memory");
+        else neuron_sync();
+    };
+    if (threadIdx.x >= kCta) {
+        // push warps: one CTA barrier per step hands over the step's spikers; they take part in
+        // the cluster barriers without anything to publish
+        int slot = far_ring_slot(P, t0);
+        const int part = (threadIdx.x - kCta) >> 5;
+        cta_sync();
+        if (list) {
+            cluster_arrive();
+            cluster_wait();
+            if (deliverFirst) {
+                cluster_arrive();
+                cluster_wait();
             }
         }
-        return;
+        for (int s = 0; s < steps; s++) {
+            const bool handOver = list && s + 1 < steps;
+            if (handOver) cluster_arrive();
+            cta_sync();
+            if (sm.abortStep == s) {
+                if (handOver) cluster_wait();
+                break;
+            }
+            push_own(P, t0 + s, slot, sm, (int)((t0 + s) & 1), part, kWarps);
+            if (++slot == P.farDepth) slot = 0;
+            if (handOver) cluster_wait();
+        }
+        return true;
     }
-    const int b = blockIdx.x / nq;
-    const int local = (blockIdx.x % nq) * kCta + threadIdx.x;
+    const int local = rank * kCta + threadIdx.x;
     const bool active = local < bs;
     const int i = b * bs + (active ? local : 0);
     const int itype = type_of(P, active ? local : 0);
@@ -1590,63 +1725,177 @@ __global__ void __launch_bounds__(kCta, 1) v1_persistent_kernel(V1Params P, cons
     const float tonic = active ? P.tonicDep[i] : 0.f;
     const float depC = tonic_current(P, itype, tonic);
     const int m = active ? P.nLGNperV1[i] : 0;
-    // this neuron's LGN synapses in shared memory, [synapse][kCta] per array: weights, the
-    // current step's spike words (copied in asynchronously a step ahead), cell ids
-    extern __shared__ __align__(16) float lgnSm[];
-    const int mx = P.maxLGN;
-    float *smW = lgnSm + threadIdx.x;
-    float *smS = lgnSm + (size_t)mx * kCta + threadIdx.x;
-    int *smI = reinterpret_cast<int *>(lgnSm + (size_t)2 * mx * kCta) + threadIdx.x;
-    for (int q = 0; q < m; q++) {
-        smI[q * kCta] = __ldg(P.lgnId + (size_t)q * P.nV1 + i);
-        smW[q * kCta] = __ldg(P.sLGN + (size_t)q * P.nV1 + i);
-    }
-    // ring slots kept incrementally (t mod lgnSlots, t mod farDepth)
-    int lgnSlot = (int)(t0 % lgnSlots);
-    int fsT = far_ring_slot(P, t0), fsPrev = far_ring_slot(P, t0 - 1);
-    if (active) lgn_words_async(lgnRing + (size_t)lgnSlot * P.lgnN, smI, smS, m);
     // this neuron's outgoing far list (static for the run)
     const int farE0 = (P.farOn && active) ? P.farOff[i] : 0;
     const int farDeg = (P.farOn && active) ? P.farOff[i + 1] - farE0 : 0;
     const int farN1 = (P.farOn && active) ? P.farN1[i] : 0;
     const bool isFarPre = P.farOn && active && P.farPre[i];
-    for (int s = 0; s < K; s++) {
+    // LGN synapses in shared memory, [synapse][kCta] per array from this thread's column: weights,
+    // the step's spike words (copied in asynchronously a step ahead), cell ids
+    const bool smemSyn = !General || (P.maxLGN <= mRows && !P.multiSpike);
+    float *smW = dyn + threadIdx.x;
+    float *smS = dyn + (size_t)mRows * kCta + threadIdx.x;
+    int *smI = reinterpret_cast<int *>(dyn + (size_t)2 * mRows * kCta) + threadIdx.x;
+    int lgnSlot = (int)(t0 % lgnSlots);
+    if (smemSyn) {
+        for (int q = 0; q < m; q++) {
+            smI[q * kCta] = __ldg(P.lgnId + (size_t)q * P.nV1 + i);
+            smW[q * kCta] = __ldg(P.sLGN + (size_t)q * P.nV1 + i);
+        }
+        if (active) lgn_words_async(lgnRing + (size_t)lgnSlot * P.lgnN, smI, smS, m);
+    }
+    // far events of step t0 - 1 that a per-step launch (or the initial spikes) left to push
+    if (P.farOn) far_push_list(P, t0 - 1, cta, nCta);
+    if (threadIdx.x == 0) {
+        sm.cnt[0] = sm.cnt[1] = 0;
+        sm.abortStep = -1;
+        sm.peerFail = 0u;
+    }
+    if (list && threadIdx.x < 2 * (kMaxBS / 32)) sm.list.ball[threadIdx.x >> 5][threadIdx.x & 31] = 0u;
+    cta_sync();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        // the last CTA to arrive: everyone has read the list that was left
+        sm.arrived = atomicAdd(barrier, 1u) + 1u;
+        if (sm.arrived == (unsigned)nCta && P.farOn)
+            P.farCount[0] = P.farCount[1] = P.farCount[2] = 0ull;
+    }
+    if (list) {
+        cluster_arrive();   // the peers run, and are done with an earlier trial's buffers
+        cluster_wait();
+        if (deliverFirst) {
+            const float w = active ? __ldcg(P.sInfo + (size_t)((t0 - 1) & 1) * P.nV1 + i) : 0.f;
+            publish_spikes(sm, (int)((t0 - 1) & 1), csize, rank, w >= 1.0f, w);
+            cluster_arrive();
+        }
+    }
+    // ring and record slots kept incrementally
+    int fsT = P.farOn ? far_ring_slot(P, t0) : 0, fsPrev = P.farOn ? far_ring_slot(P, t0 - 1) : 0;
+    int t3 = (int)(t0 % 3);
+    FFStep ff;
+    bool ok = true;
+    for (int s = 0; s < steps; s++) {
         const long long t = t0 + s;
-        const unsigned long long farSize = P.farOn ? far_list_size(P, t - 1) : 0ull;
-        if (s > 0 || deliverFirst) deliver_prev<Rng>(P, t - 1, b, local, i, active, itype, st, condState, sm, fsPrev);
+        const int par = (int)(t & 1);
+        const bool dl = s > 0 || deliverFirst;
+        if (list && dl) {
+            cluster_wait();
+            deliver_list<Rng>(P, t - 1, b, local, i, active, itype, st, condState, sm.list.sp[par ^ 1],
+                              sm.list.ball[par ^ 1]);
+        }
         const int lgnNext = lgnSlot + 1 == lgnSlots ? 0 : lgnSlot + 1;
+        const float *lgnSInfo = lgnRing + (size_t)lgnSlot * P.lgnN;
+        auto feed_forward = [&]() {
+            if (!active || (General && P.multiSpike)) return;
+            if (smemSyn) {
+                lgn_words_wait();
+                step_feedforward<Rng, true>(P, t, i, itype, tonic, depC, m, lgnSInfo, st, condState, noisyState, ff,
+                                            smW, smS);
+            } else {
+                step_feedforward<Rng, false>(P, t, i, itype, tonic, depC, m, lgnSInfo, st, condState, noisyState, ff);
+            }
+        };
+        // failure draws of the near synapses precede those of the LGN synapses: with a general
+        // neighbour list they come after the barrier
+        const bool ffEarly = list || !dl;
+        if (ffEarly) feed_forward();
+        if (s > 0 && (coupled || s == 1)) {
+            const unsigned target = (unsigned)nCta * (coupled ? (unsigned)(s + 1) : 1u);
+            ok = barrier_wait(barrier, target, sm, P.err, P.waitSpins);
+            if (!coupled && list) {
+                // the only grid barrier of the launch: the CTAs of a cluster have to agree, or one
+                // would go on publishing into the shared memory of one that has left
+                if (!ok && threadIdx.x < csize) store_at_rank(&sm.peerFail, threadIdx.x, 1u);
+                cluster_arrive();
+                cluster_wait();
+                ok = sm.peerFail == 0u;
+                if (!ok) break;
+            }
+            if (!ok) {
+                if (threadIdx.x == 0) sm.abortStep = s;
+                if (pushWarps) cta_sync();
+                // a peer that passed this barrier publishes step s into this CTA's shared memory; it
+                // fails at the next one, which this CTA does not reach
+                if (list && s + 1 < steps) {
+                    cluster_arrive();
+                    cluster_wait();
+                }
+                break;
+            }
+        }
+        if (dl) {
+            if (!list) {
+                deliver_prev<Rng>(P, t - 1, b, local, i, active, itype, st, condState, sm.near, P.farOn ? fsPrev : -1);
+            } else if (active) {
+                if (P.farClass) {
+                    FarIn fin;
+                    far_fetch(P, fsPrev, t3 == 0 ? 2 : t3 - 1, i, fin);
+                    far_apply(P, fsPrev, i, fin, st);
+                }
+                if (P.rec) record_conductances(P, t - 1, i, st);
+            }
+        }
+        if (!ffEarly) feed_forward();
         float sInfo = 0.f;
-        if (active) {
-            const float *lgnSInfo = lgnRing + (size_t)lgnSlot * P.lgnN;
-            lgn_words_wait();
-            sInfo = step_neuron<Rng, false, true>(P, t, i, itype, tonic, depC, m, nullptr, lgnSInfo, st, condState,
-                                                  noisyState, nullptr, smW, smS);
-            if (P.spikeCount && sInfo >= 1.0f) P.spikeCount[i] += (unsigned)floorf(sInfo);
-            if (sInfo >= 1.0f) prefetch_spiker(P, b, local, farE0, farDeg);
+        if (active && !(General && P.multiSpike)) sInfo = step_membrane(P, itype, depC, ff, st);
+        if (General && active && P.multiSpike)
+            sInfo = step_multi<Rng>(P, t, i, itype, tonic, depC, m, lgnSInfo, st, condState, noisyState);
+        const bool spk = active && sInfo >= 1.0f;
+        if (list && s + 1 < steps) {
+            publish_spikes(sm, par, csize, rank, spk, sInfo);
+            cluster_arrive();
         }
+        if (spk) prefetch_spiker(P, b, local, farE0, farDeg);
         if (P.farOn) {
-            far_push_range(P, t - 1, sm, blockIdx.x, nNeuron, farSize, pushShare, (int)(farSize & 0xffffffffu),
-                           fsPrev);
-            far_phase(P, t, i, active, sInfo, isFarPre, farE0, farDeg, farN1, sm, blockIdx.x, fsT);
+            if (spk && farDeg > 0) {
+                const int q = atomicAdd(&sm.cnt[par], 1);
+                sm.e0[par][q] = farE0;
+                sm.deg[par][q] = farDeg;
+                sm.si[par][q] = sInfo;
+                sm.preE[par][q] = local < P.nE;
+            }
+            far_same_step(P, t, t3, fsT, spk, sInfo, isFarPre, local < P.nE, farE0, farN1, cta == 0 && threadIdx.x == 0);
         }
+        if (active && !(General && P.multiSpike)) store_step(P, t, i, sInfo, ff.depOut, st);
+        if (P.spikeCount && spk) atomicAdd(P.spikeCount + i, (unsigned)floorf(sInfo));
+        if (coupled) {
+            cta_sync();
+            if (threadIdx.x == 0) {
+                sm.cnt[par ^ 1] = 0;   // pushed: step t + 1's spikers go there
+                if (s + 1 < steps) {
+                    __threadfence();
+                    sm.arrived = atomicAdd(barrier, 1u) + 1u;
+                }
+            }
+        }
+        // the LGN rows of all steps are complete before the launch: the next step's words are
+        // copied in while this CTA waits
+        if (smemSyn && active && s + 1 < steps) lgn_words_async(lgnRing + (size_t)lgnNext * P.lgnN, smI, smS, m);
+        if (P.farOn && !pushWarps) push_own(P, t, fsT, sm, par, threadIdx.x >> 5, kWarps);
+        lgnSlot = lgnNext;
         fsPrev = fsT;
         if (++fsT == P.farDepth) fsT = 0;
-        if (s + 1 < K) {
-            barrier_arrive(barrier, &s_arrived);
-            // the next step's LGN rows are complete before the launch: their copies run while
-            // this CTA waits at the barrier
-            if (active) lgn_words_async(lgnRing + (size_t)lgnNext * P.lgnN, smI, smS, m);
-            if (!barrier_wait(barrier, (unsigned)gridDim.x * (unsigned)(s + 1), &s_arrived, P.err, P.waitSpins))
-                break;
-        }
-        lgnSlot = lgnNext;
+        t3 = t3 == 2 ? 0 : t3 + 1;
     }
-    lgn_words_wait();
+    if (smemSyn) lgn_words_wait();
     if (active) {
         store_state(P, i, st);
+        if (!(General && P.multiSpike)) P.dep[i] = ff.depOut;
         if (Rng && P.condRng) P.rGenCond[i] = condState;
         if (Rng && P.noiseRng) P.rNoisy[i] = noisyState;
     }
+    return ok;
+}
+
+// K steps of one patch in one cooperative launch.
+template <bool Rng>
+__global__ void __launch_bounds__(2 * kCta, 1) v1_persistent_kernel(V1Params P, const long long *stepBase, int K,
+                                                                    const float *__restrict__ lgnRing, int lgnSlots,
+                                                                    int deliverFirst, unsigned *barrier) {
+    __shared__ PShared sm;
+    extern __shared__ __align__(16) float lgnSm[];
+    persistent_steps<Rng, false>(P, *stepBase, K, blockIdx.x, gridDim.x, lgnRing, lgnSlots, deliverFirst != 0,
+                          barrier, sm, lgnSm, P.maxLGN);
 }
 
 // rand_spInit (src/coredynamics.cu:5-146) for a network without initial spikes: seeds the
@@ -1875,7 +2124,7 @@ __global__ void v1_sp_push_kernel(V1Params P, const float *H, int depth) {
         const float frac = P.farFrac[e];
         const int steps = sp & 0xffff;
         if (!((sp >> 24) & 1)) {
-            if (sLast >= 1.0f && steps <= 1) far_event(P, -1, far_ring_slot(P, -1), i, sLast, post, f, steps, sp, frac, steps);
+            if (sLast >= 1.0f && steps <= 1) far_event(P, -1, far_ring_slot(P, -1), i, sLast, post, f, sp, frac, steps);
             continue;
         }
         for (int q = 0; q < depth; q++) {
@@ -1883,14 +2132,14 @@ __global__ void v1_sp_push_kernel(V1Params P, const float *H, int depth) {
             if (w < 1.0f) continue;
             const long long th = q == 0 ? -1 : (long long)q - depth - 1;
             const long long k = th + steps + 1;
-            if (k == 0 || k == 1) far_event(P, th, far_ring_slot(P, th), i, w, post, f, steps, sp, frac, (int)k);
+            if (k == 0 || k == 1) far_event(P, th, far_ring_slot(P, th), i, w, post, f, sp, frac, (int)k);
         }
         for (int q = 1; q < depth - 1; q++) {
             const float w = H[(size_t)q * nV1 + i];
             if (w < 1.0f) continue;
             const long long th = (long long)q - depth;
             for (int k = 0; k < 2; k++)
-                if (k <= steps && th + steps - k >= 0) far_event(P, th, far_ring_slot(P, th), i, w, post, f, steps, sp, frac, k);
+                if (k <= steps && th + steps - k >= 0) far_event(P, th, far_ring_slot(P, th), i, w, post, f, sp, frac, k);
         }
     }
 }
@@ -1976,55 +2225,90 @@ cudaError_t launch_v1_step(const V1Params &p, const long long *stepBase, int ste
     return cudaGetLastError();
 }
 
-// Number of CTAs of the persistent kernel and whether they can all be resident at once.
+// A cooperative launch of `grid` CTAs in clusters of csize.
+struct CoopLaunch {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    CoopLaunch(int grid, int threads, size_t smem, int csize, cudaStream_t st) {
+        cfg.gridDim = dim3(grid);
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = csize;
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = csize > 1 ? 2 : 1;
+    }
+};
+
+// CTAs of a kernel that can be resident at once, in whole clusters.
+template <class Kern>
+static int resident_ctas(Kern kern, int threads, size_t smem, int csize, int device) {
+    int n = 0;
+    if (csize > 1) {
+        CoopLaunch cl(csize, threads, smem, csize, nullptr);
+        cl.cfg.attrs = cl.attr + 1;
+        cl.cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, kern, &cl.cfg) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        return n * csize;
+    }
+    int sms = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n * sms;
+}
+
 // Dynamic shared memory of the persistent kernel: weights, spike words and ids of up to maxLGN
 // LGN synapses per thread.
 static size_t v1_persistent_smem(const V1Params &p) {
     return (size_t)3 * std::max(p.maxLGN, 1) * kCta * sizeof(float);
 }
 
-int v1_persistent_ctas(const V1Params &p, int device, bool *fits, int *pushCtas) {
+// The shape of the persistent launch: a block's CTAs as a cluster, with push warps when there are
+// far synapses and every CTA still finds an SM; else without push warps (two CTAs share an SM);
+// else single CTAs, whose near delivery then goes through global memory.
+bool v1_persistent_shape(const V1Params &p, int device, int *cluster, int *threads) {
     const int nq = (p.blockSize + kCta - 1) / kCta;
     const int n = p.nblock * nq;
-    *pushCtas = 0;
-    int perSM = 0, sms = 0;
+    int coop = 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
+    if (!coop || p.maxLGN > kMaxLgnReg) return false;
     const int maxDyn = (int)((size_t)3 * kMaxLgnReg * kCta * sizeof(float));
     cudaFuncSetAttribute(v1_persistent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxDyn);
     cudaFuncSetAttribute(v1_persistent_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxDyn);
     const size_t dyn = v1_persistent_smem(p);
-    if (needs_rng(p))
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, v1_persistent_kernel<true>, kCta, dyn);
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, v1_persistent_kernel<false>, kCta, dyn);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    int coop = 0;
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
-    *fits = coop && perSM > 0 && n <= perSM * sms && p.maxLGN <= kMaxLgnReg;
-    // far-push CTAs on the SMs the neuron CTAs leave free (at most a quarter of the neuron
-    // CTAs, at least 8 when that many are free: each one more CTA at every grid barrier)
-    if (*fits && p.farOn) *pushCtas = std::min(perSM * sms - n, std::max(8, n / 4));
-    return n;
+    const int shapes[3][2] = {{nq, 2 * kCta}, {nq, kCta}, {1, kCta}};
+    for (int k = p.farOn ? 0 : 1; k < 3; k++) {
+        const int fit = needs_rng(p) ? resident_ctas(v1_persistent_kernel<true>, shapes[k][1], dyn, shapes[k][0], device)
+                                     : resident_ctas(v1_persistent_kernel<false>, shapes[k][1], dyn, shapes[k][0], device);
+        if (fit < n) continue;
+        *cluster = shapes[k][0];
+        *threads = shapes[k][1];
+        return true;
+    }
+    return false;
 }
 
 cudaError_t launch_v1_persistent(const V1Params &p, const long long *stepBase, int K, const float *lgnRing,
                                  int lgnSlots, int deliverFirst, unsigned *barrier, cudaStream_t st) {
     const int nq = (p.blockSize + kCta - 1) / kCta;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(p.nblock * nq + p.pushCta);
-    cfg.blockDim = dim3(kCta);
-    cfg.dynamicSmemBytes = v1_persistent_smem(p);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    CoopLaunch cl(p.nblock * nq, p.threads, v1_persistent_smem(p), p.cluster, st);
     cudaError_t e = cudaMemsetAsync(barrier, 0, sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
     if (needs_rng(p))
-        return cudaLaunchKernelEx(&cfg, v1_persistent_kernel<true>, p, stepBase, K, lgnRing, lgnSlots,
+        return cudaLaunchKernelEx(&cl.cfg, v1_persistent_kernel<true>, p, stepBase, K, lgnRing, lgnSlots,
                                   deliverFirst, barrier);
-    return cudaLaunchKernelEx(&cfg, v1_persistent_kernel<false>, p, stepBase, K, lgnRing, lgnSlots,
+    return cudaLaunchKernelEx(&cl.cfg, v1_persistent_kernel<false>, p, stepBase, K, lgnRing, lgnSlots,
                               deliverFirst, barrier);
 }
 
@@ -2090,98 +2374,15 @@ __global__ void __launch_bounds__(kCta, MinB) v1_batch_step_kernel(const BatchTr
 // slotCtas CTAs (the largest trial's CTA count); slot s runs active trials s, s + nSlots, ...
 // one after the other, each for its steps of the chunk, with the trial's state in registers
 // and a barrier among the trial's own CTAs between steps (no grid-wide barrier: trials are
-// independent).  The step is the per-step kernels' (same delivery order, same arithmetic), so
-// every trial computes what the per-step batch and pv1_run compute for it.
-template <bool Rng>
-__device__ __forceinline__ void batch_trial_steps(const V1Params &P, long long t0, int steps, int cta, int nCta,
-                                                  const float *__restrict__ lgnRing, int lgnSlots, bool deliverFirst,
-                                                  unsigned *barrier, Smem &sm, unsigned *s_arrived,
-                                                  float *dyn) {
-    const int bs = P.blockSize;
-    const int nq = (bs + kCta - 1) / kCta;
-    const int b = cta / nq;
-    const int local = (cta % nq) * kCta + threadIdx.x;
-    const bool active = local < bs;
-    const int i = b * bs + (active ? local : 0);
-    const int itype = type_of(P, active ? local : 0);
-    NState st;
-    load_state(P, i, st);
-    curandStateMRG32k3a condState, noisyState;
-    if (Rng && P.condRng && active) condState = P.rGenCond[i];
-    if (Rng && P.noiseRng && active) noisyState = P.rNoisy[i];
-    const float tonic = active ? P.tonicDep[i] : 0.f;
-    const float depC = tonic_current(P, itype, tonic);
-    const int m = active ? P.nLGNperV1[i] : 0;
-    const int farE0 = (P.farOn && active) ? P.farOff[i] : 0;
-    const int farDeg = (P.farOn && active) ? P.farOff[i + 1] - farE0 : 0;
-    const int farN1 = (P.farOn && active) ? P.farN1[i] : 0;
-    const bool isFarPre = P.farOn && active && P.farPre[i];
-    // short LGN lists: ids, weights and the step's spike words in shared memory ([synapse][kCta]
-    // from the thread's column), the next step's words copied in while the trial's CTAs meet at
-    // the barrier -- as the single-patch persistent kernel does
-    const bool smemSyn = dyn && P.maxLGN <= kBatchLgn && !P.multiSpike;
-    float *smW = dyn + threadIdx.x;
-    float *smS = dyn + (size_t)kBatchLgn * kCta + threadIdx.x;
-    int *smI = reinterpret_cast<int *>(dyn + (size_t)2 * kBatchLgn * kCta) + threadIdx.x;
-    // ring slots kept incrementally (t mod lgnSlots, t mod farDepth)
-    int lgnSlot = (int)(t0 % lgnSlots);
-    int fsT = P.farOn ? far_ring_slot(P, t0) : 0, fsPrev = P.farOn ? far_ring_slot(P, t0 - 1) : 0;
-    if (smemSyn) {
-        for (int q = 0; q < m; q++) {
-            smI[q * kCta] = __ldg(P.lgnId + (size_t)q * P.nV1 + i);
-            smW[q * kCta] = __ldg(P.sLGN + (size_t)q * P.nV1 + i);
-        }
-        if (active) lgn_words_async(lgnRing + (size_t)lgnSlot * P.lgnN, smI, smS, m);
-    }
-    for (int s = 0; s < steps; s++) {
-        const long long t = t0 + s;
-        if (s > 0 || deliverFirst)
-            deliver_prev<Rng>(P, t - 1, b, local, i, active, itype, st, condState, sm, P.farOn ? fsPrev : -1);
-        const int lgnNext = lgnSlot + 1 == lgnSlots ? 0 : lgnSlot + 1;
-        float sInfo = 0.f;
-        if (active) {
-            const float *lgnSInfo = lgnRing + (size_t)lgnSlot * P.lgnN;
-            if (P.multiSpike) {
-                sInfo = step_neuron_multi<Rng>(P, t, i, itype, tonic, depC, m, lgnSInfo, st, condState, noisyState);
-            } else if (smemSyn) {
-                lgn_words_wait();
-                sInfo = step_neuron<Rng, false, true>(P, t, i, itype, tonic, depC, m, nullptr, lgnSInfo, st,
-                                                      condState, noisyState, nullptr, smW, smS);
-            } else {
-                sInfo = step_neuron<Rng, false>(P, t, i, itype, tonic, depC, m, nullptr, lgnSInfo, st, condState,
-                                                noisyState);
-            }
-            if (P.spikeCount && sInfo >= 1.0f) P.spikeCount[i] += (unsigned)floorf(sInfo);
-        }
-        if (P.farOn) {
-            far_push_list(P, t - 1, sm, cta, nCta, fsPrev);
-            far_phase(P, t, i, active, sInfo, isFarPre, farE0, farDeg, farN1, sm, cta, fsT);
-            fsPrev = fsT;
-            if (++fsT == P.farDepth) fsT = 0;
-        }
-        if (s + 1 < steps) {
-            barrier_arrive(barrier, s_arrived);
-            if (smemSyn && active) lgn_words_async(lgnRing + (size_t)lgnNext * P.lgnN, smI, smS, m);
-            if (!barrier_wait(barrier, (unsigned)nCta * (unsigned)(s + 1), s_arrived, P.err, P.waitSpins)) break;
-        }
-        lgnSlot = lgnNext;
-    }
-    if (smemSyn) lgn_words_wait();
-    if (active) {
-        store_state(P, i, st);
-        if (Rng && P.condRng) P.rGenCond[i] = condState;
-        if (Rng && P.noiseRng) P.rNoisy[i] = noisyState;
-    }
-}
-
-template <bool Rng>
+// independent).  The step is the single patch's (persistent_steps), so every trial computes
+// what the per-step batch and pv1_run compute for it.
+template <bool Rng, bool General>
 __global__ void __launch_bounds__(kCta, 2) v1_batch_persistent_kernel(const BatchTrial *__restrict__ trials,
                                                                      const int *__restrict__ activeList,
                                                                      const int *__restrict__ nActive, int slotCtas,
                                                                      int nSlots, int K, unsigned *barriers) {
-    __shared__ Smem sm;
+    __shared__ PShared sm;
     __shared__ __align__(16) BatchTrial sT;
-    __shared__ unsigned s_arrived;
     extern __shared__ __align__(16) float dyn[];   // LGN synapses: weights, words, ids [kBatchLgn][kCta] each
     const int slot = blockIdx.x / slotCtas, c = blockIdx.x % slotCtas;
     const int na = *nActive;
@@ -2198,60 +2399,43 @@ __global__ void __launch_bounds__(kCta, 2) v1_batch_persistent_kernel(const Batc
         const long long left = sT.tEnd - t0;
         const int steps = left < K ? (int)left : K;
         if (steps <= 0) continue;
-        batch_trial_steps<Rng>(sT.v, t0, steps, c, sT.nCta, sT.lgnRing, sT.lgnSlots, t0 >= sT.tDeliverFrom,
-                               barriers + q, sm, &s_arrived, dyn);
+        // a trial whose barrier gave up ends the slot: its cluster's CTAs leave it a step apart
+        if (!persistent_steps<Rng, General>(sT.v, t0, steps, c, sT.nCta, sT.lgnRing, sT.lgnSlots,
+                                            t0 >= sT.tDeliverFrom, barriers + q, sm, dyn, kBatchLgn))
+            return;
     }
 }
 
-// The kernel's shared memory (Smem, the trial block and 72 KB of LGN synapses) passes the
+// The kernel's shared memory (PShared, the trial block and 72 KB of LGN synapses) passes the
 // 48 KB a block gets without opting in; two blocks still fit an SM.
 constexpr size_t kBatchDyn = (size_t)3 * kBatchLgn * kCta * sizeof(float);
-static cudaError_t batch_persistent_smem_optin() {
-    static cudaError_t done = cudaErrorNotReady;
-    if (done == cudaErrorNotReady) {
-        const int dyn = (int)kBatchDyn;
-        done = cudaFuncSetAttribute(v1_batch_persistent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
-        if (done == cudaSuccess)
-            done = cudaFuncSetAttribute(v1_batch_persistent_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        dyn);
-    }
-    return done;
+
+using BatchKernel = void (*)(const BatchTrial *, const int *, const int *, int, int, int, unsigned *);
+static BatchKernel batch_kernel(bool rng, bool general) {
+    if (general) return rng ? v1_batch_persistent_kernel<true, true> : v1_batch_persistent_kernel<false, true>;
+    return rng ? v1_batch_persistent_kernel<true, false> : v1_batch_persistent_kernel<false, false>;
 }
 
-int v1_batch_persistent_capacity(bool rng, int device) {
-    int perSM = 0, sms = 0;
-    if (batch_persistent_smem_optin() != cudaSuccess) return 0;
-    const size_t dyn = kBatchDyn;
-    cudaError_t e = rng ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, v1_batch_persistent_kernel<true>, kCta, dyn)
-                        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, v1_batch_persistent_kernel<false>, kCta, dyn);
-    if (e != cudaSuccess) return 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
-    return perSM * sms;
+// Whether a trial needs the general kernel: LGN lists past kBatchLgn or several spikes per step.
+bool v1_batch_general(const V1Params &p) { return p.multiSpike || p.maxLGN > kBatchLgn; }
+
+int v1_batch_persistent_capacity(bool rng, bool general, int device, int csize) {
+    int coop = 0;
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop) return 0;
+    BatchKernel k = batch_kernel(rng, general);
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBatchDyn) != cudaSuccess) return 0;
+    return resident_ctas(k, kCta, kBatchDyn, csize, device);
 }
 
 cudaError_t launch_v1_batch_persistent(const BatchTrial *trials, const int *activeList, const int *nActive,
                                        int slotCtas, int nSlots, int K, unsigned *barriers, int nTrials, bool rng,
-                                       cudaStream_t st) {
-    if (nSlots <= 0 || slotCtas <= 0) return cudaErrorInvalidValue;
-    cudaError_t e = batch_persistent_smem_optin();
+                                       bool general, int csize, cudaStream_t st) {
+    if (nSlots <= 0 || slotCtas <= 0 || csize <= 0 || slotCtas % csize) return cudaErrorInvalidValue;
+    cudaError_t e = cudaMemsetAsync(barriers, 0, (size_t)nTrials * sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(barriers, 0, (size_t)nTrials * sizeof(unsigned), st);
-    if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nSlots * slotCtas);
-    cfg.blockDim = dim3(kCta);
-    cfg.dynamicSmemBytes = kBatchDyn;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (rng)
-        return cudaLaunchKernelEx(&cfg, v1_batch_persistent_kernel<true>, trials, activeList, nActive, slotCtas,
-                                  nSlots, K, barriers);
-    return cudaLaunchKernelEx(&cfg, v1_batch_persistent_kernel<false>, trials, activeList, nActive, slotCtas, nSlots,
-                              K, barriers);
+    CoopLaunch cl(nSlots * slotCtas, kCta, kBatchDyn, csize, st);
+    return cudaLaunchKernelEx(&cl.cfg, batch_kernel(rng, general), trials, activeList, nActive, slotCtas, nSlots, K,
+                              barriers);
 }
 
 template <bool Rng>
