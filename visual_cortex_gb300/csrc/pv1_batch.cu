@@ -233,6 +233,7 @@ int pv1_batch_create(pv1_plan *const *plans, uint32_t nTrials, const uint64_t *t
         T.v = v.vp;
         T.v.spikeCount = b->dCounts + b->countOff[q];
         T.lgnRing = v.lgnRing;
+        T.lgnBits = v.lgnBits;
         T.lgnSlots = v.lgnSlots;
         T.nCta = v.vp.nblock * ((v.vp.blockSize + 255) / 256);
         T.step = v.d_stepBase;
@@ -440,7 +441,9 @@ int pv1_batch_sweep(pv1_batch *b, float *ms) {
         const int rows = (int)left[q];
         const size_t cells = (size_t)L[q].p.nLGN;
         float *sp = nullptr, *fr = nullptr;
-        if (!fresh(&sp, (size_t)rows * cells) || (L[q].p.outFr && !fresh(&fr, (size_t)rows * cells))) {
+        unsigned *bits = nullptr;
+        if (!fresh(&sp, (size_t)rows * cells) || !fresh((float **)&bits, (size_t)rows * L[q].p.bitW) ||
+            (L[q].p.outFr && !fresh(&fr, (size_t)rows * cells))) {
             release();
             return bfail(b, PV1_E_NOMEM, "cudaMalloc of the sweep's LGN buffers");
         }
@@ -448,6 +451,8 @@ int pv1_batch_sweep(pv1_batch *b, float *ms) {
         if (L[q].p.outFr) L[q].p.outFr = fr;
         L[q].p.outSlots = rows;
         T[q].lgnRing = sp;
+        T[q].lgnBits = bits;
+        L[q].p.outBits = bits;
         T[q].lgnSlots = rows;
     }
     // slot schedule: longest trial first, each to the least loaded slot; the kernel's slot s

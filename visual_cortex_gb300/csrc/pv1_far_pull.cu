@@ -218,12 +218,11 @@ __global__ void far_pull_sum_kernel(V1Params P, const long long *stepBase, long 
                     for (int ig = 0; ig < kMaxNG; ig++) {
                         if (preE && ig < ngE) {
                             const float fv = __fmul_rn(__fmul_rn(nsp, f), P.pE[itype * ngE + ig]);
-                            cond_input_v(P.condE.rise[ig], P.condE.decay[ig], P.condE.dod[ig], lg[ig], lh[ig], fv, delta);
+                            cond_input(P.condE, lg[ig], lh[ig], fv, delta, ig);
                         }
                         if (!preE && ig < ngI) {
                             const float fv = __fmul_rn(__fmul_rn(nsp, f), P.pI[itype * ngI + ig]);
-                            cond_input_v(P.condI.rise[ig], P.condI.decay[ig], P.condI.dod[ig], lg[ngE + ig],
-                                         lh[ngE + ig], fv, delta);
+                            cond_input(P.condI, lg[ngE + ig], lh[ngE + ig], fv, delta, ig);
                         }
                     }
                 }

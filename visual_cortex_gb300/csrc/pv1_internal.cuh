@@ -35,8 +35,17 @@ constexpr long long kDefaultWaitSpins = 20000000;
 
 // Two-state (g, h) conductance kernel with rise and decay times: the kinetics of the
 // reference's ConductanceShape (src/condShape.h:13-41).  dod = tr/(td - tr).
+// Divisions by the two times: with hi = 1/c rounded and lo the rest of 1/c, x hi + x lo in one
+// multiplication and one fused multiply-add is the correctly rounded x / c for most c (N.
+// Brisebarre, J.-M. Muller, S. K. Raina, "Accelerating correctly rounded floating-point division
+// when the divisor is known in advance", IEEE Trans. Computers 53, 2004); quick says that
+// compute_step_decay compared it with the division for every significand of x and all the
+// times of this kernel.  Scaling x by a power of two scales both, short of underflow (|x| below
+// 2^-90 or so), where the exponential of either is 1: the arguments here are -dt..0 steps.
 struct Cond {
     float rise[kMaxNG], decay[kMaxNG], dod[kMaxNG];
+    float riseHi[kMaxNG], riseLo[kMaxNG], decayHi[kMaxNG], decayLo[kMaxNG];
+    int quick;
 };
 
 __host__ inline Cond make_cond(const float *rt, const float *dc, int n) {
@@ -45,35 +54,46 @@ __host__ inline Cond make_cond(const float *rt, const float *dc, int n) {
         c.rise[i] = rt[i];
         c.decay[i] = dc[i];
         c.dod[i] = rt[i] / (dc[i] - rt[i]);
+        c.riseHi[i] = (float)(1.0 / rt[i]);
+        c.riseLo[i] = (float)(1.0 / rt[i] - c.riseHi[i]);
+        c.decayHi[i] = (float)(1.0 / dc[i]);
+        c.decayLo[i] = (float)(1.0 / dc[i] - c.decayHi[i]);
     }
     return c;
+}
+
+__device__ __forceinline__ float div_known(float x, float c, float hi, float lo, int quick) {
+    return quick ? __fmaf_rn(x, hi, __fmul_rn(x, lo)) : x / c;
+}
+
+// exp(-dt/rise) and exp(-dt/decay) over a part dt of a step.
+__device__ __forceinline__ float exp_rise(const Cond &c, float dt, int ig) {
+    return expf(div_known(-dt, c.rise[ig], c.riseHi[ig], c.riseLo[ig], c.quick));
+}
+__device__ __forceinline__ float exp_decay(const Cond &c, float dt, int ig) {
+    return expf(div_known(-dt, c.decay[ig], c.decayHi[ig], c.decayLo[ig], c.quick));
 }
 
 // Unit input of strength f arriving `dt` before the end of the interval
 // (compute_single_input_conductance, src/condShape.h:27-32).
 __device__ __forceinline__ void cond_input(const Cond &c, float &g, float &h, float f, float dt,
                                            int ig) {
-    float etr = expf(-dt / c.rise[ig]);
-    g += f * c.dod[ig] * (expf(-dt / c.decay[ig]) - etr);
-    h += f * etr;
-}
-
-// The same input with the kernel's constants passed as values (lets a caller choose between
-// two kernels without taking the address of a kernel parameter).
-__device__ __forceinline__ void cond_input_v(float rise, float decay, float dod, float &g, float &h, float f,
-                                             float dt) {
-    float etr = expf(-dt / rise);
-    g += f * dod * (expf(-dt / decay) - etr);
+    float etr = exp_rise(c, dt, ig);
+    g += f * c.dod[ig] * (exp_decay(c, dt, ig) - etr);
     h += f * etr;
 }
 
 // Exact exponential decay of (g, h) over dt (decay_conductance, src/condShape.h:34-40).
 __device__ __forceinline__ void cond_decay(const Cond &c, float &g, float &h, float dt, int ig) {
-    float etr = expf(-dt / c.rise[ig]);
-    float etd = expf(-dt / c.decay[ig]);
+    float etr = exp_rise(c, dt, ig);
+    float etd = exp_decay(c, dt, ig);
     g = g * etd + h * c.dod[ig] * (etd - etr);
     h *= etr;
 }
+
+// x / c where inv is 1/c if c is a power of two (the product is then the quotient, whatever x
+// is), else 0.
+__device__ __forceinline__ float div_pow2(float x, float c, float inv) { return inv != 0.f ? x * inv : x / c; }
 
 // Decay factors over one full step, exp(-dt/decay) and exp(-dt/rise) per species: constant
 // for a run, computed once on the device with the same expression cond_decay evaluates, so
@@ -128,6 +148,8 @@ struct LgnParams {
     curandStateMRG32k3a *state;            // [nLGN]
     float *rate;             // [K][nLGN] rates of the chunk being computed
     float *outSInfo;         // [outSlots][nLGN] spike words, row = step % outSlots
+    unsigned *outBits;       // [outSlots][bitW] bit id of a row: cell id spiked (may be null)
+    int bitW;                // words per row, a multiple of 4
     float *outFr;            // [outSlots][nLGN] rates (may be null)
     int outSlots;
     float *recU; int *recUCount; int recCap; long long recStep0; int recSteps;
@@ -162,6 +184,7 @@ struct V1Params {
     float vE, vI, vL;
     float vR[kMaxType], vThres[kMaxType], gL[kMaxType], C[kMaxType], tRef[kMaxType];
     float vT[kMaxType], deltaT[kMaxType], tau_w[kMaxType], a[kMaxType], b[kMaxType];
+    float invC[kMaxType], invDeltaT[kMaxType], invDt;   // reciprocals of powers of two, else 0 (div_pow2)
     float pFF[kMaxType * kMaxNG], pE[kMaxType * kMaxNG], pI[kMaxType * kMaxNG];
     float synFail[kMaxType * kMaxType], synPerCon[kMaxType * kMaxType];
     float synFailFF[kMaxType], synPerConFF[kMaxType], noisyDep[kMaxType];
@@ -194,6 +217,7 @@ struct V1Params {
     // LGN -> V1
     int maxLGN;
     int lgnN;                  // row length of the LGN spike ring (nLGN)
+    int lgnW;                  // words per row of the LGN spike bits (LgnParams::bitW)
     const int *nLGNperV1;      // [nV1]
     const int *lgnId;          // [maxLGN][nV1]
     const float *sLGN;         // [maxLGN][nV1]
@@ -311,6 +335,8 @@ cudaError_t launch_lgn_spatial(cudaTextureObject_t L, cudaTextureObject_t M, cud
                                int nSample, int layer0, int nLayer, int row0, float *out,
                                cudaStream_t st);
 cudaError_t launch_lgn_step(const LgnParams &p, const long long *stepBase, int K, cudaStream_t st);
+// Spike bits of K rows of the ring (row of step *stepBase + k) from their words.
+cudaError_t launch_lgn_bits(const LgnParams &p, const long long *stepBase, int K, cudaStream_t st);
 cudaError_t launch_lgn_rate_only(const LgnParams &p, const long long *stepBase, int K, cudaStream_t st);
 
 // What the allocation-free LGN entry point needs from a plan (defined in pv1_plan.cu).
@@ -356,11 +382,11 @@ cudaError_t launch_far_pull_apply(const V1Params &p, cudaStream_t st);
 // Cluster size and threads per CTA of the persistent kernel; false if its CTAs cannot all be
 // resident at once.
 bool v1_persistent_shape(const V1Params &p, int device, int *cluster, int *threads);
-// Evaluates the full-step decay factors of the three conductance kernels on the device and
-// stores them into p (synchronous).
+// Evaluates the full-step decay factors of the three conductance kernels on the device, checks the
+// quick divisions by their times and stores both into p (synchronous).
 cudaError_t compute_step_decay(V1Params &p, cudaStream_t st);
 cudaError_t launch_v1_persistent(const V1Params &p, const long long *stepBase, int K, const float *lgnRing,
-                                 int lgnSlots, int deliverFirst, unsigned *barrier, cudaStream_t st);
+                                 const unsigned *lgnBits, int lgnSlots, int deliverFirst, unsigned *barrier, cudaStream_t st);
 cudaError_t launch_advance_step(long long *stepBase, int k, cudaStream_t st);
 
 // ---- batched trials: many independent patches stepped by the same launches ----
@@ -368,6 +394,7 @@ cudaError_t launch_advance_step(long long *stepBase, int k, cudaStream_t st);
 struct BatchTrial {
     V1Params v;
     const float *lgnRing;
+    const unsigned *lgnBits;
     int lgnSlots;
     int nCta;                  // CTAs of this patch (nblock * ceil(blockSize / 256))
     long long *step;           // the trial's device step counter (its plan's)
@@ -386,6 +413,7 @@ struct PlanBatchView {
     V1Params vp;
     LgnParams lp;
     const float *lgnRing;
+    unsigned *lgnBits;
     int lgnSlots;
     long long *d_stepBase;
     long long step;

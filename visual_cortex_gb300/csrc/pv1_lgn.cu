@@ -660,6 +660,7 @@ __device__ __forceinline__ void lgn_class_body(const LgnParams &P, long long t0,
         }
     }
     __syncthreads();
+    const unsigned lanes = __ballot_sync(0xffffffffu, on);
     if (!on) return;
     int id = P.nParvo_I + cell;
     if (cell >= P.nMagno_I) id += P.nParvo_C;
@@ -713,6 +714,10 @@ __device__ __forceinline__ void lgn_class_body(const LgnParams &P, long long t0,
         }
         const float sInfo = nsp + tsp / dt;
         P.outSInfo[(size_t)(it % P.outSlots) * P.nLGN + id] = sInfo;
+        if (P.outBits) {   // without parvo cells a warp's ids are one word of the row's bits
+            const unsigned bits = __ballot_sync(lanes, sInfo >= 1.0f);
+            if ((threadIdx.x & 31) == 0) P.outBits[(size_t)(it % P.outSlots) * P.bitW + (id >> 5)] = bits;
+        }
         if (P.nFF) ff_pre_step(P, it, id, nsp, tsp, sInfo, ffVar);
     }
     P.leftTimeRate[id] = ltr;
@@ -906,6 +911,15 @@ __global__ void __launch_bounds__(256) lgn_spike_kernel(LgnParams P, const long 
     if (P.nFF > 1) P.ffPre[(size_t)P.nLGN + id] = ffVar[1];
 }
 
+// The spike bits of K rows from their words: a warp makes one word of one row.
+__global__ void __launch_bounds__(256) lgn_bits_kernel(LgnParams P, const long long *stepBase) {
+    const int id = blockIdx.x * blockDim.x + threadIdx.x;
+    const long long row = (*stepBase + blockIdx.y) % P.outSlots;
+    const bool spk = id < P.nLGN && P.outSInfo[(size_t)row * P.nLGN + id] >= 1.0f;
+    const unsigned bits = __ballot_sync(0xffffffffu, spk);
+    if ((threadIdx.x & 31) == 0 && (id >> 5) < P.bitW) P.outBits[(size_t)row * P.bitW + (id >> 5)] = bits;
+}
+
 }  // namespace pv1
 
 // ---- launchers used by the host runtime ---------------------------------------------
@@ -967,13 +981,20 @@ cudaError_t launch_parvo_spatial(cudaTextureObject_t L, cudaTextureObject_t M, c
     return cudaGetLastError();
 }
 
+cudaError_t launch_lgn_bits(const LgnParams &p, const long long *stepBase, int K, cudaStream_t st) {
+    if (p.nLGN <= 0 || K <= 0) return cudaSuccess;
+    lgn_bits_kernel<<<dim3((p.nLGN + 255) / 256, K), 256, 0, st>>>(p, stepBase);
+    return cudaGetLastError();
+}
+
 int lgn_step_launches(const LgnParams &p, int K) {
+    const int bits = p.outBits ? 1 : 0;
     if (p.nParvo == 0) {
         if (p.nMagno <= 0) return 0;
         if (p.classCtw && K <= kClassMaxK) return 1;
-        return 2;
+        return 2 + bits;
     }
-    return (p.nMagno > 0) + 2;
+    return (p.nMagno > 0) + 2 + bits;
 }
 
 cudaError_t launch_lgn_step(const LgnParams &p, const long long *stepBase, int K, cudaStream_t st) {
@@ -989,7 +1010,8 @@ cudaError_t launch_lgn_step(const LgnParams &p, const long long *stepBase, int K
         if (e != cudaSuccess) return e;
         const int n = std::max(p.nMagno, p.nParvo);
         lgn_spike_kernel<<<dim3((n + 255) / 256, 2), 256, 0, st>>>(p, stepBase, K);
-        return cudaGetLastError();
+        e = cudaGetLastError();
+        return e == cudaSuccess && p.outBits ? launch_lgn_bits(p, stepBase, K, st) : e;
     }
     if (p.nMagno <= 0) return cudaSuccess;
     if (p.classCtw && K <= kClassMaxK) {
@@ -1008,7 +1030,8 @@ cudaError_t launch_lgn_step(const LgnParams &p, const long long *stepBase, int K
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     lgn_spike_kernel<<<(p.nMagno + 255) / 256, 256, 0, st>>>(p, stepBase, K);
-    return cudaGetLastError();
+    e = cudaGetLastError();
+    return e == cudaSuccess && p.outBits ? launch_lgn_bits(p, stepBase, K, st) : e;
 }
 
 cudaError_t launch_lgn_class_batch(const BatchLgn *trials, int nTrials, int maxCellCtas, int K, cudaStream_t st) {

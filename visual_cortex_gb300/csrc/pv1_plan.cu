@@ -66,6 +66,7 @@ struct pv1_plan {
     int nFrame = 0;
     // LGN spike ring
     float *d_lgnRing = nullptr, *d_lgnFr = nullptr;
+    unsigned *d_lgnBits = nullptr;   // spike bits of the ring's rows (persistent V1 kernels)
     int lgnSlots = 0;
     // an external LGN source (pv1_set_lgn_source): rows [extStep0, extStep0 + extSteps)
     const float *extLgn = nullptr;
@@ -218,6 +219,11 @@ int lgn_stage(pv1_plan *p, long long t0, int k, const long long *d_step, cudaStr
                                     (size_t)cnt * row, cudaMemcpyDeviceToDevice, st));
         done += cnt;
     }
+    if (p->lp.outBits) {
+        cudaError_t e = launch_lgn_bits(p->lp, d_step, k, st);
+        if (e != cudaSuccess) return fail(p, PV1_E_CUDA, std::string("lgn_bits: ") + cudaGetErrorString(e));
+        if (launches) *launches += 1;
+    }
     return PV1_OK;
 }
 
@@ -230,7 +236,7 @@ int issue_chunk(pv1_plan *p, long long t0, int k, int deliverFirst, long long *l
     if (r) return r;
     cudaError_t e = cudaSuccess;
     if (p->persistent) {
-        e = launch_v1_persistent(p->vp, p->d_stepBase, k, p->d_lgnRing, p->lgnSlots, deliverFirst, p->d_barrier,
+        e = launch_v1_persistent(p->vp, p->d_stepBase, k, p->d_lgnRing, p->d_lgnBits, p->lgnSlots, deliverFirst, p->d_barrier,
                                  p->stream);
         if (e != cudaSuccess) return fail(p, PV1_E_CUDA, std::string("v1_persistent: ") + cudaGetErrorString(e));
         n += 1;
@@ -295,6 +301,7 @@ int plan_lgn_view(pv1_plan *p, PlanLgnView *out) {
     int r = ensure_all_frames(p);
     if (r) return r;
     out->lp = p->lp;
+    out->lp.outBits = nullptr;   // its rows go to the caller's buffer
     out->stream = p->stream;
     out->step = p->step;
     out->device = p->device;
@@ -320,6 +327,9 @@ int plan_batch_view(pv1_plan *p, PlanBatchView *out) {
     out->vp = p->vp;
     out->lp = p->lp;
     out->lgnRing = p->d_lgnRing;
+    out->lgnBits = p->d_lgnBits;
+    out->lp.outBits = p->d_lgnBits;
+    out->vp.lgnW = p->lp.bitW;
     out->lgnSlots = p->lgnSlots;
     out->d_stepBase = p->d_stepBase;
     out->step = p->step;
@@ -400,6 +410,15 @@ int pv1_plan_create(const pv1_v1_config *cfg, pv1_plan **out) {
     v.condFF = make_cond(c.riseFF, c.decayFF, c.ngFF);
     v.condE = make_cond(c.riseE, c.decayE, c.ngE);
     v.condI = make_cond(c.riseI, c.decayI, c.ngI);
+    auto pow2_inverse = [](float x) {
+        int e;
+        return x > 0 && std::frexp(x, &e) == 0.5f && std::abs(e) < 100 ? 1.0f / x : 0.0f;
+    };
+    v.invDt = pow2_inverse(c.dt);
+    for (int j = 0; j < kMaxType; j++) {
+        v.invC[j] = pow2_inverse(c.C[j]);
+        v.invDeltaT[j] = pow2_inverse(c.deltaT[j]);
+    }
     v.vE = c.vE;
     v.vI = c.vI;
     v.vL = c.vL;
@@ -683,6 +702,8 @@ int lgn_setup_impl(pv1_plan *p, const pv1_lgn_config *lc, const pv1_lgn_parvo_co
     // LGN spike ring (rows = step % lgnSlots)
     p->lgnSlots = std::max(2 * p->K, 2);   // two chunks: the one V1 reads, the one the LGN writes
     r = dev_alloc(p, &p->d_lgnRing, (size_t)p->lgnSlots * nLGN);
+    L.bitW = (nLGN + 127) / 128 * 4;
+    if (r == PV1_OK) r = dev_alloc(p, &p->d_lgnBits, (size_t)p->lgnSlots * L.bitW);
     if (r) return r;
     L.outSInfo = p->d_lgnRing;
     L.outFr = nullptr;
@@ -1769,7 +1790,10 @@ int pv1_set_record(pv1_plan *p, int flags, uint32_t slots) {
     if (want != p->lgnSlots) {
         free_one(p, p->d_lgnRing);
         p->lgnSlots = want;
+        free_one(p, p->d_lgnBits);
         int r = dev_alloc(p, &p->d_lgnRing, (size_t)want * p->nLGN);
+        if (r) return r;
+        r = dev_alloc(p, &p->d_lgnBits, (size_t)want * p->lp.bitW);
         if (r) return r;
     }
     if (flags & PV1_REC_LGN_FR) {
@@ -1809,8 +1833,10 @@ static int choose_mode(pv1_plan *p) {
     if (p->modeChosen) return PV1_OK;
     p->vp.cluster = 1;
     p->vp.threads = 256;
+    p->vp.lgnW = p->lp.bitW;
     p->persistent = p->allowPersistent && !p->vp.multiSpike && !p->vp.farPullOn && !p->vp.nearPullOn && !p->vp.ffMode &&
                     v1_persistent_shape(p->vp, p->device, &p->vp.cluster, &p->vp.threads);
+    p->lp.outBits = p->persistent ? p->d_lgnBits : nullptr;
     if (p->persistent && !p->d_barrier) {
         int r = dev_alloc(p, &p->d_barrier, 2);
         if (r) return r;
@@ -1901,8 +1927,8 @@ int pv1_run(pv1_plan *p, uint32_t nsteps, int sync) {
             for (int c = 0; c < nFull; c++) {
                 if (c > 0) PV1_CUDA(p, cudaStreamWaitEvent(p->stream, p->evLgn, 0));
                 PV1_CUDA(p, cudaEventRecord(p->evFree, p->stream));   // chunk c-1's V1 is done
-                e = launch_v1_persistent(p->vp, p->d_stepBase, K, p->d_lgnRing, p->lgnSlots, 1, p->d_barrier,
-                                         p->stream);
+                e = launch_v1_persistent(p->vp, p->d_stepBase, K, p->d_lgnRing, p->d_lgnBits, p->lgnSlots, 1,
+                                         p->d_barrier, p->stream);
                 if (e == cudaSuccess) e = launch_advance_step(p->d_stepBase, K, p->stream);
                 if (e != cudaSuccess) return fail(p, PV1_E_CUDA, std::string("v1_persistent: ") + cudaGetErrorString(e));
                 p->launches += 2;
@@ -2067,8 +2093,8 @@ int pv1_time_kernels(pv1_plan *p, uint32_t nsteps, float *v1_ms, float *lgn_ms, 
         PV1_CUDA(p, launch_lgn_step(p->lp, p->d_stepBase, K, p->stream));
         PV1_CUDA(p, cudaEventRecord(ev[3 * c + 1], p->stream));
         if (p->persistent) {
-            PV1_CUDA(p, launch_v1_persistent(p->vp, p->d_stepBase, K, p->d_lgnRing, p->lgnSlots, deliverFirst,
-                                             p->d_barrier, p->stream));
+            PV1_CUDA(p, launch_v1_persistent(p->vp, p->d_stepBase, K, p->d_lgnRing, p->d_lgnBits, p->lgnSlots,
+                                             deliverFirst, p->d_barrier, p->stream));
         } else {
             for (int s = 0; s < K; s++)
                 PV1_CUDA(p, launch_v1_step(p->vp, p->d_stepBase, s, p->d_lgnRing, p->lgnSlots,

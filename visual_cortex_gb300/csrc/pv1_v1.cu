@@ -35,7 +35,11 @@ constexpr int kWarps = kCta / 32;
 constexpr int kMaxBS = 1024;
 constexpr int kLgnBatch = 8;
 constexpr int kMaxLgnReg = 32;        // LGN synapses kept in shared memory by the persistent kernel
-constexpr int kBatchLgn = 24;         // the same in the batched persistent kernel (two blocks per SM)
+// The same in the batched persistent kernel, and the words of an LGN row's spike bits: with PShared
+// and the trial block its shared memory still fits an SM twice.
+constexpr int kBatchLgn = 24;
+constexpr int kBatchBits = 512;
+constexpr size_t kBatchDyn = ((size_t)2 * kBatchLgn * kCta + 2 * kBatchBits) * sizeof(float);
 constexpr int kConBatch = 8;          // conMat rows fetched together
 
 __device__ __forceinline__ int type_of(const V1Params &P, int local) {
@@ -66,19 +70,6 @@ __device__ __forceinline__ RecOff rec_off(const V1Params &P) {
     o.hI = o.hE + P.ngE * n;
     return o;
 }
-
-// Starts the copies of one step's LGN spike words of a neuron's m synapses into shared memory
-// (ids and destinations [synapse][kCta] from this thread's column); lgn_words_wait completes
-// them.  Each thread reads back only what it copied, so no CTA barrier is needed.
-__device__ __forceinline__ void lgn_words_async(const float *__restrict__ ring, const int *ids, float *dst, int m) {
-    for (int q = 0; q < m; q++) {
-        const unsigned d = (unsigned)__cvta_generic_to_shared(dst + q * kCta);
-        const float *src = ring + ids[q * kCta];
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-__device__ __forceinline__ void lgn_words_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // Per-neuron dynamic state (registers).
 struct NState {
@@ -188,8 +179,8 @@ __device__ __forceinline__ int compact_spikers(const V1Params &P, const float *_
             for (int ig = 0; ig < kMaxNG; ig++) {
                 if (ig < (isE ? P.ngE : P.ngI)) {
                     float g = 0.f, h = 0.f;
-                    cond_input_v(isE ? P.condE.rise[ig] : P.condI.rise[ig], isE ? P.condE.decay[ig] : P.condI.decay[ig],
-                                 isE ? P.condE.dod[ig] : P.condI.dod[ig], g, h, nsp, dt - tsp);
+                    if (isE) cond_input(P.condE, g, h, nsp, dt - tsp, ig);
+                    else cond_input(P.condI, g, h, nsp, dt - tsp, ig);
                     sm.og[ig][pos] = g;
                     sm.oh[ig][pos] = h;
                 }
@@ -414,11 +405,9 @@ __device__ __forceinline__ void deliver_prev(const V1Params &P, long long tp, in
 #pragma unroll
                         for (int ig = 0; ig < kMaxNG; ig++) {
                             if (preE && ig < ngE)
-                                cond_input_v(P.condE.rise[ig], P.condE.decay[ig], P.condE.dod[ig], lgE[ig], lhE[ig],
-                                             nsp * f * ipE[ig], delta);
+                                cond_input(P.condE, lgE[ig], lhE[ig], nsp * f * ipE[ig], delta, ig);
                             if (!preE && ig < ngI)
-                                cond_input_v(P.condI.rise[ig], P.condI.decay[ig], P.condI.dod[ig], lgI[ig], lhI[ig],
-                                             nsp * f * ipI[ig], delta);
+                                cond_input(P.condI, lgI[ig], lhI[ig], nsp * f * ipI[ig], delta, ig);
                         }
                     }
                 }
@@ -549,6 +538,15 @@ __device__ __forceinline__ void lgn_input(const V1Params &P, int itype, float sF
     }
 }
 
+// The LGN spikes of one step as a persistent thread knows them: which of its synapses received one,
+// the first two spike words, and ids and weights in shared memory ([synapse][kCta] from its column).
+struct LgnIn {
+    unsigned mask;
+    float w0, w1;
+    const int *ids;
+    const float *wts;
+};
+
 // What the feed-forward half of a membrane step hands to the integration half.
 struct FFStep {
     float g0[kMaxNG];          // feed-forward conductances at the start of the integrated interval
@@ -558,14 +556,13 @@ struct FFStep {
 // Phase B, first half: noise and the feed-forward conductances of step t (decay over the step and
 // the LGN input, src/coredynamics.cu:1422-1502); st.gFF/hFF leave at their end-of-step values.
 // Nothing here depends on what other neurons do in step t - 1, so the persistent kernels run it
-// while they wait for them.  With SmemSyn the spike words and weights of the neuron's synapses
-// are in shared memory (smS, smW: [synapse][kCta] from the thread's column); otherwise ids and
-// words are loaded batch by batch and weights only for synapses that received a spike.
+// while they wait for them.  With SmemSyn the spikes are known (in); otherwise ids and words are
+// loaded batch by batch and weights only for synapses that received a spike.
 template <bool Rng, bool SmemSyn>
 __device__ __forceinline__ void step_feedforward(const V1Params &P, long long t, int i, int itype, float tonic,
                                                  float depC, int m, const float *__restrict__ lgnSInfo, NState &st,
                                                  curandStateMRG32k3a &condState, curandStateMRG32k3a &noisyState,
-                                                 FFStep &ff, const float *smW = nullptr, const float *smS = nullptr) {
+                                                 FFStep &ff, const LgnIn &in = LgnIn{}) {
     const int nV1 = P.nV1;
     const float dt = P.dt;
     const int ngFF = P.ngFF;
@@ -620,17 +617,14 @@ __device__ __forceinline__ void step_feedforward(const V1Params &P, long long t,
         if (rs >= 0 && rs < P.recSteps) recFF = P.recFF + ((size_t)rs * nV1 + i) * P.recCap;
     }
     if constexpr (SmemSyn) {
-        // the step's spike words (copied in by lgn_words_async) and the weights in shared
-        // memory, [synapse][kCta] from this thread's column: no global load
-        unsigned mask = 0u;
-#pragma unroll
-        for (int q = 0; q < kMaxLgnReg; q++)
-            if (q < m) mask |= (smS[q * kCta] >= 1.0f ? 1u : 0u) << q;
-        while (mask) {
+        // the synapses that received a spike, in synapse order; the first two words are here
+        unsigned mask = in.mask;
+        for (int k = 0; mask; k++) {
             const int q = __ffs(mask) - 1;
             mask &= mask - 1;
-            lgn_input<Rng>(P, itype, smS[q * kCta], smW[q * kCta], backingUp, tBack, pf, nSynFF, g0, h0, g1, h1,
-                           condState, recFF, nFF);
+            const float sFF = k == 0 ? in.w0 : (k == 1 ? in.w1 : __ldcg(lgnSInfo + in.ids[q * kCta]));
+            lgn_input<Rng>(P, itype, sFF, in.wts[q * kCta], backingUp, tBack, pf, nSynFF, g0, h0, g1, h1, condState,
+                           recFF, nFF);
         }
     } else if (m <= kMaxLgnReg) {
         // ids and spike words in chunks of 16 (all loads of a chunk in flight together); the
@@ -692,7 +686,7 @@ __device__ __forceinline__ float step_membrane(const V1Params &P, int itype, flo
     const float vR = P.vR[itype], vThres = P.vThres[itype], gL = P.gL[itype];
     const float Cm = P.C[itype], tRef = P.tRef[itype], vT = P.vT[itype];
     const float deltaT = P.deltaT[itype], tau_w = P.tau_w[itype], aa = P.a[itype];
-    const float bb = P.b[itype];
+    const float bb = P.b[itype], invC = P.invC[itype], invDeltaT = P.invDeltaT[itype];
     const float v0 = st.v;
     float w0 = st.w;
     float tBack = st.tBack;
@@ -757,14 +751,16 @@ __device__ __forceinline__ float step_membrane(const V1Params &P, int itype, flo
         }
         float nz0, nz1;
         if (P.tau_noise > 0) { nz0 = noise0; nz1 = noise1; }
-        else { noise1 /= dt; nz0 = noise1; nz1 = noise1; }
+        else { noise1 = div_pow2(noise1, dt, P.invDt); nz0 = noise1; nz1 = noise1; }
         {
             const float dTgL = deltaT * gL;
-            const float fk1 = (-a0 * v0 + b0 + dTgL * expf((v0 - vT) / deltaT) - w0) / Cm + nz0;
+            const float fk1 =
+                div_pow2(-a0 * v0 + b0 + dTgL * expf(div_pow2(v0 - vT, deltaT, invDeltaT)) - w0, Cm, invC) + nz0;
             const float gk1 = (aa * (v0 - P.vL) - w0) / tau_w;
             const float v1 = v0 + new_dt * fk1;
             const float w1 = w0 + new_dt * gk1;
-            const float fk2 = (-a1 * v1 + b1 + dTgL * expf((v1 - vT) / deltaT) - w1) / Cm + nz1;
+            const float fk2 =
+                div_pow2(-a1 * v1 + b1 + dTgL * expf(div_pow2(v1 - vT, deltaT, invDeltaT)) - w1, Cm, invC) + nz1;
             const float gk2 = (aa * (v1 - P.vL) - w1) / tau_w;
             w = w0 + new_dt * (gk1 + gk2) / 2;
             v = v0 + new_dt * (fk1 + fk2) / 2;
@@ -1459,65 +1455,119 @@ __global__ void __launch_bounds__(kCta) v1_step_kernel(V1Params P, const long lo
 
 // ---- K steps in one launch (persistent kernels) ----
 // What a step of a patch waits for, and how the kernels below keep it short:
-//   * the spikes of its own block (near delivery).  The CTAs of a block form a cluster: each
-//     thread that spikes writes its spike word into the shared memory of every CTA of the block
-//     and each warp its ballot word, and a cluster barrier (split into arrive and wait) hands
-//     them over.  Every warp then walks the block's ballot words itself: no global round trip, no
-//     CTA barrier.  Two buffers (parity of the step): a CTA writes step t + 1's only after the
-//     cluster barrier of step t, which its peers reach after they have read step t - 1's.
+//   * the spikes of its own block (near delivery).  The CTAs of a block form a cluster: a thread
+//     that spikes writes its unit conductances into the shared memory of every CTA of the block and
+//     each warp its ballot word, as asynchronous stores that count towards an mbarrier there; a
+//     step's phase completes when every warp of the block has announced its bytes and they have
+//     landed.  No fence and no CTA barrier: every warp walks the block's ballot words itself.
+//     Two buffers (parity of the step): a warp writes step t + 1's only after the phase of step
+//     t, in which its peers announced that they had read step t - 1's.
 //   * the far events arriving in the step, in the global ring.  A grid barrier per step orders the
 //     same-step pushes before their delivery; a block without far synapses or foreign
 //     neighbours needs none (one barrier per launch, after its first step, still bounds the
 //     start of the grid).  Between its arrival and its wait a CTA does everything of the next step
-//     that does not depend on other blocks: the near delivery, the feed-forward conductances, the
-//     copies of the next LGN words.
+//     that does not depend on other blocks: the near delivery and the feed-forward conductances.
+//   * the LGN spikes: one bit per cell, a row per step copied to shared memory a step ahead by the
+//     bulk-copy engine; a neuron tests the bits of its synapses and reads the words of those that
+//     spiked (the words of all of them, 20 scattered copies per thread and step, took 1,850 cycles
+//     of an 11,000-cycle step).
 //   * the later far events of a spike only have to be in the ring one barrier later: the CTA's
 //     spikers are listed in shared memory and pushed by kCta further threads of the CTA (push
 //     warps) during the next step, or by the neuron threads themselves between arrival and
 //     wait where the registers do not allow the extra warps.
 // Bound by the latency of one warp's instruction stream (two warps per scheduler).  Measured per
-// 800-step call: one block 5,740 -> 4,440 us, 4 blocks with noise and failures (301 steps) 3,179 ->
-// 2,339, 8 blocks with far synapses (203 steps) 2,282 -> 2,155, the 32-block patch with its
-// movie 13,577 -> 12,933; 12 trials of 4 blocks in one sweep 30,285 -> 29,291.
+// call, against general CTAs with a full grid barrier per step and LGN words per synapse: one block
+// 800 steps 5,715 -> 3,541 us, 4 blocks with noise and failures 301 steps 3,151 -> 2,076, 8 blocks
+// with far synapses 203 steps 2,261 -> 1,863, the 32-block patch with its movie 800 steps 13,193 ->
+// 11,433; 12 trials of 4 blocks in one sweep 29,755 -> 25,952.
 constexpr unsigned kBarrierAbort = 0x80000000u;
 constexpr int kPushU = 2;       // far items a lane fetches together
+constexpr int kMaxBitWords = 2048;   // LGN spike bits kept in shared memory (two rows of up to 65,536 cells)
+constexpr int kMbarSpins = 1 << 24;  // polls of an mbarrier before it counts as lost
 
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
-__device__ __forceinline__ void store_at_rank(void *smem, int rank, unsigned v) {
-    const unsigned a = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile(
-        "{ .reg .b32 r; mapa.shared::cluster.u32 r, %0, %1; st.shared::cluster.u32 [r], %2; }" ::"r"(a), "r"(rank),
-        "r"(v)
-        : "memory");
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ unsigned smem_at(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ unsigned at_rank(unsigned addr, int rank) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void send_word(unsigned addr, unsigned bar, unsigned v) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(v), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void send_float4(unsigned addr, unsigned bar, float4 v) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
+                 "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)),
+                 "r"(__float_as_uint(v.w)), "r"(bar)
+                 : "memory");
+}
+// One arrival at a peer's mbarrier that announces `bytes` of asynchronous stores.
+__device__ __forceinline__ void announce(unsigned bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
+    for (int i = 0; i < kMbarSpins; i++) {
+        unsigned ok;
+        asm volatile(
+            "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
 }
 
 // Shared memory of a persistent CTA.
-struct PShared {
+struct __align__(16) PShared {
     union {
         struct {
-            float sp[2][kMaxBS];            // spike words of the block's spikers, by parity of the step
+            float4 unit[2][kMaxBS];         // g, h per species of the block's spikers, by parity of the step
             unsigned ball[2][kMaxBS / 32];  // who spiked
         } list;
         Smem near;                          // general neighbour lists
     };
+    uint64_t nearBar[2], bitBar[2];
     // this CTA's far spikers, by parity of the step
     int cnt[2];
     int e0[2][kCta], deg[2][kCta];
     float si[2][kCta];
     unsigned char preE[2][kCta];
-    unsigned arrived, peerFail;
+    unsigned peerFail;
     int ok, abortStep;
 };
+static_assert(kMaxNG == 2, "a spiker's unit conductances are two (g, h) pairs");
+
+// Phases of the mbarriers (bit k: the parity the next wait on that barrier expects); they run on over
+// the trials of a batch.
+struct Phases {
+    unsigned near0 = 0, near1 = 0, bit0 = 0, bit1 = 0;
+};
+
+// Sets up the mbarriers, once per launch; every thread of the CTA (and of its cluster) calls it.
+__device__ __forceinline__ void init_barriers(PShared &sm, int csize) {
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < 2; k++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_at(&sm.nearBar[k])), "r"(csize * kWarps));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_at(&sm.bitBar[k])));
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+}
 
 // Grid (or trial) barrier on a monotonic arrival counter, zeroed before each launch.  wait()
 // polls with a bounded number of attempts; a CTA that gives up sets kErrBarrier and the abort bit
 // of the counter, which releases and fails every other waiter.
 __device__ __forceinline__ bool barrier_wait(unsigned *count, unsigned target, PShared &sm, int *err, long long limit) {
     if (threadIdx.x == 0) {
-        unsigned c = sm.arrived;   // the counter as this CTA's arrival left it
+        unsigned c = 0;
         long long spins = 0;
-        while ((c & ~kBarrierAbort) < target && !(c & kBarrierAbort)) {
+        while (true) {
             if (++spins > limit) {
                 atomicOr(err, kErrBarrier);
                 atomicOr(count, kBarrierAbort);
@@ -1526,38 +1576,114 @@ __device__ __forceinline__ bool barrier_wait(unsigned *count, unsigned target, P
             }
             if (spins > 64) __nanosleep(32);
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
+            if ((c & ~kBarrierAbort) >= target || (c & kBarrierAbort)) break;
         }
-        __threadfence();
         sm.ok = (c & kBarrierAbort) ? 0 : 1;
     }
     neuron_sync();
     return sm.ok != 0;
 }
 
-// This step's spikes of the CTA (rank `rank` of the block's csize CTAs) to every CTA of the block.
-__device__ __forceinline__ void publish_spikes(PShared &sm, int par, int csize, int rank, bool spk, float sInfo) {
+// This step's spikes of the warp (CTA `rank` of the block's csize) to every CTA of the block: unit
+// conductances (output_g/h of compute_V, src/coredynamics.cu:2008-2041) and the ballot word.  poison:
+// tells the peers that this CTA gave up.
+__device__ __forceinline__ void publish_spikes(const V1Params &P, PShared &sm, int par, int csize, int rank, bool spk,
+                                               float sInfo, bool isE, bool poison = false) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned bal = __ballot_sync(0xffffffffu, spk);
-    if (lane < csize) store_at_rank(&sm.list.ball[par][rank * kWarps + warp], lane, bal);
-    if (spk)
-        for (int r = 0; r < csize; r++)
-            store_at_rank(&sm.list.sp[par][rank * kCta + threadIdx.x], r, __float_as_uint(sInfo));
+    const unsigned bar = smem_at(&sm.nearBar[par]);
+    if (spk) {
+        const float nsp = floorf(sInfo);
+        const float tsp = (sInfo - nsp) * P.dt;
+        float g[kMaxNG] = {0.f, 0.f}, h[kMaxNG] = {0.f, 0.f};
+#pragma unroll
+        for (int ig = 0; ig < kMaxNG; ig++) {
+            if (isE) {
+                if (ig < P.ngE) cond_input(P.condE, g[ig], h[ig], nsp, P.dt - tsp, ig);
+            } else {
+                if (ig < P.ngI) cond_input(P.condI, g[ig], h[ig], nsp, P.dt - tsp, ig);
+            }
+        }
+        const float4 u = make_float4(g[0], h[0], g[1], h[1]);
+        if (csize == 1) {
+            sm.list.unit[par][threadIdx.x] = u;
+        } else {
+            const unsigned to = smem_at(&sm.list.unit[par][rank * kCta + threadIdx.x]);
+            for (int r = 0; r < csize; r++) send_float4(at_rank(to, r), at_rank(bar, r), u);
+        }
+    }
+    if (csize == 1) {   // a block of one CTA is no cluster: plain stores and a plain arrival
+        __syncwarp();
+        if (lane == 0) {
+            sm.list.ball[par][warp] = bal;
+            if (poison) sm.peerFail = 1u;
+            asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+        }
+    } else if (lane < csize) {
+        const unsigned peer = at_rank(bar, lane);
+        const bool tell = poison && warp == 0;
+        send_word(at_rank(smem_at(&sm.list.ball[par][rank * kWarps + warp]), lane), peer, bal);
+        if (tell) send_word(at_rank(smem_at(&sm.peerFail), lane), peer, 1u);
+        announce(peer, 4u + 16u * __popc(bal) + (tell ? 4u : 0u));
+    }
 }
 
-// Near delivery of step tp from the block's published spikes (near list: the own block alone): up
-// to 32 spikers at a time, one lane each evaluating its unit conductance (output_g/h of compute_V,
-// src/coredynamics.cu:2008-2041), the others' conMat rows read eight together.  Ascending
-// neuron order and the arithmetic of deliver_prev.
+// Waits for the block's spikes of the step with parity par; false if they never came.
+__device__ __forceinline__ bool wait_spikes(PShared &sm, int par, Phases &ph) {
+    const bool in = mbar_wait(smem_at(&sm.nearBar[par]), par ? ph.near1 : ph.near0);
+    if (par) ph.near1 ^= 1u;
+    else ph.near0 ^= 1u;
+    return in;
+}
+
+// The bits of the LGN row of a step into shared memory (thread 0 issues the copy).
+__device__ __forceinline__ void fetch_bits(PShared &sm, unsigned *dst, const unsigned *row, int words, int buf) {
+    if (threadIdx.x == 0) {
+        const unsigned bar = smem_at(&sm.bitBar[buf]);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(words * 4) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         smem_at(dst)),
+                     "l"(row), "r"(words * 4), "r"(bar)
+                     : "memory");
+    }
+}
+
+// Which of a neuron's m LGN synapses (ids in shared memory, [synapse][kCta] from the thread's column,
+// rows padded to a multiple of 4) received a spike, and the first two spike words.
+__device__ __forceinline__ LgnIn lgn_spikes(const unsigned *bits, const float *__restrict__ lgnSInfo, const int *ids,
+                                            const float *wts, int m, int rows) {
+    LgnIn in{0u, 0.f, 0.f, ids, wts};
+    for (int q0 = 0; q0 < rows; q0 += 4) {
+        unsigned hit = 0u;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int id = ids[(q0 + k) * kCta];
+            hit |= ((bits[id >> 5] >> (id & 31)) & 1u) << k;
+        }
+        in.mask |= hit << q0;
+    }
+    in.mask &= m < 32 ? (1u << m) - 1u : 0xffffffffu;
+    if (in.mask) {
+        const unsigned rest = in.mask & (in.mask - 1);
+        in.w0 = __ldcg(lgnSInfo + ids[(__ffs(in.mask) - 1) * kCta]);
+        if (rest) in.w1 = __ldcg(lgnSInfo + ids[(__ffs(rest) - 1) * kCta]);
+    }
+    return in;
+}
+
+// Near delivery of step tp from the block's published spikes (near list: the own block alone), four
+// conMat rows read together.  Ascending neuron order and the arithmetic of deliver_prev.
 template <bool Rng>
 __device__ __forceinline__ void deliver_list(const V1Params &P, long long tp, int b, int local, int i, bool active,
-                                             int itype, NState &st, curandStateMRG32k3a &condState, const float *sp,
+                                             int itype, NState &st, curandStateMRG32k3a &condState, const float4 *unit,
                                              const unsigned *ball) {
     const int lane = threadIdx.x & 31;
     const int bs = P.blockSize, nE = P.nE, ngE = P.ngE, ngI = P.ngI;
     const unsigned wb = ball[lane];
     unsigned nz = __ballot_sync(0xffffffffu, wb != 0);
     float *recNear = nullptr;
-    int nDraw = 0, cntE = 0;
+    int nDraw = 0, cntE = 0, done = 0;
     if constexpr (Rng) {
         if (P.recNear && active) {
             const long long rs = tp - P.recStep0;
@@ -1572,73 +1698,51 @@ __device__ __forceinline__ void deliver_list(const V1Params &P, long long tp, in
         for (int ig = 0; ig < kMaxNG; ig++) lgE[ig] = lhE[ig] = lgI[ig] = lhI[ig] = 0.f;
         const float *col = P.conMat + (size_t)b * P.nnbMax * bs * bs + local;
         unsigned cur = 0u;
-        int w = 0, done = 0;
-        while (nz || cur) {
-            int j = 0, n = 0;
-            while (n < 32) {
-                if (!cur) {
-                    if (!nz) break;
+        int w = 0;
+        while (nz | cur) {
+            constexpr int kB = 4;
+            int j[kB];
+            float sv[kB];
+#pragma unroll
+            for (int k = 0; k < kB; k++) {
+                if (!cur && nz) {
                     w = __ffs(nz) - 1;
                     nz &= nz - 1;
                     cur = __shfl_sync(0xffffffffu, wb, w);
                 }
-                const int bit = __ffs(cur) - 1;
+                j[k] = cur ? w * 32 + __ffs(cur) - 1 : -1;
                 cur &= cur - 1;
-                if (lane == n) j = w * 32 + bit;
-                n++;
+                sv[k] = (j[k] >= 0 && active) ? __ldg(col + (size_t)j[k] * bs) : 0.f;
             }
-            float og[kMaxNG], oh[kMaxNG];
-            for (int r0 = 0; r0 < n; r0 += kConBatch) {
-                float sv[kConBatch];
 #pragma unroll
-                for (int k = 0; k < kConBatch; k++) {
-                    const int jr = __shfl_sync(0xffffffffu, j, (r0 + k) & 31);
-                    sv[k] = (r0 + k < n && active) ? __ldg(col + (size_t)jr * bs) : 0.f;
+            for (int k = 0; k < kB; k++) {
+                if (j[k] < 0) break;
+                const bool isE = j[k] < nE;
+                float strength = sv[k];
+                if constexpr (Rng) {
+                    if (strength > 0 && P.condRng)
+                        strength = near_failure(P, strength, isE, isE ? done : done - cntE, itype, condState, recNear,
+                                                nDraw);
+                    done++;
                 }
-                if (r0 == 0) {
-                    const float sI = sp[j];
-                    const float nsp = floorf(sI);
-                    const float tsp = (sI - nsp) * P.dt;
-                    const bool isE = j < nE;
+                if (strength > 0) {
+                    const float4 u = unit[j[k]];
+                    const float g[kMaxNG] = {u.x, u.z}, h[kMaxNG] = {u.y, u.w};
 #pragma unroll
                     for (int ig = 0; ig < kMaxNG; ig++) {
-                        og[ig] = oh[ig] = 0.f;
-                        if (lane < n && ig < (isE ? ngE : ngI))
-                            cond_input_v(isE ? P.condE.rise[ig] : P.condI.rise[ig],
-                                         isE ? P.condE.decay[ig] : P.condI.decay[ig],
-                                         isE ? P.condE.dod[ig] : P.condI.dod[ig], og[ig], oh[ig], nsp, P.dt - tsp);
-                    }
-                }
-#pragma unroll
-                for (int k = 0; k < kConBatch; k++) {
-                    if (r0 + k >= n) break;
-                    const int r = r0 + k;
-                    const bool isE = __shfl_sync(0xffffffffu, j, r) < nE;
-                    float strength = sv[k];
-                    if constexpr (Rng) {
-                        if (strength > 0 && P.condRng)
-                            strength = near_failure(P, strength, isE, isE ? done + r : done + r - cntE, itype, condState,
-                                                    recNear, nDraw);
-                    }
-#pragma unroll
-                    for (int ig = 0; ig < kMaxNG; ig++) {
-                        const float g = __shfl_sync(0xffffffffu, og[ig], r), h = __shfl_sync(0xffffffffu, oh[ig], r);
-                        if (strength > 0) {
-                            if (isE && ig < ngE) {
-                                const float str = strength * P.pE[itype * ngE + ig];
-                                lgE[ig] += str * g;
-                                lhE[ig] += str * h;
-                            }
-                            if (!isE && ig < ngI) {
-                                const float str = strength * P.pI[itype * ngI + ig];
-                                lgI[ig] += str * g;
-                                lhI[ig] += str * h;
-                            }
+                        if (isE && ig < ngE) {
+                            const float str = strength * P.pE[itype * ngE + ig];
+                            lgE[ig] += str * g[ig];
+                            lhE[ig] += str * h[ig];
+                        }
+                        if (!isE && ig < ngI) {
+                            const float str = strength * P.pI[itype * ngI + ig];
+                            lgI[ig] += str * g[ig];
+                            lhI[ig] += str * h[ig];
                         }
                     }
                 }
             }
-            done += n;
         }
 #pragma unroll
         for (int ig = 0; ig < kMaxNG; ig++) {
@@ -1661,23 +1765,21 @@ __device__ __forceinline__ void push_own(const V1Params &P, long long t, int tSl
     }
 }
 
-// `steps` steps of the patch P from step t0 for CTA `cta` of its nCta CTAs (csize of them to a
-// cluster), with the neuron state, the generators and (up to mCap) the LGN synapses of its neurons
-// held on the SM.  Threads past kCta are push warps.  dyn: LGN weights, spike words and ids
-// [mRows][kCta] each.  General: patches with more than mRows LGN synapses or with several spikes per
-// step are accepted too.  False if a barrier gave up.
+// `steps` steps of the patch P from step t0 for CTA `cta` of its nCta CTAs, with the neuron state, the
+// generators and (up to mRows) the LGN synapses of its neurons held on the SM.  Threads past
+// kCta are push warps.  dyn: LGN weights and ids [mRows][kCta] each (mRows a multiple of 4), then two
+// rows of LGN spike bits of bitRoom words (0: the bits are read from global memory).  General:
+// patches with more than mRows LGN synapses or with several spikes per step are accepted too.
+// False if a barrier gave up.
 template <bool Rng, bool General>
-__device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0, int steps, int cta, int nCta,
-                                                 const float *__restrict__ lgnRing, int lgnSlots, bool deliverFirst,
-                                                 unsigned *barrier, PShared &sm, float *dyn,
-                                                 int mRows) {
+__device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0, int steps, int cta, int nCta, int csize,
+                                                 const float *__restrict__ lgnRing, const unsigned *__restrict__ lgnBits,
+                                                 int lgnSlots, bool deliverFirst, unsigned *barrier, PShared &sm,
+                                                 Phases &ph, float *dyn, int mRows, int bitRoom) {
     const int bs = P.blockSize;
     const int nq = (bs + kCta - 1) / kCta;
     const int b = cta / nq, rank = cta % nq;
     const bool pushWarps = blockDim.x > kCta;
-    // as launched: a tool that relaunches the kernel without clusters gets the general path
-    int csize;
-    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(csize));
     const bool list = P.noDelay && P.nearSelf && csize == nq;
     const bool coupled = P.farOn || (P.noDelay && !list);
     auto cta_sync = [&]() {
@@ -1685,30 +1787,16 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
         else neuron_sync();
     };
     if (threadIdx.x >= kCta) {
-        // push warps: one CTA barrier per step hands over the step's spikers; they take part in
-        // the cluster barriers without anything to publish
+        // push warps: one CTA barrier per step hands over the step's spikers
         int slot = far_ring_slot(P, t0);
         const int part = (threadIdx.x - kCta) >> 5;
         cta_sync();
-        if (list) {
-            cluster_arrive();
-            cluster_wait();
-            if (deliverFirst) {
-                cluster_arrive();
-                cluster_wait();
-            }
-        }
+        if (list && csize > 1) cluster_sync();
         for (int s = 0; s < steps; s++) {
-            const bool handOver = list && s + 1 < steps;
-            if (handOver) cluster_arrive();
             cta_sync();
-            if (sm.abortStep == s) {
-                if (handOver) cluster_wait();
-                break;
-            }
+            if (sm.abortStep == s) break;
             push_own(P, t0 + s, slot, sm, (int)((t0 + s) & 1), part, kWarps);
             if (++slot == P.farDepth) slot = 0;
-            if (handOver) cluster_wait();
         }
         return true;
     }
@@ -1716,6 +1804,7 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
     const bool active = local < bs;
     const int i = b * bs + (active ? local : 0);
     const int itype = type_of(P, active ? local : 0);
+    const bool isE = local < P.nE;
 
     NState st;
     load_state(P, i, st);
@@ -1730,19 +1819,19 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
     const int farDeg = (P.farOn && active) ? P.farOff[i + 1] - farE0 : 0;
     const int farN1 = (P.farOn && active) ? P.farN1[i] : 0;
     const bool isFarPre = P.farOn && active && P.farPre[i];
-    // LGN synapses in shared memory, [synapse][kCta] per array from this thread's column: weights,
-    // the step's spike words (copied in asynchronously a step ahead), cell ids
+    // LGN synapses in shared memory, [synapse][kCta] per array from this thread's column
     const bool smemSyn = !General || (P.maxLGN <= mRows && !P.multiSpike);
+    const int rows = (P.maxLGN + 3) & ~3;
     float *smW = dyn + threadIdx.x;
-    float *smS = dyn + (size_t)mRows * kCta + threadIdx.x;
-    int *smI = reinterpret_cast<int *>(dyn + (size_t)2 * mRows * kCta) + threadIdx.x;
+    int *smI = reinterpret_cast<int *>(dyn + (size_t)mRows * kCta) + threadIdx.x;
+    unsigned *smB = reinterpret_cast<unsigned *>(dyn + (size_t)2 * mRows * kCta);
+    const bool smemBits = P.lgnW <= bitRoom;
     int lgnSlot = (int)(t0 % lgnSlots);
     if (smemSyn) {
-        for (int q = 0; q < m; q++) {
-            smI[q * kCta] = __ldg(P.lgnId + (size_t)q * P.nV1 + i);
-            smW[q * kCta] = __ldg(P.sLGN + (size_t)q * P.nV1 + i);
+        for (int q = 0; q < rows; q++) {
+            smI[q * kCta] = q < m ? __ldg(P.lgnId + (size_t)q * P.nV1 + i) : 0;
+            if (q < m) smW[q * kCta] = __ldg(P.sLGN + (size_t)q * P.nV1 + i);
         }
-        if (active) lgn_words_async(lgnRing + (size_t)lgnSlot * P.lgnN, smI, smS, m);
     }
     // far events of step t0 - 1 that a per-step launch (or the initial spikes) left to push
     if (P.farOn) far_push_list(P, t0 - 1, cta, nCta);
@@ -1756,20 +1845,18 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
     if (threadIdx.x == 0) {
         __threadfence();
         // the last CTA to arrive: everyone has read the list that was left
-        sm.arrived = atomicAdd(barrier, 1u) + 1u;
-        if (sm.arrived == (unsigned)nCta && P.farOn)
+        if (atomicAdd(barrier, 1u) + 1u == (unsigned)nCta && P.farOn)
             P.farCount[0] = P.farCount[1] = P.farCount[2] = 0ull;
     }
     if (list) {
-        cluster_arrive();   // the peers run, and are done with an earlier trial's buffers
-        cluster_wait();
+        if (csize > 1) cluster_sync();   // the peers run, and are done with an earlier trial's buffers
         if (deliverFirst) {
             const float w = active ? __ldcg(P.sInfo + (size_t)((t0 - 1) & 1) * P.nV1 + i) : 0.f;
-            publish_spikes(sm, (int)((t0 - 1) & 1), csize, rank, w >= 1.0f, w);
-            cluster_arrive();
+            publish_spikes(P, sm, (int)((t0 - 1) & 1), csize, rank, w >= 1.0f, w, isE);
         }
     }
-    // ring and record slots kept incrementally
+    if (smemSyn && smemBits) fetch_bits(sm, smB, lgnBits + (size_t)lgnSlot * P.lgnW, P.lgnW, 0);
+    // ring slots kept incrementally
     int fsT = P.farOn ? far_ring_slot(P, t0) : 0, fsPrev = P.farOn ? far_ring_slot(P, t0 - 1) : 0;
     int t3 = (int)(t0 % 3);
     FFStep ff;
@@ -1779,47 +1866,61 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
         const int par = (int)(t & 1);
         const bool dl = s > 0 || deliverFirst;
         if (list && dl) {
-            cluster_wait();
-            deliver_list<Rng>(P, t - 1, b, local, i, active, itype, st, condState, sm.list.sp[par ^ 1],
-                              sm.list.ball[par ^ 1]);
+            if (!wait_spikes(sm, par ^ 1, ph)) {
+                atomicOr(P.err, kErrBarrier);
+                sm.peerFail = 1u;
+            }
+            if (sm.peerFail) {   // a CTA of the block gave up: all of them leave here
+                ok = false;
+                if (threadIdx.x == 0) sm.abortStep = s;
+                if (pushWarps) cta_sync();
+                break;
+            }
+        } else if (!coupled) {
+            neuron_sync();
         }
         const int lgnNext = lgnSlot + 1 == lgnSlots ? 0 : lgnSlot + 1;
         const float *lgnSInfo = lgnRing + (size_t)lgnSlot * P.lgnN;
+        LgnIn in{};
+        if (smemSyn) {
+            // the other buffer was read in step s - 1, before the spikes (or barrier) just waited for
+            const unsigned *bits = lgnBits + (size_t)lgnSlot * P.lgnW;
+            if (smemBits) {
+                const int buf = s & 1;
+                if (s + 1 < steps)
+                    fetch_bits(sm, smB + (buf ^ 1) * bitRoom, lgnBits + (size_t)lgnNext * P.lgnW, P.lgnW, buf ^ 1);
+                if (mbar_wait(smem_at(&sm.bitBar[buf]), buf ? ph.bit1 : ph.bit0)) bits = smB + buf * bitRoom;
+                if (buf) ph.bit1 ^= 1u;
+                else ph.bit0 ^= 1u;
+            }
+            if (active) in = lgn_spikes(bits, lgnSInfo, smI, smW, m, rows);
+        }
+        if (list && dl)
+            deliver_list<Rng>(P, t - 1, b, local, i, active, itype, st, condState, sm.list.unit[par ^ 1],
+                              sm.list.ball[par ^ 1]);
         auto feed_forward = [&]() {
             if (!active || (General && P.multiSpike)) return;
-            if (smemSyn) {
-                lgn_words_wait();
-                step_feedforward<Rng, true>(P, t, i, itype, tonic, depC, m, lgnSInfo, st, condState, noisyState, ff,
-                                            smW, smS);
-            } else {
+            if (smemSyn)
+                step_feedforward<Rng, true>(P, t, i, itype, tonic, depC, m, lgnSInfo, st, condState, noisyState, ff, in);
+            else
                 step_feedforward<Rng, false>(P, t, i, itype, tonic, depC, m, lgnSInfo, st, condState, noisyState, ff);
-            }
         };
         // failure draws of the near synapses precede those of the LGN synapses: with a general
         // neighbour list they come after the barrier
         const bool ffEarly = list || !dl;
         if (ffEarly) feed_forward();
-        if (s > 0 && (coupled || s == 1)) {
+        if (s > 0 && nCta > 1 && (coupled || s == 1)) {
             const unsigned target = (unsigned)nCta * (coupled ? (unsigned)(s + 1) : 1u);
-            ok = barrier_wait(barrier, target, sm, P.err, P.waitSpins);
-            if (!coupled && list) {
-                // the only grid barrier of the launch: the CTAs of a cluster have to agree, or one
-                // would go on publishing into the shared memory of one that has left
-                if (!ok && threadIdx.x < csize) store_at_rank(&sm.peerFail, threadIdx.x, 1u);
-                cluster_arrive();
-                cluster_wait();
-                ok = sm.peerFail == 0u;
-                if (!ok) break;
-            }
-            if (!ok) {
+            if (!barrier_wait(barrier, target, sm, P.err, P.waitSpins)) {
+                ok = false;
+                // peers that passed this barrier still send step s to this CTA: it tells them to leave and
+                // stays until all of the block have sent
+                if (list && s + 1 < steps) {
+                    publish_spikes(P, sm, par, csize, rank, false, 0.f, isE, true);
+                    wait_spikes(sm, par, ph);
+                }
                 if (threadIdx.x == 0) sm.abortStep = s;
                 if (pushWarps) cta_sync();
-                // a peer that passed this barrier publishes step s into this CTA's shared memory; it
-                // fails at the next one, which this CTA does not reach
-                if (list && s + 1 < steps) {
-                    cluster_arrive();
-                    cluster_wait();
-                }
                 break;
             }
         }
@@ -1841,10 +1942,7 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
         if (General && active && P.multiSpike)
             sInfo = step_multi<Rng>(P, t, i, itype, tonic, depC, m, lgnSInfo, st, condState, noisyState);
         const bool spk = active && sInfo >= 1.0f;
-        if (list && s + 1 < steps) {
-            publish_spikes(sm, par, csize, rank, spk, sInfo);
-            cluster_arrive();
-        }
+        if (list && s + 1 < steps) publish_spikes(P, sm, par, csize, rank, spk, sInfo, isE);
         if (spk) prefetch_spiker(P, b, local, farE0, farDeg);
         if (P.farOn) {
             if (spk && farDeg > 0) {
@@ -1852,32 +1950,31 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
                 sm.e0[par][q] = farE0;
                 sm.deg[par][q] = farDeg;
                 sm.si[par][q] = sInfo;
-                sm.preE[par][q] = local < P.nE;
+                sm.preE[par][q] = isE;
             }
-            far_same_step(P, t, t3, fsT, spk, sInfo, isFarPre, local < P.nE, farE0, farN1, cta == 0 && threadIdx.x == 0);
+            far_same_step(P, t, t3, fsT, spk, sInfo, isFarPre, isE, farE0, farN1, cta == 0 && threadIdx.x == 0);
         }
-        if (active && !(General && P.multiSpike)) store_step(P, t, i, sInfo, ff.depOut, st);
-        if (P.spikeCount && spk) atomicAdd(P.spikeCount + i, (unsigned)floorf(sInfo));
+        // spike words other CTAs read in the next step (general neighbour lists) come before the arrival
+        const bool storeFirst = !list || (General && P.multiSpike);
+        if (storeFirst && active && !(General && P.multiSpike)) store_step(P, t, i, sInfo, ff.depOut, st);
         if (coupled) {
             cta_sync();
             if (threadIdx.x == 0) {
                 sm.cnt[par ^ 1] = 0;   // pushed: step t + 1's spikers go there
                 if (s + 1 < steps) {
                     __threadfence();
-                    sm.arrived = atomicAdd(barrier, 1u) + 1u;
+                    atomicAdd(barrier, 1u);
                 }
             }
         }
-        // the LGN rows of all steps are complete before the launch: the next step's words are
-        // copied in while this CTA waits
-        if (smemSyn && active && s + 1 < steps) lgn_words_async(lgnRing + (size_t)lgnNext * P.lgnN, smI, smS, m);
+        if (!storeFirst && active) store_step(P, t, i, sInfo, ff.depOut, st);
+        if (P.spikeCount && spk) atomicAdd(P.spikeCount + i, (unsigned)floorf(sInfo));
         if (P.farOn && !pushWarps) push_own(P, t, fsT, sm, par, threadIdx.x >> 5, kWarps);
         lgnSlot = lgnNext;
         fsPrev = fsT;
         if (++fsT == P.farDepth) fsT = 0;
         t3 = t3 == 2 ? 0 : t3 + 1;
     }
-    if (smemSyn) lgn_words_wait();
     if (active) {
         store_state(P, i, st);
         if (!(General && P.multiSpike)) P.dep[i] = ff.depOut;
@@ -1887,15 +1984,27 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
     return ok;
 }
 
+// CTAs per cluster, as launched: a tool that relaunches the kernel without clusters gets the
+// general path.
+__device__ __forceinline__ int cluster_ctas() {
+    int n;
+    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
+    return n;
+}
+
 // K steps of one patch in one cooperative launch.
 template <bool Rng>
 __global__ void __launch_bounds__(2 * kCta, 1) v1_persistent_kernel(V1Params P, const long long *stepBase, int K,
-                                                                    const float *__restrict__ lgnRing, int lgnSlots,
-                                                                    int deliverFirst, unsigned *barrier) {
+                                                                    const float *__restrict__ lgnRing,
+                                                                    const unsigned *__restrict__ lgnBits, int lgnSlots,
+                                                                    int deliverFirst, unsigned *barrier, int bitRoom) {
     __shared__ PShared sm;
     extern __shared__ __align__(16) float lgnSm[];
-    persistent_steps<Rng, false>(P, *stepBase, K, blockIdx.x, gridDim.x, lgnRing, lgnSlots, deliverFirst != 0,
-                          barrier, sm, lgnSm, P.maxLGN);
+    Phases ph;
+    const int csize = cluster_ctas();
+    init_barriers(sm, csize);
+    persistent_steps<Rng, false>(P, *stepBase, K, blockIdx.x, gridDim.x, csize, lgnRing, lgnBits, lgnSlots,
+                                 deliverFirst != 0, barrier, sm, ph, lgnSm, (P.maxLGN + 3) & ~3, bitRoom);
 }
 
 // rand_spInit (src/coredynamics.cu:5-146) for a network without initial spikes: seeds the
@@ -2018,8 +2127,8 @@ __global__ void __launch_bounds__(1024) v1_sp_init_kernel(V1Params P, unsigned l
     for (int ig = 0; ig < kMaxNG; ig++) {
         if (ig < ng) {
             float g = 0.f, h = 0.f;
-            if (isE) cond_input_v(P.condE.rise[ig], P.condE.decay[ig], P.condE.dod[ig], g, h, 1.f, dt - tsp);
-            else cond_input_v(P.condI.rise[ig], P.condI.decay[ig], P.condI.dod[ig], g, h, 1.f, dt - tsp);
+            if (isE) cond_input(P.condE, g, h, 1.f, dt - tsp, ig);
+            else cond_input(P.condI, g, h, 1.f, dt - tsp, ig);
             const size_t r = isE ? (size_t)ig * nE + sid : (size_t)ig * nI + (size_t)nE * P.ngE + sid;
             ogTab[base + r] = g;
             ohTab[base + r] = h;
@@ -2191,20 +2300,50 @@ __global__ void step_decay_kernel(Cond cFF, Cond cE, Cond cI, float dt, StepDeca
     }
 }
 
+// Compares div_known with the division for every significand x in [1, 2) and every time of the
+// kernel conds[blockIdx.y]; a difference clears its flag.
+__global__ void __launch_bounds__(256) quick_division_kernel(Cond c0, Cond c1, Cond c2, int n0, int n1, int n2, int *ok) {
+    const Cond &c = blockIdx.y == 0 ? c0 : (blockIdx.y == 1 ? c1 : c2);
+    const int n = blockIdx.y == 0 ? n0 : (blockIdx.y == 1 ? n1 : n2);
+    const float x = __uint_as_float(0x3f800000u + blockIdx.x * blockDim.x + threadIdx.x);
+    bool same = true;
+    for (int ig = 0; ig < kMaxNG; ig++) {
+        if (ig >= n) break;
+        same = same && div_known(x, c.rise[ig], c.riseHi[ig], c.riseLo[ig], 1) == x / c.rise[ig];
+        same = same && div_known(x, c.decay[ig], c.decayHi[ig], c.decayLo[ig], 1) == x / c.decay[ig];
+    }
+    if (!same) ok[blockIdx.y] = 0;
+}
+
 cudaError_t compute_step_decay(V1Params &p, cudaStream_t st) {
-    StepDecay *d = nullptr;
-    cudaError_t e = cudaMalloc(&d, 3 * sizeof(StepDecay));
+    struct Out {
+        StepDecay dec[3];
+        int ok[3];
+    } h, *d = nullptr;
+    cudaError_t e = cudaMalloc(&d, sizeof(Out));
     if (e != cudaSuccess) return e;
-    step_decay_kernel<<<1, 32, 0, st>>>(p.condFF, p.condE, p.condI, p.dt, d);
-    StepDecay h[3];
-    e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, st);
+    e = cudaMemsetAsync(d, 1, sizeof(Out), st);
+    step_decay_kernel<<<1, 32, 0, st>>>(p.condFF, p.condE, p.condI, p.dt, d->dec);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    quick_division_kernel<<<dim3((1 << 23) / 256, 3), 256, 0, st>>>(p.condFF, p.condE, p.condI, p.ngFF, p.ngE, p.ngI,
+                                                                  d->ok);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     cudaFree(d);
     if (e != cudaSuccess) return e;
-    p.decFF = h[0];
-    p.decE = h[1];
-    p.decI = h[2];
+    p.decFF = h.dec[0];
+    p.decE = h.dec[1];
+    p.decI = h.dec[2];
+    // times far from 1 could take the products of the check out of the normal range
+    auto plain = [](const Cond &c, int n) {
+        bool in = true;
+        for (int k = 0; k < n; k++) in = in && c.rise[k] > 1e-6f && c.rise[k] < 1e6f && c.decay[k] > 1e-6f && c.decay[k] < 1e6f;
+        return in;
+    };
+    p.condFF.quick = h.ok[0] != 0 && plain(p.condFF, p.ngFF);
+    p.condE.quick = h.ok[1] != 0 && plain(p.condE, p.ngE);
+    p.condI.quick = h.ok[2] != 0 && plain(p.condI, p.ngI);
     return cudaSuccess;
 }
 
@@ -2268,10 +2407,11 @@ static int resident_ctas(Kern kern, int threads, size_t smem, int csize, int dev
     return n * sms;
 }
 
-// Dynamic shared memory of the persistent kernel: weights, spike words and ids of up to maxLGN
-// LGN synapses per thread.
+// Dynamic shared memory of the persistent kernel: weights and ids of the LGN synapses of each thread,
+// two rows of LGN spike bits.
+static int v1_persistent_bits(const V1Params &p) { return p.lgnW <= kMaxBitWords ? p.lgnW : 0; }
 static size_t v1_persistent_smem(const V1Params &p) {
-    return (size_t)3 * std::max(p.maxLGN, 1) * kCta * sizeof(float);
+    return ((size_t)2 * ((p.maxLGN + 3) & ~3) * kCta + 2 * v1_persistent_bits(p)) * sizeof(float);
 }
 
 // The shape of the persistent launch: a block's CTAs as a cluster, with push warps when there are
@@ -2283,7 +2423,7 @@ bool v1_persistent_shape(const V1Params &p, int device, int *cluster, int *threa
     int coop = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
     if (!coop || p.maxLGN > kMaxLgnReg) return false;
-    const int maxDyn = (int)((size_t)3 * kMaxLgnReg * kCta * sizeof(float));
+    const int maxDyn = (int)(((size_t)2 * kMaxLgnReg * kCta + 2 * kMaxBitWords) * sizeof(float));
     cudaFuncSetAttribute(v1_persistent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxDyn);
     cudaFuncSetAttribute(v1_persistent_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxDyn);
     const size_t dyn = v1_persistent_smem(p);
@@ -2300,16 +2440,14 @@ bool v1_persistent_shape(const V1Params &p, int device, int *cluster, int *threa
 }
 
 cudaError_t launch_v1_persistent(const V1Params &p, const long long *stepBase, int K, const float *lgnRing,
-                                 int lgnSlots, int deliverFirst, unsigned *barrier, cudaStream_t st) {
+                                 const unsigned *lgnBits, int lgnSlots, int deliverFirst, unsigned *barrier,
+                                 cudaStream_t st) {
     const int nq = (p.blockSize + kCta - 1) / kCta;
     CoopLaunch cl(p.nblock * nq, p.threads, v1_persistent_smem(p), p.cluster, st);
     cudaError_t e = cudaMemsetAsync(barrier, 0, sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
-    if (needs_rng(p))
-        return cudaLaunchKernelEx(&cl.cfg, v1_persistent_kernel<true>, p, stepBase, K, lgnRing, lgnSlots,
-                                  deliverFirst, barrier);
-    return cudaLaunchKernelEx(&cl.cfg, v1_persistent_kernel<false>, p, stepBase, K, lgnRing, lgnSlots,
-                              deliverFirst, barrier);
+    return cudaLaunchKernelEx(&cl.cfg, needs_rng(p) ? v1_persistent_kernel<true> : v1_persistent_kernel<false>, p, stepBase,
+                              K, lgnRing, lgnBits, lgnSlots, deliverFirst, barrier, v1_persistent_bits(p));
 }
 
 cudaError_t launch_v1_rng_init(curandStateMRG32k3a *cond, curandStateMRG32k3a *noisy,
@@ -2383,7 +2521,10 @@ __global__ void __launch_bounds__(kCta, 2) v1_batch_persistent_kernel(const Batc
                                                                      int nSlots, int K, unsigned *barriers) {
     __shared__ PShared sm;
     __shared__ __align__(16) BatchTrial sT;
-    extern __shared__ __align__(16) float dyn[];   // LGN synapses: weights, words, ids [kBatchLgn][kCta] each
+    extern __shared__ __align__(16) float dyn[];   // LGN synapses: weights, ids [kBatchLgn][kCta] each; spike bits
+    Phases ph;
+    const int csize = cluster_ctas();
+    init_barriers(sm, csize);
     const int slot = blockIdx.x / slotCtas, c = blockIdx.x % slotCtas;
     const int na = *nActive;
     for (int j = slot; j < na; j += nSlots) {
@@ -2400,15 +2541,12 @@ __global__ void __launch_bounds__(kCta, 2) v1_batch_persistent_kernel(const Batc
         const int steps = left < K ? (int)left : K;
         if (steps <= 0) continue;
         // a trial whose barrier gave up ends the slot: its cluster's CTAs leave it a step apart
-        if (!persistent_steps<Rng, General>(sT.v, t0, steps, c, sT.nCta, sT.lgnRing, sT.lgnSlots,
-                                            t0 >= sT.tDeliverFrom, barriers + q, sm, dyn, kBatchLgn))
+        if (!persistent_steps<Rng, General>(sT.v, t0, steps, c, sT.nCta, csize, sT.lgnRing, sT.lgnBits, sT.lgnSlots,
+                                            t0 >= sT.tDeliverFrom, barriers + q, sm, ph, dyn, kBatchLgn, kBatchBits))
             return;
     }
 }
 
-// The kernel's shared memory (PShared, the trial block and 72 KB of LGN synapses) passes the
-// 48 KB a block gets without opting in; two blocks still fit an SM.
-constexpr size_t kBatchDyn = (size_t)3 * kBatchLgn * kCta * sizeof(float);
 
 using BatchKernel = void (*)(const BatchTrial *, const int *, const int *, int, int, int, unsigned *);
 static BatchKernel batch_kernel(bool rng, bool general) {
