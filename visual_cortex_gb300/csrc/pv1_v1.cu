@@ -300,10 +300,10 @@ __device__ __forceinline__ void near_ring_take(const V1Params &P, int farSlot, i
     }
 }
 
-// The conductances of step tp's record, complete once its spikes are delivered.
-__device__ __forceinline__ void record_conductances(const V1Params &P, long long tp, int i, const NState &st) {
+// The conductances of a step's record (ring slot recSlot), complete once its spikes are delivered.
+__device__ __forceinline__ void record_conductances(const V1Params &P, int recSlot, int i, const NState &st) {
     const int nV1 = P.nV1;
-    float *r = P.rec + (tp % P.recSlots) * P.recStride;
+    float *r = P.rec + recSlot * P.recStride;
     const RecOff o = rec_off(P);
 #pragma unroll
     for (int ig = 0; ig < kMaxNG; ig++) {
@@ -492,7 +492,7 @@ __device__ __forceinline__ void deliver_prev(const V1Params &P, long long tp, in
     }
     // far events (sum_G adds them after the near delivery); the ring slot is cleared
     if (far) far_apply(P, farSlot, i, fin, st);
-    if (P.rec && active) record_conductances(P, tp, i, st);
+    if (P.rec && active) record_conductances(P, (int)(tp % P.recSlots), i, st);
 }
 
 // The tonic drive of the AdEx constructor (src/coredynamics.cuh:41-49).
@@ -756,12 +756,12 @@ __device__ __forceinline__ float step_membrane(const V1Params &P, int itype, flo
             const float dTgL = deltaT * gL;
             const float fk1 =
                 div_pow2(-a0 * v0 + b0 + dTgL * expf(div_pow2(v0 - vT, deltaT, invDeltaT)) - w0, Cm, invC) + nz0;
-            const float gk1 = (aa * (v0 - P.vL) - w0) / tau_w;
+            const float gk1 = div_sparse(aa * (v0 - P.vL) - w0, tau_w);
             const float v1 = v0 + new_dt * fk1;
             const float w1 = w0 + new_dt * gk1;
             const float fk2 =
                 div_pow2(-a1 * v1 + b1 + dTgL * expf(div_pow2(v1 - vT, deltaT, invDeltaT)) - w1, Cm, invC) + nz1;
-            const float gk2 = (aa * (v1 - P.vL) - w1) / tau_w;
+            const float gk2 = div_sparse(aa * (v1 - P.vL) - w1, tau_w);
             w = w0 + new_dt * (gk1 + gk2) / 2;
             v = v0 + new_dt * (fk1 + fk2) / 2;
         }
@@ -789,14 +789,14 @@ __device__ __forceinline__ float step_membrane(const V1Params &P, int itype, flo
     return spikeCount > 0 ? 1.0f + tsp / dt : v;
 }
 
-// The step's spike word to global memory and to the records.
+// The step's spike word to global memory and to the records (ring slot recSlot).
 __device__ __forceinline__ void store_step(const V1Params &P, long long t, int i, float sInfo, float depOut,
-                                           const NState &st) {
+                                           const NState &st, int recSlot) {
     const int nV1 = P.nV1;
     __stcg(P.sInfo + (size_t)(t & 1) * nV1 + i, sInfo);
-    if (P.recSpk) P.recSpk[(size_t)(t % P.recSlots) * nV1 + i] = sInfo;
+    if (P.recSpk) P.recSpk[(size_t)recSlot * nV1 + i] = sInfo;
     if (P.rec) {
-        float *r = P.rec + (t % P.recSlots) * P.recStride;
+        float *r = P.rec + recSlot * P.recStride;
         const RecOff o = rec_off(P);
         r[o.sinfo + i] = sInfo;
         r[o.dep + i] = depOut;
@@ -819,7 +819,7 @@ __device__ __forceinline__ float step_neuron(const V1Params &P, long long t, int
     step_feedforward<Rng, false>(P, t, i, itype, tonic, depC, m, lgnSInfo, st, condState, noisyState, ff);
     const float sInfo = step_membrane(P, itype, depC, ff, st);
     P.dep[i] = ff.depOut;
-    store_step(P, t, i, sInfo, ff.depOut, st);
+    store_step(P, t, i, sInfo, ff.depOut, st, P.recSpk || P.rec ? (int)(t % P.recSlots) : 0);
     return sInfo;
 }
 
@@ -1859,6 +1859,8 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
     // ring slots kept incrementally
     int fsT = P.farOn ? far_ring_slot(P, t0) : 0, fsPrev = P.farOn ? far_ring_slot(P, t0 - 1) : 0;
     int t3 = (int)(t0 % 3);
+    const bool rec = P.recSpk || P.rec;
+    int recSlot = rec ? (int)(t0 % P.recSlots) : 0, recPrev = rec ? (int)((t0 + P.recSlots - 1) % P.recSlots) : 0;
     FFStep ff;
     bool ok = true;
     for (int s = 0; s < steps; s++) {
@@ -1933,7 +1935,7 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
                     far_fetch(P, fsPrev, t3 == 0 ? 2 : t3 - 1, i, fin);
                     far_apply(P, fsPrev, i, fin, st);
                 }
-                if (P.rec) record_conductances(P, t - 1, i, st);
+                if (P.rec) record_conductances(P, recPrev, i, st);
             }
         }
         if (!ffEarly) feed_forward();
@@ -1956,21 +1958,21 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
         }
         // spike words other CTAs read in the next step (general neighbour lists) come before the arrival
         const bool storeFirst = !list || (General && P.multiSpike);
-        if (storeFirst && active && !(General && P.multiSpike)) store_step(P, t, i, sInfo, ff.depOut, st);
+        if (storeFirst && active && !(General && P.multiSpike)) store_step(P, t, i, sInfo, ff.depOut, st, recSlot);
         if (coupled) {
             cta_sync();
             if (threadIdx.x == 0) {
                 sm.cnt[par ^ 1] = 0;   // pushed: step t + 1's spikers go there
-                if (s + 1 < steps) {
-                    __threadfence();
-                    atomicAdd(barrier, 1u);
-                }
+                if (s + 1 < steps)
+                    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(barrier) : "memory");
             }
         }
-        if (!storeFirst && active) store_step(P, t, i, sInfo, ff.depOut, st);
+        if (!storeFirst && active) store_step(P, t, i, sInfo, ff.depOut, st, recSlot);
         if (P.spikeCount && spk) atomicAdd(P.spikeCount + i, (unsigned)floorf(sInfo));
         if (P.farOn && !pushWarps) push_own(P, t, fsT, sm, par, threadIdx.x >> 5, kWarps);
         lgnSlot = lgnNext;
+        recPrev = recSlot;
+        if (++recSlot == P.recSlots) recSlot = 0;
         fsPrev = fsT;
         if (++fsT == P.farDepth) fsT = 0;
         t3 = t3 == 2 ? 0 : t3 + 1;
