@@ -247,7 +247,7 @@ int pv1_batch_create(pv1_plan *const *plans, uint32_t nTrials, const uint64_t *t
         b->step[q] = v.step;
         b->end[q] = T.tEnd;
         b->totalTiles += T.nCta;
-        b->maxCellCtas = std::max(b->maxCellCtas, (v.lp.nMagno + 127) / 128);
+        b->maxCellCtas = std::max(b->maxCellCtas, (v.lp.nMagno + kClassCells - 1) / kClassCells);
         if (!v.lp.classCtw) b->allClass = false;
         if (v.vp.condRng || v.vp.noiseRng) b->rng = true;
         if (v1_batch_general(v.vp)) b->general = true;

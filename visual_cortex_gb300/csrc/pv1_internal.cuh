@@ -20,6 +20,7 @@ constexpr int kMaxSeg = 255;   // frames one temporal window may span (segments 
 constexpr int kClassMaxK = 64;
 constexpr int kClassMaxSeg = 48;
 constexpr int kClassMaxSlots = 64;
+constexpr int kClassCells = 32;   // cells per CTA
 
 // Error word bits raised by kernels (never trap).
 constexpr int kMaxLgnMulti = 64;       // LGN synapses per neuron in the multi-spike step
@@ -125,6 +126,7 @@ struct SegTable {
     const int *nseg;     // [nPhase]
     const int *rel;      // [nPhase][maxSeg]
     const int *j0;       // [nPhase][maxSeg+1] (j0[s+1] = end of segment s)
+    const float *weight; // [nPhase][maxSeg] sums of the class's temporal weights (single-class plans)
 };
 
 // Number of stimulus frames read once step `it` has started.

@@ -570,8 +570,6 @@ __device__ __forceinline__ int frame_number(const FrameSched &fs, int currentFra
     return currentFrame - 1 - back;
 }
 
-constexpr int kClassCta = 128;
-
 // Presynaptic LTP traces of LGN cell id over step it (LGN_nonlinear with learning 1-3,
 // src/discrete_input_convol.cu:1774-1808), one per learning type (FF->E, then FF->I), each with
 // its own tauLTP: the value at the start of the step and, when the cell spiked, the value right
@@ -602,153 +600,262 @@ __device__ __forceinline__ void ff_pre_step(const LgnParams &P, long long it, in
 
 
 
-// The whole LGN step for a chunk of K steps when every magno cell has the same temporal
-// weights (one temporal kernel class): the window segment weights W[s][q] (differences of the
-// shared cumulative weights) and the frame slot of every segment are computed once per CTA;
-// each thread (one cell) stages the S values of the chunk's frames in shared memory, then for
-// each step contracts them with W, applies the logistic rate and draws the Poisson spikes.
+// The whole LGN step for a chunk of K steps when every magno cell has the same temporal weights (one
+// temporal kernel class).  A CTA owns kClassCells cells.  The weights of the window segments come
+// from a table per frame phase; the CTA lays them out by frame slot, so that the rates of eight
+// consecutive steps of a cell are eight accumulators over the chunk's frames: one value of S and two
+// 16-byte reads of weights for eight products.  Every warp takes eight steps; the rates are independent
+// of each other, only the Poisson generator is a chain, run by one warp (lane = cell) over the chunk:
+// each lane advances through the steps without a spike by itself, so that the draws of different
+// cells, at different steps, are made together.
 // The arithmetic per (cell, step) is the one of lgn_rate_kernel + lgn_spike_kernel: same
 // segment weights, same summation order, same generator calls.
-__device__ __forceinline__ void lgn_class_body(const LgnParams &P, long long t0, int K, int cellBase) {
-    extern __shared__ float sS[];                       // [kClassMaxSlots][kClassCta]
-    __shared__ float sW[kClassMaxK][kClassMaxSeg];
-    __shared__ unsigned char sSlot[kClassMaxK][kClassMaxSeg];
-    __shared__ int sNseg[kClassMaxK];
-    __shared__ int sFlo, sNU;
-    const FrameSched fs = P.fs;
-    if (threadIdx.x == 0) {
-        const int cf0 = frames_read_after_step(fs, t0);
-        const int ph0 = (int)((fs.magnoComp + (t0 + 1) * (long long)fs.denorm) % fs.ntPerFrame);
-        const int te0 = fs.frameOffset + (ph0 <= fs.magnoComp ? 2 : 1);
-        sFlo = frame_number(fs, cf0, te0 + P.seg.rel[(size_t)ph0 * P.seg.maxSeg]);
-        const long long t1 = t0 + K - 1;
-        const int cf1 = frames_read_after_step(fs, t1);
-        const int ph1 = (int)((fs.magnoComp + (t1 + 1) * (long long)fs.denorm) % fs.ntPerFrame);
-        const int te1 = fs.frameOffset + (ph1 <= fs.magnoComp ? 2 : 1);
-        const int n1 = P.seg.nseg[ph1];
-        const int Fhi = frame_number(fs, cf1, te1 + P.seg.rel[(size_t)ph1 * P.seg.maxSeg + n1 - 1]);
-        sNU = Fhi - sFlo + 1;
-        if (sNU > kClassMaxSlots || sNU < 1) atomicOr(P.err, kErrBounds);
-    }
-    __syncthreads();
-    const int Flo = sFlo, nU = min(max(sNU, 1), kClassMaxSlots);
-    for (int s = threadIdx.x; s < K; s += blockDim.x) {
-        const long long it = t0 + s;
-        const int cf = frames_read_after_step(fs, it);
-        const int phase = (int)((fs.magnoComp + (it + 1) * (long long)fs.denorm) % fs.ntPerFrame);
-        const int te = fs.frameOffset + (phase <= fs.magnoComp ? 2 : 1);
-        const int nseg = P.seg.nseg[phase];
-        sNseg[s] = nseg;
-        const int *rel = P.seg.rel + (size_t)phase * P.seg.maxSeg;
-        const int *j0 = P.seg.j0 + (size_t)phase * (P.seg.maxSeg + 1);
-        double ca = P.classCtw[j0[0]];
-        for (int q = 0; q < nseg; q++) {
-            const double cb = P.classCtw[j0[q + 1]];
-            sW[s][q] = (float)(cb - ca);
-            ca = cb;
-            const int slot = frame_number(fs, cf, te + rel[q]) - Flo;
-            sSlot[s][q] = (unsigned char)min(max(slot, 0), kClassMaxSlots - 1);
+// Bound by latency: a chunk's tables, its rates and its Poisson chain in turn.  Calls of 16 steps of one
+// block (512 cells; the stage runs before the V1 launch) went from 148 to 128 us, the sweep of 12 trials
+// of 2,048 cells from 25,246 to 23,939 us, with it.
+struct ClassShared {
+    float S[kClassMaxSlots][kClassCells];
+    float4 W[kClassMaxSlots][kClassMaxK / 4];    // weight of a frame slot in each step
+    float rT[kClassMaxK][kClassCells];           // dt * rate; then the spike word
+    float rate[kClassMaxK][kClassCells];
+    unsigned long long valid[kClassMaxK];        // frame slots a step's window covers
+    int phase[kClassMaxK], cf[kClassMaxK], tail[kClassMaxK], nseg[kClassMaxK];
+    int Flo, nU;
+};
+constexpr int kClassThreads = 256;
+constexpr int kClassGroup = 8;   // steps a warp contracts together
+
+// get_spike for one step of a cell whose next spike falls in it (src/discrete_input_convol.cu:1589-1619):
+// the number of spikes and the time of the last one; leaves the carried integral for the next step.
+__device__ __forceinline__ unsigned draw_spikes(const LgnParams &P, long long it, int id, float rate, float rT, float &ltr,
+                                                float &lnl, curandStateMRG32k3a &st, float &tsp) {
+    float next_rT = lnl - ltr, old_rT;
+    unsigned nsp = 0;
+    do {
+        const float u = curand_uniform(&st);
+        if (P.recU) {
+            const long long rs = it - P.recStep0;
+            if (rs >= 0 && rs < P.recSteps) {
+                const size_t base = (size_t)rs * P.nLGN + id;
+                if ((int)nsp < P.recCap) P.recU[base * P.recCap + nsp] = u;
+                else atomicOr(P.err, kErrRecordOverflow);
+                P.recUCount[base] = nsp + 1;
+            }
         }
-    }
-    const int cell = cellBase + threadIdx.x;
-    const bool on = cell < P.nMagno;
-    if (on) {
-        for (int u = 0; u < nU; u++) {
-            const int F = Flo + u;
-            const int row = F < 0 ? fs.initRow : F % fs.nFrame;
-            sS[u * kClassCta + threadIdx.x] = __ldg(P.S + (size_t)row * P.nMagno + cell);
-        }
-    }
-    __syncthreads();
-    const unsigned lanes = __ballot_sync(0xffffffffu, on);
-    if (!on) return;
-    int id = P.nParvo_I + cell;
-    if (cell >= P.nMagno_I) id += P.nParvo_C;
-    const float absk = P.absk[cell];
-    const float mx = P.maxConvol[id];
-    const float C50 = P.c50[id], Kc = P.sharp[id], LA = P.la[id], LB = P.lb[id];
-    float ltr = P.leftTimeRate[id];
-    float lnl = P.lastNegLogRand[id];
-    curandStateMRG32k3a st = P.state[id];
-    float ffVar[2] = {P.nFF > 0 ? P.ffPre[id] : 0.f, P.nFF > 1 ? P.ffPre[(size_t)P.nLGN + id] : 0.f};
-    const float dt = P.dt;
-    for (int s = 0; s < K; s++) {
-        const long long it = t0 + s;
-        float convol = 0.f;
-        const int nseg = sNseg[s];
-        for (int q = 0; q < nseg; q++) convol += sS[sSlot[s][q] * kClassCta + threadIdx.x] * sW[s][q];
-        // LGN_nonlinear (src/discrete_input_convol.cu:1660-1730)
-        float current = (convol * absk) * P.convolRatio;
-        if (current < 0) current = 0;
-        const float X = (float)(1.0 / (double)(1 + expf(Kc * (C50 - current / mx))));
-        const float fr = P.frRatio * mx * (LA * X + LB);
-        if (P.outFr) P.outFr[(size_t)(it % P.outSlots) * P.nLGN + id] = fr;
-        // get_spike (src/discrete_input_convol.cu:1589-1619)
-        const float rate = fr / 1000.0f;
-        const float rT = dt * rate;
-        float next_rT = lnl - ltr;
-        unsigned nsp = 0;
-        float tsp = 0.f;
-        if (next_rT > rT) {
-            ltr += rT;
-        } else {
-            float old_rT;
-            do {
-                const float u = curand_uniform(&st);
-                if (P.recU) {
-                    const long long rs = it - P.recStep0;
-                    if (rs >= 0 && rs < P.recSteps) {
-                        const size_t base = (size_t)rs * P.nLGN + id;
-                        if ((int)nsp < P.recCap) P.recU[base * P.recCap + nsp] = u;
-                        else atomicOr(P.err, kErrRecordOverflow);
-                        P.recUCount[base] = nsp + 1;
-                    }
-                }
-                lnl = fmaxf(-logf(u), 0.0f * rate);
-                old_rT = next_rT;
-                next_rT += lnl;
-                nsp++;
-            } while (next_rT <= rT);
-            ltr = rT - old_rT;
-            tsp = old_rT / (rate * nsp);
-        }
-        const float sInfo = nsp + tsp / dt;
-        P.outSInfo[(size_t)(it % P.outSlots) * P.nLGN + id] = sInfo;
-        if (P.outBits) {   // without parvo cells a warp's ids are one word of the row's bits
-            const unsigned bits = __ballot_sync(lanes, sInfo >= 1.0f);
-            if ((threadIdx.x & 31) == 0) P.outBits[(size_t)(it % P.outSlots) * P.bitW + (id >> 5)] = bits;
-        }
-        if (P.nFF) ff_pre_step(P, it, id, nsp, tsp, sInfo, ffVar);
-    }
-    P.leftTimeRate[id] = ltr;
-    P.lastNegLogRand[id] = lnl;
-    P.state[id] = st;
-    if (P.nFF > 0) P.ffPre[id] = ffVar[0];
-    if (P.nFF > 1) P.ffPre[(size_t)P.nLGN + id] = ffVar[1];
+        lnl = fmaxf(-logf(u), 0.0f * rate);
+        old_rT = next_rT;
+        next_rT += lnl;
+        nsp++;
+    } while (next_rT <= rT);
+    ltr = rT - old_rT;
+    tsp = old_rT / (rate * nsp);
+    return nsp;
 }
 
-__global__ void __launch_bounds__(kClassCta) lgn_class_kernel(LgnParams P, const long long *stepBase, int K) {
-    lgn_class_body(P, *stepBase, K, blockIdx.x * kClassCta);
+// LGN_nonlinear's rate for a linear response (src/discrete_input_convol.cu:1660-1730).  The reference
+// takes the reciprocal in double and rounds it to float: the correctly rounded float reciprocal (a
+// quotient of 24-bit numbers is never that close to the middle of two floats).
+__device__ __forceinline__ float logistic_rate(const LgnParams &P, float response, float mx, float C50, float Kc, float LA,
+                                               float LB) {
+    float current = response * P.convolRatio;
+    if (current < 0) current = 0;
+    const float X = __frcp_rn(1 + expf(Kc * (C50 - div_sparse(current, mx))));
+    return P.frRatio * mx * (LA * X + LB);
+}
+
+__device__ __forceinline__ void lgn_class_body(const LgnParams &P, long long t0, int K, int cellBase, ClassShared &sm) {
+    const FrameSched fs = P.fs;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto step_tables = [&](long long it, int &cf, int &phase, int &tail) {
+        cf = frames_read_after_step(fs, it);
+        phase = (int)((fs.magnoComp + (it + 1) * (long long)fs.denorm) % fs.ntPerFrame);
+        tail = fs.frameOffset + (phase <= fs.magnoComp ? 2 : 1);
+    };
+    if ((int)threadIdx.x < K) {
+        const int s = threadIdx.x;
+        int cf, phase, tail;
+        step_tables(t0 + s, cf, phase, tail);
+        const int nseg = P.seg.nseg[phase];
+        sm.cf[s] = cf;
+        sm.phase[s] = phase;
+        sm.tail[s] = tail;
+        sm.nseg[s] = nseg;
+        sm.valid[s] = 0ull;
+        // first and last frame of the chunk's windows
+        const int *rel = P.seg.rel + (size_t)phase * P.seg.maxSeg;
+        if (s == 0) sm.Flo = frame_number(fs, cf, tail + rel[0]);
+        if (s == K - 1) sm.nU = frame_number(fs, cf, tail + rel[nseg - 1]);
+    }
+    __syncthreads();
+    const int Flo = sm.Flo;
+    const int span = sm.nU - Flo + 1;
+    const int nU = min(max(span, 1), kClassMaxSlots);
+    if (threadIdx.x == 0 && span != nU) atomicOr(P.err, kErrBounds);
+    float *W = reinterpret_cast<float *>(sm.W);
+    for (int k = threadIdx.x; k < K * P.seg.maxSeg; k += kClassThreads) {
+        const int s = k / P.seg.maxSeg, q = k - s * P.seg.maxSeg;
+        if (q >= sm.nseg[s]) continue;
+        const size_t at = (size_t)sm.phase[s] * P.seg.maxSeg + q;
+        const float w = __ldg(P.seg.weight + at);
+        const int slot =
+            min(max(frame_number(fs, sm.cf[s], sm.tail[s] + __ldg(P.seg.rel + at)) - Flo, 0), kClassMaxSlots - 1);
+        W[slot * kClassMaxK + s] = w;
+        atomicOr(&sm.valid[s], 1ull << slot);
+    }
+    const int cell = cellBase + lane;
+    const bool on = cell < P.nMagno;
+    for (int u = warp; u < nU; u += kClassThreads / 32) {
+        const int F = Flo + u;
+        const int row = F < 0 ? fs.initRow : F % fs.nFrame;
+        sm.S[u][lane] = on ? __ldg(P.S + (size_t)row * P.nMagno + cell) : 0.f;
+    }
+    int id = P.nParvo_I + cell;
+    if (cell >= P.nMagno_I) id += P.nParvo_C;
+    float absk = 0.f, mx = 1.f, C50 = 0.f, Kc = 0.f, LA = 0.f, LB = 0.f;
+    if (on) {
+        absk = P.absk[cell]; mx = P.maxConvol[id]; C50 = P.c50[id]; Kc = P.sharp[id]; LA = P.la[id]; LB = P.lb[id];
+    }
+    const int row0 = (int)(t0 % P.outSlots);
+    __syncthreads();
+    for (int s0 = warp * kClassGroup; s0 < K; s0 += (kClassThreads / 32) * kClassGroup) {
+        const int n = min(kClassGroup, K - s0);
+        unsigned long long any = 0ull, all = ~0ull;
+        for (int j = 0; j < n; j++) {
+            any |= sm.valid[s0 + j];
+            all &= sm.valid[s0 + j];
+        }
+        float acc[kClassGroup];
+#pragma unroll
+        for (int j = 0; j < kClassGroup; j++) acc[j] = 0.f;
+        for (int u = 0; u < nU; u++) {
+            if (!((any >> u) & 1)) continue;
+            const float x = sm.S[u][lane];
+            const float4 a = sm.W[u][s0 / 4], b = sm.W[u][s0 / 4 + 1];
+            const float w[kClassGroup] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            if ((all >> u) & 1) {
+#pragma unroll
+                for (int j = 0; j < kClassGroup; j++) acc[j] += x * w[j];
+            } else {
+#pragma unroll
+                for (int j = 0; j < kClassGroup; j++)
+                    if (j < n && ((sm.valid[s0 + j] >> u) & 1)) acc[j] += x * w[j];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kClassGroup; j++) {
+            if (j < n) {
+                const float fr = logistic_rate(P, acc[j] * absk, mx, C50, Kc, LA, LB);
+                int row = row0 + s0 + j;
+                if (row >= P.outSlots) row %= P.outSlots;
+                if (P.outFr && on) P.outFr[(size_t)row * P.nLGN + id] = fr;
+                const float rate = fr / 1000.0f;
+                sm.rate[s0 + j][lane] = rate;
+                sm.rT[s0 + j][lane] = P.dt * rate;
+            }
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        float ltr = 0.f, lnl = 0.f;
+        curandStateMRG32k3a st;
+        if (on) {
+            ltr = P.leftTimeRate[id];
+            lnl = P.lastNegLogRand[id];
+            st = P.state[id];
+        }
+        float *rT = &sm.rT[0][lane];
+        const float *rate = &sm.rate[0][lane];
+        const float dt = P.dt;
+        if (P.nFF == 0) {
+            int c = on ? 0 : K;
+            while (__any_sync(0xffffffffu, c < K)) {
+                // to the step of the next spike: four steps at a time as long as none of them has it
+                for (; c + 4 <= K; c += 4) {
+                    const float r0 = rT[c * kClassCells], r1 = rT[(c + 1) * kClassCells];
+                    const float r2 = rT[(c + 2) * kClassCells], r3 = rT[(c + 3) * kClassCells];
+                    const float l1 = ltr + r0, l2 = l1 + r1, l3 = l2 + r2;
+                    if (!(lnl - ltr > r0 && lnl - l1 > r1 && lnl - l2 > r2 && lnl - l3 > r3)) break;
+                    ltr = l3 + r3;
+#pragma unroll
+                    for (int k = 0; k < 4; k++) rT[(c + k) * kClassCells] = 0.f;
+                }
+                bool hit = false;
+                for (; c < K; c++) {
+                    const float r = rT[c * kClassCells];
+                    if (!(lnl - ltr > r)) {
+                        hit = true;
+                        break;
+                    }
+                    ltr += r;
+                    rT[c * kClassCells] = 0.f;
+                }
+                __syncwarp();
+                if (hit) {
+                    float tsp;
+                    const unsigned nsp =
+                        draw_spikes(P, t0 + c, id, rate[c * kClassCells], rT[c * kClassCells], ltr, lnl, st, tsp);
+                    rT[c * kClassCells] = nsp + tsp / dt;
+                    c++;
+                }
+            }
+        } else if (on) {
+            float ffVar[2] = {P.ffPre[id], P.nFF > 1 ? P.ffPre[(size_t)P.nLGN + id] : 0.f};
+            for (int s = 0; s < K; s++) {
+                const float r = rT[s * kClassCells];
+                unsigned nsp = 0;
+                float tsp = 0.f;
+                if (lnl - ltr > r) ltr += r;
+                else nsp = draw_spikes(P, t0 + s, id, rate[s * kClassCells], r, ltr, lnl, st, tsp);
+                const float sInfo = nsp + tsp / dt;
+                rT[s * kClassCells] = sInfo;
+                ff_pre_step(P, t0 + s, id, nsp, tsp, sInfo, ffVar);
+            }
+            P.ffPre[id] = ffVar[0];
+            if (P.nFF > 1) P.ffPre[(size_t)P.nLGN + id] = ffVar[1];
+        }
+        if (on) {
+            P.leftTimeRate[id] = ltr;
+            P.lastNegLogRand[id] = lnl;
+            P.state[id] = st;
+        }
+    }
+    __syncthreads();
+    for (int s = warp; s < K; s += kClassThreads / 32) {
+        int row = row0 + s;
+        if (row >= P.outSlots) row %= P.outSlots;
+        const float sInfo = sm.rT[s][lane];
+        if (on) P.outSInfo[(size_t)row * P.nLGN + id] = sInfo;
+        if (P.outBits) {   // without parvo cells the CTA's ids are one word of the row's bits
+            const unsigned bits = __ballot_sync(0xffffffffu, on && sInfo >= 1.0f);
+            if (lane == 0) P.outBits[(size_t)row * P.bitW + (id >> 5)] = bits;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kClassThreads) lgn_class_kernel(LgnParams P, const long long *stepBase, int K) {
+    __shared__ ClassShared sm;
+    lgn_class_body(P, *stepBase, K, blockIdx.x * kClassCells, sm);
 }
 
 // The single-class LGN stage for every trial of a batch: grid (cell CTAs, trials); each CTA
 // copies its trial's parameters to shared memory and runs the same body for the steps the
 // trial still has among the next K (in pieces of at most kClassMaxK steps).
-__global__ void __launch_bounds__(kClassCta) lgn_class_batch_kernel(const BatchLgn *__restrict__ trials, int K) {
+__global__ void __launch_bounds__(kClassThreads) lgn_class_batch_kernel(const BatchLgn *__restrict__ trials, int K) {
+    __shared__ ClassShared sm;
     __shared__ __align__(16) BatchLgn sT;
     const int *src = reinterpret_cast<const int *>(trials + blockIdx.y);
     int *dst = reinterpret_cast<int *>(&sT);
-    for (int w = threadIdx.x; w < (int)(sizeof(BatchLgn) / sizeof(int)); w += kClassCta) dst[w] = src[w];
+    for (int w = threadIdx.x; w < (int)(sizeof(BatchLgn) / sizeof(int)); w += kClassThreads) dst[w] = src[w];
     __syncthreads();
     const long long t0 = *sT.step;
     const long long left = sT.tEnd - t0;
     const int k = left < K ? (int)left : K;
-    if (k <= 0 || (int)blockIdx.x * kClassCta >= sT.p.nMagno) return;
+    if (k <= 0 || (int)blockIdx.x * kClassCells >= sT.p.nMagno) return;
     // chunks of at most kClassMaxK steps (the shared tables of one chunk's frames); the cells'
     // carried state passes from one chunk to the next through global memory
     for (int off = 0; off < k; off += kClassMaxK) {
         if (off) __syncthreads();
-        lgn_class_body(sT.p, t0 + off, min(kClassMaxK, k - off), blockIdx.x * kClassCta);
+        lgn_class_body(sT.p, t0 + off, min(kClassMaxK, k - off), blockIdx.x * kClassCells, sm);
     }
 }
 
@@ -789,12 +896,8 @@ __global__ void __launch_bounds__(256) lgn_rate_kernel(LgnParams P, const long l
         convol += S[(size_t)s_row[q] * nm] * wseg;
         ca = cb;
     }
-    // LGN_nonlinear (src/discrete_input_convol.cu:1660-1730)
-    const float mx = P.maxConvol[id];
-    float current = (convol * P.absk[cell]) * P.convolRatio;
-    if (current < 0) current = 0;
-    const float X = (float)(1.0 / (double)(1 + expf(P.sharp[id] * (P.c50[id] - current / mx))));
-    const float fr = P.frRatio * mx * (P.la[id] * X + P.lb[id]);
+    const float fr =
+        logistic_rate(P, convol * P.absk[cell], P.maxConvol[id], P.c50[id], P.sharp[id], P.la[id], P.lb[id]);
     P.rate[(size_t)s * P.nLGN + id] = fr;
     if (P.outFr) P.outFr[(size_t)(it % P.outSlots) * P.nLGN + id] = fr;
 }
@@ -838,12 +941,7 @@ __global__ void __launch_bounds__(256) lgn_parvo_rate_kernel(LgnParams P, const 
         caS = cbS;
     }
     const float convol = convolC * P.pk[cell] + convolS * P.pk[np + cell];
-    // LGN_nonlinear (src/discrete_input_convol.cu:1660-1730)
-    const float mx = P.maxConvol[id];
-    float current = convol * P.convolRatio;
-    if (current < 0) current = 0;
-    const float X = (float)(1.0 / (double)(1 + expf(P.sharp[id] * (P.c50[id] - current / mx))));
-    const float fr = P.frRatio * mx * (P.la[id] * X + P.lb[id]);
+    const float fr = logistic_rate(P, convol, P.maxConvol[id], P.c50[id], P.sharp[id], P.la[id], P.lb[id]);
     P.rate[(size_t)s * P.nLGN + id] = fr;
     if (P.outFr) P.outFr[(size_t)(it % P.outSlots) * P.nLGN + id] = fr;
 }
@@ -874,32 +972,10 @@ __global__ void __launch_bounds__(256) lgn_spike_kernel(LgnParams P, const long 
         const float fr = P.rate[(size_t)s * P.nLGN + id];
         const float rate = fr / 1000.0f;
         const float rT = dt * rate;
-        float next_rT = lnl - ltr;
         unsigned nsp = 0;
         float tsp = 0.f;
-        if (next_rT > rT) {
-            ltr += rT;
-        } else {
-            float old_rT;
-            do {
-                float u = curand_uniform(&st);
-                if (P.recU) {
-                    long long rs = it - P.recStep0;
-                    if (rs >= 0 && rs < P.recSteps) {
-                        size_t base = (size_t)rs * P.nLGN + id;
-                        if ((int)nsp < P.recCap) P.recU[base * P.recCap + nsp] = u;
-                        else atomicOr(P.err, kErrRecordOverflow);
-                        P.recUCount[base] = nsp + 1;
-                    }
-                }
-                lnl = fmaxf(-logf(u), 0.0f * rate);
-                old_rT = next_rT;
-                next_rT += lnl;
-                nsp++;
-            } while (next_rT <= rT);
-            ltr = rT - old_rT;
-            tsp = old_rT / (rate * nsp);
-        }
+        if (lnl - ltr > rT) ltr += rT;
+        else nsp = draw_spikes(P, it, id, rate, rT, ltr, lnl, st, tsp);
         const float sInfo = nsp + tsp / dt;
         P.outSInfo[(size_t)(it % P.outSlots) * P.nLGN + id] = sInfo;
         if (P.nFF) ff_pre_step(P, it, id, nsp, tsp, sInfo, ffVar);
@@ -1015,14 +1091,7 @@ cudaError_t launch_lgn_step(const LgnParams &p, const long long *stepBase, int K
     }
     if (p.nMagno <= 0) return cudaSuccess;
     if (p.classCtw && K <= kClassMaxK) {
-        const size_t smem = (size_t)kClassMaxSlots * kClassCta * sizeof(float);
-        static bool attrSet = false;
-        if (!attrSet) {
-            cudaError_t e = cudaFuncSetAttribute(lgn_class_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return e;
-            attrSet = true;
-        }
-        lgn_class_kernel<<<(p.nMagno + kClassCta - 1) / kClassCta, kClassCta, smem, st>>>(p, stepBase, K);
+        lgn_class_kernel<<<(p.nMagno + kClassCells - 1) / kClassCells, kClassThreads, 0, st>>>(p, stepBase, K);
         return cudaGetLastError();
     }
     dim3 grid((p.nMagno + 255) / 256, K);
@@ -1037,15 +1106,7 @@ cudaError_t launch_lgn_step(const LgnParams &p, const long long *stepBase, int K
 cudaError_t launch_lgn_class_batch(const BatchLgn *trials, int nTrials, int maxCellCtas, int K, cudaStream_t st) {
     if (nTrials <= 0 || maxCellCtas <= 0) return cudaSuccess;
     if (K <= 0) return cudaErrorInvalidValue;
-    const size_t smem = (size_t)kClassMaxSlots * kClassCta * sizeof(float);
-    static bool attrSet = false;
-    if (!attrSet) {
-        cudaError_t e = cudaFuncSetAttribute(lgn_class_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e != cudaSuccess) return e;
-        attrSet = true;
-    }
-    lgn_class_batch_kernel<<<dim3(maxCellCtas, nTrials), kClassCta, smem, st>>>(trials, K);
+    lgn_class_batch_kernel<<<dim3(maxCellCtas, nTrials), kClassThreads, 0, st>>>(trials, K);
     return cudaGetLastError();
 }
 

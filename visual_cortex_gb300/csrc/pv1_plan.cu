@@ -819,6 +819,18 @@ int lgn_setup_impl(pv1_plan *p, const pv1_lgn_config *lc, const pv1_lgn_parvo_co
             PV1_CUDA(p, cudaMemcpy2D(d_cls, sizeof(double), d_ctw, (size_t)nMagno * sizeof(double), sizeof(double),
                                      (size_t)nKS + 1, cudaMemcpyDeviceToDevice));
             L.classCtw = d_cls;
+            // the segment sums of every frame phase, as lgn_rate_kernel forms them
+            std::vector<double> cls((size_t)nKS + 1);
+            PV1_CUDA(p, cudaMemcpy(cls.data(), d_cls, cls.size() * sizeof(double), cudaMemcpyDeviceToHost));
+            std::vector<float> wt((size_t)c.ntPerFrame * maxSeg, 0.f);
+            for (size_t ph = 0; ph < c.ntPerFrame; ph++)
+                for (int q = 0; q < nseg[ph]; q++)
+                    wt[ph * maxSeg + q] = (float)(cls[j0[ph * (maxSeg + 1) + q + 1]] - cls[j0[ph * (maxSeg + 1) + q]]);
+            float *d_wt;
+            r = dev_upload(p, &d_wt, wt.data(), wt.size());
+            if (r) return r;
+            PV1_CUDA(p, cudaStreamSynchronize(p->stream));
+            L.seg.weight = d_wt;
         }
     }
     int e = check_device_error(p);
