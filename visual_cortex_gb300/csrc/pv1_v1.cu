@@ -191,10 +191,15 @@ __device__ __forceinline__ int compact_spikers(const V1Params &P, const float *_
     return total;
 }
 
-// Sends to L2 what the next step reads because neuron i (local index `local` of block b)
-// spiked: its rows of the near tiles that list block b (read by the delivery, whole 16-byte
-// aligned rows), and the whole 16-byte chunks of its far synapse list (read by the push).
-// Hints only: nothing waits on them.
+__device__ __forceinline__ void prefetch_far(const V1Params &P, int e0, int deg) {
+    const unsigned bytes = (unsigned)deg * 16u;
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(P.farRec + e0), "r"(bytes) : "memory");
+}
+
+// Sends to L2 what is read when neuron i (local index `local` of block b) spikes: its rows of the near
+// tiles that list block b (read by the delivery, whole 16-byte aligned rows), and the whole
+// 16-byte chunks of `farDeg` synapses of its far list (read by the push).  Hints only: nothing
+// waits on them.
 __device__ __forceinline__ void prefetch_spiker(const V1Params &P, int b, int local, int farE0, int farDeg) {
     if (P.noDelay && P.nearRevOff && (P.blockSize & 3) == 0) {
         const unsigned bytes = (unsigned)P.blockSize * 4u;
@@ -203,10 +208,7 @@ __device__ __forceinline__ void prefetch_spiker(const V1Params &P, int b, int lo
             asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(row), "r"(bytes) : "memory");
         }
     }
-    if (farDeg > 0) {
-        const unsigned bytes = (unsigned)farDeg * 16u;
-        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(P.farRec + farE0), "r"(bytes) : "memory");
-    }
+    if (farDeg > 0) prefetch_far(P, farE0, farDeg);
 }
 
 // The excitatory filtered rate of learning 1, 2 and 4, advanced over step tp in the near
@@ -495,6 +497,29 @@ __device__ __forceinline__ void deliver_prev(const V1Params &P, long long tp, in
     if (P.rec && active) record_conductances(P, (int)(tp % P.recSlots), i, st);
 }
 
+// What a step reads of its neuron's type: the persistent kernels keep it in shared memory, as a few
+// 16-byte reads in place of a dozen indexed reads of the kernel's parameters.
+struct __align__(16) TypeConst {
+    float4 level;      // vR, vThres, vT, tRef
+    float4 membrane;   // gL, C, 1/C (div_pow2), tau_w
+    float4 adex;       // deltaT, 1/deltaT (div_pow2), a, b
+    float pFF[kMaxNG], pE[kMaxNG], pI[kMaxNG];
+};
+
+__device__ __forceinline__ TypeConst type_const(const V1Params &P, int itype) {
+    TypeConst k;
+    k.level = make_float4(P.vR[itype], P.vThres[itype], P.vT[itype], P.tRef[itype]);
+    k.membrane = make_float4(P.gL[itype], P.C[itype], P.invC[itype], P.tau_w[itype]);
+    k.adex = make_float4(P.deltaT[itype], P.invDeltaT[itype], P.a[itype], P.b[itype]);
+#pragma unroll
+    for (int ig = 0; ig < kMaxNG; ig++) {
+        k.pFF[ig] = ig < P.ngFF ? P.pFF[itype * P.ngFF + ig] : 0.f;
+        k.pE[ig] = ig < P.ngE ? P.pE[itype * P.ngE + ig] : 0.f;
+        k.pI[ig] = ig < P.ngI ? P.pI[itype * P.ngI + ig] : 0.f;
+    }
+    return k;
+}
+
 // The tonic drive of the AdEx constructor (src/coredynamics.cuh:41-49).
 __device__ __forceinline__ float tonic_current(const V1Params &P, int itype, float tonic) {
     const float vT = P.vT[itype], gL = P.gL[itype], aa = P.a[itype], deltaT = P.deltaT[itype];
@@ -505,7 +530,7 @@ __device__ __forceinline__ float tonic_current(const V1Params &P, int itype, flo
 
 // One LGN synapse with spike word sFF and weight f (src/coredynamics.cu:1476-1500).
 template <bool Rng>
-__device__ __forceinline__ void lgn_input(const V1Params &P, int itype, float sFF, float f, bool backingUp,
+__device__ __forceinline__ void lgn_input(const V1Params &P, const float *pFF, float sFF, float f, bool backingUp,
                                           float tBack, float pf, float nSynFF, float *g0, float *h0,
                                           float *g1, float *h1, curandStateMRG32k3a &condState,
                                           float *recFF, int &nFF) {
@@ -530,7 +555,7 @@ __device__ __forceinline__ void lgn_input(const V1Params &P, int itype, float sF
 #pragma unroll
         for (int ig = 0; ig < kMaxNG; ig++) {
             if (ig < P.ngFF) {
-                const float str = f * P.pFF[itype * P.ngFF + ig];
+                const float str = f * pFF[ig];
                 if (backingUp && ddt > 0) cond_input(P.condFF, g0[ig], h0[ig], str * nspFF, ddt, ig);
                 cond_input(P.condFF, g1[ig], h1[ig], str * nspFF, dt - tspFF, ig);
             }
@@ -539,13 +564,15 @@ __device__ __forceinline__ void lgn_input(const V1Params &P, int itype, float sF
 }
 
 // The LGN spikes of one step as a persistent thread knows them: which of its synapses received one,
-// the first two spike words, and ids and weights in shared memory ([synapse][kCta] from its column).
+// the first two spike words, ids ([group of four][kCta] from its column) and weights ([synapse][kCta]).
 struct LgnIn {
     unsigned mask;
     float w0, w1;
-    const int *ids;
+    const int4 *ids;
     const float *wts;
 };
+
+__device__ __forceinline__ int synapse_id(const int4 *ids, int q);
 
 // What the feed-forward half of a membrane step hands to the integration half.
 struct FFStep {
@@ -559,8 +586,8 @@ struct FFStep {
 // while they wait for them.  With SmemSyn the spikes are known (in); otherwise ids and words are
 // loaded batch by batch and weights only for synapses that received a spike.
 template <bool Rng, bool SmemSyn>
-__device__ __forceinline__ void step_feedforward(const V1Params &P, long long t, int i, int itype, float tonic,
-                                                 float depC, int m, const float *__restrict__ lgnSInfo, NState &st,
+__device__ __forceinline__ void step_feedforward(const V1Params &P, const TypeConst &tc, long long t, int i, int itype,
+                                                 float tonic, float depC, int m, const float *__restrict__ lgnSInfo, NState &st,
                                                  curandStateMRG32k3a &condState, curandStateMRG32k3a &noisyState,
                                                  FFStep &ff, const LgnIn &in = LgnIn{}) {
     const int nV1 = P.nV1;
@@ -622,8 +649,8 @@ __device__ __forceinline__ void step_feedforward(const V1Params &P, long long t,
         for (int k = 0; mask; k++) {
             const int q = __ffs(mask) - 1;
             mask &= mask - 1;
-            const float sFF = k == 0 ? in.w0 : (k == 1 ? in.w1 : __ldcg(lgnSInfo + in.ids[q * kCta]));
-            lgn_input<Rng>(P, itype, sFF, in.wts[q * kCta], backingUp, tBack, pf, nSynFF, g0, h0, g1, h1, condState,
+            const float sFF = k == 0 ? in.w0 : (k == 1 ? in.w1 : __ldcg(lgnSInfo + synapse_id(in.ids, q)));
+            lgn_input<Rng>(P, tc.pFF, sFF, in.wts[q * kCta], backingUp, tBack, pf, nSynFF, g0, h0, g1, h1, condState,
                            recFF, nFF);
         }
     } else if (m <= kMaxLgnReg) {
@@ -647,7 +674,7 @@ __device__ __forceinline__ void step_feedforward(const V1Params &P, long long t,
             const size_t lid = (size_t)q * nV1 + i;
             const float sFF = __ldcg(lgnSInfo + __ldg(P.lgnId + lid));
             const float f = __ldg(P.sLGN + lid);
-            lgn_input<Rng>(P, itype, sFF, f, backingUp, tBack, pf, nSynFF, g0, h0, g1, h1, condState, recFF,
+            lgn_input<Rng>(P, tc.pFF, sFF, f, backingUp, tBack, pf, nSynFF, g0, h0, g1, h1, condState, recFF,
                            nFF);
         }
     } else {
@@ -665,7 +692,7 @@ __device__ __forceinline__ void step_feedforward(const V1Params &P, long long t,
 #pragma unroll
             for (int k = 0; k < kLgnBatch; k++) {
                 if (q0 + k < m)
-                    lgn_input<Rng>(P, itype, sp[k], fs[k], backingUp, tBack, pf, nSynFF, g0, h0, g1, h1, condState,
+                    lgn_input<Rng>(P, tc.pFF, sp[k], fs[k], backingUp, tBack, pf, nSynFF, g0, h0, g1, h1, condState,
                                    recFF, nFF);
             }
         }
@@ -680,13 +707,14 @@ __device__ __forceinline__ void step_feedforward(const V1Params &P, long long t,
 
 // Phase B, second half: cortical conductances, integration and threshold of step t
 // (src/coredynamics.cu:1380-1590).  Returns the spike word.
-__device__ __forceinline__ float step_membrane(const V1Params &P, int itype, float depC, const FFStep &ff, NState &st) {
+__device__ __forceinline__ float step_membrane(const V1Params &P, const TypeConst &tc, float depC, const FFStep &ff,
+                                               NState &st) {
     const float dt = P.dt;
     const int ngE = P.ngE, ngI = P.ngI, ngFF = P.ngFF;
-    const float vR = P.vR[itype], vThres = P.vThres[itype], gL = P.gL[itype];
-    const float Cm = P.C[itype], tRef = P.tRef[itype], vT = P.vT[itype];
-    const float deltaT = P.deltaT[itype], tau_w = P.tau_w[itype], aa = P.a[itype];
-    const float bb = P.b[itype], invC = P.invC[itype], invDeltaT = P.invDeltaT[itype];
+    const float4 lvl = tc.level, mem = tc.membrane, adx = tc.adex;
+    const float vR = lvl.x, vThres = lvl.y, vT = lvl.z, tRef = lvl.w;
+    const float gL = mem.x, Cm = mem.y, invC = mem.z, tau_w = mem.w;
+    const float deltaT = adx.x, invDeltaT = adx.y, aa = adx.z, bb = adx.w;
     const float v0 = st.v;
     float w0 = st.w;
     float tBack = st.tBack;
@@ -816,8 +844,9 @@ __device__ __forceinline__ float step_neuron(const V1Params &P, long long t, int
                                              int m, const float *__restrict__ lgnSInfo, NState &st,
                                              curandStateMRG32k3a &condState, curandStateMRG32k3a &noisyState) {
     FFStep ff;
-    step_feedforward<Rng, false>(P, t, i, itype, tonic, depC, m, lgnSInfo, st, condState, noisyState, ff);
-    const float sInfo = step_membrane(P, itype, depC, ff, st);
+    const TypeConst tc = type_const(P, itype);
+    step_feedforward<Rng, false>(P, tc, t, i, itype, tonic, depC, m, lgnSInfo, st, condState, noisyState, ff);
+    const float sInfo = step_membrane(P, tc, depC, ff, st);
     P.dep[i] = ff.depOut;
     store_step(P, t, i, sInfo, ff.depOut, st, P.recSpk || P.rec ? (int)(t % P.recSlots) : 0);
     return sInfo;
@@ -1532,6 +1561,7 @@ struct __align__(16) PShared {
         Smem near;                          // general neighbour lists
     };
     uint64_t nearBar[2], bitBar[2];
+    TypeConst type[kMaxType];
     // this CTA's far spikers, by parity of the step
     int cnt[2];
     int e0[2][kCta], deg[2][kCta];
@@ -1649,25 +1679,26 @@ __device__ __forceinline__ void fetch_bits(PShared &sm, unsigned *dst, const uns
     }
 }
 
-// Which of a neuron's m LGN synapses (ids in shared memory, [synapse][kCta] from the thread's column,
-// rows padded to a multiple of 4) received a spike, and the first two spike words.
-__device__ __forceinline__ LgnIn lgn_spikes(const unsigned *bits, const float *__restrict__ lgnSInfo, const int *ids,
-                                            const float *wts, int m, int rows) {
+// Synapse q's id among a thread's ids in shared memory ([group of four][kCta] from its column).
+__device__ __forceinline__ int synapse_id(const int4 *ids, int q) {
+    return reinterpret_cast<const int *>(ids + (q >> 2) * kCta)[q & 3];
+}
+
+// Which of a neuron's m LGN synapses (in groups of four) received a spike, and the first two words.
+__device__ __forceinline__ LgnIn lgn_spikes(const unsigned *bits, const float *__restrict__ lgnSInfo, const int4 *ids,
+                                            const float *wts, int m, int groups) {
     LgnIn in{0u, 0.f, 0.f, ids, wts};
-    for (int q0 = 0; q0 < rows; q0 += 4) {
-        unsigned hit = 0u;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int id = ids[(q0 + k) * kCta];
-            hit |= ((bits[id >> 5] >> (id & 31)) & 1u) << k;
-        }
-        in.mask |= hit << q0;
+    auto bit = [&](int id) { return (bits[id >> 5] >> (id & 31)) & 1u; };
+#pragma unroll 2
+    for (int g = 0; g < groups; g++) {
+        const int4 id = ids[g * kCta];
+        in.mask |= (bit(id.x) | bit(id.y) << 1 | bit(id.z) << 2 | bit(id.w) << 3) << (4 * g);
     }
     in.mask &= m < 32 ? (1u << m) - 1u : 0xffffffffu;
     if (in.mask) {
         const unsigned rest = in.mask & (in.mask - 1);
-        in.w0 = __ldcg(lgnSInfo + ids[(__ffs(in.mask) - 1) * kCta]);
-        if (rest) in.w1 = __ldcg(lgnSInfo + ids[(__ffs(rest) - 1) * kCta]);
+        in.w0 = __ldcg(lgnSInfo + synapse_id(ids, __ffs(in.mask) - 1));
+        if (rest) in.w1 = __ldcg(lgnSInfo + synapse_id(ids, __ffs(rest) - 1));
     }
     return in;
 }
@@ -1675,8 +1706,8 @@ __device__ __forceinline__ LgnIn lgn_spikes(const unsigned *bits, const float *_
 // Near delivery of step tp from the block's published spikes (near list: the own block alone), four
 // conMat rows read together.  Ascending neuron order and the arithmetic of deliver_prev.
 template <bool Rng>
-__device__ __forceinline__ void deliver_list(const V1Params &P, long long tp, int b, int local, int i, bool active,
-                                             int itype, NState &st, curandStateMRG32k3a &condState, const float4 *unit,
+__device__ __forceinline__ void deliver_list(const V1Params &P, const TypeConst &tc, long long tp, int b, int local, int i,
+                                             bool active, int itype, NState &st, curandStateMRG32k3a &condState, const float4 *unit,
                                              const unsigned *ball) {
     const int lane = threadIdx.x & 31;
     const int bs = P.blockSize, nE = P.nE, ngE = P.ngE, ngI = P.ngI;
@@ -1731,12 +1762,12 @@ __device__ __forceinline__ void deliver_list(const V1Params &P, long long tp, in
 #pragma unroll
                     for (int ig = 0; ig < kMaxNG; ig++) {
                         if (isE && ig < ngE) {
-                            const float str = strength * P.pE[itype * ngE + ig];
+                            const float str = strength * tc.pE[ig];
                             lgE[ig] += str * g[ig];
                             lhE[ig] += str * h[ig];
                         }
                         if (!isE && ig < ngI) {
-                            const float str = strength * P.pI[itype * ngI + ig];
+                            const float str = strength * tc.pI[ig];
                             lgI[ig] += str * g[ig];
                             lhI[ig] += str * h[ig];
                         }
@@ -1823,13 +1854,13 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
     const bool smemSyn = !General || (P.maxLGN <= mRows && !P.multiSpike);
     const int rows = (P.maxLGN + 3) & ~3;
     float *smW = dyn + threadIdx.x;
-    int *smI = reinterpret_cast<int *>(dyn + (size_t)mRows * kCta) + threadIdx.x;
+    int4 *smI = reinterpret_cast<int4 *>(dyn + (size_t)mRows * kCta) + threadIdx.x;
     unsigned *smB = reinterpret_cast<unsigned *>(dyn + (size_t)2 * mRows * kCta);
     const bool smemBits = P.lgnW <= bitRoom;
     int lgnSlot = (int)(t0 % lgnSlots);
     if (smemSyn) {
         for (int q = 0; q < rows; q++) {
-            smI[q * kCta] = q < m ? __ldg(P.lgnId + (size_t)q * P.nV1 + i) : 0;
+            reinterpret_cast<int *>(smI + (q >> 2) * kCta)[q & 3] = q < m ? __ldg(P.lgnId + (size_t)q * P.nV1 + i) : 0;
             if (q < m) smW[q * kCta] = __ldg(P.sLGN + (size_t)q * P.nV1 + i);
         }
     }
@@ -1840,6 +1871,8 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
         sm.abortStep = -1;
         sm.peerFail = 0u;
     }
+    if (threadIdx.x < kMaxType) sm.type[threadIdx.x] = type_const(P, threadIdx.x);
+    const TypeConst &tc = sm.type[itype];
     if (list && threadIdx.x < 2 * (kMaxBS / 32)) sm.list.ball[threadIdx.x >> 5][threadIdx.x & 31] = 0u;
     cta_sync();
     if (threadIdx.x == 0) {
@@ -1895,17 +1928,17 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
                 if (buf) ph.bit1 ^= 1u;
                 else ph.bit0 ^= 1u;
             }
-            if (active) in = lgn_spikes(bits, lgnSInfo, smI, smW, m, rows);
+            if (active) in = lgn_spikes(bits, lgnSInfo, smI, smW, m, rows >> 2);
         }
         if (list && dl)
-            deliver_list<Rng>(P, t - 1, b, local, i, active, itype, st, condState, sm.list.unit[par ^ 1],
+            deliver_list<Rng>(P, tc, t - 1, b, local, i, active, itype, st, condState, sm.list.unit[par ^ 1],
                               sm.list.ball[par ^ 1]);
         auto feed_forward = [&]() {
             if (!active || (General && P.multiSpike)) return;
             if (smemSyn)
-                step_feedforward<Rng, true>(P, t, i, itype, tonic, depC, m, lgnSInfo, st, condState, noisyState, ff, in);
+                step_feedforward<Rng, true>(P, tc, t, i, itype, tonic, depC, m, lgnSInfo, st, condState, noisyState, ff, in);
             else
-                step_feedforward<Rng, false>(P, t, i, itype, tonic, depC, m, lgnSInfo, st, condState, noisyState, ff);
+                step_feedforward<Rng, false>(P, tc, t, i, itype, tonic, depC, m, lgnSInfo, st, condState, noisyState, ff);
         };
         // failure draws of the near synapses precede those of the LGN synapses: with a general
         // neighbour list they come after the barrier
@@ -1940,12 +1973,19 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
         }
         if (!ffEarly) feed_forward();
         float sInfo = 0.f;
-        if (active && !(General && P.multiSpike)) sInfo = step_membrane(P, itype, depC, ff, st);
+        const float vBefore = st.v;
+        if (active && !(General && P.multiSpike)) sInfo = step_membrane(P, tc, depC, ff, st);
         if (General && active && P.multiSpike)
             sInfo = step_multi<Rng>(P, t, i, itype, tonic, depC, m, lgnSInfo, st, condState, noisyState);
         const bool spk = active && sInfo >= 1.0f;
         if (list && s + 1 < steps) publish_spikes(P, sm, par, csize, rank, spk, sInfo, isE);
-        if (spk) prefetch_spiker(P, b, local, farE0, farDeg);
+        // a neuron that enters the last tenth below its threshold will likely spike some steps from now:
+        // what its delivery and its same-step push wait for is then already in L2
+        if (active && !spk) {
+            const float near = tc.level.y - 0.1f * (tc.level.y - tc.level.x);
+            if (vBefore < near && st.v >= near) prefetch_spiker(P, b, local, farE0, farN1);
+        }
+        if (spk && farDeg > farN1) prefetch_far(P, farE0 + farN1, farDeg - farN1);
         if (P.farOn) {
             if (spk && farDeg > 0) {
                 const int q = atomicAdd(&sm.cnt[par], 1);
