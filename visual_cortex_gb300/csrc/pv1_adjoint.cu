@@ -24,6 +24,7 @@
 // the adjoint (sum over posts of C[p][n] * lambda_hI[n] for every I neuron p) is a
 // warp-cooperative mat-vec over the block's C rows per step.  Gradients: dL/dW by atomic adds
 // at the (sparse) LGN events, dL/d(EdE, ErE, dodE, EdI, ErI, dodI) reduced in FP64.
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <string>
@@ -44,8 +45,9 @@ struct AdjArgs {
     int N, nI, nWin, nSeg;
     int split;   // CTAs per (trial, block)
     // dynamic shared memory, in bytes from its start (-1: not there): event masks of the CTA's neurons,
-    // their event lists by LGN cell (offsets, entries), synapse weights
+    // their event lists by LGN cell (offsets, entries), synapse weights, inhibitory weights
     int maskAt, offAt, entAt, wAt;
+    int gabaAt, gabaRoom;   // the block's inhibitory weights
     int smemBytes;
 };
 
@@ -128,8 +130,9 @@ __device__ __forceinline__ float adj_neuron_step(const pv1_adj_problem &P, AStat
 // count towards an mbarrier; the same mbarrier tells that every warp has set its bits.  Two
 // buffers by parity of the step: a warp reaches step t + 2's only after the phase of step t + 1, which
 // its peers announce after they have used step t's.
-// Measured: forward and backward of 4,096 neurons x 16 trials x 4,000 steps 40,384 -> 23,737 us, of two
-// blocks of 128 neurons x 320 steps with the recurrent term 3,784 -> 3,193 us.
+// Measured, with the staged inhibitory weights below: forward and backward of 4,096 neurons x 16 trials x
+// 4,000 steps 40,384 -> 22,120 us (23,737 without them), of two blocks of 128 neurons x 320 steps with
+// the recurrent term 3,784 -> 2,914 us.
 struct AdjShared {
     unsigned ball[2][32];
     unsigned *mask[2], *many[2];   // per neuron of the CTA: synapses with an event; those with a count above 1
@@ -329,54 +332,123 @@ __device__ __forceinline__ unsigned lgn_inputs(const AdjArgs &A, const uint8_t *
     return mask;
 }
 
-// The weights of the block's spiking I neurons (ball: the step's ballots) onto this neuron, ascending: all
-// but the last (up to) eight are added to hI here, those are left in pend (absent: 0 with pendN).  They
-// are added at the start of the next step, behind the work that does not need them.
+// The CTA's columns of the block's I -> all weights without their zeros, in shared memory: they are read
+// between a step's spikes and the next step's threshold, where a read from L2 was a third of the
+// step.  Per I neuron and 32 columns (a warp): the bits of the non-zero columns and the place of the first
+// one's weight.  (hI is never -0, so leaving out the zeros does not change it.)
+struct GabaView {
+    const float *C;            // [nI][blockSize]
+    const unsigned *bits;      // [nI][columns / 32], null: the weights did not fit, read C
+    const unsigned *first;     // [nI][columns / 32]
+    const float *w;
+    int words;                 // columns / 32
+};
+
+// Builds it at dyn + A.gabaAt within A.gabaRoom bytes (every thread of the CTA calls it).
+__device__ __forceinline__ GabaView stage_gaba(const AdjArgs &A, uint8_t *dyn, const float *C, int col0, AdjShared &sm) {
+    GabaView v{C, nullptr, nullptr, nullptr, (int)blockDim.x / 32};
+    const int words = v.words, cells = A.nI * words, bs = (int)A.p.blockSize;
+    if (A.gabaAt < 0) return v;
+    unsigned *bits = reinterpret_cast<unsigned *>(dyn + A.gabaAt), *first = bits + cells;
+    float *w = reinterpret_cast<float *>(first + cells);
+    const int cap = (A.gabaRoom - cells * 8) / 4;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const float *col = C + col0 + threadIdx.x;   // warp w holds column word w
+    if (threadIdx.x == 0) sm.scan[0] = 0;
+    __syncthreads();
+    for (int p0 = 0; p0 < A.nI; p0 += 4) {
+        float x[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) x[u] = p0 + u < A.nI ? __ldg(col + (size_t)(p0 + u) * bs) : 0.f;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (p0 + u >= A.nI) break;
+            const unsigned m = __ballot_sync(0xffffffffu, x[u] != 0.f);
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&sm.scan[0], __popc(m));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            const int k = (p0 + u) * words + warp;
+            if (lane == 0) {
+                bits[k] = m;
+                first[k] = (unsigned)at;
+            }
+            const int mine = at + __popc(m & ((1u << lane) - 1u));
+            if (x[u] != 0.f && mine < cap) w[mine] = x[u];
+        }
+    }
+    __syncthreads();
+    const bool fits = sm.scan[0] <= cap;
+    __syncthreads();
+    if (fits) {
+        v.bits = bits;
+        v.first = first;
+        v.w = w;
+    }
+    return v;
+}
+
+// The weights of the block's spiking I neurons (ball: the step's ballots) onto this neuron, ascending.  Read
+// from shared memory they are added to hI here; read from global memory, all but the last (up to)
+// four are, and those are left in pend, to be added at the start of the next step, behind the
+// work that does not need them.
 struct Pending {
-    float w[8];
+    float w[4];
     int n;
 };
 
-__device__ __forceinline__ void gaba_inputs(const AdjArgs &A, const float *C, int local, const unsigned *ball, float &hI,
+__device__ __forceinline__ void gaba_inputs(const AdjArgs &A, const GabaView &v, int local, const unsigned *ball, float &hI,
                                             Pending &pd) {
     const pv1_adj_problem &P = A.p;
     const int nWarp = ((int)P.blockSize + 31) / 32;
     const int lane = threadIdx.x & 31, w0 = (int)P.nE / 32;
     const unsigned mine = lane >= w0 && lane < nWarp ? ball[lane] : 0u;
-    unsigned nz = __ballot_sync(0xffffffffu, mine != 0), cur = 0u;
-    int w = 0;
+    unsigned nz = __ballot_sync(0xffffffffu, mine != 0);
     pd.n = 0;
+    if (!nz) return;
+    unsigned cur = 0u;
+    int w = 0;
+    auto next = [&]() {   // the next spiking I neuron; only while there is one
+        if (!cur) {
+            w = __ffs(nz) - 1;
+            nz &= nz - 1;
+            cur = __shfl_sync(0xffffffffu, mine, w);
+        }
+        const int pre = w * 32 + __ffs(cur) - 1 - (int)P.nE;
+        cur &= cur - 1;
+        return pre;
+    };
+    if (v.bits) {
+        const int word = threadIdx.x >> 5;
+        while (nz | cur) {
+            const int k = next() * v.words + word;
+            const unsigned m = v.bits[k];
+            if ((m >> lane) & 1u) hI = hI + v.w[v.first[k] + __popc(m & ((1u << lane) - 1u))];
+        }
+        return;
+    }
     while (nz | cur) {
         // a full batch left from before is followed by more: add it
-        if (pd.n == 8) {
+        if (pd.n == 4) {
 #pragma unroll
-            for (int j = 0; j < 8; j++) hI = hI + pd.w[j];
-            pd.n = 0;
+            for (int j = 0; j < 4; j++) hI = hI + pd.w[j];
         }
+        pd.n = 0;
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            if (!cur && nz) {
-                w = __ffs(nz) - 1;
-                nz &= nz - 1;
-                cur = __shfl_sync(0xffffffffu, mine, w);
-            }
-            if (cur) {
-                const int pre = w * 32 + __ffs(cur) - 1 - (int)P.nE;
-                cur &= cur - 1;
-                pd.w[j] = __ldg(C + (size_t)pre * P.blockSize + local);
-                pd.n = j + 1;
-            }
+        for (int j = 0; j < 4; j++) {
+            if (!(nz | cur)) break;
+            pd.w[j] = __ldg(v.C + (size_t)next() * P.blockSize + local);
+            pd.n = j + 1;
         }
     }
 }
 
 __device__ __forceinline__ void add_pending(float &hI, Pending &pd) {
-    if (pd.n) {
 #pragma unroll
-        for (int j = 0; j < 8; j++)
-            if (j < pd.n) hI = hI + pd.w[j];
-        pd.n = 0;
+    for (int j = 0; j < 4; j++) {
+        if (j >= pd.n) break;
+        hI = hI + pd.w[j];
     }
+    pd.n = 0;
 }
 
 // Copies the neuron's synapse weights into the CTA's shared memory (column per thread) where there is
@@ -419,7 +491,7 @@ struct StepOut {
 };
 
 __device__ __forceinline__ StepOut exchange_step(const AdjArgs &A, AdjShared &sm, AState &s, float I0, bool isE, int local,
-                                                 const float *C, const uint8_t *x, int par, unsigned &phase,
+                                                 const GabaView &gv, const uint8_t *x, int par, unsigned &phase,
                                                  const SynView &sv, Pending &pd) {
     StepOut o;
     float gE1, hE1, gI1, hI1;
@@ -428,7 +500,7 @@ __device__ __forceinline__ StepOut exchange_step(const AdjArgs &A, AdjShared &sm
     send_ballot(sm, par, local >> 5, bal, A.split);
     if (!wait_block(sm, par, phase)) o.vnext = nanf("");   // never seen: the run's outputs say so
     o.mask = lgn_inputs(A, x, sm, par, hE1, sv, o.many);
-    gaba_inputs(A, C, local, sm.ball[par], hI1, pd);
+    gaba_inputs(A, gv, local, sm.ball[par], hI1, pd);
     s.v = o.vnext;
     s.gE = gE1; s.hE = hE1; s.gI = gI1; s.hI = hI1;
     return o;
@@ -453,6 +525,7 @@ __global__ void __launch_bounds__(MaxThreads, 1) adj_forward_kernel(AdjArgs A) {
     const uint8_t *row = A.b.X + (size_t)b * P.T * P.nLGN;
     init_exchange(A, dyn, sm, n - threadIdx.x);
     const SynView sv = stage_synapses(A, dyn, n);
+    const GabaView gv = stage_gaba(A, dyn, C, local - threadIdx.x, sm);
     const bool fits = row_fits(A);
     RowShare share = fetch_row(A, row, fits);
     unsigned phase = 0u;
@@ -473,7 +546,7 @@ __global__ void __launch_bounds__(MaxThreads, 1) adj_forward_kernel(AdjArgs A) {
             toCk = (int)P.seg;
         }
         toCk--;
-        const StepOut r = exchange_step(A, sm, s, I0, isE, local, C, row, par, phase, sv, pd);
+        const StepOut r = exchange_step(A, sm, s, I0, isE, local, gv, row, par, phase, sv, pd);
         cnt += r.spk ? 1.f : 0.f;
         vsum += r.vnext;
         if (--toWin == 0) {
@@ -540,6 +613,7 @@ __global__ void __launch_bounds__(MaxThreads, 1) adj_backward_kernel(AdjArgs A) 
     const uint8_t *Xb = A.b.X + (size_t)b * P.T * P.nLGN;
     init_exchange(A, dyn, sm, n - threadIdx.x);
     const SynView sv = stage_synapses(A, dyn, n);
+    const GabaView gv = stage_gaba(A, dyn, C, local - threadIdx.x, sm);
     const bool fits = row_fits(A);
     unsigned phase = 0u;
     Pending pd;
@@ -565,7 +639,7 @@ __global__ void __launch_bounds__(MaxThreads, 1) adj_backward_kernel(AdjArgs A) 
             if (t + 1 < t1) share = fetch_row(A, row + P.nLGN, fits);
             add_pending(s.hI, pd);
             o[0] = s.v; o[bs] = s.gE; o[2 * bs] = s.hE; o[3 * bs] = s.gI; o[4 * bs] = s.hI;
-            const StepOut r = exchange_step(A, sm, s, I0, isE, local, C, row, t & 1, phase, sv, pd);
+            const StepOut r = exchange_step(A, sm, s, I0, isE, local, gv, row, t & 1, phase, sv, pd);
             o[5 * bs] = (float)((r.refr ? 1 : 0) | (r.spk ? 2 : 0) | (r.many ? 4 : 0));
             o[6 * bs] = __uint_as_float(r.mask);
         }
@@ -728,6 +802,15 @@ void adj_smem_plan(AdjArgs &A) {
         A.entAt = take(ent);
     }
     A.wAt = take((size_t)A.p.K * threads * sizeof(float));
+    // the rest, as far as the weights could need it, for the inhibitory ones
+    const size_t words = (size_t)A.nI * (threads / 32) * 8, all = words + (size_t)A.nI * threads * sizeof(float);
+    const size_t rest = std::min(room - at, all);
+    A.gabaAt = -1;
+    A.gabaRoom = 0;
+    if (rest > words + all / 16) {
+        A.gabaRoom = (int)rest;
+        A.gabaAt = take(rest);
+    }
     A.smemBytes = (int)at;
 }
 
