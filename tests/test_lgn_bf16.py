@@ -121,3 +121,29 @@ def test_simulation_driven_by_the_bf16_lgn_stage(native):
     assert lgn[True] > 300 and lgn[False] > 300, lgn
     assert rates[True] > 0.5 and rates[False] > 0.5, rates
     assert abs(rates[True] - rates[False]) < 0.1 * rates[False], rates
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cells,steps", [(131, 129), (130, 300), (4, 128), (260, 1)])
+def test_odd_sizes_are_parts_of_a_larger_stage(native, cells, steps):
+    """Cells and steps past the last whole tile, and cell counts whose rows the copy out cannot take: the
+    spike words and rates are, bit for bit, those of the same cells and steps in a stage of whole
+    tiles (a cell's generator depends on its index alone)."""
+    import dataclasses
+    from visual_cortex_gb300 import lgn_bf16 as L
+    full = L.make_workload(nCells=384, size=48, nFrame=24, side=15, T=384, seed=4)
+    part = dataclasses.replace(full, T=steps, W=full.W[:-(-steps // L.TILE_N)], f0=full.f0[:-(-steps // L.TILE_N)],
+                               **{k: getattr(full, k)[:cells] for k in
+                                  ("SW", "cx", "cy", "k", "c50", "sharp", "spont", "la", "lb", "maxConvol")})
+    out = []
+    for wl in (full, part):
+        tc = L.LgnTensorCore(wl, fr_every=1)
+        try:
+            tc.run(tensor_cores=True, seed=9)
+            out.append(tc.fetch(spikes=True)[1:])
+        finally:
+            tc.close()
+    (sp, fr), (sp1, fr1) = out
+    np.testing.assert_array_equal(fr1, fr[:steps, :cells])
+    np.testing.assert_array_equal(sp1, sp[:steps, :cells])
+    assert (sp >= 1).sum() > 100

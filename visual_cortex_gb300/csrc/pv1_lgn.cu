@@ -632,7 +632,7 @@ __device__ __forceinline__ unsigned draw_spikes(const LgnParams &P, long long it
     float next_rT = lnl - ltr, old_rT;
     unsigned nsp = 0;
     do {
-        const float u = curand_uniform(&st);
+        const float u = mrg_uniform(&st);
         if (P.recU) {
             const long long rs = it - P.recStep0;
             if (rs >= 0 && rs < P.recSteps) {

@@ -9,13 +9,13 @@
 // MMA's M); time advances in tiles of 128 steps (N); the frames a tile's steps read lie in a
 // 64-frame window (K).  Per tile: TMA loads the S window (128 cells x 64 frames, bf16, 128B
 // swizzle) and the tile's W (128 steps x 64 frames), one thread issues four
-// tcgen05.mma.kind::f16 (K = 16 each) into an FP32 accumulator in tensor memory; two
-// warpgroups read the lanes (cells) back with tcgen05.ld, 32 steps at a time, and evaluate the
-// logistic rate of LGN_nonlinear (src/discrete_input_convol.cu:1637-1730) for half the steps
-// each; the first group then runs the exact-time Poisson generator of get_spike (:1587-1635)
-// step by step, carrying each cell's generator state across tiles, while the next tile is
-// loaded and multiplied.  Every wait on an mbarrier is bounded; a timeout sets the error word and the
-// CTA stops issuing work, frees its tensor memory and returns.
+// tcgen05.mma.kind::f16 (K = 16 each) into an FP32 accumulator in tensor memory; eight warps
+// read the lanes (cells) back with tcgen05.ld and evaluate the logistic rate of LGN_nonlinear
+// (src/discrete_input_convol.cu:1637-1730); four warps run the exact-time Poisson generator of get_spike
+// (:1587-1635), a chain per cell, over the tile's steps.
+// Every stage works on another tile: two tiles of operands, accumulators and rates.  Every wait on an
+// mbarrier is bounded; a timeout sets the error word, every role stops and the CTA frees its tensor
+// memory and returns.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <curand_kernel.h>
@@ -67,28 +67,6 @@ __device__ __forceinline__ float lgn_rate(const TcArgs &A, float convol, float a
     return A.frRatio * mx * (LA * X + LB);
 }
 
-// Steps t0..t0+n-1 of one cell through get_spike from rT values in shared memory (stride
-// kTcM floats), spike words to out (stride nCells floats); four steps per pass with their
-// shared-memory loads issued together.
-__device__ __forceinline__ float lgn_poisson(float rT, float &ltr, float &lnl, curandStateMRG32k3a &st);
-__device__ __forceinline__ void lgn_poisson_run(const float *rT, int stride, int n, float *out, size_t nCells,
-                                                float &ltr, float &lnl, curandStateMRG32k3a &st) {
-    int c = 0;
-    for (; c + 4 <= n; c += 4) {
-        const float r0 = rT[(c + 0) * stride], r1 = rT[(c + 1) * stride];
-        const float r2 = rT[(c + 2) * stride], r3 = rT[(c + 3) * stride];
-        out[0] = lgn_poisson(r0, ltr, lnl, st);
-        out[nCells] = lgn_poisson(r1, ltr, lnl, st);
-        out[2 * nCells] = lgn_poisson(r2, ltr, lnl, st);
-        out[3 * nCells] = lgn_poisson(r3, ltr, lnl, st);
-        out += 4 * nCells;
-    }
-    for (; c < n; c++) {
-        out[0] = lgn_poisson(rT[c * stride], ltr, lnl, st);
-        out += nCells;
-    }
-}
-
 // get_spike (src/discrete_input_convol.cu:1589-1619) for one step given rT = dt * rate: the
 // only sequential part of the stage (the carried integral and the generator state).
 __device__ __forceinline__ float lgn_poisson(float rT, float &ltr, float &lnl, curandStateMRG32k3a &st) {
@@ -100,7 +78,7 @@ __device__ __forceinline__ float lgn_poisson(float rT, float &ltr, float &lnl, c
     unsigned nsp = 0;
     float old_rT;
     do {
-        const float u = curand_uniform(&st);
+        const float u = pv1::mrg_uniform(&st);
         lnl = fmaxf(-logf(u), 0.0f);
         old_rT = next_rT;
         next_rT += lnl;
@@ -108,6 +86,59 @@ __device__ __forceinline__ float lgn_poisson(float rT, float &ltr, float &lnl, c
     } while (next_rT <= rT);
     ltr = rT - old_rT;
     return nsp + old_rT / (rT * nsp);   // nsp + tsp / dt
+}
+
+// Steps 0..n-1 of a warp's cells (one per lane) through get_spike: rT, the cell's dt * rate of each step
+// (16-byte aligned), out its spike words in global memory (stride nCells), zero on entry.  Every
+// lane advances to the step of its own next spike and the draws of all lanes, at different steps, are made
+// together: stepping the lanes together instead made a draw whenever any of 32 cells spiked.
+// The advance takes sixteen steps on one test.  With l the carried integral before a step and r >= 0 its
+// rT, the step has no spike if lnl - l > r; if the integral after all sixteen, times 1.00001, is below lnl
+// (and so are then, rates being non-negative, the sums before it) that holds for each of them with room for
+// the roundings, which are below 2^-24 of lnl.  Otherwise the steps are tested one by one.
+__device__ __forceinline__ void lgn_poisson_run(const float *rT, int n, float *out, size_t nCells, float &ltr, float &lnl,
+                                                curandStateMRG32k3a &st) {
+    int c = 0;
+    while (__any_sync(0xffffffffu, c < n)) {
+        bool hit = false;
+        while (c < n) {
+            if ((c & 3) == 0 && c + 16 <= n) {
+                float l = ltr;
+                unsigned sign = 0u;
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const float4 r = *reinterpret_cast<const float4 *>(rT + c + 4 * k);
+                    l = l + r.x;
+                    l = l + r.y;
+                    l = l + r.z;
+                    l = l + r.w;
+                    sign |= __float_as_uint(r.x) | __float_as_uint(r.y);
+                    sign |= __float_as_uint(r.z) | __float_as_uint(r.w);
+                }
+                if (l * 1.00001f < lnl && !(sign >> 31)) {
+                    ltr = l;
+                    c += 16;
+                    continue;
+                }
+            }
+            // one step, or up to the next multiple of four
+            do {
+                const float r = rT[c];
+                if (!(lnl - ltr > r)) {
+                    hit = true;
+                    break;
+                }
+                ltr += r;
+                c++;
+            } while (c < n && (c & 3));
+            if (hit) break;
+        }
+        __syncwarp();
+        if (hit) {
+            out[(size_t)c * nCells] = lgn_poisson(rT[c], ltr, lnl, st);
+            c++;
+        }
+    }
 }
 
 // Epilogue of 32 consecutive steps t0..t0+31 of one cell: rates first (independent), then the
@@ -141,12 +172,15 @@ __device__ __forceinline__ void lgn_epilogue32(const TcArgs &A, int cell, int t0
 __device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+    asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                  : "memory");
 }
-// Bounded wait for the phase with the given parity; false on timeout.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity) {
+// Bounded wait for the phase with the given parity; false on timeout or when another role gave up.
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, const volatile int *stop) {
     for (long long i = 0; i < kWaitSpins; i++) {
         unsigned ok;
         asm volatile(
@@ -155,6 +189,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity) {
             : "r"(smem_u32(bar)), "r"(parity)
             : "memory");
         if (ok) return true;
+        if (*stop) return false;
         if (i > 64) __nanosleep(32);
     }
     return false;
@@ -165,6 +200,13 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
             smem_u32(dst)),
         "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
         : "memory");
+}
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, int x, int y, const void *src) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                     reinterpret_cast<uint64_t>(map)),
+                 "r"(x), "r"(y), "r"(smem_u32(src))
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
 // Shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups 1024 B apart.
 __device__ __forceinline__ uint64_t umma_desc_sw128(unsigned addr) {
@@ -190,6 +232,11 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
 }
+__device__ __forceinline__ float tmem_ld1(unsigned taddr) {
+    unsigned r;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\n\ttcgen05.wait::ld.sync.aligned;" : "=r"(r) : "r"(taddr));
+    return __uint_as_float(r);
+}
 __device__ __forceinline__ void tmem_ld32(unsigned taddr, float *v) {
     unsigned r[32];
     asm volatile(
@@ -205,123 +252,200 @@ __device__ __forceinline__ void tmem_ld32(unsigned taddr, float *v) {
     for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
 
-// Two warpgroups.  Per tile: the MMA result is read back by both (warp w reads the lanes of
-// quadrant w % 4; the first group columns 0-63, the second 64-127), each thread turning its 64
-// sums into rates (the independent part) stored to shared memory R [step][cell]; then the first
-// group runs the generator of its cell through the 128 steps from R while one thread of the
-// second group already loads and multiplies the next tile into the (now free) tensor memory.
-constexpr int kTcThreads = 256;
-constexpr unsigned kTcSmem = 1024 + 2 * kTileBytes + kTcN * kTcM * 4;   // alignment, tiles, R
+// Roles of the CTA's warps: 0-3 the generators (warp w: cells 32 w .. 32 w + 31), 4-11 the rates (warp w
+// reads the accumulator lanes of quadrant w % 4, columns 0-63 or 64-127), 12 the copies in and the
+// MMAs, 13 the zeros of the spike words, stored by TMA from one zero block ahead of the generators,
+// which then store the few words that are not.  Tile i uses buffer i % 2; per buffer:
+//   load   operands have landed (TMA)            mma    accumulator is complete (tcgen05.commit)
+//   read   the rate warps are done with the accumulator
+//   rates  R holds the tile's dt * rate          free   the generators are done with R
+//   zero   the tile's words are zero in memory
+// Measured: the whole run (seeding, this kernel, the recorded rates read back) of 16,384 cells x 16,000 steps
+// 1,495 -> 984 us, against two warpgroups that took rates and generators of a tile in turn and stored
+// every word from the generator's lanes; the generators are what is left (four warps of divergent chains).
+// R is [cell][step] with rows of kRRow floats: 16-byte accesses of consecutive lanes fall into all banks.
+constexpr int kTcThreads = 14 * 32;
+constexpr int kRRow = kTcN + 4;
+constexpr unsigned kRBytes = kTcM * kRRow * 4;
+constexpr int kZeroSteps = 32;
+constexpr unsigned kZeroBytes = kZeroSteps * kTcM * 4;
+constexpr unsigned kTcSmem = 1024 + 2 * 2 * kTileBytes + 2 * kRBytes + kZeroBytes;   // alignment, operand tiles, R, zeros
+
+struct TcBarriers {
+    uint64_t load[2], mma[2], read[2], rates[2], free[2], zero[2];
+};
 
 __global__ void __launch_bounds__(kTcThreads, 1) lgn_tc_kernel(TcArgs A, const __grid_constant__ CUtensorMap mapS,
-                                                               const __grid_constant__ CUtensorMap mapW) {
+                                                               const __grid_constant__ CUtensorMap mapW,
+                                                               const __grid_constant__ CUtensorMap mapOut, int storeTma) {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t barFull, barMma;
+    __shared__ __align__(8) TcBarriers bar;
     __shared__ unsigned tmemSlot;
-    __shared__ int abortFlag;
+    __shared__ int stop;
     uint8_t *base = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t *tileS = base;
-    uint8_t *tileW = base + kTileBytes;
-    float *R = reinterpret_cast<float *>(base + 2 * kTileBytes);   // [kTcN][kTcM]
+    auto tileS = [&](int k) { return base + k * 2 * kTileBytes; };
+    auto tileW = [&](int k) { return base + k * 2 * kTileBytes + kTileBytes; };
+    auto R = [&](int k) { return reinterpret_cast<float *>(base + 4 * kTileBytes + k * kRBytes); };   // [kTcM][kRRow]
+    float4 *zeros = reinterpret_cast<float4 *>(base + 4 * kTileBytes + 2 * kRBytes);                  // [kZeroSteps][kTcM]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int quad = warp & 3, half = warp >> 2;
     const int cell0 = blockIdx.x * kTcM;
-    const int cl = quad * 32 + lane;   // this thread's lane of the accumulator = its cell
-    const int issuer = 4 * 32;         // first thread of the second group issues the copies and MMAs
     if (threadIdx.x == 0) {
-        mbar_init(&barFull, 1);
-        mbar_init(&barMma, 1);
+        for (int k = 0; k < 2; k++) {
+            mbar_init(&bar.load[k], 1);
+            mbar_init(&bar.mma[k], 1);
+            mbar_init(&bar.read[k], 8);
+            mbar_init(&bar.rates[k], 8);
+            mbar_init(&bar.free[k], 4);
+            mbar_init(&bar.zero[k], 1);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        abortFlag = 0;
+        stop = 0;
     }
+    for (int q = threadIdx.x; q < (int)(kZeroBytes / 16); q += kTcThreads) zeros[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmemSlot)),
-                     "r"(kTcN));
+                     "r"(2 * kTcN));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const unsigned tmem = tmemSlot;
-    const int cell = cell0 + cl;
-    const bool on = cell < A.nCells;
-    float absk = 0.f, mx = 1.f, C50 = 0.f, Kc = 0.f, LA = 0.f, LB = 0.f, ltr = 0.f, lnl = 0.f;
-    curandStateMRG32k3a st;
-    if (on) {
-        absk = A.absk[cell]; mx = A.maxConvol[cell]; C50 = A.c50[cell]; Kc = A.sharp[cell];
-        LA = A.la[cell]; LB = A.lb[cell];
-        if (half == 0) {
+    const volatile int *stopped = &stop;
+    auto wait = [&](uint64_t *b, unsigned parity) {
+        if (mbar_wait(b, parity, stopped)) return true;
+        atomicOr(A.err, kErrBarrier);
+        stop = 1;
+        return false;
+    };
+    if (warp < 4) {
+        // generators
+        const int cl = warp * 32 + lane, cell = cell0 + cl;
+        const bool on = cell < A.nCells;
+        float ltr = 0.f, lnl = 0.f;
+        curandStateMRG32k3a st;
+        if (on) {
             ltr = A.ltr[cell];
             lnl = A.lnl[cell];
             st = A.state[cell];
         }
-    }
-    const float rmx = 1.0f / mx;
-    const float scale = A.dt * 1e-3f;   // rate in spikes/ms times dt
-    // tile i: TMA of its S window and W, four MMAs into tensor memory, bounded waits
-    auto load_and_multiply = [&](int i) {
-        const unsigned parity = (unsigned)(i & 1);
-        mbar_expect_tx(&barFull, 2 * kTileBytes);
-        tma_load_2d(tileS, &mapS, A.f0[i], cell0, &barFull);
-        tma_load_2d(tileW, &mapW, 0, i * kTcN, &barFull);
-        if (!mbar_wait(&barFull, parity)) {
-            atomicOr(A.err, kErrBarrier);
-            abortFlag = 1;
-            mbar_wait(&barFull, parity);   // once more, bounded: let the copies in flight land
-            return;
+        for (int i = 0; i < A.nTiles; i++) {
+            const int k = i & 1;
+            if (!wait(&bar.rates[k], (i >> 1) & 1) || !wait(&bar.zero[k], (i >> 1) & 1)) break;
+            const int n = min(kTcN, A.T - i * kTcN);
+            float *out = A.sInfo + (size_t)i * kTcN * A.nCells + cell;
+            if (!storeTma && on)
+                for (int c = 0; c < n; c++) out[(size_t)c * A.nCells] = 0.f;
+            lgn_poisson_run(R(k) + cl * kRRow, on ? n : 0, out, (size_t)A.nCells, ltr, lnl, st);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar.free[k]);
         }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint64_t da = umma_desc_sw128(smem_u32(tileS));
-        const uint64_t db = umma_desc_sw128(smem_u32(tileW));
-#pragma unroll
-        for (int k = 0; k < kTcK / 16; k++)   // K = 16 per MMA: +32 bytes inside the swizzle atom
-            umma_bf16(tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), k > 0);
-        umma_commit(&barMma);
-        if (!mbar_wait(&barMma, parity)) {
-            atomicOr(A.err, kErrBarrier);
-            abortFlag = 1;
-            mbar_wait(&barMma, parity);    // once more, bounded, before the memory is freed
+        if (on) {
+            A.ltr[cell] = ltr;
+            A.lnl[cell] = lnl;
+            A.state[cell] = st;
         }
-    };
-    if (threadIdx.x == issuer && A.nTiles > 0) load_and_multiply(0);
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    for (int i = 0; i < A.nTiles; i++) {
-        if (abortFlag) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        // rates of this thread's cell at its group's 64 steps of the tile
-        for (int c0 = half * (kTcN / 2); c0 < (half + 1) * (kTcN / 2); c0 += 32) {
-            float v[32];
-            tmem_ld32(tmem + ((unsigned)(quad * 32) << 16) + (unsigned)c0, v);
-            if (on) {
-                int ph = (i * kTcN + c0) % A.frEvery;   // steps since the last recorded rate
+    } else if (warp < 12) {
+        // rates
+        const int quad = warp & 3, half = (warp - 4) >> 2;
+        const int cl = quad * 32 + lane, cell = cell0 + cl;
+        const bool on = cell < A.nCells;
+        float absk = 0.f, mx = 1.f, C50 = 0.f, Kc = 0.f, LA = 0.f, LB = 0.f;
+        if (on) {
+            absk = A.absk[cell]; mx = A.maxConvol[cell]; C50 = A.c50[cell]; Kc = A.sharp[cell];
+            LA = A.la[cell]; LB = A.lb[cell];
+        }
+        const float rmx = 1.0f / mx;
+        const float scale = A.dt * 1e-3f;   // rate in spikes/ms times dt
+        for (int i = 0; i < A.nTiles; i++) {
+            const int k = i & 1;
+            if (!wait(&bar.mma[k], (i >> 1) & 1)) break;
+            if (i >= 2 && !wait(&bar.free[k], ((i >> 1) - 1) & 1)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            float *out = R(k) + cl * kRRow;
+            for (int c0 = half * (kTcN / 2); c0 < (half + 1) * (kTcN / 2); c0 += 32) {
+                const unsigned lanes = tmem + ((unsigned)(quad * 32) << 16) + (unsigned)(k * kTcN + c0);
+                float v[32];
+                tmem_ld32(lanes, v);
 #pragma unroll
-                for (int j = 0; j < 32; j++) {
-                    const float fr = lgn_rate(A, v[j], absk, mx, rmx, C50, Kc, LA, LB);
-                    const int t = i * kTcN + c0 + j;
-                    if (A.fr && ph == 0 && t < A.T) A.fr[(size_t)(t / A.frEvery) * A.nCells + cell] = fr;
-                    ph = ph + 1 == A.frEvery ? 0 : ph + 1;
-                    R[(c0 + j) * kTcM + cl] = fr * scale;
+                for (int j = 0; j < 32; j += 4) {
+                    float4 r;
+                    r.x = lgn_rate(A, v[j], absk, mx, rmx, C50, Kc, LA, LB) * scale;
+                    r.y = lgn_rate(A, v[j + 1], absk, mx, rmx, C50, Kc, LA, LB) * scale;
+                    r.z = lgn_rate(A, v[j + 2], absk, mx, rmx, C50, Kc, LA, LB) * scale;
+                    r.w = lgn_rate(A, v[j + 3], absk, mx, rmx, C50, Kc, LA, LB) * scale;
+                    *reinterpret_cast<float4 *>(out + c0 + j) = r;
+                }
+                if (A.fr) {
+                    // the steps whose rates are recorded: their sums are read once more
+                    const int t0 = i * kTcN + c0, end = min(t0 + 32, A.T);
+                    for (int row = (t0 + A.frEvery - 1) / A.frEvery; row * A.frEvery < end; row++) {
+                        const float x = tmem_ld1(lanes + (unsigned)(row * A.frEvery - t0));
+                        if (on) A.fr[(size_t)row * A.nCells + cell] = lgn_rate(A, x, absk, mx, rmx, C50, Kc, LA, LB);
+                    }
                 }
             }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&bar.read[k]);
+                mbar_arrive(&bar.rates[k]);
+            }
         }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();   // R holds the tile; tensor memory and both tiles are free
-        if (threadIdx.x == issuer && i + 1 < A.nTiles) load_and_multiply(i + 1);
-        if (half == 0 && on)
-            lgn_poisson_run(R + cl, kTcM, min(kTcN, A.T - i * kTcN), A.sInfo + (size_t)i * kTcN * A.nCells + cell,
-                            (size_t)A.nCells, ltr, lnl, st);
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();   // R is read; the next tile is in tensor memory
-    }
-    (void)lane;
-    if (on && half == 0) {
-        A.ltr[cell] = ltr;
-        A.lnl[cell] = lnl;
-        A.state[cell] = st;
+    } else if (warp == 12) {
+        if (lane == 0) {
+            auto load = [&](int i) {
+                const int k = i & 1;
+                mbar_expect_tx(&bar.load[k], 2 * kTileBytes);
+                tma_load_2d(tileS(k), &mapS, A.f0[i], cell0, &bar.load[k]);
+                tma_load_2d(tileW(k), &mapW, 0, i * kTcN, &bar.load[k]);
+            };
+            int loaded = 0, done = 0;   // tiles asked for, tiles multiplied
+            for (; loaded < 2 && loaded < A.nTiles; loaded++) load(loaded);
+            for (int i = 0; i < A.nTiles; i++) {
+                const int k = i & 1;
+                if (!wait(&bar.load[k], (i >> 1) & 1)) break;
+                if (i >= 2 && !wait(&bar.read[k], ((i >> 1) - 1) & 1)) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t da = umma_desc_sw128(smem_u32(tileS(k)));
+                const uint64_t db = umma_desc_sw128(smem_u32(tileW(k)));
+#pragma unroll
+                for (int q = 0; q < kTcK / 16; q++)   // K = 16 per MMA: +32 bytes inside the swizzle atom
+                    umma_bf16(tmem + (unsigned)(k * kTcN), da + (uint64_t)(2 * q), db + (uint64_t)(2 * q), q > 0);
+                umma_commit(&bar.mma[k]);
+                done = i + 1;
+                if (loaded < A.nTiles) {
+                    if (!wait(&bar.mma[k], (i >> 1) & 1)) break;
+                    load(loaded++);
+                }
+            }
+            // after a failure: copies and products still in flight are waited for, with a limit, before
+            // the memory under them is given up
+            const int never = 0;
+            if (stop)
+                for (int i = max(0, loaded - 2); i < loaded; i++) {
+                    if (i >= done) mbar_wait(&bar.load[i & 1], (i >> 1) & 1, &never);
+                    else mbar_wait(&bar.mma[i & 1], (i >> 1) & 1, &never);
+                }
+        }
+    } else {
+        if (lane == 0) {
+            for (int i = 0; i < A.nTiles; i++) {
+                const int k = i & 1;
+                // two tiles ahead of the generators at most: a barrier's phases are waited for in turn
+                if (i >= 2 && !wait(&bar.free[k], ((i >> 1) - 1) & 1)) break;
+                if (storeTma) {
+                    for (int t = i * kTcN; t < min((i + 1) * kTcN, A.T); t += kZeroSteps) tma_store_2d(&mapOut, cell0, t, zeros);
+                    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // written, not only read
+                    asm volatile("fence.proxy.async;" ::: "memory");            // before the generators' own stores
+                }
+                mbar_arrive(&bar.zero[k]);
+            }
+        }
     }
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTcN));
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kTcN));
 }
 
 // The same tiles on CUDA cores in FP32: the thread's row of the S window in registers, the
@@ -430,7 +554,8 @@ struct pv1_lgn_tc {
     int nFext = 0, nTiles = 0;
     __nv_bfloat16 *S16 = nullptr, *W16 = nullptr;
     float *S32 = nullptr, *W32 = nullptr;
-    CUtensorMap mapS{}, mapW{};
+    CUtensorMap mapS{}, mapW{}, mapOut{};
+    bool storeTma = false;
     int *d_err = nullptr;
 };
 
@@ -460,7 +585,9 @@ int talloc(pv1_lgn_tc *p, T **ptr, size_t n, const void *host = nullptr) {
     return PV1_OK;
 }
 
-int encode_map(pv1_lgn_tc *p, CUtensorMap *map, void *base, uint64_t inner, uint64_t outer) {
+// A 2D map of `outer` rows of `inner` elements: bf16 operands (box kTcM x kTcK, 128-byte swizzle) or
+// fp32 spike words (box kZeroSteps x kTcM, rows as they are).
+int encode_map(pv1_lgn_tc *p, CUtensorMap *map, void *base, uint64_t inner, uint64_t outer, bool words) {
     static EncodeTiledFn fn = nullptr;
     if (!fn) {
         void *f = nullptr;
@@ -470,11 +597,12 @@ int encode_map(pv1_lgn_tc *p, CUtensorMap *map, void *base, uint64_t inner, uint
         fn = (EncodeTiledFn)f;
     }
     const cuuint64_t dims[2] = {inner, outer};
-    const cuuint64_t strides[1] = {inner * 2};   // bytes, multiple of 16 (inner multiple of 8)
-    const cuuint32_t box[2] = {(cuuint32_t)kTcK, (cuuint32_t)kTcM};
+    const cuuint64_t strides[1] = {inner * (words ? 4 : 2)};   // bytes, a multiple of 16
+    const cuuint32_t box[2] = {words ? (cuuint32_t)kTcM : (cuuint32_t)kTcK, words ? (cuuint32_t)kZeroSteps : (cuuint32_t)kTcM};
     const cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+    CUresult r = fn(map, words ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides,
+                    box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    words ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return tfail(p, PV1_E_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
     return PV1_OK;
@@ -544,10 +672,16 @@ int pv1_lgn_tc_create(const pv1_lgn_tc_config *cfg, const float *frames, const f
     const size_t nW = (size_t)nTiles * kTcN * kTcK;
     to_bf16_kernel<<<(unsigned)((nW + 255) / 256), 256, 0, p->stream>>>(p->W32, p->W16, nW);
     PV1_TCUDA(p, cudaGetLastError());
-    r = encode_map(p, &p->mapS, p->S16, c.nFext, nC);
+    r = encode_map(p, &p->mapS, p->S16, c.nFext, nC, false);
     if (r) return r;
-    r = encode_map(p, &p->mapW, p->W16, kTcK, (uint64_t)nTiles * kTcN);
+    r = encode_map(p, &p->mapW, p->W16, kTcK, (uint64_t)nTiles * kTcN, false);
     if (r) return r;
+    // the copy out needs rows of whole 16-byte units; other cell counts are stored by the generator threads
+    p->storeTma = nC % 4 == 0;
+    if (p->storeTma) {
+        r = encode_map(p, &p->mapOut, d_sInfo, nC, c.T, true);
+        if (r) return r;
+    }
     TcArgs &a = p->a;
     a.nCells = (int)nC; a.nFext = (int)c.nFext; a.T = (int)c.T; a.nTiles = nTiles; a.frEvery = (int)c.frEvery;
     a.dt = c.dt; a.convolRatio = c.convolRatio; a.frRatio = c.frRatio;
@@ -571,11 +705,10 @@ int pv1_lgn_tc_run(pv1_lgn_tc *p, int tensorCores, uint64_t seed, float *ms) {
     PV1_TCUDA(p, cudaEventRecord(e0, p->stream));
     const int grid = (a.nCells + kTcM - 1) / kTcM;
     if (tensorCores) {
-        // 60 KB per CTA keeps at most 3 CTAs on an SM: 3 x 128 tensor-memory columns <= 512,
-        // so no CTA ever waits in tcgen05.alloc
+        // 213 KB per CTA keep one CTA on an SM, so none ever waits in tcgen05.alloc
         const int smem = (int)kTcSmem;
         PV1_TCUDA(p, cudaFuncSetAttribute(lgn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        lgn_tc_kernel<<<grid, kTcThreads, smem, p->stream>>>(a, p->mapS, p->mapW);
+        lgn_tc_kernel<<<grid, kTcThreads, smem, p->stream>>>(a, p->mapS, p->mapW, p->mapOut, p->storeTma ? 1 : 0);
     } else {
         lgn_f32_kernel<<<grid, 128, 0, p->stream>>>(a);
     }

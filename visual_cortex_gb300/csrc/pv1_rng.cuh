@@ -95,4 +95,27 @@ __device__ __forceinline__ void mrg_seed(unsigned long long seed, unsigned long 
     }
 }
 
+// The next uniform of (0, 1], curand_uniform(s) bit for bit: the recurrence and the combination of its two
+// parts as published (see the top of the file), in integers.  cuRAND evaluates them in double precision,
+// whose rate is a small fraction of single's here.  Measured on the LGN stage of the sweep of 12 trials: the
+// sweep 23,376 -> 22,970 us; 16 steps of one block 128.1 -> 126.2 us.
+__device__ __forceinline__ float mrg_uniform(curandStateMRG32k3a *s) {
+    auto fold = [](unsigned long long a, unsigned long long b, unsigned long long C) {   // a + b mod 2^32 - C
+        unsigned long long t = (a >> 32) * C + (a & 0xffffffffull) + (b >> 32) * C + (b & 0xffffffffull);
+        t = (t >> 32) * C + (t & 0xffffffffull);
+        const unsigned long long m = 4294967296ull - C;
+        return (unsigned)(t >= m ? t - m : t);
+    };
+    const unsigned p1 = fold(1403580ull * s->s1[1], (kMrgM1 - 810728ull) * s->s1[0], 209ull);
+    s->s1[0] = s->s1[1];
+    s->s1[1] = s->s1[2];
+    s->s1[2] = p1;
+    const unsigned p2 = fold(527612ull * s->s2[2], (kMrgM2 - 1370589ull) * s->s2[0], 22853ull);
+    s->s2[0] = s->s2[1];
+    s->s2[1] = s->s2[2];
+    s->s2[2] = p2;
+    const unsigned z = p1 > p2 ? p1 - p2 : (unsigned)(p1 + kMrgM1 - p2);
+    return (float)((double)z * (1.0 / 4294967087.0));   // 1 .. m1 to (0, 1]
+}
+
 }  // namespace pv1
