@@ -768,12 +768,18 @@ int adj_check(const pv1_adj_problem *p, const pv1_adj_buffers *b, AdjArgs *A, bo
     A->nI = (int)(p->blockSize - p->nE);
     A->nWin = (int)(p->T / p->win);
     A->nSeg = (int)((p->T + p->seg - 1) / p->seg);
+    // CTAs per block where the caller leaves it open.  Two halve a step's work per SM and cost an exchange
+    // over the cluster: measured forward and backward of 480 steps without the recurrent term, one CTA
+    // against two: 128 neurons 1,981 and 2,057 us, 256 neurons 2,245 and 2,163, 1,024 neurons 4,449 and
+    // 3,125.  With it the backward exchanges every step's adjoints: 128 neurons 2,455 and 4,431, 1,024
+    // neurons 9,687 and 15,865.
     int split = (int)p->ctaSplit;
     if (split == 0) {
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        split = (p->blockSize % 64 == 0 && (long long)p->B * p->nblock * 2 <= sms) ? 2 : 1;
+        const bool wide = p->blockSize >= 256 && p->blockSize % 64 == 0 && !(backward && p->recGrad);
+        split = (wide && (long long)p->B * p->nblock * 2 <= sms) ? 2 : 1;
     }
     if (split != 1 && (split != 2 || p->blockSize % 64)) {
         g_adjErr = "ctaSplit must be 0, 1 or 2 (2 needs blockSize a multiple of 64)";
