@@ -378,8 +378,8 @@ int pv1_set_step(pv1_plan *plan, int64_t step);
  * (tauAvg[0] when nLearnTypeE > 0; 0 reproduces the zeroed struct the reference passes
  * otherwise).  Derived rates as learnFF_post computes them (src/condShape.h:137-152),
  * exp_homeo = expf(-dt / decayTimeHomeoFF) (src/patch.cu:1330); the homeostasis totals start
- * from the current weights (src/patch.cu:4335-4352).  Plans with learning run one launch per
- * step (no persistent kernel, no batches) and one spike per step at most;
+ * from the current weights (src/patch.cu:4335-4352).  Plans with learning are not stepped by the
+ * cooperative kernel (pv1_persistent_mode) and not batched, and spike once per step at most;
  * PV1_E_UNSUPPORTED otherwise. */
 typedef struct pv1_ff_learning {
     int32_t learning;            /* 1, 2, 3 or 4 */
@@ -480,7 +480,9 @@ int pv1_set_wait_limit(pv1_plan *plan, int64_t spins);
 
 /* allow = 1/0 enables/disables the persistent cooperative V1 kernel (one launch per chunk of
  * steps, state in registers, bounded grid barrier between steps); allow = -1 only queries.
- * Returns 1 if the plan steps with the persistent kernel, 0 if with one launch per step. */
+ * Returns 1 if the plan steps with the persistent kernel, 0 if not: with one launch per step or,
+ * for plasticity in networks whose blocks are independent, with one launch of a cluster per block
+ * and chunk of steps (allow = 0 turns that off too). */
 int pv1_persistent_mode(pv1_plan *plan, int allow);
 
 /* ---- Batched trials ------------------------------------------------------------------

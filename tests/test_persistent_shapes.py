@@ -37,19 +37,24 @@ def _foreign(wl):
     return wl
 
 
-def _run(wl, modes, chunks):
+def _run(wl, modes, chunks, learning=None):
     from visual_cortex_gb300 import _native as N
     from visual_cortex_gb300.model import Simulation
     sim = Simulation(wl.spec, wl.net, wl.lgn, wl.stim, wl.init, wl.seeds)
     try:
+        if learning is not None:
+            sim.set_ff_learning(learning)
         sim.set_record(N.REC_SPIKES, sum(chunks) + 1)
         for k, n in enumerate(chunks):
             want = modes[k % len(modes)]
-            assert sim.persistent(int(want)) == want
+            assert sim.persistent(int(want)) == (want and learning is None)
             sim.run(n)
         out = {"raster": sim.fetch_spikes(0, sum(chunks))}
         for s in ("v", "w", "gE", "hE", "gI", "hI", "gFF", "hFF", "tBack", "dep"):
             out[s] = sim.state(s)
+        if learning is not None:
+            for s in ("sLGN", "ff_post", "ff_pre", "total_ff"):
+                out[s] = sim.state(s)
     finally:
         sim.close()
     return out
@@ -83,3 +88,23 @@ def test_foreign_near_blocks(native, far):
                                       height=64, nt=400, adex_inh=True, nFrame=40, wFF=0.35, far_partners=far))
     chunks = [65, 1, 100]
     _same(_run(wl, [False], chunks), _run(wl, [True], chunks))
+
+
+@pytest.mark.parametrize("mode,homeo,name", [(1, 0, "no_far"), (2, 2, "no_far"), (3, 1, "far"), (4, 1, "no_far"),
+                                             (3, 2, "noise_failure")])
+def test_plasticity_in_the_persistent_kernel(native, mode, homeo, name):
+    """LGN->V1 learning, which runs in the same kernel where blocks are independent (not as the cooperative
+    mode the plan reports): weights, post and presynaptic traces and homeostasis totals as the per-step
+    kernel leaves them, also when the two take turns."""
+    from visual_cortex_gb300.model import FFLearning
+    learning = FFLearning(tauLTP=16.8, tauLTD=33.7, tauTrip=114.0, tauAvg=1000.0, targetFR=8.0 if mode == 1 else 0.0,
+                          A_LGN=0.02, r_LTD=1.0, gmaxLGN=0.6, gminLGN=0.0, sRatioLGN=1.0, decayTimeHomeoFF=250.0,
+                          applyHomeo=homeo, learning=mode, nLearnTypeFF_I=1 if mode == 2 else 0, tauLTP_I=16.8,
+                          tauLTD_I=33.7, tauTrip_I=114.0, tauAvg_I=1000.0, A_LGN_I=0.01, r_LTD_I=1.0, gmaxLGN_I=0.6,
+                          gminLGN_I=0.0, sRatioLGN_I=1.0, tauAvgCortical=500.0)
+    wl = _workload(name)
+    chunks = [65, 1, 70, 64]
+    ref = _run(wl, [False], chunks, learning)
+    assert np.abs(ref["sLGN"] - np.asarray(wl.net.sLGN, np.float32).ravel()).max() > (1e-4 if mode != 4 else -1)
+    _same(ref, _run(wl, [True], chunks, learning))
+    _same(ref, _run(wl, [True, False], chunks, learning))

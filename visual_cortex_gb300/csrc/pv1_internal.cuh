@@ -391,6 +391,7 @@ bool v1_persistent_shape(const V1Params &p, int device, int *cluster, int *threa
 // Evaluates the full-step decay factors of the three conductance kernels on the device, checks the
 // quick divisions by their times and stores both into p (synchronous).
 cudaError_t compute_step_decay(V1Params &p, cudaStream_t st);
+// barrier null: the blocks do not wait on one another (no cooperative launch).
 cudaError_t launch_v1_persistent(const V1Params &p, const long long *stepBase, int K, const float *lgnRing,
                                  const unsigned *lgnBits, int lgnSlots, int deliverFirst, unsigned *barrier, cudaStream_t st);
 cudaError_t launch_advance_step(long long *stepBase, int k, cudaStream_t st);

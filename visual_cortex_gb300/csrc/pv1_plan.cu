@@ -73,6 +73,7 @@ struct pv1_plan {
     long long extStep0 = 0, extSteps = 0;
     int K = 64;  // steps per LGN launch / per persistent V1 launch / per graph
     bool persistent = false;     // V1 steps run as one cooperative launch per chunk
+    bool chunked = false;        // one launch per chunk: persistent, or independent clusters (plasticity)
     // the LGN of chunk c+1 runs on its own stream while the persistent V1 kernel runs chunk c
     cudaStream_t lgnStream = nullptr;
     cudaEvent_t evLgn = nullptr, evFree = nullptr;
@@ -235,8 +236,9 @@ int issue_chunk(pv1_plan *p, long long t0, int k, int deliverFirst, long long *l
     int r = lgn_stage(p, t0, k, p->d_stepBase, p->stream, &n);
     if (r) return r;
     cudaError_t e = cudaSuccess;
-    if (p->persistent) {
-        e = launch_v1_persistent(p->vp, p->d_stepBase, k, p->d_lgnRing, p->d_lgnBits, p->lgnSlots, deliverFirst, p->d_barrier,
+    if (p->chunked) {
+        e = launch_v1_persistent(p->vp, p->d_stepBase, k, p->d_lgnRing, p->d_lgnBits, p->lgnSlots, deliverFirst,
+                                 p->persistent ? p->d_barrier : nullptr,
                                  p->stream);
         if (e != cudaSuccess) return fail(p, PV1_E_CUDA, std::string("v1_persistent: ") + cudaGetErrorString(e));
         n += 1;
@@ -1846,9 +1848,14 @@ static int choose_mode(pv1_plan *p) {
     p->vp.cluster = 1;
     p->vp.threads = 256;
     p->vp.lgnW = p->lp.bitW;
-    p->persistent = p->allowPersistent && !p->vp.multiSpike && !p->vp.farPullOn && !p->vp.nearPullOn && !p->vp.ffMode &&
-                    v1_persistent_shape(p->vp, p->device, &p->vp.cluster, &p->vp.threads);
-    p->lp.outBits = p->persistent ? p->d_lgnBits : nullptr;
+    const bool fits = p->allowPersistent && !p->vp.multiSpike && !p->vp.farPullOn && !p->vp.nearPullOn &&
+                      v1_persistent_shape(p->vp, p->device, &p->vp.cluster, &p->vp.threads);
+    p->persistent = fits && !p->vp.ffMode;
+    // with plasticity the same kernel runs where its blocks do not wait on one another: clusters
+    // launched without the cooperative attribute and without a grid barrier
+    p->chunked = p->persistent || (fits && p->vp.ffMode && !p->vp.farOn && p->vp.noDelay && p->vp.nearSelf &&
+                                   p->vp.cluster * 256 >= (int)p->cfg.blockSize);
+    p->lp.outBits = p->chunked ? p->d_lgnBits : nullptr;
     if (p->persistent && !p->d_barrier) {
         int r = dev_alloc(p, &p->d_barrier, 2);
         if (r) return r;
@@ -1917,7 +1924,7 @@ int pv1_run(pv1_plan *p, uint32_t nsteps, int sync) {
         done += k;
     }
     if (nsteps - done >= (uint32_t)K) {
-        if (p->persistent && p->lgnSlots >= 2 * K) {
+        if (p->chunked && p->lgnSlots >= 2 * K) {
             // one cooperative V1 launch per chunk on the plan's stream; the LGN of the next chunk
             // of this run (never beyond it) on the LGN stream meanwhile, into the other half of
             // the ring, after the V1 launch that read that half has finished
@@ -1940,7 +1947,7 @@ int pv1_run(pv1_plan *p, uint32_t nsteps, int sync) {
                 if (c > 0) PV1_CUDA(p, cudaStreamWaitEvent(p->stream, p->evLgn, 0));
                 PV1_CUDA(p, cudaEventRecord(p->evFree, p->stream));   // chunk c-1's V1 is done
                 e = launch_v1_persistent(p->vp, p->d_stepBase, K, p->d_lgnRing, p->d_lgnBits, p->lgnSlots, 1,
-                                         p->d_barrier, p->stream);
+                                         p->persistent ? p->d_barrier : nullptr, p->stream);
                 if (e == cudaSuccess) e = launch_advance_step(p->d_stepBase, K, p->stream);
                 if (e != cudaSuccess) return fail(p, PV1_E_CUDA, std::string("v1_persistent: ") + cudaGetErrorString(e));
                 p->launches += 2;
@@ -1957,7 +1964,7 @@ int pv1_run(pv1_plan *p, uint32_t nsteps, int sync) {
                 }
                 done += K;
             }
-        } else if (p->persistent) {
+        } else if (p->chunked) {
             // a cooperative launch per chunk: issued directly (4 launches per K steps)
             while (nsteps - done >= (uint32_t)K) {
                 r = issue_chunk(p, p->step + (long long)done, K, 1, &p->launches);
@@ -2104,9 +2111,9 @@ int pv1_time_kernels(pv1_plan *p, uint32_t nsteps, float *v1_ms, float *lgn_ms, 
         PV1_CUDA(p, cudaEventRecord(ev[3 * c], p->stream));
         PV1_CUDA(p, launch_lgn_step(p->lp, p->d_stepBase, K, p->stream));
         PV1_CUDA(p, cudaEventRecord(ev[3 * c + 1], p->stream));
-        if (p->persistent) {
+        if (p->chunked) {
             PV1_CUDA(p, launch_v1_persistent(p->vp, p->d_stepBase, K, p->d_lgnRing, p->d_lgnBits, p->lgnSlots,
-                                             deliverFirst, p->d_barrier, p->stream));
+                                             deliverFirst, p->persistent ? p->d_barrier : nullptr, p->stream));
         } else {
             for (int s = 0; s < K; s++)
                 PV1_CUDA(p, launch_v1_step(p->vp, p->d_stepBase, s, p->d_lgnRing, p->lgnSlots,

@@ -215,18 +215,17 @@ __device__ __forceinline__ void prefetch_spiker(const V1Params &P, int b, int lo
 // delivery as recal_G_mat_nd_fast does (src/coredynamics.cu:2866-2890): from the value stored
 // at the spike time when the neuron spiked (slot 1), else the step start (slot 0), plus the
 // spike count, decayed over the rest of the step with the cortical E types' tauAvg.
-__device__ __forceinline__ void learn_avg_delivery(const V1Params &P, float postSInfo, int b, int local) {
+__device__ __forceinline__ void learn_avg_delivery(const V1Params &P, float postSInfo, const float *avg0, const float *avg1,
+                                                   float *out) {
     const float dt = P.dt;
     const float postNsp = floorf(postSInfo);
     const float postTsp = postSInfo > 0 ? postSInfo - postNsp : 1.f;
-    const int cPick = postNsp > 0 ? 1 : 0;
-    float *vAvg = P.ffPost + P.ffOffAvgE + 2 * (b * P.nE + local);
-    float lAvgE = vAvg[cPick];
+    float lAvgE = postNsp > 0 ? *avg1 : *avg0;
     float delta_t = dt;
     if (postNsp > 0) delta_t = dt * (1 - postTsp);
     lAvgE += postNsp;
     lAvgE *= expf(-delta_t / P.tauAvgCortical);
-    vAvg[0] = lAvgE;
+    *out = lAvgE;
 }
 
 // Ring slot of step t in the far/near event rings.
@@ -471,7 +470,10 @@ __device__ __forceinline__ void deliver_prev(const V1Params &P, long long tp, in
         neuron_sync();
     }
     if (recNear) P.recNearCount[(size_t)(tp - P.recStep0) * nV1 + i] = nNearDraw;
-    if (P.ffMode && P.ffMode != 3 && active && local < P.nE) learn_avg_delivery(P, __ldcg(sPrev + i), b, local);
+    if (P.ffMode && P.ffMode != 3 && active && local < P.nE) {
+        float *vAvg = P.ffPost + P.ffOffAvgE + 2 * (b * P.nE + local);
+        learn_avg_delivery(P, __ldcg(sPrev + i), vAvg, vAvg + 1, vAvg);
+    }
 #pragma unroll
     for (int ig = 0; ig < kMaxNG; ig++) {
         st.gE[ig] += lgE[ig]; st.hE[ig] += lhE[ig];
@@ -852,6 +854,41 @@ __device__ __forceinline__ float step_neuron(const V1Params &P, long long t, int
     return sInfo;
 }
 
+// Where a neuron's learning variables live: in global memory (per-step kernel), or in shared memory for the
+// K steps of a launch (persistent kernel), with the synapses' weights and ids.
+struct LearnVars {
+    float *ltd, *trip, *avg0, *avg1;   // post traces; filtered rate (avg1: at the spike time, E with learning != 3)
+    float *total, *target;             // total LGN weight and its target
+    float *wts;                        // weights, wStride apart
+    size_t wStride;
+};
+
+// Global places of neuron i's learning variables.
+__device__ __forceinline__ LearnVars learn_vars(const V1Params &P, int i, int local) {
+    const bool isE = local < P.nE;
+    const int nEt = P.nE * P.nblock, nIt = P.nI * P.nblock, b = i / P.blockSize;
+    const int id = isE ? b * P.nE + local : b * P.nI + (local - P.nE);   // eid / iid
+    LearnVars v;
+    v.ltd = (isE ? P.ffPost : P.ffPost + P.ffOffI) + id;
+    v.trip = (isE ? P.ffPost + nEt : P.ffPost + P.ffOffI + nIt) + id;
+    v.avg0 = isE ? P.ffPost + P.ffOffAvgE + 2 * id : P.ffPost + P.ffOffAvgI + id;
+    v.avg1 = v.avg0 + 1;
+    v.total = P.totalFF + i;
+    v.target = P.totalFF + P.nV1 + i;
+    v.wts = P.sLGNw + i;
+    v.wStride = P.nV1;
+    return v;
+}
+
+// Decay factors over a whole step of a type's post traces (the expressions learn_ff evaluates for other
+// intervals).
+struct LearnDecay {
+    float ltd, trip, avg;
+};
+__device__ __forceinline__ LearnDecay learn_decay(const V1Params &P, const FFType &T) {
+    return LearnDecay{expf(-P.dt / T.tauLTD), expf(-P.dt / T.tauTrip), expf(-P.dt / T.tauAvg)};
+}
+
 // LGN->V1 plasticity after the membrane step of neuron i (learning 1-3): the learning block
 // of compute_V_collect_spike_learnFF_fast (src/coredynamics.cu:1631-1993) with one FF->E type
 // for excitatory posts and, with learning 2, one FF->I type for inhibitory posts.  The post
@@ -868,9 +905,21 @@ __device__ __forceinline__ float step_neuron(const V1Params &P, long long t, int
 // presynaptic trace 0 (layer 1 + 3j of the LGN surface with j counting from 0,
 // src/coredynamics.cu:1905-1912), which is the FF->E type's trace when both types learn.
 // Float arithmetic in the reference's order.
-__device__ __noinline__ void learn_ff(const V1Params &P, long long t, int i, int local, int m, float sInfo,
-                                      const float *__restrict__ lgnSInfo, const float *__restrict__ preRow,
-                                      int nLGN) {
+//
+// A warp's instructions bound it: every synapse of every lane in synapse order, with few warps per SM to
+// hide the latency of each.  What a synapse whose cell did not spike shares with the others is computed once
+// (the decay of its trace to tsp), and the words and traces of kLearnChunk synapses are read together (one
+// by one, each waited for its own reads: 15 of the 26 us of a per-step launch).  In the persistent
+// kernel (in: the step's LGN spikes; else null) only the words of cells that spiked are read, and weights, ids and the
+// neuron's variables stay in shared memory for the K steps.  200 steps of 2 x 1,024 neurons with 20
+// synapses: 6,407 us as launches per step, 2,280 us so (2,741 with each synapse's own expf and reads, 2,941
+// with words and traces in registers for all ten synapses' paths: spills).
+constexpr int kLearnChunk = 10;
+constexpr int kLearnVars = 6;   // learning variables a persistent thread keeps in shared memory
+
+__device__ __forceinline__ void learn_ff(const V1Params &P, int i, int local, int m, float sInfo,
+                                         const float *__restrict__ lgnSInfo, const float *__restrict__ preRow, int nLGN,
+                                         const LearnVars &v, const LearnDecay &decay, const LgnIn *in) {
     const bool isE = local < P.nE;
     if (!isE && !P.ffI) return;
     const FFType &T = P.ffT[isE ? 0 : 1];
@@ -883,18 +932,11 @@ __device__ __noinline__ void learn_ff(const V1Params &P, long long t, int i, int
         nsp = 0;
         tsp = dt;
     }
-    const int nV1 = P.nV1;
-    const int nEt = P.nE * P.nblock, nIt = P.nI * P.nblock;
-    const int b = i / P.blockSize;
-    const int id = isE ? b * P.nE + local : b * P.nI + (local - P.nE);   // eid / iid
-    float *vLTD = isE ? P.ffPost : P.ffPost + P.ffOffI;
-    float *vTrip = isE ? P.ffPost + nEt : P.ffPost + P.ffOffI + nIt;
-    float *vAvg = isE ? P.ffPost + P.ffOffAvgE + 2 * id : P.ffPost + P.ffOffAvgI + id;
     // row 0: the step start; row 1: the spike time
     float lLTD[2], lTrip[2], lAvg[2];
-    lLTD[0] = vLTD[id];
-    lTrip[0] = vTrip[id];
-    lAvg[0] = vAvg[0];
+    lLTD[0] = *v.ltd;
+    lTrip[0] = *v.trip;
+    lAvg[0] = *v.avg0;
     lLTD[1] = lTrip[1] = lAvg[1] = 0.f;
     if (nsp > 0) {
         lLTD[1] = lLTD[0];
@@ -903,12 +945,12 @@ __device__ __noinline__ void learn_ff(const V1Params &P, long long t, int i, int
         lTrip[1] *= expf(-tsp / T.tauTrip);
         lAvg[1] = lAvg[0];
         lAvg[1] *= expf(-tsp / T.tauAvg);
-        if (isE && P.ffMode != 3) vAvg[1] = lAvg[1];
+        if (isE && P.ffMode != 3) *v.avg1 = lAvg[1];
     }
     float new0 = 0.f, change = 0.f, delta_f = 0.f;
     if (P.applyHomeo) {
-        const float f0 = P.totalFF[i];
-        const float finf = P.totalFF[nV1 + i];
+        const float f0 = *v.total;
+        const float finf = *v.target;
         const float d = f0 - finf;
         if (d > 0 || P.symmetricHomeo) {
             new0 = d * P.expHomeo + finf;
@@ -918,70 +960,77 @@ __device__ __noinline__ void learn_ff(const V1Params &P, long long t, int i, int
             change = P.applyHomeo == 1 ? 1.f : 0.f;
         }
     }
-    for (int q = 0; q < m; q++) {
-        const size_t lid = (size_t)q * nV1 + i;
-        float f = P.sLGNw[lid];
-        if (f == 0 && !P.rebound) continue;
-        if (P.applyHomeo == 1) f *= change;
-        else if (P.applyHomeo == 2) f += change;
-        const int cell = __ldg(P.lgnId + lid);
-        const float sFF = __ldcg(lgnSInfo + cell);
-        const unsigned nspFF = (unsigned)floorf(sFF);
-        const float tspFF = (sFF > 0 ? sFF - (float)nspFF : 1.f) * dt;
-        if (nspFF > 0) {  // LTD, whether or not the neuron spiked
-            int cPick;
-            float delta_t;
-            if (tspFF < tsp) {
-                cPick = 0;
-                delta_t = tspFF;
-            } else {
-                cPick = 1;
-                delta_t = tspFF - tsp;
+    // the presynaptic trace decays over the same time for every LGN cell that did not spike before the neuron
+    const float eLTP = nsp > 0 ? expf(-tsp / T.tauLTP) : 0.f;
+    for (int q0 = 0; q0 < m; q0 += kLearnChunk) {
+        float sFF[kLearnChunk], lpre[kLearnChunk];
+        auto cell = [&](int q) { return in ? synapse_id(in->ids, q) : __ldg(P.lgnId + (size_t)q * P.nV1 + i); };
+#pragma unroll
+        for (int k = 0; k < kLearnChunk; k++) {
+            const int q = q0 + k;
+            sFF[k] = lpre[k] = 0.f;
+            if (q < m && (!in || (in->mask >> q) & 1u)) sFF[k] = __ldcg(lgnSInfo + cell(q));
+        }
+        if (nsp > 0) {
+#pragma unroll
+            for (int k = 0; k < kLearnChunk; k++)
+                if (q0 + k < m) lpre[k] = __ldcg(preRow + cell(q0 + k));
+        }
+#pragma unroll
+        for (int k = 0; k < kLearnChunk; k++) {
+            const int q = q0 + k;
+            if (q >= m) break;
+            float *w = v.wts + q * v.wStride;
+            float f = *w;
+            if (f == 0 && !P.rebound) continue;
+            if (P.applyHomeo == 1) f *= change;
+            else if (P.applyHomeo == 2) f += change;
+            float pre = lpre[k], e = eLTP;
+            if (sFF[k] > 0) {
+                const float nspFF = floorf(sFF[k]);
+                const float tspFF = (sFF[k] - nspFF) * dt;
+                if (nspFF > 0) {  // LTD, whether or not the neuron spiked
+                    const int cPick = tspFF < tsp ? 0 : 1;
+                    const float delta_t = tspFF < tsp ? tspFF : tspFF - tsp;
+                    float A_LTD = T.A_ratio;
+                    if (T.targetFR > 0) A_LTD *= T.tauLTP * lAvg[cPick] * lAvg[cPick];
+                    const float df = lLTD[cPick] * expf(-delta_t / T.tauLTD) * A_LTD;
+                    f -= df;
+                    if (P.applyHomeo) delta_f -= df;
+                }
+                if (nsp > 0 && tspFF < tsp) {
+                    pre = __ldcg(preRow + nLGN + cell(q));
+                    e = expf(-(tsp - tspFF) / T.tauLTP);
+                }
             }
-            float A_LTD = T.A_ratio;
-            if (T.targetFR > 0) A_LTD *= T.tauLTP * lAvg[cPick] * lAvg[cPick];
-            const float df = lLTD[cPick] * expf(-delta_t / T.tauLTD) * A_LTD;
-            f -= df;
-            if (P.applyHomeo) delta_f -= df;
-        }
-        if (nsp > 0) {  // LTP, whether or not the LGN cell spiked
-            float lpre, delta_t;
-            if (tspFF < tsp) {
-                lpre = __ldcg(preRow + nLGN + cell);
-                delta_t = tsp - tspFF;
-            } else {
-                lpre = __ldcg(preRow + cell);
-                delta_t = tsp;
+            if (nsp > 0) {  // LTP, whether or not the LGN cell spiked
+                const float df = pre * e * lTrip[1] * T.A_LTP;
+                if (P.applyHomeo) delta_f += df;
+                f += df;
             }
-            const float df = lpre * expf(-delta_t / T.tauLTP) * lTrip[1] * T.A_LTP;
-            if (P.applyHomeo) delta_f += df;
-            f += df;
+            if (f < T.gmin) {
+                if (P.applyHomeo) delta_f += T.gmin - f;
+                f = T.gmin;
+            }
+            if (f > T.gmax) {
+                if (P.applyHomeo) delta_f -= f - T.gmax;
+                f = T.gmax;
+            }
+            *w = f;
         }
-        if (f < T.gmin) {
-            if (P.applyHomeo) delta_f += T.gmin - f;
-            f = T.gmin;
-        }
-        if (f > T.gmax) {
-            if (P.applyHomeo) delta_f -= f - T.gmax;
-            f = T.gmax;
-        }
-        P.sLGNw[lid] = f;
     }
-    if (P.applyHomeo) P.totalFF[i] = new0 + delta_f;
+    if (P.applyHomeo) *v.total = new0 + delta_f;
     // the post traces take this step's spikes and decay to its end
-    float delta_t = dt;
-    const int cPick = nsp > 0 ? 1 : 0;
-    if (nsp > 0) delta_t -= tsp;
-    lLTD[cPick] += nsp;
-    lTrip[cPick] += nsp;
-    lLTD[cPick] *= expf(-delta_t / T.tauLTD);
-    lTrip[cPick] *= expf(-delta_t / T.tauTrip);
-    vLTD[id] = lLTD[cPick];
-    vTrip[id] = lTrip[cPick];
-    if (!isE || P.ffMode == 3) {
-        lAvg[cPick] += nsp;
-        lAvg[cPick] *= expf(-delta_t / T.tauAvg);
-        vAvg[0] = lAvg[cPick];
+    const bool avg = !isE || P.ffMode == 3;
+    if (nsp > 0) {
+        const float delta_t = dt - tsp;
+        *v.ltd = (lLTD[1] + nsp) * expf(-delta_t / T.tauLTD);
+        *v.trip = (lTrip[1] + nsp) * expf(-delta_t / T.tauTrip);
+        if (avg) *v.avg0 = (lAvg[1] + nsp) * expf(-delta_t / T.tauAvg);
+    } else {
+        *v.ltd = lLTD[0] * decay.ltd;
+        *v.trip = lTrip[0] * decay.trip;
+        if (avg) *v.avg0 = lAvg[0] * decay.avg;
     }
 }
 
@@ -1458,8 +1507,9 @@ __device__ __forceinline__ void v1_step_body(const V1Params &P, long long t, int
         if (P.spikeCount && sInfo >= 1.0f) P.spikeCount[i] += (unsigned)floorf(sInfo);
         if (P.farPullOn || P.nearPullOn) P.sRing[(size_t)(t % P.sDepth) * P.nV1 + i] = sInfo;
         if (P.ffLearn)
-            learn_ff(P, t, i, local, P.nLGNperV1[i], sInfo, lgnSInfo,
-                     P.ffPreRing + (size_t)(t % lgnSlots) * P.ffTypes * 2 * P.lgnN, P.lgnN);
+            learn_ff(P, i, local, P.nLGNperV1[i], sInfo, lgnSInfo,
+                     P.ffPreRing + (size_t)(t % lgnSlots) * P.ffTypes * 2 * P.lgnN, P.lgnN, learn_vars(P, i, local),
+                     learn_decay(P, P.ffT[local < P.nE ? 0 : 1]), nullptr);
     }
     if (P.farOn) {
         const int e0 = active ? P.farOff[i] : 0;
@@ -1801,8 +1851,9 @@ __device__ __forceinline__ void push_own(const V1Params &P, long long t, int tSl
 // kCta are push warps.  dyn: LGN weights and ids [mRows][kCta] each (mRows a multiple of 4), then two
 // rows of LGN spike bits of bitRoom words (0: the bits are read from global memory).  General:
 // patches with more than mRows LGN synapses or with several spikes per step are accepted too.
-// False if a barrier gave up.
-template <bool Rng, bool General>
+// Learn: with LGN->V1 plasticity (the weights change in shared memory and go back at the end).  False if a
+// barrier gave up.
+template <bool Rng, bool General, bool Learn>
 __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0, int steps, int cta, int nCta, int csize,
                                                  const float *__restrict__ lgnRing, const unsigned *__restrict__ lgnBits,
                                                  int lgnSlots, bool deliverFirst, unsigned *barrier, PShared &sm,
@@ -1861,7 +1912,7 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
     if (smemSyn) {
         for (int q = 0; q < rows; q++) {
             reinterpret_cast<int *>(smI + (q >> 2) * kCta)[q & 3] = q < m ? __ldg(P.lgnId + (size_t)q * P.nV1 + i) : 0;
-            if (q < m) smW[q * kCta] = __ldg(P.sLGN + (size_t)q * P.nV1 + i);
+            if (q < m) smW[q * kCta] = __ldcg(P.sLGN + (size_t)q * P.nV1 + i);
         }
     }
     // far events of step t0 - 1 that a per-step launch (or the initial spikes) left to push
@@ -1875,7 +1926,7 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
     const TypeConst &tc = sm.type[itype];
     if (list && threadIdx.x < 2 * (kMaxBS / 32)) sm.list.ball[threadIdx.x >> 5][threadIdx.x & 31] = 0u;
     cta_sync();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && barrier) {
         __threadfence();
         // the last CTA to arrive: everyone has read the list that was left
         if (atomicAdd(barrier, 1u) + 1u == (unsigned)nCta && P.farOn)
@@ -1896,6 +1947,27 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
     int recSlot = rec ? (int)(t0 % P.recSlots) : 0, recPrev = rec ? (int)((t0 + P.recSlots - 1) % P.recSlots) : 0;
     FFStep ff;
     bool ok = true;
+    float sLast = 0.f;   // the spike word of the step before (Learn)
+    // this neuron's learning variables in shared memory behind the spike bits, one column per thread
+    LearnVars lv;
+    LearnDecay decay;
+    if constexpr (Learn) {
+        float *col = dyn + (size_t)2 * mRows * kCta + 2 * bitRoom + threadIdx.x;
+        lv = LearnVars{col, col + kCta, col + 2 * kCta, col + 3 * kCta, col + 4 * kCta, col + 5 * kCta, smW, kCta};
+        decay = learn_decay(P, P.ffT[isE ? 0 : 1]);
+        if (active && (isE || P.ffI)) {
+            const LearnVars g = learn_vars(P, i, local);
+            if (P.ffLearn) {
+                *lv.ltd = *g.ltd;
+                *lv.trip = *g.trip;
+                *lv.total = *g.total;
+                *lv.target = *g.target;
+            }
+            *lv.avg0 = *g.avg0;
+            if (isE) *lv.avg1 = *g.avg1;
+        }
+    }
+    if constexpr (Learn) sLast = active && deliverFirst ? __ldcg(P.sInfo + (size_t)((t0 - 1) & 1) * P.nV1 + i) : 0.f;
     for (int s = 0; s < steps; s++) {
         const long long t = t0 + s;
         const int par = (int)(t & 1);
@@ -1930,6 +2002,9 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
             }
             if (active) in = lgn_spikes(bits, lgnSInfo, smI, smW, m, rows >> 2);
         }
+        if constexpr (Learn) {   // the filtered rate of learning 1, 2 and 4, advanced over step t - 1
+            if (list && dl && P.ffMode != 3 && active && isE) learn_avg_delivery(P, sLast, lv.avg0, lv.avg1, lv.avg0);
+        }
         if (list && dl)
             deliver_list<Rng>(P, tc, t - 1, b, local, i, active, itype, st, condState, sm.list.unit[par ^ 1],
                               sm.list.ball[par ^ 1]);
@@ -1944,7 +2019,7 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
         // neighbour list they come after the barrier
         const bool ffEarly = list || !dl;
         if (ffEarly) feed_forward();
-        if (s > 0 && nCta > 1 && (coupled || s == 1)) {
+        if (s > 0 && nCta > 1 && barrier && (coupled || s == 1)) {
             const unsigned target = (unsigned)nCta * (coupled ? (unsigned)(s + 1) : 1u);
             if (!barrier_wait(barrier, target, sm, P.err, P.waitSpins)) {
                 ok = false;
@@ -1979,6 +2054,12 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
             sInfo = step_multi<Rng>(P, t, i, itype, tonic, depC, m, lgnSInfo, st, condState, noisyState);
         const bool spk = active && sInfo >= 1.0f;
         if (list && s + 1 < steps) publish_spikes(P, sm, par, csize, rank, spk, sInfo, isE);
+        if constexpr (Learn) {
+            sLast = sInfo;
+            if (active && P.ffLearn)
+                learn_ff(P, i, local, m, sInfo, lgnSInfo, P.ffPreRing + (size_t)lgnSlot * P.ffTypes * 2 * P.lgnN, P.lgnN, lv,
+                         decay, &in);
+        }
         // a neuron that enters the last tenth below its threshold will likely spike some steps from now:
         // what its delivery and its same-step push wait for is then already in L2
         if (active && !spk) {
@@ -2017,6 +2098,20 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
         if (++fsT == P.farDepth) fsT = 0;
         t3 = t3 == 2 ? 0 : t3 + 1;
     }
+    if constexpr (Learn) {
+        if (active && P.ffLearn)
+            for (int q = 0; q < m; q++) P.sLGNw[(size_t)q * P.nV1 + i] = smW[q * kCta];
+        if (active && (isE || P.ffI)) {
+            const LearnVars g = learn_vars(P, i, local);
+            if (P.ffLearn) {
+                *g.ltd = *lv.ltd;
+                *g.trip = *lv.trip;
+                *g.total = *lv.total;
+            }
+            *g.avg0 = *lv.avg0;
+            if (isE) *g.avg1 = *lv.avg1;
+        }
+    }
     if (active) {
         store_state(P, i, st);
         if (!(General && P.multiSpike)) P.dep[i] = ff.depOut;
@@ -2035,7 +2130,7 @@ __device__ __forceinline__ int cluster_ctas() {
 }
 
 // K steps of one patch in one cooperative launch.
-template <bool Rng>
+template <bool Rng, bool Learn>
 __global__ void __launch_bounds__(2 * kCta, 1) v1_persistent_kernel(V1Params P, const long long *stepBase, int K,
                                                                     const float *__restrict__ lgnRing,
                                                                     const unsigned *__restrict__ lgnBits, int lgnSlots,
@@ -2045,7 +2140,7 @@ __global__ void __launch_bounds__(2 * kCta, 1) v1_persistent_kernel(V1Params P, 
     Phases ph;
     const int csize = cluster_ctas();
     init_barriers(sm, csize);
-    persistent_steps<Rng, false>(P, *stepBase, K, blockIdx.x, gridDim.x, csize, lgnRing, lgnBits, lgnSlots,
+    persistent_steps<Rng, false, Learn>(P, *stepBase, K, blockIdx.x, gridDim.x, csize, lgnRing, lgnBits, lgnSlots,
                                  deliverFirst != 0, barrier, sm, ph, lgnSm, (P.maxLGN + 3) & ~3, bitRoom);
 }
 
@@ -2406,11 +2501,11 @@ cudaError_t launch_v1_step(const V1Params &p, const long long *stepBase, int ste
     return cudaGetLastError();
 }
 
-// A cooperative launch of `grid` CTAs in clusters of csize.
+// A launch of `grid` CTAs in clusters of csize, cooperative or not.
 struct CoopLaunch {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
-    CoopLaunch(int grid, int threads, size_t smem, int csize, cudaStream_t st) {
+    CoopLaunch(int grid, int threads, size_t smem, int csize, cudaStream_t st, bool coop = true) {
         cfg.gridDim = dim3(grid);
         cfg.blockDim = dim3(threads);
         cfg.dynamicSmemBytes = smem;
@@ -2421,8 +2516,8 @@ struct CoopLaunch {
         attr[1].val.clusterDim.x = csize;
         attr[1].val.clusterDim.y = 1;
         attr[1].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = csize > 1 ? 2 : 1;
+        cfg.attrs = coop ? attr : attr + 1;
+        cfg.numAttrs = (coop ? 1 : 0) + (csize > 1 ? 1 : 0);
     }
 };
 
@@ -2431,9 +2526,7 @@ template <class Kern>
 static int resident_ctas(Kern kern, int threads, size_t smem, int csize, int device) {
     int n = 0;
     if (csize > 1) {
-        CoopLaunch cl(csize, threads, smem, csize, nullptr);
-        cl.cfg.attrs = cl.attr + 1;
-        cl.cfg.numAttrs = 1;
+        CoopLaunch cl(csize, threads, smem, csize, nullptr, false);
         if (cudaOccupancyMaxActiveClusters(&n, kern, &cl.cfg) != cudaSuccess) {
             cudaGetLastError();
             return 0;
@@ -2453,7 +2546,14 @@ static int resident_ctas(Kern kern, int threads, size_t smem, int csize, int dev
 // two rows of LGN spike bits.
 static int v1_persistent_bits(const V1Params &p) { return p.lgnW <= kMaxBitWords ? p.lgnW : 0; }
 static size_t v1_persistent_smem(const V1Params &p) {
-    return ((size_t)2 * ((p.maxLGN + 3) & ~3) * kCta + 2 * v1_persistent_bits(p)) * sizeof(float);
+    return ((size_t)2 * ((p.maxLGN + 3) & ~3) * kCta + 2 * v1_persistent_bits(p) + (p.ffMode ? kLearnVars * kCta : 0)) *
+           sizeof(float);
+}
+
+using PersistentKernel = void (*)(V1Params, const long long *, int, const float *, const unsigned *, int, int, unsigned *, int);
+static PersistentKernel persistent_kernel(const V1Params &p) {
+    if (p.ffMode) return needs_rng(p) ? v1_persistent_kernel<true, true> : v1_persistent_kernel<false, true>;
+    return needs_rng(p) ? v1_persistent_kernel<true, false> : v1_persistent_kernel<false, false>;
 }
 
 // The shape of the persistent launch: a block's CTAs as a cluster, with push warps when there are
@@ -2465,15 +2565,16 @@ bool v1_persistent_shape(const V1Params &p, int device, int *cluster, int *threa
     int coop = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
     if (!coop || p.maxLGN > kMaxLgnReg) return false;
-    const int maxDyn = (int)(((size_t)2 * kMaxLgnReg * kCta + 2 * kMaxBitWords) * sizeof(float));
-    cudaFuncSetAttribute(v1_persistent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxDyn);
-    cudaFuncSetAttribute(v1_persistent_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxDyn);
+    const int maxDyn = (int)(((size_t)2 * kMaxLgnReg * kCta + 2 * kMaxBitWords + kLearnVars * kCta) * sizeof(float));
+    const PersistentKernel kern = persistent_kernel(p);
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, maxDyn) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
     const size_t dyn = v1_persistent_smem(p);
     const int shapes[3][2] = {{nq, 2 * kCta}, {nq, kCta}, {1, kCta}};
     for (int k = p.farOn ? 0 : 1; k < 3; k++) {
-        const int fit = needs_rng(p) ? resident_ctas(v1_persistent_kernel<true>, shapes[k][1], dyn, shapes[k][0], device)
-                                     : resident_ctas(v1_persistent_kernel<false>, shapes[k][1], dyn, shapes[k][0], device);
-        if (fit < n) continue;
+        if (resident_ctas(kern, shapes[k][1], dyn, shapes[k][0], device) < n) continue;
         *cluster = shapes[k][0];
         *threads = shapes[k][1];
         return true;
@@ -2485,11 +2586,13 @@ cudaError_t launch_v1_persistent(const V1Params &p, const long long *stepBase, i
                                  const unsigned *lgnBits, int lgnSlots, int deliverFirst, unsigned *barrier,
                                  cudaStream_t st) {
     const int nq = (p.blockSize + kCta - 1) / kCta;
-    CoopLaunch cl(p.nblock * nq, p.threads, v1_persistent_smem(p), p.cluster, st);
-    cudaError_t e = cudaMemsetAsync(barrier, 0, sizeof(unsigned), st);
-    if (e != cudaSuccess) return e;
-    return cudaLaunchKernelEx(&cl.cfg, needs_rng(p) ? v1_persistent_kernel<true> : v1_persistent_kernel<false>, p, stepBase,
-                              K, lgnRing, lgnBits, lgnSlots, deliverFirst, barrier, v1_persistent_bits(p));
+    CoopLaunch cl(p.nblock * nq, p.threads, v1_persistent_smem(p), p.cluster, st, barrier != nullptr);
+    if (barrier) {
+        const cudaError_t e = cudaMemsetAsync(barrier, 0, sizeof(unsigned), st);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaLaunchKernelEx(&cl.cfg, persistent_kernel(p), p, stepBase, K, lgnRing, lgnBits, lgnSlots, deliverFirst,
+                              barrier, v1_persistent_bits(p));
 }
 
 cudaError_t launch_v1_rng_init(curandStateMRG32k3a *cond, curandStateMRG32k3a *noisy,
@@ -2583,7 +2686,7 @@ __global__ void __launch_bounds__(kCta, 2) v1_batch_persistent_kernel(const Batc
         const int steps = left < K ? (int)left : K;
         if (steps <= 0) continue;
         // a trial whose barrier gave up ends the slot: its cluster's CTAs leave it a step apart
-        if (!persistent_steps<Rng, General>(sT.v, t0, steps, c, sT.nCta, csize, sT.lgnRing, sT.lgnBits, sT.lgnSlots,
+        if (!persistent_steps<Rng, General, false>(sT.v, t0, steps, c, sT.nCta, csize, sT.lgnRing, sT.lgnBits, sT.lgnSlots,
                                             t0 >= sT.tDeliverFrom, barriers + q, sm, ph, dyn, kBatchLgn, kBatchBits))
             return;
     }
