@@ -18,10 +18,9 @@
 // Adding the previous step's delivery before this step's decay is the same sequence of
 // float operations as the reference's separate kernels.
 //
-// Two kernels run these phases: v1_step_kernel does one step per launch (state in HBM), and
-// v1_persistent_kernel runs K steps in one cooperative launch with the neuron state, the
-// LGN synapse ids and the generators held in registers and a bounded grid barrier between
-// steps.  Both are instantiated with and without the random-number paths (noise, synaptic
+// v1_step_kernel runs these phases one step per launch (state in HBM).  v1_persistent_kernel and, for the
+// trials of a sweep, v1_batch_persistent_kernel run K steps in one launch with the neuron state and the
+// generators in registers and the LGN synapses in shared memory.  All are instantiated with and without the random-number paths (noise, synaptic
 // failure); the host picks the variant.  Per-species arrays use compile-time indices so that
 // they stay in registers.
 #include <algorithm>
@@ -1550,15 +1549,17 @@ __global__ void __launch_bounds__(kCta) v1_step_kernel(V1Params P, const long lo
 //     bulk-copy engine; a neuron tests the bits of its synapses and reads the words of those that
 //     spiked (the words of all of them, 20 scattered copies per thread and step, took 1,850 cycles
 //     of an 11,000-cycle step).
-//   * the later far events of a spike only have to be in the ring one barrier later: the CTA's
-//     spikers are listed in shared memory and pushed by kCta further threads of the CTA (push
-//     warps) during the next step, or by the neuron threads themselves between arrival and
-//     wait where the registers do not allow the extra warps.
+//   * the far pushes.  The CTA's spikers are listed in shared memory for kCta further threads of the
+//     CTA (push warps): they push the same-step events, arrive at the grid barrier and then push the later
+//     events, while the neuron threads are in the next step (waiting for their own pushes and the
+//     release behind them, the neuron threads lost 2,300 of an 18,600-cycle step of 32 blocks).  Where the registers do
+//     not allow the extra warps (two CTAs per SM) the neuron threads push themselves, between arrival and
+//     wait.
 // Bound by the latency of one warp's instruction stream (two warps per scheduler).  Measured per
 // call, against general CTAs with a full grid barrier per step and LGN words per synapse: one block
-// 800 steps 5,715 -> 3,541 us, 4 blocks with noise and failures 301 steps 3,151 -> 2,076, 8 blocks
-// with far synapses 203 steps 2,261 -> 1,863, the 32-block patch with its movie 800 steps 13,193 ->
-// 11,433; 12 trials of 4 blocks in one sweep 29,755 -> 25,952.
+// 800 steps 5,715 -> 3,380 us, 4 blocks with noise and failures 301 steps 3,151 -> 1,990, 8 blocks
+// with far synapses 203 steps 2,261 -> 1,636, the 32-block patch with its movie 800 steps 13,400 ->
+// 10,320; 12 trials of 4 blocks in one sweep 29,755 -> 21,660.
 constexpr unsigned kBarrierAbort = 0x80000000u;
 constexpr int kPushU = 2;       // far items a lane fetches together
 constexpr int kMaxBitWords = 2048;   // LGN spike bits kept in shared memory (two rows of up to 65,536 cells)
@@ -1614,7 +1615,7 @@ struct __align__(16) PShared {
     TypeConst type[kMaxType];
     // this CTA's far spikers, by parity of the step
     int cnt[2];
-    int e0[2][kCta], deg[2][kCta];
+    int e0[2][kCta], deg[2][kCta], n1[2][kCta];
     float si[2][kCta];
     unsigned char preE[2][kCta];
     unsigned peerFail;
@@ -1834,15 +1835,17 @@ __device__ __forceinline__ void deliver_list(const V1Params &P, const TypeConst 
     if (Rng && recNear) P.recNearCount[(size_t)(tp - P.recStep0) * P.nV1 + i] = nDraw;
 }
 
-// The later far events of the CTA's spikers of step t (list of its parity), by nWarps warps.
+// The later (or, sameStep, the same-step) far events of the CTA's spikers of step t (list of its parity),
+// by nWarps warps.
 __device__ __forceinline__ void push_own(const V1Params &P, long long t, int tSlot, const PShared &sm, int par, int part,
-                                         int nWarps) {
+                                         int nWarps, bool sameStep = false) {
     const int n = sm.cnt[par], lane = threadIdx.x & 31;
     for (int c0 = 0; c0 < n; c0 += 32) {
         const int q = c0 + lane;
         const bool in = q < n;
-        push_spikers<kPushU>(P, t, tSlot, in ? sm.e0[par][q] : 0, in ? sm.deg[par][q] : 0, in ? sm.si[par][q] : 1.f,
-                             in && sm.preE[par][q], false, part, nWarps);
+        push_spikers<kPushU>(P, t, tSlot, in ? sm.e0[par][q] : 0,
+                             in ? (sameStep ? sm.n1 : sm.deg)[par][q] : 0, in ? sm.si[par][q] : 1.f,
+                             in && sm.preE[par][q], sameStep, part, nWarps);
     }
 }
 
@@ -1853,7 +1856,7 @@ __device__ __forceinline__ void push_own(const V1Params &P, long long t, int tSl
 // patches with more than mRows LGN synapses or with several spikes per step are accepted too.
 // Learn: with LGN->V1 plasticity (the weights change in shared memory and go back at the end).  False if a
 // barrier gave up.
-template <bool Rng, bool General, bool Learn>
+template <bool Rng, bool General, bool Learn, bool Push>
 __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0, int steps, int cta, int nCta, int csize,
                                                  const float *__restrict__ lgnRing, const unsigned *__restrict__ lgnBits,
                                                  int lgnSlots, bool deliverFirst, unsigned *barrier, PShared &sm,
@@ -1861,23 +1864,44 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
     const int bs = P.blockSize;
     const int nq = (bs + kCta - 1) / kCta;
     const int b = cta / nq, rank = cta % nq;
-    const bool pushWarps = blockDim.x > kCta;
+    const bool pushWarps = Push && blockDim.x > kCta;
     const bool list = P.noDelay && P.nearSelf && csize == nq;
     const bool coupled = P.farOn || (P.noDelay && !list);
     auto cta_sync = [&]() {
         if (pushWarps) asm volatile("bar.sync 0, %0;" ::"n"(2 * kCta) : "memory");
         else neuron_sync();
     };
-    if (threadIdx.x >= kCta) {
+    // The push warps also push a step's same-step events and arrive at the grid barrier, and the neuron
+    // threads do not wait for that: they go on with the next step up to the grid barrier, behind which the push
+    // warps have let go of the lists of step s - 1.
+    const bool handoff = pushWarps && coupled && list && nCta > 1;
+    auto hand_over = [&]() {
+        if (handoff) asm volatile("bar.arrive 2, %0;" ::"n"(2 * kCta) : "memory");
+        else if (pushWarps) cta_sync();
+    };
+    if (pushWarps && threadIdx.x >= kCta) {
         // push warps: one CTA barrier per step hands over the step's spikers
         int slot = far_ring_slot(P, t0);
         const int part = (threadIdx.x - kCta) >> 5;
         cta_sync();
         if (list && csize > 1) cluster_sync();
         for (int s = 0; s < steps; s++) {
-            cta_sync();
+            const int par = (int)((t0 + s) & 1);
+            if (handoff) asm volatile("bar.sync 2, %0;" ::"n"(2 * kCta) : "memory");
+            else cta_sync();
             if (sm.abortStep == s) break;
-            push_own(P, t0 + s, slot, sm, (int)((t0 + s) & 1), part, kWarps);
+            if (handoff) {
+                if (sm.cnt[par] > 0) {
+                    push_own(P, t0 + s, slot, sm, par, part, kWarps, true);
+                    asm volatile("bar.sync 3, %0;" ::"n"(kCta) : "memory");
+                }
+                if (threadIdx.x == kCta) {
+                    sm.cnt[par ^ 1] = 0;
+                    if (s + 1 < steps)
+                        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(barrier) : "memory");
+                }
+            }
+            push_own(P, t0 + s, slot, sm, par, part, kWarps);
             if (++slot == P.farDepth) slot = 0;
         }
         return true;
@@ -1980,7 +2004,7 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
             if (sm.peerFail) {   // a CTA of the block gave up: all of them leave here
                 ok = false;
                 if (threadIdx.x == 0) sm.abortStep = s;
-                if (pushWarps) cta_sync();
+                hand_over();
                 break;
             }
         } else if (!coupled) {
@@ -2030,7 +2054,7 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
                     wait_spikes(sm, par, ph);
                 }
                 if (threadIdx.x == 0) sm.abortStep = s;
-                if (pushWarps) cta_sync();
+                hand_over();
                 break;
             }
         }
@@ -2072,15 +2096,19 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
                 const int q = atomicAdd(&sm.cnt[par], 1);
                 sm.e0[par][q] = farE0;
                 sm.deg[par][q] = farDeg;
+                sm.n1[par][q] = farN1;
                 sm.si[par][q] = sInfo;
                 sm.preE[par][q] = isE;
             }
-            far_same_step(P, t, t3, fsT, spk, sInfo, isFarPre, isE, farE0, farN1, cta == 0 && threadIdx.x == 0);
+            far_same_step(P, t, t3, fsT, spk, sInfo, isFarPre, isE, farE0, handoff ? 0 : farN1,
+                          cta == 0 && threadIdx.x == 0);
         }
         // spike words other CTAs read in the next step (general neighbour lists) come before the arrival
         const bool storeFirst = !list || (General && P.multiSpike);
         if (storeFirst && active && !(General && P.multiSpike)) store_step(P, t, i, sInfo, ff.depOut, st, recSlot);
-        if (coupled) {
+        if (handoff) {
+            hand_over();
+        } else if (coupled) {
             cta_sync();
             if (threadIdx.x == 0) {
                 sm.cnt[par ^ 1] = 0;   // pushed: step t + 1's spikers go there
@@ -2140,7 +2168,7 @@ __global__ void __launch_bounds__(2 * kCta, 1) v1_persistent_kernel(V1Params P, 
     Phases ph;
     const int csize = cluster_ctas();
     init_barriers(sm, csize);
-    persistent_steps<Rng, false, Learn>(P, *stepBase, K, blockIdx.x, gridDim.x, csize, lgnRing, lgnBits, lgnSlots,
+    persistent_steps<Rng, false, Learn, true>(P, *stepBase, K, blockIdx.x, gridDim.x, csize, lgnRing, lgnBits, lgnSlots,
                                  deliverFirst != 0, barrier, sm, ph, lgnSm, (P.maxLGN + 3) & ~3, bitRoom);
 }
 
@@ -2686,7 +2714,7 @@ __global__ void __launch_bounds__(kCta, 2) v1_batch_persistent_kernel(const Batc
         const int steps = left < K ? (int)left : K;
         if (steps <= 0) continue;
         // a trial whose barrier gave up ends the slot: its cluster's CTAs leave it a step apart
-        if (!persistent_steps<Rng, General, false>(sT.v, t0, steps, c, sT.nCta, csize, sT.lgnRing, sT.lgnBits, sT.lgnSlots,
+        if (!persistent_steps<Rng, General, false, false>(sT.v, t0, steps, c, sT.nCta, csize, sT.lgnRing, sT.lgnBits, sT.lgnSlots,
                                             t0 >= sT.tDeliverFrom, barriers + q, sm, ph, dyn, kBatchLgn, kBatchBits))
             return;
     }
