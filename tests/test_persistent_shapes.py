@@ -108,3 +108,36 @@ def test_plasticity_in_the_persistent_kernel(native, mode, homeo, name):
     assert np.abs(ref["sLGN"] - np.asarray(wl.net.sLGN, np.float32).ravel()).max() > (1e-4 if mode != 4 else -1)
     _same(ref, _run(wl, [True], chunks, learning))
     _same(ref, _run(wl, [True, False], chunks, learning))
+
+
+@pytest.mark.parametrize("n,nblock,dur", [(22, 2, (5.0, 20.0)), (2, 3, (4.0, 9.0))])
+def test_sweep_with_push_warps(native, n, nblock, dur):
+    """Trials with far synapses take turns on the slots of the kernel with push warps (one CTA per SM), or have
+    one each: every trial ends as it does alone."""
+    from visual_cortex_gb300 import synth
+    from visual_cortex_gb300.batch import Batch
+    from visual_cortex_gb300.model import Simulation
+    trials = synth.batch_trials(n_trials=n, nblock=nblock, n_lgn=512, width=64, height=64, nFrame=60, far_partners=60,
+                                dur_ms=dur, seed=3)
+    make = lambda wl: Simulation(wl.spec, wl.net, wl.lgn, wl.stim, wl.init, wl.seeds)
+    batched = [make(tr.wl) for tr in trials]
+    try:
+        b = Batch(batched, [tr.steps for tr in trials], autotune=False)
+        try:
+            if n < 8:
+                b.run(max_steps=20)
+            assert b.sweep() > 0
+        finally:
+            b.close()
+        for q, tr in enumerate(trials):
+            alone = make(tr.wl)
+            try:
+                alone.persistent(0)
+                alone.run(tr.steps)
+                for k in ("v", "w", "tBack", "gE", "hE", "gI", "hI", "gFF", "hFF"):
+                    np.testing.assert_array_equal(batched[q].state(k), alone.state(k), err_msg=f"trial {q} {k}")
+            finally:
+                alone.close()
+    finally:
+        for s in batched:
+            s.close()

@@ -39,6 +39,7 @@ struct pv1_batch {
     int *dActive = nullptr, *dNActive = nullptr;   // active trial list (persistent variant)
     unsigned *dBar = nullptr;                      // per-trial barrier counters
     int slotCtas = 0, nSlots = 0, csize = 1;       // persistent variant: CTAs per slot, slots, CTAs per cluster
+    int nPush = 0;                                 // slots of its form with push warps, one CTA per SM (0: not used)
     int totalTiles = 0;
     int maxCellCtas = 0;
     bool allClass = true;
@@ -119,6 +120,13 @@ int refresh_tiles(pv1_batch *b) {
     return PV1_OK;
 }
 
+// A step of the persistent form with push warps (one CTA per SM, fewer slots) over a step of the form
+// without (two CTAs per SM where the slots need it).  A sweep takes the form whose longest slot ends first.
+// Measured per step with far synapses: trials of 4 blocks 7.2 against 9.5 us (4 trials), 7.5 against 9.9 (9), and
+// where the plain form doubles up 7.5 against 10.6 (12 trials) to 11.2 (18); of 2 blocks 7.3 against 8.7 (18)
+// and 10.4 (36); of 8 blocks 7.7 against 10.5 (4) and 11.7 (8).
+constexpr double kPushStep = 0.7;
+
 // One chunk of k steps for every active trial, on the batch stream (direct or under capture).
 int issue(pv1_batch *b, int k, int minB, long long *launches) {
     long long n = 0;
@@ -136,8 +144,10 @@ int issue(pv1_batch *b, int k, int minB, long long *launches) {
         }
     }
     if (minB == 0) {
-        e = launch_v1_batch_persistent(b->dT, b->dActive, b->dNActive, b->slotCtas, b->nSlots, k, b->dBar, b->n,
-                                       b->rng, b->general, b->csize, b->stream);
+        // with push warps where every trial still finds a slot: the slots run once per chunk
+        const bool push = b->nPush >= b->n;
+        e = launch_v1_batch_persistent(b->dT, b->dActive, b->dNActive, b->slotCtas, push ? b->nPush : b->nSlots, k, b->dBar,
+                                       b->n, b->rng, b->general, push, b->csize, b->stream);
         if (e != cudaSuccess) return bfail(b, PV1_E_CUDA, std::string("v1 batch persistent: ") + cudaGetErrorString(e));
         n += 1;
     } else {
@@ -273,12 +283,16 @@ int pv1_batch_create(pv1_plan *const *plans, uint32_t nTrials, const uint64_t *t
     b->csize = (b->hT[0].v.blockSize + 255) / 256;
     for (int q = 1; q < b->n; q++)
         if ((b->hT[q].v.blockSize + 255) / 256 != b->csize) b->csize = 1;
-    int cap = v1_batch_persistent_capacity(b->rng, b->general, b->device, b->csize);
+    int cap = v1_batch_persistent_capacity(b->rng, b->general, false, b->device, b->csize);
     if (b->csize > 1 && cap < b->slotCtas) {
         b->csize = 1;
-        cap = v1_batch_persistent_capacity(b->rng, b->general, b->device, 1);
+        cap = v1_batch_persistent_capacity(b->rng, b->general, false, b->device, 1);
     }
     b->nSlots = b->slotCtas > 0 ? std::min(cap / b->slotCtas, b->n) : 0;
+    bool far = true;
+    for (int q = 0; q < b->n; q++) far = far && b->hT[q].v.farOn;
+    if (far && b->nSlots > 0)
+        b->nPush = std::min(v1_batch_persistent_capacity(b->rng, b->general, true, b->device, b->csize) / b->slotCtas, b->n);
     if (b->nSlots > 0) b->minB = 0;
     PV1_BCUDA(b, cudaStreamSynchronize(b->stream));
     return refresh_tiles(b);
@@ -460,19 +474,26 @@ int pv1_batch_sweep(pv1_batch *b, float *ms) {
     std::vector<int> order(b->n);
     for (int q = 0; q < b->n; q++) order[q] = q;
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return left[x] > left[y]; });
-    std::vector<std::vector<int>> per(b->nSlots);
-    std::vector<long long> load(b->nSlots, 0);
-    for (int q : order) {
-        if (!left[q]) continue;
-        const int sl = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-        per[sl].push_back(q);
-        load[sl] += left[q];
-    }
-    size_t depth = 0;
-    for (auto &v : per) depth = std::max(depth, v.size());
-    std::vector<int> list(depth * b->nSlots, -1);
-    for (int sl = 0; sl < b->nSlots; sl++)
-        for (size_t k = 0; k < per[sl].size(); k++) list[k * b->nSlots + sl] = per[sl][k];
+    auto schedule = [&](int nSlots, std::vector<int> &list) {
+        std::vector<std::vector<int>> per(nSlots);
+        std::vector<long long> load(nSlots, 0);
+        for (int q : order) {
+            if (!left[q]) continue;
+            const int sl = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+            per[sl].push_back(q);
+            load[sl] += left[q];
+        }
+        size_t depth = 0;
+        for (auto &v : per) depth = std::max(depth, v.size());
+        list.assign(depth * nSlots, -1);
+        for (int sl = 0; sl < nSlots; sl++)
+            for (size_t k = 0; k < per[sl].size(); k++) list[k * nSlots + sl] = per[sl][k];
+        return *std::max_element(load.begin(), load.end());
+    };
+    std::vector<int> list, listPush;
+    const long long steps = schedule(b->nSlots, list);
+    const bool push = b->nPush > 0 && kPushStep * (double)schedule(b->nPush, listPush) <= (double)steps;
+    if (push) list.swap(listPush);
     const int nList = (int)list.size();
     BatchTrial *dTs = nullptr;
     BatchLgn *dLs = nullptr;
@@ -503,8 +524,8 @@ int pv1_batch_sweep(pv1_batch *b, float *ms) {
     if (e == cudaSuccess) {
         cudaError_t e1 = launch_lgn_class_batch(dLs, b->n, b->maxCellCtas, (int)maxLeft, b->stream);
         if (e1 == cudaSuccess)
-            e1 = launch_v1_batch_persistent(dTs, dList, dNList, b->slotCtas, b->nSlots, (int)maxLeft, b->dBar, b->n,
-                                            b->rng, b->general, b->csize, b->stream);
+            e1 = launch_v1_batch_persistent(dTs, dList, dNList, b->slotCtas, push ? b->nPush : b->nSlots, (int)maxLeft,
+                                            b->dBar, b->n, b->rng, b->general, push, b->csize, b->stream);
         if (e1 == cudaSuccess) e1 = launch_batch_advance(dTs, b->n, (int)maxLeft, b->dSimTime, b->stream);
         cudaError_t e2 = cudaStreamEndCapture(b->stream, &g);
         e = e1 != cudaSuccess ? e1 : e2;

@@ -444,10 +444,10 @@ int v1_batch_regs(int minB, bool rng);
 // Batched trials in one cooperative launch per chunk (slots of slotCtas CTAs in clusters of csize,
 // per-trial barriers).
 bool v1_batch_general(const V1Params &p);
-int v1_batch_persistent_capacity(bool rng, bool general, int device, int csize);
+int v1_batch_persistent_capacity(bool rng, bool general, bool push, int device, int csize);
 cudaError_t launch_v1_batch_persistent(const BatchTrial *trials, const int *activeList, const int *nActive,
                                        int slotCtas, int nSlots, int K, unsigned *barriers, int nTrials, bool rng,
-                                       bool general, int csize, cudaStream_t st);
+                                       bool general, bool push, int csize, cudaStream_t st);
 
 // Fixed-point scale for far-delivery accumulation: integer adds are associative, so the
 // sum of events does not depend on their order and runs are reproducible.

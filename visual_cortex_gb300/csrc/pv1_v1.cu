@@ -1559,7 +1559,7 @@ __global__ void __launch_bounds__(kCta) v1_step_kernel(V1Params P, const long lo
 // call, against general CTAs with a full grid barrier per step and LGN words per synapse: one block
 // 800 steps 5,715 -> 3,380 us, 4 blocks with noise and failures 301 steps 3,151 -> 1,990, 8 blocks
 // with far synapses 203 steps 2,261 -> 1,636, the 32-block patch with its movie 800 steps 13,400 ->
-// 10,320; 12 trials of 4 blocks in one sweep 29,755 -> 21,660.
+// 10,320; 12 trials of 4 blocks in one sweep 29,755 -> 16,170.
 constexpr unsigned kBarrierAbort = 0x80000000u;
 constexpr int kPushU = 2;       // far items a lane fetches together
 constexpr int kMaxBitWords = 2048;   // LGN spike bits kept in shared memory (two rows of up to 65,536 cells)
@@ -1877,7 +1877,7 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
     const bool handoff = pushWarps && coupled && list && nCta > 1;
     auto hand_over = [&]() {
         if (handoff) asm volatile("bar.arrive 2, %0;" ::"n"(2 * kCta) : "memory");
-        else if (pushWarps) cta_sync();
+        else if (pushWarps && coupled) cta_sync();
     };
     if (pushWarps && threadIdx.x >= kCta) {
         // push warps: one CTA barrier per step hands over the step's spikers
@@ -1885,11 +1885,11 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
         const int part = (threadIdx.x - kCta) >> 5;
         cta_sync();
         if (list && csize > 1) cluster_sync();
-        for (int s = 0; s < steps; s++) {
+        for (int s = 0; s < steps && coupled; s++) {
             const int par = (int)((t0 + s) & 1);
             if (handoff) asm volatile("bar.sync 2, %0;" ::"n"(2 * kCta) : "memory");
             else cta_sync();
-            if (sm.abortStep == s) break;
+            if (sm.abortStep == s) return false;
             if (handoff) {
                 if (sm.cnt[par] > 0) {
                     push_own(P, t0 + s, slot, sm, par, part, kWarps, true);
@@ -2686,12 +2686,12 @@ __global__ void __launch_bounds__(kCta, MinB) v1_batch_step_kernel(const BatchTr
 // one after the other, each for its steps of the chunk, with the trial's state in registers
 // and a barrier among the trial's own CTAs between steps (no grid-wide barrier: trials are
 // independent).  The step is the single patch's (persistent_steps), so every trial computes
-// what the per-step batch and pv1_run compute for it.
-template <bool Rng, bool General>
-__global__ void __launch_bounds__(kCta, 2) v1_batch_persistent_kernel(const BatchTrial *__restrict__ trials,
-                                                                     const int *__restrict__ activeList,
-                                                                     const int *__restrict__ nActive, int slotCtas,
-                                                                     int nSlots, int K, unsigned *barriers) {
+// what the per-step batch and pv1_run compute for it.  Push: with push warps, one CTA per SM (batches whose
+// trials all have far synapses; the host chooses the form).
+template <bool Rng, bool General, bool Push>
+__global__ void __launch_bounds__(Push ? 2 * kCta : kCta, Push ? 1 : 2)
+    v1_batch_persistent_kernel(const BatchTrial *__restrict__ trials, const int *__restrict__ activeList,
+                               const int *__restrict__ nActive, int slotCtas, int nSlots, int K, unsigned *barriers) {
     __shared__ PShared sm;
     __shared__ __align__(16) BatchTrial sT;
     extern __shared__ __align__(16) float dyn[];   // LGN synapses: weights, ids [kBatchLgn][kCta] each; spike bits
@@ -2706,7 +2706,7 @@ __global__ void __launch_bounds__(kCta, 2) v1_batch_persistent_kernel(const Batc
         __syncthreads();
         const int *src = reinterpret_cast<const int *>(trials + q);
         int *dst = reinterpret_cast<int *>(&sT);
-        for (int w = threadIdx.x; w < (int)(sizeof(BatchTrial) / sizeof(int)); w += kCta) dst[w] = src[w];
+        for (int w = threadIdx.x; w < (int)(sizeof(BatchTrial) / sizeof(int)); w += blockDim.x) dst[w] = src[w];
         __syncthreads();
         if (c >= sT.nCta) continue;
         const long long t0 = *sT.step;
@@ -2714,7 +2714,7 @@ __global__ void __launch_bounds__(kCta, 2) v1_batch_persistent_kernel(const Batc
         const int steps = left < K ? (int)left : K;
         if (steps <= 0) continue;
         // a trial whose barrier gave up ends the slot: its cluster's CTAs leave it a step apart
-        if (!persistent_steps<Rng, General, false, false>(sT.v, t0, steps, c, sT.nCta, csize, sT.lgnRing, sT.lgnBits, sT.lgnSlots,
+        if (!persistent_steps<Rng, General, false, Push>(sT.v, t0, steps, c, sT.nCta, csize, sT.lgnRing, sT.lgnBits, sT.lgnSlots,
                                             t0 >= sT.tDeliverFrom, barriers + q, sm, ph, dyn, kBatchLgn, kBatchBits))
             return;
     }
@@ -2722,30 +2722,34 @@ __global__ void __launch_bounds__(kCta, 2) v1_batch_persistent_kernel(const Batc
 
 
 using BatchKernel = void (*)(const BatchTrial *, const int *, const int *, int, int, int, unsigned *);
-static BatchKernel batch_kernel(bool rng, bool general) {
-    if (general) return rng ? v1_batch_persistent_kernel<true, true> : v1_batch_persistent_kernel<false, true>;
-    return rng ? v1_batch_persistent_kernel<true, false> : v1_batch_persistent_kernel<false, false>;
+template <bool Push>
+static BatchKernel batch_kernel_of(bool rng, bool general) {
+    if (general) return rng ? v1_batch_persistent_kernel<true, true, Push> : v1_batch_persistent_kernel<false, true, Push>;
+    return rng ? v1_batch_persistent_kernel<true, false, Push> : v1_batch_persistent_kernel<false, false, Push>;
+}
+static BatchKernel batch_kernel(bool rng, bool general, bool push) {
+    return push ? batch_kernel_of<true>(rng, general) : batch_kernel_of<false>(rng, general);
 }
 
 // Whether a trial needs the general kernel: LGN lists past kBatchLgn or several spikes per step.
 bool v1_batch_general(const V1Params &p) { return p.multiSpike || p.maxLGN > kBatchLgn; }
 
-int v1_batch_persistent_capacity(bool rng, bool general, int device, int csize) {
+int v1_batch_persistent_capacity(bool rng, bool general, bool push, int device, int csize) {
     int coop = 0;
     if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop) return 0;
-    BatchKernel k = batch_kernel(rng, general);
+    BatchKernel k = batch_kernel(rng, general, push);
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBatchDyn) != cudaSuccess) return 0;
-    return resident_ctas(k, kCta, kBatchDyn, csize, device);
+    return resident_ctas(k, push ? 2 * kCta : kCta, kBatchDyn, csize, device);
 }
 
 cudaError_t launch_v1_batch_persistent(const BatchTrial *trials, const int *activeList, const int *nActive,
                                        int slotCtas, int nSlots, int K, unsigned *barriers, int nTrials, bool rng,
-                                       bool general, int csize, cudaStream_t st) {
+                                       bool general, bool push, int csize, cudaStream_t st) {
     if (nSlots <= 0 || slotCtas <= 0 || csize <= 0 || slotCtas % csize) return cudaErrorInvalidValue;
     cudaError_t e = cudaMemsetAsync(barriers, 0, (size_t)nTrials * sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
-    CoopLaunch cl(nSlots * slotCtas, kCta, kBatchDyn, csize, st);
-    return cudaLaunchKernelEx(&cl.cfg, batch_kernel(rng, general), trials, activeList, nActive, slotCtas, nSlots, K,
+    CoopLaunch cl(nSlots * slotCtas, push ? 2 * kCta : kCta, kBatchDyn, csize, st);
+    return cudaLaunchKernelEx(&cl.cfg, batch_kernel(rng, general, push), trials, activeList, nActive, slotCtas, nSlots, K,
                               barriers);
 }
 
