@@ -37,7 +37,7 @@ struct pv1_batch {
     int2 *dTiles = nullptr;
     int *dNTiles = nullptr;
     int *dActive = nullptr, *dNActive = nullptr;   // active trial list (persistent variant)
-    unsigned *dBar = nullptr;                      // per-trial barrier counters
+    unsigned *dBar = nullptr;                      // per-trial barrier counters, two each
     int slotCtas = 0, nSlots = 0, csize = 1;       // persistent variant: CTAs per slot, slots, CTAs per cluster
     int nPush = 0;                                 // slots of its form with push warps, one CTA per SM (0: not used)
     int totalTiles = 0;
@@ -275,7 +275,7 @@ int pv1_batch_create(pv1_plan *const *plans, uint32_t nTrials, const uint64_t *t
     r |= balloc(b, &b->dNTiles, 1);
     r |= balloc(b, &b->dActive, nTrials);
     r |= balloc(b, &b->dNActive, 1);
-    r |= balloc(b, &b->dBar, nTrials);
+    r |= balloc(b, &b->dBar, 2 * (size_t)nTrials);
     if (r) return r;
     // persistent variant: slots as large as the largest trial, as many as stay co-resident
     for (int q = 0; q < b->n; q++) b->slotCtas = std::max(b->slotCtas, b->hT[q].nCta);

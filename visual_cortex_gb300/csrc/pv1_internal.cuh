@@ -391,7 +391,7 @@ bool v1_persistent_shape(const V1Params &p, int device, int *cluster, int *threa
 // Evaluates the full-step decay factors of the three conductance kernels on the device, checks the
 // quick divisions by their times and stores both into p (synchronous).
 cudaError_t compute_step_decay(V1Params &p, cudaStream_t st);
-// barrier null: the blocks do not wait on one another (no cooperative launch).
+// barrier: two counters; null: the blocks do not wait on one another (no cooperative launch).
 cudaError_t launch_v1_persistent(const V1Params &p, const long long *stepBase, int K, const float *lgnRing,
                                  const unsigned *lgnBits, int lgnSlots, int deliverFirst, unsigned *barrier, cudaStream_t st);
 cudaError_t launch_advance_step(long long *stepBase, int k, cudaStream_t st);
@@ -442,7 +442,7 @@ cudaError_t launch_batch_rates(const BatchTrial *trials, const unsigned *counts,
                                double *meanRate, cudaStream_t st);
 int v1_batch_regs(int minB, bool rng);
 // Batched trials in one cooperative launch per chunk (slots of slotCtas CTAs in clusters of csize,
-// per-trial barriers).
+// per-trial barriers of two counters each).
 bool v1_batch_general(const V1Params &p);
 int v1_batch_persistent_capacity(bool rng, bool general, bool push, int device, int csize);
 cudaError_t launch_v1_batch_persistent(const BatchTrial *trials, const int *activeList, const int *nActive,

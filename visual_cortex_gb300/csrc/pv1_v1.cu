@@ -1641,9 +1641,10 @@ __device__ __forceinline__ void init_barriers(PShared &sm, int csize) {
     __syncthreads();
 }
 
-// Grid (or trial) barrier on a monotonic arrival counter, zeroed before each launch.  wait()
-// polls with a bounded number of attempts; a CTA that gives up sets kErrBarrier and the abort bit
-// of the counter, which releases and fails every other waiter.
+// Grid (or trial) barrier: two monotonic arrival counters, zeroed before each launch: the ends of the
+// CTAs' steps, and the CTAs that have started.  barrier_wait polls one of them with a bounded number
+// of attempts; a CTA that gives up sets kErrBarrier and the abort bit of the counter, which
+// releases and fails every other waiter.
 __device__ __forceinline__ bool barrier_wait(unsigned *count, unsigned target, PShared &sm, int *err, long long limit) {
     if (threadIdx.x == 0) {
         unsigned c = 0;
@@ -1952,8 +1953,9 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
     cta_sync();
     if (threadIdx.x == 0 && barrier) {
         __threadfence();
-        // the last CTA to arrive: everyone has read the list that was left
-        if (atomicAdd(barrier, 1u) + 1u == (unsigned)nCta && P.farOn)
+        // the last CTA to come here: everyone has read the list that was left.  A word of its own: step
+        // 0 has no wait, so a CTA can arrive at the end of it before another one has come here
+        if (atomicAdd(barrier + 1, 1u) + 1u == (unsigned)nCta && P.farOn)
             P.farCount[0] = P.farCount[1] = P.farCount[2] = 0ull;
     }
     if (list) {
@@ -2044,8 +2046,9 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
         const bool ffEarly = list || !dl;
         if (ffEarly) feed_forward();
         if (s > 0 && nCta > 1 && barrier && (coupled || s == 1)) {
-            const unsigned target = (unsigned)nCta * (coupled ? (unsigned)(s + 1) : 1u);
-            if (!barrier_wait(barrier, target, sm, P.err, P.waitSpins)) {
+            // every CTA's arrival of step s - 1; uncoupled, that every CTA has started
+            const unsigned target = (unsigned)nCta * (coupled ? (unsigned)s : 1u);
+            if (!barrier_wait(coupled ? barrier : barrier + 1, target, sm, P.err, P.waitSpins)) {
                 ok = false;
                 // peers that passed this barrier still send step s to this CTA: it tells them to leave and
                 // stays until all of the block have sent
@@ -2616,7 +2619,7 @@ cudaError_t launch_v1_persistent(const V1Params &p, const long long *stepBase, i
     const int nq = (p.blockSize + kCta - 1) / kCta;
     CoopLaunch cl(p.nblock * nq, p.threads, v1_persistent_smem(p), p.cluster, st, barrier != nullptr);
     if (barrier) {
-        const cudaError_t e = cudaMemsetAsync(barrier, 0, sizeof(unsigned), st);
+        const cudaError_t e = cudaMemsetAsync(barrier, 0, 2 * sizeof(unsigned), st);
         if (e != cudaSuccess) return e;
     }
     return cudaLaunchKernelEx(&cl.cfg, persistent_kernel(p), p, stepBase, K, lgnRing, lgnBits, lgnSlots, deliverFirst,
@@ -2715,7 +2718,7 @@ __global__ void __launch_bounds__(Push ? 2 * kCta : kCta, Push ? 1 : 2)
         if (steps <= 0) continue;
         // a trial whose barrier gave up ends the slot: its cluster's CTAs leave it a step apart
         if (!persistent_steps<Rng, General, false, Push>(sT.v, t0, steps, c, sT.nCta, csize, sT.lgnRing, sT.lgnBits, sT.lgnSlots,
-                                            t0 >= sT.tDeliverFrom, barriers + q, sm, ph, dyn, kBatchLgn, kBatchBits))
+                                            t0 >= sT.tDeliverFrom, barriers + 2 * q, sm, ph, dyn, kBatchLgn, kBatchBits))
             return;
     }
 }
@@ -2746,7 +2749,7 @@ cudaError_t launch_v1_batch_persistent(const BatchTrial *trials, const int *acti
                                        int slotCtas, int nSlots, int K, unsigned *barriers, int nTrials, bool rng,
                                        bool general, bool push, int csize, cudaStream_t st) {
     if (nSlots <= 0 || slotCtas <= 0 || csize <= 0 || slotCtas % csize) return cudaErrorInvalidValue;
-    cudaError_t e = cudaMemsetAsync(barriers, 0, (size_t)nTrials * sizeof(unsigned), st);
+    cudaError_t e = cudaMemsetAsync(barriers, 0, (size_t)2 * nTrials * sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
     CoopLaunch cl(nSlots * slotCtas, push ? 2 * kCta : kCta, kBatchDyn, csize, st);
     return cudaLaunchKernelEx(&cl.cfg, batch_kernel(rng, general, push), trials, activeList, nActive, slotCtas, nSlots, K,
