@@ -128,8 +128,10 @@ __device__ __forceinline__ float adj_neuron_step(const pv1_adj_problem &P, AStat
 // mask.  A neuron then visits its set bits in ascending synapse order, so that its sums are those
 // of the full walk.  The warps' ballots go to every CTA of the block as asynchronous stores that
 // count towards an mbarrier; the same mbarrier tells that every warp has set its bits.  Two
-// buffers by parity of the step: a warp reaches step t + 2's only after the phase of step t + 1, which
-// its peers announce after they have used step t's.
+// buffers by parity of a running count of exchanges: a warp reaches exchange e + 2's only after the
+// phase of exchange e + 1, which its peers announce after they have used exchange e's.  (Not by parity
+// of the step: the backward goes from the last step to the segment before, which can have the
+// same one.)
 // Measured, with the staged inhibitory weights below: forward and backward of 4,096 neurons x 16 trials x
 // 4,000 steps 40,384 -> 22,120 us (23,737 without them), of two blocks of 128 neurons x 320 steps with
 // the recurrent term 3,784 -> 2,914 us.
@@ -217,7 +219,7 @@ __device__ __forceinline__ RowShare fetch_row(const AdjArgs &A, const uint8_t *r
     return r;
 }
 
-// The events of a count row into the masks of step parity par: each thread its share of the cells.
+// The events of a count row into the masks of exchange parity par: each thread its share of the cells.
 __device__ __forceinline__ void mark_events(const AdjArgs &A, const uint8_t *dyn, const uint8_t *row, const RowShare &r,
                                             bool fits, AdjShared &sm, int par) {
     if (A.entAt < 0) return;
@@ -242,7 +244,7 @@ __device__ __forceinline__ void mark_events(const AdjArgs &A, const uint8_t *dyn
     }
 }
 
-// Announces this warp's part of step t (its bits are set, its ballot is on the way) to every CTA of the
+// Announces this warp's part of an exchange (its bits are set, its ballot is on the way) to every CTA of the
 // block.
 __device__ __forceinline__ void send_ballot(AdjShared &sm, int par, int word, unsigned bal, int split) {
     const int lane = threadIdx.x & 31;
@@ -267,7 +269,7 @@ __device__ __forceinline__ void send_ballot(AdjShared &sm, int par, int word, un
     }
 }
 
-// Bounded wait for the phase of step t's parity; false if it never completes.
+// Bounded wait for the phase of an exchange's parity; false if it never completes.
 __device__ __forceinline__ bool wait_block(AdjShared &sm, int par, unsigned &phase) {
     const unsigned bar = smem_u32(&sm.bar[par]);
     const unsigned want = (phase >> par) & 1u;
@@ -616,6 +618,7 @@ __global__ void __launch_bounds__(MaxThreads, 1) adj_backward_kernel(AdjArgs A) 
     const GabaView gv = stage_gaba(A, dyn, C, local - threadIdx.x, sm);
     const bool fits = row_fits(A);
     unsigned phase = 0u;
+    int par = 0;   // of the next exchange
     Pending pd;
     pd.n = 0;
     // adjoints of the state after the current step
@@ -634,12 +637,12 @@ __global__ void __launch_bounds__(MaxThreads, 1) adj_backward_kernel(AdjArgs A) 
         const uint8_t *row = Xb + (size_t)t0 * P.nLGN;
         RowShare share = fetch_row(A, row, fits);
         float *o = scr;
-        for (int t = t0; t < t1; t++, row += P.nLGN, o += scrStep) {
-            mark_events(A, dyn, row, share, fits, sm, t & 1);
+        for (int t = t0; t < t1; t++, row += P.nLGN, o += scrStep, par ^= 1) {
+            mark_events(A, dyn, row, share, fits, sm, par);
             if (t + 1 < t1) share = fetch_row(A, row + P.nLGN, fits);
             add_pending(s.hI, pd);
             o[0] = s.v; o[bs] = s.gE; o[2 * bs] = s.hE; o[3 * bs] = s.gI; o[4 * bs] = s.hI;
-            const StepOut r = exchange_step(A, sm, s, I0, isE, local, gv, row, t & 1, phase, sv, pd);
+            const StepOut r = exchange_step(A, sm, s, I0, isE, local, gv, row, par, phase, sv, pd);
             o[5 * bs] = (float)((r.refr ? 1 : 0) | (r.spk ? 2 : 0) | (r.many ? 4 : 0));
             o[6 * bs] = __uint_as_float(r.mask);
         }
