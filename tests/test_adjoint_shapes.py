@@ -66,3 +66,20 @@ def test_count_rows(native, nLGN, counts, rec_grad):
 def test_room_for_inhibitory_weights(native, nE, density):
     """Blocks with more inhibitory neurons, more weights and not more than shared memory takes."""
     _check(*_patch(60, 16, 20, bs=1024, nE=nE, nblock=1, seed=nE, density=density, drive=2.0, cta_split=1))
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3, 4])
+def test_counts_at_any_address(native, offset):
+    """Count rows are bytes: they may start anywhere."""
+    import torch
+    patch, W = _patch(130, 64, 65, seed=4)
+    room = torch.zeros(patch.X.numel() + 4, dtype=torch.uint8, device="cuda")
+    view = room[offset:offset + patch.X.numel()].view(patch.X.shape)
+    view.copy_(patch.X)
+    assert view.data_ptr() % 4 == offset % 4
+    want = _gradients(patch, W, lambda p, *a: p.forward(*a))
+    patch.X = view
+    got = _gradients(patch, W, lambda p, *a: p.forward(*a))
+    assert float(want[0].sum()) > 0
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    assert float((got[2] - want[2]).abs().max() / want[2].abs().max()) < 1e-5

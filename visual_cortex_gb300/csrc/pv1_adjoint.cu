@@ -197,14 +197,15 @@ __device__ __forceinline__ void mark_cell(const unsigned *off, const unsigned sh
     }
 }
 
-// A thread's share of a count row, fetched a step ahead: up to two words of four cells each (rows of
+// A thread's share of a count row, fetched a step ahead: up to two words of four cells each (aligned rows of
 // whole words with no more than eight cells per thread), else nothing (the row is read when marked).
 struct RowShare {
     unsigned w[2];
 };
 
 __device__ __forceinline__ bool row_fits(const AdjArgs &A) {
-    return A.entAt >= 0 && A.p.nLGN % 4 == 0 && A.p.nLGN <= 8 * blockDim.x;
+    return A.entAt >= 0 && A.p.nLGN % 4 == 0 && A.p.nLGN <= 8 * blockDim.x &&
+           reinterpret_cast<uintptr_t>(A.b.X) % 4 == 0;
 }
 
 __device__ __forceinline__ RowShare fetch_row(const AdjArgs &A, const uint8_t *row, bool fits) {
