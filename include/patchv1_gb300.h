@@ -573,6 +573,8 @@ typedef struct {
     float *scratch;       /* [B*nblock][seg][6][blockSize] recompute buffer */
 } pv1_adj_buffers;
 
+/* The kernels' waits are bounded (about a second): where one runs out, its neurons' potentials, and with
+ * them vbar and the gradients, are NaN. */
 uint64_t pv1_adj_checkpoint_floats(const pv1_adj_problem *p);
 uint64_t pv1_adj_scratch_floats(const pv1_adj_problem *p);
 int pv1_adj_forward(const pv1_adj_problem *p, const pv1_adj_buffers *b, void *stream);

@@ -270,21 +270,22 @@ __device__ __forceinline__ void send_ballot(AdjShared &sm, int par, int word, un
     }
 }
 
-// Bounded wait for the phase of an exchange's parity; false if it never completes.
+// Bounded wait of a warp for the phase of an exchange's parity; false if it does not complete.  A poll suspends
+// the warp for up to 3.9 us: the limit is a second.
+constexpr int kAdjSpins = 1 << 18;
 __device__ __forceinline__ bool wait_block(AdjShared &sm, int par, unsigned &phase) {
     const unsigned bar = smem_u32(&sm.bar[par]);
     const unsigned want = (phase >> par) & 1u;
-    phase ^= 1u << par;
-    for (int i = 0; i < (1 << 24); i++) {
-        unsigned ok;
+    unsigned ok = 0u;
+    for (int i = 0; i < kAdjSpins && !ok; i++)
         asm volatile(
             "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
             : "=r"(ok)
             : "r"(bar), "r"(want)
             : "memory");
-        if (ok) return true;
-    }
-    return false;
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    phase ^= 1u << par;
+    return true;
 }
 
 // The neuron's LGN events of a step into hE, synapse order; returns their mask.  Without event lists
@@ -485,8 +486,18 @@ __device__ __forceinline__ void init_exchange(const AdjArgs &A, uint8_t *dyn, Ad
     block_sync(A.split);   // every CTA of the block is set up before the first remote store
 }
 
+// The end of a CTA's exchanges: no CTA leaves while a peer's stores are on their way to it.
+__device__ __forceinline__ void leave_exchange(AdjShared &sm, int split, unsigned phase, int lost) {
+    if (split == 1) return;
+    cg::this_cluster().sync();
+    if (lost >= 0) wait_block(sm, lost, phase);   // what was late: everyone has sent by now
+}
+
 // One forward step of a neuron with its exchange: shared by the forward and the recompute of the
 // backward.  vnext, spk, refr: the step's results; mask, many: its LGN events.
+// lost: the parity of the exchange whose wait ran out, else -1.  From then on the warp neither sends nor
+// waits, so that what is left takes no time and the peers' waits run out as well, once each; its
+// potentials are NaN, which the outputs show.
 struct StepOut {
     float vnext;
     bool spk, refr, many;
@@ -495,13 +506,16 @@ struct StepOut {
 
 __device__ __forceinline__ StepOut exchange_step(const AdjArgs &A, AdjShared &sm, AState &s, float I0, bool isE, int local,
                                                  const GabaView &gv, const uint8_t *x, int par, unsigned &phase,
-                                                 const SynView &sv, Pending &pd) {
+                                                 const SynView &sv, Pending &pd, int &lost) {
     StepOut o;
     float gE1, hE1, gI1, hI1;
     o.vnext = adj_neuron_step(A.p, s, I0, isE, o.spk, o.refr, gE1, hE1, gI1, hI1);
     const unsigned bal = __ballot_sync(0xffffffffu, o.spk);
-    send_ballot(sm, par, local >> 5, bal, A.split);
-    if (!wait_block(sm, par, phase)) o.vnext = nanf("");   // never seen: the run's outputs say so
+    if (lost < 0) {
+        send_ballot(sm, par, local >> 5, bal, A.split);
+        if (!wait_block(sm, par, phase)) lost = par;
+    }
+    if (lost >= 0) o.vnext = nanf("");
     o.mask = lgn_inputs(A, x, sm, par, hE1, sv, o.many);
     gaba_inputs(A, gv, local, sm.ball[par], hI1, pd);
     s.v = o.vnext;
@@ -532,6 +546,7 @@ __global__ void __launch_bounds__(MaxThreads, 1) adj_forward_kernel(AdjArgs A) {
     const bool fits = row_fits(A);
     RowShare share = fetch_row(A, row, fits);
     unsigned phase = 0u;
+    int lost = -1;
     Pending pd;
     pd.n = 0;
     int toCk = 0, toWin = (int)P.win;
@@ -549,7 +564,7 @@ __global__ void __launch_bounds__(MaxThreads, 1) adj_forward_kernel(AdjArgs A) {
             toCk = (int)P.seg;
         }
         toCk--;
-        const StepOut r = exchange_step(A, sm, s, I0, isE, local, gv, row, par, phase, sv, pd);
+        const StepOut r = exchange_step(A, sm, s, I0, isE, local, gv, row, par, phase, sv, pd, lost);
         cnt += r.spk ? 1.f : 0.f;
         vsum += r.vnext;
         if (--toWin == 0) {
@@ -561,7 +576,7 @@ __global__ void __launch_bounds__(MaxThreads, 1) adj_forward_kernel(AdjArgs A) {
             toWin = (int)P.win;
         }
     }
-    if (split > 1) cg::this_cluster().sync();   // no CTA leaves while a peer's stores are on their way to it
+    leave_exchange(sm, split, phase, lost);
 }
 
 __device__ __forceinline__ void block_add_double(double v, double *out, double *red) {
@@ -620,6 +635,7 @@ __global__ void __launch_bounds__(MaxThreads, 1) adj_backward_kernel(AdjArgs A) 
     const bool fits = row_fits(A);
     unsigned phase = 0u;
     int par = 0;   // of the next exchange
+    int lost = -1;
     Pending pd;
     pd.n = 0;
     // adjoints of the state after the current step
@@ -643,7 +659,7 @@ __global__ void __launch_bounds__(MaxThreads, 1) adj_backward_kernel(AdjArgs A) 
             if (t + 1 < t1) share = fetch_row(A, row + P.nLGN, fits);
             add_pending(s.hI, pd);
             o[0] = s.v; o[bs] = s.gE; o[2 * bs] = s.hE; o[3 * bs] = s.gI; o[4 * bs] = s.hI;
-            const StepOut r = exchange_step(A, sm, s, I0, isE, local, gv, row, par, phase, sv, pd);
+            const StepOut r = exchange_step(A, sm, s, I0, isE, local, gv, row, par, phase, sv, pd, lost);
             o[5 * bs] = (float)((r.refr ? 1 : 0) | (r.spk ? 2 : 0) | (r.many ? 4 : 0));
             o[6 * bs] = __uint_as_float(r.mask);
         }
@@ -742,7 +758,7 @@ __global__ void __launch_bounds__(MaxThreads, 1) adj_backward_kernel(AdjArgs A) 
     block_add_double(dEdI, A.b.gC + 3, red);
     block_add_double(dErI, A.b.gC + 4, red);
     block_add_double(ddodI, A.b.gC + 5, red);
-    if (split > 1) cg::this_cluster().sync();   // no CTA leaves while a peer's stores are on their way to it
+    leave_exchange(sm, split, phase, lost);
 }
 
 int adj_check(const pv1_adj_problem *p, const pv1_adj_buffers *b, AdjArgs *A, bool backward) {
