@@ -83,3 +83,38 @@ def test_counts_at_any_address(native, offset):
     assert float(want[0].sum()) > 0
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
     assert float((got[2] - want[2]).abs().max() / want[2].abs().max()) < 1e-5
+
+
+def test_two_threads_with_different_sizes(native):
+    """Problems of different shared-memory sizes launched from two threads on their own streams."""
+    import ctypes as C
+    import threading
+    import torch
+    from visual_cortex_gb300.adjoint import AdjBuffers
+    ptr = lambda t: C.c_void_p(t.data_ptr())
+    calls, keep = [], []
+    for q, kw in enumerate((dict(bs=512, nE=384, K=30, nLGN=4096), dict(bs=256, nE=192, K=16, nLGN=1024))):
+        patch, W = _patch(1, 1, 1, B=1, nblock=1, seed=q, **kw)
+        prob = patch._problem(patch.consts(torch.tensor(5.0), torch.tensor(7.0)))
+        out = [torch.empty(patch.cfg.N, device="cuda") for _ in range(2)]
+        ck = torch.empty(int(native.lib.pv1_adj_checkpoint_floats(C.byref(prob))), device="cuda")
+        buf = AdjBuffers(ids=ptr(patch.ids), W=ptr(W), X=ptr(patch.X), Crec=ptr(patch.Crec), I0=ptr(patch.I0),
+                         v0=ptr(patch.v0), rates=ptr(out[0]), vbar=ptr(out[1]), ck=ptr(ck))
+        stream = torch.cuda.Stream()
+        calls.append((prob, buf, C.c_void_p(stream.cuda_stream)))
+        keep.append((patch, W, out, ck, stream))
+    torch.cuda.synchronize()
+    failed = [0, 0]
+
+    def work(q):
+        prob, buf, stream = calls[q]
+        for _ in range(20000):
+            failed[q] += native.lib.pv1_adj_forward(C.byref(prob), C.byref(buf), stream) != 0
+
+    threads = [threading.Thread(target=work, args=(q,)) for q in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert failed == [0, 0]

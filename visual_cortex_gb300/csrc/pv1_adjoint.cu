@@ -810,9 +810,10 @@ int adj_check(const pv1_adj_problem *p, const pv1_adj_buffers *b, AdjArgs *A, bo
 }
 
 // Dynamic shared memory: the masks, the event lists if they fit, then the weights if they fit.
+constexpr size_t kAdjRoom = 200 * 1024;
 void adj_smem_plan(AdjArgs &A) {
     const int threads = (int)(A.p.blockSize / A.split);
-    const size_t room = 200 * 1024;
+    const size_t room = kAdjRoom;
     size_t at = 0;
     auto take = [&](size_t bytes) {
         if (at + bytes > room) return -1;
@@ -846,10 +847,9 @@ cudaError_t adj_launch(Kern kern, const AdjArgs &A, cudaStream_t st) {
     cfg.gridDim = dim3(A.p.nblock * A.split, A.p.B);
     cfg.blockDim = dim3(A.p.blockSize / A.split);
     cfg.dynamicSmemBytes = (size_t)A.smemBytes;
-    if (cfg.dynamicSmemBytes > 24 * 1024) {   // with the kernels' own shared memory this can pass 48 KB
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, A.smemBytes);
-        if (e != cudaSuccess) return e;
-    }
+    // the same limit for every problem: it belongs to the kernel, and another thread may be about to launch it
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAdjRoom);
+    if (e != cudaSuccess) return e;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
