@@ -313,11 +313,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) lgn_tc_kernel(TcArgs A, const _
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const unsigned tmem = tmemSlot;
     const volatile int *stopped = &stop;
-    auto wait = [&](uint64_t *b, unsigned parity) {
-        if (mbar_wait(b, parity, stopped)) return true;
+    auto give_up = [&]() {
         atomicOr(A.err, kErrBarrier);
         stop = 1;
         return false;
+    };
+    // of a role of one lane, and of a whole warp: the lanes poll on their own and can find different
+    // answers when another role stops, while what follows is for all of them together
+    auto wait_lane = [&](uint64_t *b, unsigned parity) { return mbar_wait(b, parity, stopped) || give_up(); };
+    auto wait = [&](uint64_t *b, unsigned parity) {
+        return __all_sync(0xffffffffu, mbar_wait(b, parity, stopped)) || give_up();
     };
     if (warp < 4) {
         // generators
@@ -405,8 +410,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) lgn_tc_kernel(TcArgs A, const _
             for (; loaded < 2 && loaded < A.nTiles; loaded++) load(loaded);
             for (int i = 0; i < A.nTiles; i++) {
                 const int k = i & 1;
-                if (!wait(&bar.load[k], (i >> 1) & 1)) break;
-                if (i >= 2 && !wait(&bar.read[k], ((i >> 1) - 1) & 1)) break;
+                if (!wait_lane(&bar.load[k], (i >> 1) & 1)) break;
+                if (i >= 2 && !wait_lane(&bar.read[k], ((i >> 1) - 1) & 1)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t da = umma_desc_sw128(smem_u32(tileS(k)));
                 const uint64_t db = umma_desc_sw128(smem_u32(tileW(k)));
@@ -416,7 +421,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) lgn_tc_kernel(TcArgs A, const _
                 umma_commit(&bar.mma[k]);
                 done = i + 1;
                 if (loaded < A.nTiles) {
-                    if (!wait(&bar.mma[k], (i >> 1) & 1)) break;
+                    if (!wait_lane(&bar.mma[k], (i >> 1) & 1)) break;
                     load(loaded++);
                 }
             }
@@ -434,7 +439,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) lgn_tc_kernel(TcArgs A, const _
             for (int i = 0; i < A.nTiles; i++) {
                 const int k = i & 1;
                 // two tiles ahead of the generators at most: a barrier's phases are waited for in turn
-                if (i >= 2 && !wait(&bar.free[k], ((i >> 1) - 1) & 1)) break;
+                if (i >= 2 && !wait_lane(&bar.free[k], ((i >> 1) - 1) & 1)) break;
                 if (storeTma) {
                     for (int t = i * kTcN; t < min((i + 1) * kTcN, A.T); t += kZeroSteps) tma_store_2d(&mapOut, cell0, t, zeros);
                     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // written, not only read
