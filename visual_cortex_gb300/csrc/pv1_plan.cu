@@ -147,6 +147,21 @@ int dev_upload(pv1_plan *p, T **ptr, const T *host, size_t n) {
     return PV1_OK;
 }
 
+// A copy behind everything on the plan's stream, complete on return.  (The blocking copies run on the legacy
+// stream: neither what the plan's own stream still has to do nor what it is given next is ordered
+// with them.)
+int copy_now(pv1_plan *p, void *dst, const void *src, size_t bytes, cudaMemcpyKind kind) {
+    PV1_CUDA(p, cudaMemcpyAsync(dst, src, bytes, kind, p->stream));
+    PV1_CUDA(p, cudaStreamSynchronize(p->stream));
+    return PV1_OK;
+}
+
+#define PV1_COPY(p, dst, src, bytes, kind)                              \
+    do {                                                                \
+        const int r_ = copy_now((p), (dst), (src), (bytes), (kind));    \
+        if (r_) return r_;                                              \
+    } while (0)
+
 void free_one(pv1_plan *p, void *ptr) {
     auto it = std::find(p->allocs.begin(), p->allocs.end(), ptr);
     if (it != p->allocs.end()) {
@@ -809,7 +824,7 @@ int lgn_setup_impl(pv1_plan *p, const pv1_lgn_config *lc, const pv1_lgn_parvo_co
     L.classCtw = nullptr;
     if (nMagno > 0 && nParvo == 0) {
         std::vector<float> tw((size_t)nMagno * nKS);
-        PV1_CUDA(p, cudaMemcpy(tw.data(), p->d_TW, tw.size() * sizeof(float), cudaMemcpyDeviceToHost));
+        PV1_COPY(p, tw.data(), p->d_TW, tw.size() * sizeof(float), cudaMemcpyDeviceToHost);
         bool same = true;
         for (int m = 1; m < nMagno && same; m++)
             same = std::memcmp(tw.data(), tw.data() + (size_t)m * nKS, nKS * sizeof(float)) == 0;
@@ -818,12 +833,12 @@ int lgn_setup_impl(pv1_plan *p, const pv1_lgn_config *lc, const pv1_lgn_parvo_co
             double *d_cls;
             r = dev_alloc(p, &d_cls, (size_t)nKS + 1);
             if (r) return r;
-            PV1_CUDA(p, cudaMemcpy2D(d_cls, sizeof(double), d_ctw, (size_t)nMagno * sizeof(double), sizeof(double),
-                                     (size_t)nKS + 1, cudaMemcpyDeviceToDevice));
+            PV1_CUDA(p, cudaMemcpy2DAsync(d_cls, sizeof(double), d_ctw, (size_t)nMagno * sizeof(double), sizeof(double),
+                                          (size_t)nKS + 1, cudaMemcpyDeviceToDevice, p->stream));
             L.classCtw = d_cls;
             // the segment sums of every frame phase, as lgn_rate_kernel forms them
             std::vector<double> cls((size_t)nKS + 1);
-            PV1_CUDA(p, cudaMemcpy(cls.data(), d_cls, cls.size() * sizeof(double), cudaMemcpyDeviceToHost));
+            PV1_COPY(p, cls.data(), d_cls, cls.size() * sizeof(double), cudaMemcpyDeviceToHost);
             std::vector<float> wt((size_t)c.ntPerFrame * maxSeg, 0.f);
             for (size_t ph = 0; ph < c.ntPerFrame; ph++)
                 for (int q = 0; q < nseg[ph]; q++)
@@ -860,9 +875,9 @@ int pv1_lgn_get_parvo_tables(pv1_plan *p, float *TW, float *SW, float *SC) {
     if (p->nParvo == 0) return fail(p, PV1_E_STATE, "no parvo cells");
     PV1_CUDA(p, cudaStreamSynchronize(p->stream));
     const size_t np = p->nParvo, ns = p->pSample;
-    if (TW) PV1_CUDA(p, cudaMemcpy(TW, p->d_pTW, np * 2 * p->pcfg.nKernelSample * sizeof(float), cudaMemcpyDeviceToHost));
-    if (SW) PV1_CUDA(p, cudaMemcpy(SW, p->d_pSW, ns * sizeof(float), cudaMemcpyDeviceToHost));
-    if (SC) PV1_CUDA(p, cudaMemcpy(SC, p->d_pSC, 4 * np * ns * sizeof(float), cudaMemcpyDeviceToHost));
+    if (TW) PV1_COPY(p, TW, p->d_pTW, np * 2 * p->pcfg.nKernelSample * sizeof(float), cudaMemcpyDeviceToHost);
+    if (SW) PV1_COPY(p, SW, p->d_pSW, ns * sizeof(float), cudaMemcpyDeviceToHost);
+    if (SC) PV1_COPY(p, SC, p->d_pSC, 4 * np * ns * sizeof(float), cudaMemcpyDeviceToHost);
     return PV1_OK;
 }
 
@@ -873,7 +888,7 @@ int pv1_lgn_get_parvo_spatial(pv1_plan *p, float *PS) {
     int r = ensure_all_frames(p);
     if (r) return r;
     PV1_CUDA(p, cudaStreamSynchronize(p->stream));
-    PV1_CUDA(p, cudaMemcpy(PS, p->d_pS, (size_t)(p->nFrame + 1) * 2 * p->nParvo * sizeof(float), cudaMemcpyDeviceToHost));
+    PV1_COPY(p, PS, p->d_pS, (size_t)(p->nFrame + 1) * 2 * p->nParvo * sizeof(float), cudaMemcpyDeviceToHost);
     return PV1_OK;
 }
 
@@ -882,10 +897,10 @@ int pv1_lgn_get_tables(pv1_plan *p, float *TW, float *SW, float *SC, float *maxC
     if (!p->lgnReady) return fail(p, PV1_E_STATE, "LGN not set up");
     PV1_CUDA(p, cudaStreamSynchronize(p->stream));
     const size_t nm = p->nMagno;
-    if (TW) PV1_CUDA(p, cudaMemcpy(TW, p->d_TW, nm * p->lcfg.nKernelSample * sizeof(float), cudaMemcpyDeviceToHost));
-    if (SW) PV1_CUDA(p, cudaMemcpy(SW, p->d_SW, nm * p->mSample * sizeof(float), cudaMemcpyDeviceToHost));
-    if (SC) PV1_CUDA(p, cudaMemcpy(SC, p->d_SC, 2 * nm * p->mSample * sizeof(float), cudaMemcpyDeviceToHost));
-    if (maxConvol) PV1_CUDA(p, cudaMemcpy(maxConvol, p->d_maxConvol, p->nLGN * sizeof(float), cudaMemcpyDeviceToHost));
+    if (TW) PV1_COPY(p, TW, p->d_TW, nm * p->lcfg.nKernelSample * sizeof(float), cudaMemcpyDeviceToHost);
+    if (SW) PV1_COPY(p, SW, p->d_SW, nm * p->mSample * sizeof(float), cudaMemcpyDeviceToHost);
+    if (SC) PV1_COPY(p, SC, p->d_SC, 2 * nm * p->mSample * sizeof(float), cudaMemcpyDeviceToHost);
+    if (maxConvol) PV1_COPY(p, maxConvol, p->d_maxConvol, p->nLGN * sizeof(float), cudaMemcpyDeviceToHost);
     return PV1_OK;
 }
 
@@ -1053,7 +1068,7 @@ int pv1_lgn_get_spatial(pv1_plan *p, float *S) {
     int r = ensure_all_frames(p);
     if (r) return r;
     PV1_CUDA(p, cudaStreamSynchronize(p->stream));
-    PV1_CUDA(p, cudaMemcpy(S, p->d_S, (size_t)(p->nFrame + 1) * p->nMagno * sizeof(float), cudaMemcpyDeviceToHost));
+    PV1_COPY(p, S, p->d_S, (size_t)(p->nFrame + 1) * p->nMagno * sizeof(float), cudaMemcpyDeviceToHost);
     return PV1_OK;
 }
 
@@ -1176,8 +1191,8 @@ int pv1_set_ff_learning(pv1_plan *p, const pv1_ff_learning *l) {
     std::vector<float> s((size_t)v.maxLGN * n), tot(2 * n, 0.f);
     std::vector<int> m(n);
     PV1_CUDA(p, cudaStreamSynchronize(p->stream));
-    if (!s.empty()) PV1_CUDA(p, cudaMemcpy(s.data(), v.sLGN, s.size() * sizeof(float), cudaMemcpyDeviceToHost));
-    PV1_CUDA(p, cudaMemcpy(m.data(), v.nLGNperV1, n * sizeof(int), cudaMemcpyDeviceToHost));
+    if (!s.empty()) PV1_COPY(p, s.data(), v.sLGN, s.size() * sizeof(float), cudaMemcpyDeviceToHost);
+    PV1_COPY(p, m.data(), v.nLGNperV1, n * sizeof(int), cudaMemcpyDeviceToHost);
     for (size_t i = 0; i < n; i++) {
         float t = 0.f;
         for (int j = 0; j < m[i]; j++) t += s[(size_t)j * n + i];
@@ -2500,7 +2515,7 @@ int pv1_get_state(pv1_plan *p, int which, float *out) {
         default: return fail(p, PV1_E_ARG, "unknown state id");
     }
     if (!src) return fail(p, PV1_E_STATE, "state not allocated");
-    PV1_CUDA(p, cudaMemcpy(out, src, cnt * sizeof(float), cudaMemcpyDeviceToHost));
+    PV1_COPY(p, out, src, cnt * sizeof(float), cudaMemcpyDeviceToHost);
     return PV1_OK;
 }
 
@@ -2536,7 +2551,7 @@ int pv1_put_state(pv1_plan *p, int which, const float *in) {
         default: return fail(p, PV1_E_ARG, "state id cannot be written");
     }
     if (!dst) return fail(p, PV1_E_STATE, "state not allocated");
-    PV1_CUDA(p, cudaMemcpy(dst, in, cnt * sizeof(float), cudaMemcpyHostToDevice));
+    PV1_COPY(p, dst, in, cnt * sizeof(float), cudaMemcpyHostToDevice);
     return PV1_OK;
 }
 
@@ -2590,8 +2605,8 @@ int pv1_fetch_draws(pv1_plan *p, int kind, float *draws, int32_t *counts) {
         case 3: src = v.recNear; cnt = steps * nV1 * cap; csrc = v.recNearCount; ccnt = steps * nV1; break;
         default: return fail(p, PV1_E_ARG, "unknown draw kind");
     }
-    if (draws) PV1_CUDA(p, cudaMemcpy(draws, src, cnt * sizeof(float), cudaMemcpyDeviceToHost));
-    if (counts && csrc) PV1_CUDA(p, cudaMemcpy(counts, csrc, ccnt * sizeof(int), cudaMemcpyDeviceToHost));
+    if (draws) PV1_COPY(p, draws, src, cnt * sizeof(float), cudaMemcpyDeviceToHost);
+    if (counts && csrc) PV1_COPY(p, counts, csrc, ccnt * sizeof(int), cudaMemcpyDeviceToHost);
     return PV1_OK;
 }
 
