@@ -2060,6 +2060,8 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
                 hand_over();
                 break;
             }
+        } else if (s > 0 && coupled) {
+            neuron_sync();   // one CTA: thread 0 has made room for this step's spikers
         }
         if (dl) {
             if (!list) {
