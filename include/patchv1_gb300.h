@@ -471,9 +471,10 @@ int pv1_time_kernels(pv1_plan *plan, uint32_t nsteps, float *v1_ms, float *lgn_m
  * refused here with PV1_E_STATE. */
 int pv1_lgn_spikes_noalloc(pv1_plan *plan, uint32_t nsteps, float *d_sinfo, float *d_fr);
 
-/* Polls of a barrier wait (the persistent kernel's grid barrier between steps, the batched
- * kernel's per-trial barrier) before it gives up; spins < 0 restores the default (2e7 polls,
- * about a second).  A wait that gives up releases every other waiter, the kernel returns, and
+/* Polls of a wait for other CTAs (the persistent kernel's grid barrier between steps, the batched
+ * kernel's per-trial barrier; the spikes of a block's CTAs, whose polls are longer and counted as
+ * 64 each) before it gives up; spins < 0 restores the default (2e7 polls, about a second).
+ * A wait that gives up releases every other waiter, the kernel returns, and
  * the run reports PV1_E_DEVICE ("a barrier wait gave up") instead of hanging: the GPU context
  * stays usable.  No counterpart in the reference (its kernels never wait on one another). */
 int pv1_set_wait_limit(pv1_plan *plan, int64_t spins);

@@ -1563,7 +1563,11 @@ __global__ void __launch_bounds__(kCta) v1_step_kernel(V1Params P, const long lo
 constexpr unsigned kBarrierAbort = 0x80000000u;
 constexpr int kPushU = 2;       // far items a lane fetches together
 constexpr int kMaxBitWords = 2048;   // LGN spike bits kept in shared memory (two rows of up to 65,536 cells)
-constexpr int kMbarSpins = 1 << 24;  // polls of an mbarrier before it counts as lost
+// Polls of an mbarrier before it counts as lost.  A poll suspends its warp for up to 3.9 us, one of the grid
+// barrier takes about 50 ns: a wait for other CTAs gets one for kGridPolls of the plan's limit, a
+// wait for the CTA's own warps and copies a second.
+constexpr int kMbarSpins = 1 << 18;
+constexpr int kGridPolls = 64;
 
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
@@ -1589,17 +1593,22 @@ __device__ __forceinline__ void announce(unsigned bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                  : "memory");
 }
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
-    for (int i = 0; i < kMbarSpins; i++) {
-        unsigned ok;
+// Bounded wait of a whole warp for a phase; false (for all its lanes) if it does not complete, or, with
+// stop, once a warp of the block has given up.
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, int spins, const int *stop = nullptr) {
+    unsigned ok = 0u;
+    for (int i = 0; i <= spins; i++) {
         asm volatile(
             "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
             : "=r"(ok)
             : "r"(bar), "r"(parity)
             : "memory");
-        if (ok) return true;
+        if (ok || (stop && *(volatile const int *)stop)) break;
     }
-    return false;
+    return __all_sync(0xffffffffu, ok);
+}
+__device__ __forceinline__ void store_remote(unsigned addr, unsigned v) {
+    asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
 // Shared memory of a persistent CTA.
@@ -1618,8 +1627,9 @@ struct __align__(16) PShared {
     int e0[2][kCta], deg[2][kCta], n1[2][kCta];
     float si[2][kCta];
     unsigned char preE[2][kCta];
-    unsigned peerFail;
-    int ok, abortStep;
+    int stop;                       // a warp of the block gave up: the waits for spikes end
+    unsigned left[kMaxBS / 32];     // leave_block: the block's warps
+    int abortStep;
 };
 static_assert(kMaxNG == 2, "a spiker's unit conductances are two (g, h) pairs");
 
@@ -1641,12 +1651,30 @@ __device__ __forceinline__ void init_barriers(PShared &sm, int csize) {
     __syncthreads();
 }
 
+// Giving up.  A wait that runs out must not leave anyone waiting for good, nor end a CTA to which others
+// still send.  So a warp whose wait for spikes or bits ran out (lost) tells all who may wait for it
+// (give_up) and leaves where its CTA can tell that it does: at the next meeting of the CTA's warps, if
+// there is one (a warp must not miss a barrier of a fixed number of threads), else where it is.  A step's
+// meeting is behind its wait for the grid, and for all warps alike.  At the end the warps of a block
+// tell each other how far they came; if one gave up they make up the announcements that are missing
+// and stay until what they were sent has arrived (leave_block).
+__device__ __forceinline__ void give_up(PShared &sm, int csize, int *err, unsigned *count) {
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) {
+        atomicOr(err, kErrBarrier);
+        if (count) atomicOr(count, kBarrierAbort);
+    }
+    if (csize == 1) *(volatile int *)&sm.stop = 1;
+    else if (lane < csize) store_remote(at_rank(smem_at(&sm.stop), lane), 1u);
+}
+
 // Grid (or trial) barrier: two monotonic arrival counters, zeroed before each launch: the ends of the
-// CTAs' steps, and the CTAs that have started.  barrier_wait polls one of them with a bounded number
-// of attempts; a CTA that gives up sets kErrBarrier and the abort bit of the counter, which
-// releases and fails every other waiter.
-__device__ __forceinline__ bool barrier_wait(unsigned *count, unsigned target, PShared &sm, int *err, long long limit) {
-    if (threadIdx.x == 0) {
+// CTAs' steps, and the CTAs that have started.  meet: the neuron threads of a CTA meet, after one
+// counter (if given) has reached its target.  False for all of them if a warp is lost, if that
+// takes more than `limit` polls (sets kErrBarrier and the abort bit of the counter, which releases
+// and fails every other waiter) or if the abort bit is set.
+__device__ __forceinline__ bool meet(unsigned *count, unsigned target, bool lost, int *err, long long limit) {
+    if (count && threadIdx.x == 0 && !lost) {
         unsigned c = 0;
         long long spins = 0;
         while (true) {
@@ -1660,17 +1688,21 @@ __device__ __forceinline__ bool barrier_wait(unsigned *count, unsigned target, P
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
             if ((c & ~kBarrierAbort) >= target || (c & kBarrierAbort)) break;
         }
-        sm.ok = (c & kBarrierAbort) ? 0 : 1;
+        lost = (c & kBarrierAbort) != 0;
     }
-    neuron_sync();
-    return sm.ok != 0;
+    __syncwarp();
+    unsigned any;
+    asm volatile("{ .reg .pred p, q; setp.ne.u32 p, %1, 0; bar.red.or.pred q, 1, %2, p; selp.u32 %0, 1, 0, q; }"
+                 : "=r"(any)
+                 : "r"((unsigned)lost), "n"(kCta)
+                 : "memory");
+    return any == 0;
 }
 
 // This step's spikes of the warp (CTA `rank` of the block's csize) to every CTA of the block: unit
-// conductances (output_g/h of compute_V, src/coredynamics.cu:2008-2041) and the ballot word.  poison:
-// tells the peers that this CTA gave up.
+// conductances (output_g/h of compute_V, src/coredynamics.cu:2008-2041) and the ballot word.
 __device__ __forceinline__ void publish_spikes(const V1Params &P, PShared &sm, int par, int csize, int rank, bool spk,
-                                               float sInfo, bool isE, bool poison = false) {
+                                               float sInfo, bool isE) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned bal = __ballot_sync(0xffffffffu, spk);
     const unsigned bar = smem_at(&sm.nearBar[par]);
@@ -1698,24 +1730,48 @@ __device__ __forceinline__ void publish_spikes(const V1Params &P, PShared &sm, i
         __syncwarp();
         if (lane == 0) {
             sm.list.ball[par][warp] = bal;
-            if (poison) sm.peerFail = 1u;
             asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
         }
     } else if (lane < csize) {
         const unsigned peer = at_rank(bar, lane);
-        const bool tell = poison && warp == 0;
         send_word(at_rank(smem_at(&sm.list.ball[par][rank * kWarps + warp]), lane), peer, bal);
-        if (tell) send_word(at_rank(smem_at(&sm.peerFail), lane), peer, 1u);
-        announce(peer, 4u + 16u * __popc(bal) + (tell ? 4u : 0u));
+        announce(peer, 4u + 16u * __popc(bal));
     }
 }
 
-// Waits for the block's spikes of the step with parity par; false if they never came.
-__device__ __forceinline__ bool wait_spikes(PShared &sm, int par, Phases &ph) {
-    const bool in = mbar_wait(smem_at(&sm.nearBar[par]), par ? ph.near1 : ph.near0);
+// Waits for the block's spikes of the step with parity par; false if they did not come.
+__device__ __forceinline__ bool wait_spikes(PShared &sm, int par, Phases &ph, int spins, const int *stop) {
+    if (!mbar_wait(smem_at(&sm.nearBar[par]), par ? ph.near1 : ph.near0, spins, stop)) return false;
     if (par) ph.near1 ^= 1u;
     else ph.near0 ^= 1u;
-    return in;
+    return true;
+}
+
+// The end of a block's steps, for all threads of its csize CTAs (a cluster if exchange, with the spikes
+// sent between them).  sent: the first step from t0 whose spikes this warp did not publish, due: the first
+// one whose spikes it did not take.  False for all of them if one of them failed.  The warps of a block
+// are at most a step apart in what they published, so that what is made up goes to the phases the
+// peers still wait for.
+__device__ __noinline__ bool leave_block(PShared &sm, bool exchange, int csize, int rank, long long t0, int sent, int due,
+                                         bool failed, Phases ph) {
+    if (!exchange || csize == 1) return __syncthreads_or(failed) == 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < kWarps && lane < csize)
+        store_remote(at_rank(smem_at(&sm.left[rank * kWarps + warp]), lane), (unsigned)sent | (failed ? 0x80000000u : 0u));
+    cluster_sync();
+    const unsigned v = lane < csize * kWarps ? sm.left[lane] : 0u;
+    if (!__any_sync(0xffffffffu, v >> 31)) return true;
+    if (warp >= kWarps) return false;
+    const int last = (int)__reduce_max_sync(0xffffffffu, v & 0x7fffffffu);
+    for (int q = sent; q < last; q++)
+        if (lane < csize) announce(at_rank(smem_at(&sm.nearBar[(t0 + q) & 1]), lane), 0u);
+    for (int q = due; q < last; q++) {
+        // a barrier's last phase is complete only after those before it
+        if (q + 2 >= last) wait_spikes(sm, (int)((t0 + q) & 1), ph, kMbarSpins, nullptr);
+        else if ((t0 + q) & 1) ph.near1 ^= 1u;
+        else ph.near0 ^= 1u;
+    }
+    return false;
 }
 
 // The bits of the LGN row of a step into shared memory (thread 0 issues the copy).
@@ -1890,7 +1946,7 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
             const int par = (int)((t0 + s) & 1);
             if (handoff) asm volatile("bar.sync 2, %0;" ::"n"(2 * kCta) : "memory");
             else cta_sync();
-            if (sm.abortStep == s) return false;
+            if (sm.abortStep == s) break;
             if (handoff) {
                 if (sm.cnt[par] > 0) {
                     push_own(P, t0 + s, slot, sm, par, part, kWarps, true);
@@ -1905,7 +1961,7 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
             push_own(P, t0 + s, slot, sm, par, part, kWarps);
             if (++slot == P.farDepth) slot = 0;
         }
-        return true;
+        return leave_block(sm, list, csize, rank, t0, 0, 0, false, ph);
     }
     const int local = rank * kCta + threadIdx.x;
     const bool active = local < bs;
@@ -1945,7 +2001,7 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
     if (threadIdx.x == 0) {
         sm.cnt[0] = sm.cnt[1] = 0;
         sm.abortStep = -1;
-        sm.peerFail = 0u;
+        sm.stop = 0;
     }
     if (threadIdx.x < kMaxType) sm.type[threadIdx.x] = type_const(P, threadIdx.x);
     const TypeConst &tc = sm.type[itype];
@@ -1965,14 +2021,21 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
             publish_spikes(P, sm, (int)((t0 - 1) & 1), csize, rank, w >= 1.0f, w, isE);
         }
     }
-    if (smemSyn && smemBits) fetch_bits(sm, smB, lgnBits + (size_t)lgnSlot * P.lgnW, P.lgnW, 0);
     // ring slots kept incrementally
     int fsT = P.farOn ? far_ring_slot(P, t0) : 0, fsPrev = P.farOn ? far_ring_slot(P, t0 - 1) : 0;
     int t3 = (int)(t0 % 3);
     const bool rec = P.recSpk || P.rec;
     int recSlot = rec ? (int)(t0 % P.recSlots) : 0, recPrev = rec ? (int)((t0 + P.recSlots - 1) % P.recSlots) : 0;
     FFStep ff;
-    bool ok = true;
+    // waits for other CTAs: the counter of the grid barrier, the limit for spikes
+    unsigned *count = barrier && nCta > 1 ? (coupled ? barrier : barrier + 1) : nullptr;
+    const int spins = csize > 1 ? (int)min(P.waitSpins / kGridPolls, (long long)kMbarSpins << 8) : kMbarSpins;
+    int s = 0;
+    int lost = -1;   // 2 x the step whose wait for spikes ran out, + 1 if it was the one for the bits
+    auto lose = [&](int where) {
+        lost = where;
+        give_up(sm, list ? csize : 1, P.err, count);
+    };
     float sLast = 0.f;   // the spike word of the step before (Learn)
     // this neuron's learning variables in shared memory behind the spike bits, one column per thread
     LearnVars lv;
@@ -1994,22 +2057,14 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
         }
     }
     if constexpr (Learn) sLast = active && deliverFirst ? __ldcg(P.sInfo + (size_t)((t0 - 1) & 1) * P.nV1 + i) : 0.f;
-    for (int s = 0; s < steps; s++) {
+    if (smemSyn && smemBits) fetch_bits(sm, smB, lgnBits + (size_t)lgnSlot * P.lgnW, P.lgnW, 0);
+    for (; s < steps; s++) {
         const long long t = t0 + s;
         const int par = (int)(t & 1);
         const bool dl = s > 0 || deliverFirst;
-        if (list && dl) {
-            if (!wait_spikes(sm, par ^ 1, ph)) {
-                atomicOr(P.err, kErrBarrier);
-                sm.peerFail = 1u;
-            }
-            if (sm.peerFail) {   // a CTA of the block gave up: all of them leave here
-                ok = false;
-                if (threadIdx.x == 0) sm.abortStep = s;
-                hand_over();
-                break;
-            }
-        } else if (!coupled) {
+        if (list && dl && lost < 0) {
+            if (!wait_spikes(sm, par ^ 1, ph, spins, &sm.stop)) lose(2 * s);
+        } else if (!coupled && !list) {
             neuron_sync();
         }
         const int lgnNext = lgnSlot + 1 == lgnSlots ? 0 : lgnSlot + 1;
@@ -2018,13 +2073,17 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
         if (smemSyn) {
             // the other buffer was read in step s - 1, before the spikes (or barrier) just waited for
             const unsigned *bits = lgnBits + (size_t)lgnSlot * P.lgnW;
-            if (smemBits) {
+            if (smemBits && lost < 0) {
                 const int buf = s & 1;
                 if (s + 1 < steps)
                     fetch_bits(sm, smB + (buf ^ 1) * bitRoom, lgnBits + (size_t)lgnNext * P.lgnW, P.lgnW, buf ^ 1);
-                if (mbar_wait(smem_at(&sm.bitBar[buf]), buf ? ph.bit1 : ph.bit0)) bits = smB + buf * bitRoom;
-                if (buf) ph.bit1 ^= 1u;
-                else ph.bit0 ^= 1u;
+                if (mbar_wait(smem_at(&sm.bitBar[buf]), buf ? ph.bit1 : ph.bit0, kMbarSpins)) {
+                    bits = smB + buf * bitRoom;
+                    if (buf) ph.bit1 ^= 1u;
+                    else ph.bit0 ^= 1u;
+                } else {
+                    lose(2 * s + 1);
+                }
             }
             if (active) in = lgn_spikes(bits, lgnSInfo, smI, smW, m, rows >> 2);
         }
@@ -2045,23 +2104,16 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
         // neighbour list they come after the barrier
         const bool ffEarly = list || !dl;
         if (ffEarly) feed_forward();
-        if (s > 0 && nCta > 1 && barrier && (coupled || s == 1)) {
-            // every CTA's arrival of step s - 1; uncoupled, that every CTA has started
-            const unsigned target = (unsigned)nCta * (coupled ? (unsigned)s : 1u);
-            if (!barrier_wait(coupled ? barrier : barrier + 1, target, sm, P.err, P.waitSpins)) {
-                ok = false;
-                // peers that passed this barrier still send step s to this CTA: it tells them to leave and
-                // stays until all of the block have sent
-                if (list && s + 1 < steps) {
-                    publish_spikes(P, sm, par, csize, rank, false, 0.f, isE, true);
-                    wait_spikes(sm, par, ph);
-                }
+        if (s > 0 && (coupled || (s == 1 && count))) {
+            // behind every CTA's arrival of step s - 1; uncoupled, behind the start of every CTA
+            if (!meet(count, (unsigned)nCta * (coupled ? (unsigned)s : 1u), lost >= 0, P.err, P.waitSpins)) {
+                if (lost < 0) give_up(sm, list ? csize : 1, P.err, count);
                 if (threadIdx.x == 0) sm.abortStep = s;
                 hand_over();
                 break;
             }
-        } else if (s > 0 && coupled) {
-            neuron_sync();   // one CTA: thread 0 has made room for this step's spikers
+        } else if (lost >= 0 && list && !coupled && (s > 0 || !count)) {
+            break;
         }
         if (dl) {
             if (!list) {
@@ -2151,7 +2203,8 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
         if (Rng && P.condRng) P.rGenCond[i] = condState;
         if (Rng && P.noiseRng) P.rNoisy[i] = noisyState;
     }
-    return ok;
+    const int sent = min(s, steps - 1);
+    return leave_block(sm, list, csize, rank, t0, sent, lost < 0 ? sent : (lost - 1) >> 1, s < steps || lost >= 0, ph);
 }
 
 // CTAs per cluster, as launched: a tool that relaunches the kernel without clusters gets the
