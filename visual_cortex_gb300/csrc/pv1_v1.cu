@@ -2204,6 +2204,12 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
         if (Rng && P.noiseRng) P.rNoisy[i] = noisyState;
     }
     const int sent = min(s, steps - 1);
+    if (smemSyn && smemBits && threadIdx.x < 32 && (s < steps || lost >= 0)) {
+        // gave up: no CTA ends under a copy into it.  Copies are asked for a step ahead, and not any more once lost
+        const int first = lost < 0 ? s + 1 : lost >> 1, last = lost < 0 ? s + 1 : (lost + 1) >> 1;
+        for (int q = first; q <= last && q < steps; q++)
+            mbar_wait(smem_at(&sm.bitBar[q & 1]), q & 1 ? ph.bit1 : ph.bit0, kMbarSpins);
+    }
     return leave_block(sm, list, csize, rank, t0, sent, lost < 0 ? sent : (lost - 1) >> 1, s < steps || lost >= 0, ph);
 }
 
