@@ -1593,17 +1593,23 @@ __device__ __forceinline__ void announce(unsigned bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                  : "memory");
 }
+// One poll of a phase.
+__device__ __forceinline__ unsigned mbar_poll(unsigned bar, unsigned parity) {
+    unsigned ok;
+    asm volatile(
+        "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok;
+}
 // Bounded wait of a whole warp for a phase; false (for all its lanes) if it does not complete, or, with
 // stop, once a warp of the block has given up.
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, int spins, const int *stop = nullptr) {
-    unsigned ok = 0u;
-    for (int i = 0; i <= spins; i++) {
-        asm volatile(
-            "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (ok || (stop && *(volatile const int *)stop)) break;
+__device__ __noinline__ bool mbar_wait(unsigned bar, unsigned parity, int spins, const int *stop) {
+    unsigned ok = mbar_poll(bar, parity);
+    for (int i = 0; i < spins && !ok; i++) {
+        if (stop && *(volatile const int *)stop) break;
+        ok = mbar_poll(bar, parity);
     }
     return __all_sync(0xffffffffu, ok);
 }
@@ -1658,7 +1664,7 @@ __device__ __forceinline__ void init_barriers(PShared &sm, int csize) {
 // meeting is behind its wait for the grid, and for all warps alike.  At the end the warps of a block
 // tell each other how far they came; if one gave up they make up the announcements that are missing
 // and stay until what they were sent has arrived (leave_block).
-__device__ __forceinline__ void give_up(PShared &sm, int csize, int *err, unsigned *count) {
+__device__ __noinline__ void give_up(PShared &sm, int csize, int *err, unsigned *count) {
     const int lane = threadIdx.x & 31;
     if (lane == 0) {
         atomicOr(err, kErrBarrier);
@@ -1739,14 +1745,6 @@ __device__ __forceinline__ void publish_spikes(const V1Params &P, PShared &sm, i
     }
 }
 
-// Waits for the block's spikes of the step with parity par; false if they did not come.
-__device__ __forceinline__ bool wait_spikes(PShared &sm, int par, Phases &ph, int spins, const int *stop) {
-    if (!mbar_wait(smem_at(&sm.nearBar[par]), par ? ph.near1 : ph.near0, spins, stop)) return false;
-    if (par) ph.near1 ^= 1u;
-    else ph.near0 ^= 1u;
-    return true;
-}
-
 // The end of a block's steps, for all threads of its csize CTAs (a cluster if exchange, with the spikes
 // sent between them).  sent: the first step from t0 whose spikes this warp did not publish, due: the first
 // one whose spikes it did not take.  False for all of them if one of them failed.  The warps of a block
@@ -1767,8 +1765,9 @@ __device__ __noinline__ bool leave_block(PShared &sm, bool exchange, int csize, 
         if (lane < csize) announce(at_rank(smem_at(&sm.nearBar[(t0 + q) & 1]), lane), 0u);
     for (int q = due; q < last; q++) {
         // a barrier's last phase is complete only after those before it
-        if (q + 2 >= last) wait_spikes(sm, (int)((t0 + q) & 1), ph, kMbarSpins, nullptr);
-        else if ((t0 + q) & 1) ph.near1 ^= 1u;
+        const int par = (int)((t0 + q) & 1);
+        if (q + 2 >= last) mbar_wait(smem_at(&sm.nearBar[par]), par ? ph.near1 : ph.near0, kMbarSpins, nullptr);
+        if (par) ph.near1 ^= 1u;
         else ph.near0 ^= 1u;
     }
     return false;
@@ -2032,10 +2031,6 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
     const int spins = csize > 1 ? (int)min(P.waitSpins / kGridPolls, (long long)kMbarSpins << 8) : kMbarSpins;
     int s = 0;
     int lost = -1;   // 2 x the step whose wait for spikes ran out, + 1 if it was the one for the bits
-    auto lose = [&](int where) {
-        lost = where;
-        give_up(sm, list ? csize : 1, P.err, count);
-    };
     float sLast = 0.f;   // the spike word of the step before (Learn)
     // this neuron's learning variables in shared memory behind the spike bits, one column per thread
     LearnVars lv;
@@ -2062,11 +2057,30 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
         const long long t = t0 + s;
         const int par = (int)(t & 1);
         const bool dl = s > 0 || deliverFirst;
-        if (list && dl && lost < 0) {
-            if (!wait_spikes(sm, par ^ 1, ph, spins, &sm.stop)) lose(2 * s);
-        } else if (!coupled && !list) {
-            neuron_sync();
+        const int buf = s & 1;
+        if (lost < 0) {
+            // step t - 1's spikes and step t's bits: mostly both are there, or come, at the first poll
+            const bool spikes = list && dl, copied = smemSyn && smemBits;
+            const unsigned nearBar = smem_at(&sm.nearBar[par ^ 1]), bitBar = smem_at(&sm.bitBar[buf]);
+            const unsigned nearPar = par ? ph.near0 : ph.near1, bitPar = buf ? ph.bit1 : ph.bit0;
+            unsigned ok = 1u;
+            if (spikes) ok = mbar_poll(nearBar, nearPar);
+            if (copied) ok &= mbar_poll(bitBar, bitPar);
+            if (!__all_sync(0xffffffffu, ok)) {
+                if (spikes && !mbar_wait(nearBar, nearPar, spins, &sm.stop)) lost = 2 * s;
+                else if (copied && !mbar_wait(bitBar, bitPar, kMbarSpins, nullptr)) lost = 2 * s + 1;
+                if (lost >= 0) give_up(sm, list ? csize : 1, P.err, count);
+            }
+            if (spikes && lost != 2 * s) {
+                if (par) ph.near0 ^= 1u;
+                else ph.near1 ^= 1u;
+            }
+            if (copied && lost < 0) {
+                if (buf) ph.bit1 ^= 1u;
+                else ph.bit0 ^= 1u;
+            }
         }
+        if (!coupled && !list) neuron_sync();
         const int lgnNext = lgnSlot + 1 == lgnSlots ? 0 : lgnSlot + 1;
         const float *lgnSInfo = lgnRing + (size_t)lgnSlot * P.lgnN;
         LgnIn in{};
@@ -2074,16 +2088,9 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
             // the other buffer was read in step s - 1, before the spikes (or barrier) just waited for
             const unsigned *bits = lgnBits + (size_t)lgnSlot * P.lgnW;
             if (smemBits && lost < 0) {
-                const int buf = s & 1;
+                bits = smB + buf * bitRoom;
                 if (s + 1 < steps)
                     fetch_bits(sm, smB + (buf ^ 1) * bitRoom, lgnBits + (size_t)lgnNext * P.lgnW, P.lgnW, buf ^ 1);
-                if (mbar_wait(smem_at(&sm.bitBar[buf]), buf ? ph.bit1 : ph.bit0, kMbarSpins)) {
-                    bits = smB + buf * bitRoom;
-                    if (buf) ph.bit1 ^= 1u;
-                    else ph.bit0 ^= 1u;
-                } else {
-                    lose(2 * s + 1);
-                }
             }
             if (active) in = lgn_spikes(bits, lgnSInfo, smI, smW, m, rows >> 2);
         }
@@ -2206,9 +2213,8 @@ __device__ __forceinline__ bool persistent_steps(const V1Params &P, long long t0
     const int sent = min(s, steps - 1);
     if (smemSyn && smemBits && threadIdx.x < 32 && (s < steps || lost >= 0)) {
         // gave up: no CTA ends under a copy into it.  Copies are asked for a step ahead, and not any more once lost
-        const int first = lost < 0 ? s + 1 : lost >> 1, last = lost < 0 ? s + 1 : (lost + 1) >> 1;
-        for (int q = first; q <= last && q < steps; q++)
-            mbar_wait(smem_at(&sm.bitBar[q & 1]), q & 1 ? ph.bit1 : ph.bit0, kMbarSpins);
+        const int q = lost < 0 ? s + 1 : lost >> 1;
+        if (q < steps) mbar_wait(smem_at(&sm.bitBar[q & 1]), q & 1 ? ph.bit1 : ph.bit0, kMbarSpins, nullptr);
     }
     return leave_block(sm, list, csize, rank, t0, sent, lost < 0 ? sent : (lost - 1) >> 1, s < steps || lost >= 0, ph);
 }
