@@ -552,9 +552,9 @@ typedef struct {
                          * recurrent spike input is held constant in the backward (stop-gradient),
                          * the usual cure for the exploding recurrent surrogate gradient */
     uint32_t ctaSplit;  /* CTAs per (trial, block), joined in a thread-block cluster: 1 or 2;
-                         * 0 = 2 when blockSize is a multiple of 64 and B * nblock * 2 CTAs fit
-                         * the SMs, else 1.  Results do not depend on it (up to the order of the
-                         * FP64 atomic sums of dL/d(kernel constants)). */
+                         * 0 = 2 when blockSize is a multiple of 64 from 256 on and B * nblock * 2
+                         * CTAs fit the SMs, but 1 in a backward with recGrad, else 1.  Results do
+                         * not depend on it (up to the order of the atomic sums of the gradients). */
 } pv1_adj_problem;
 
 typedef struct {
@@ -571,7 +571,7 @@ typedef struct {
     const float *gV;      /* [B][nWin][N] dL/dvbar (may be null) */
     float *gW;            /* out [K][N] dL/dW, accumulated (zero it first) */
     double *gC;           /* out [6] dL/d(EdE, ErE, dodE, EdI, ErI, dodI), accumulated */
-    float *scratch;       /* [B*nblock][seg][6][blockSize] recompute buffer */
+    float *scratch;       /* [B*nblock][seg][7][blockSize] recompute buffer */
 } pv1_adj_buffers;
 
 /* The kernels' waits are bounded (about a second): where one runs out, its neurons' potentials, and with

@@ -133,8 +133,8 @@ __device__ __forceinline__ float adj_neuron_step(const pv1_adj_problem &P, AStat
 // of the step: the backward goes from the last step to the segment before, which can have the
 // same one.)
 // Measured, with the staged inhibitory weights below: forward and backward of 4,096 neurons x 16 trials x
-// 4,000 steps 40,384 -> 22,120 us (23,737 without them), of two blocks of 128 neurons x 320 steps with
-// the recurrent term 3,784 -> 2,914 us.
+// 4,000 steps 40,384 -> 22,530 us (some 1,600 more without them), of two blocks of 128 neurons x 320 steps
+// with the recurrent term 3,784 -> 2,914 us (1,737 with one CTA per block, as adj_check chooses now).
 struct AdjShared {
     unsigned ball[2][32];
     unsigned *mask[2], *many[2];   // per neuron of the CTA: synapses with an event; those with a count above 1

@@ -261,7 +261,7 @@ __device__ __forceinline__ void tmem_ld32(unsigned taddr, float *v) {
 //   rates  R holds the tile's dt * rate          free   the generators are done with R
 //   zero   the tile's words are zero in memory
 // Measured: the whole run (seeding, this kernel, the recorded rates read back) of 16,384 cells x 16,000 steps
-// 1,495 -> 984 us, against two warpgroups that took rates and generators of a tile in turn and stored
+// 1,495 -> 991 us, against two warpgroups that took rates and generators of a tile in turn and stored
 // every word from the generator's lanes; the generators are what is left (four warps of divergent chains).
 // R is [cell][step] with rows of kRRow floats: 16-byte accesses of consecutive lanes fall into all banks.
 constexpr int kTcThreads = 14 * 32;

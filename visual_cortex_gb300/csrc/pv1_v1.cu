@@ -911,7 +911,7 @@ __device__ __forceinline__ LearnDecay learn_decay(const V1Params &P, const FFTyp
 // by one, each waited for its own reads: 15 of the 26 us of a per-step launch).  In the persistent
 // kernel (in: the step's LGN spikes; else null) only the words of cells that spiked are read, and weights, ids and the
 // neuron's variables stay in shared memory for the K steps.  200 steps of 2 x 1,024 neurons with 20
-// synapses: 6,407 us as launches per step, 2,280 us so (2,741 with each synapse's own expf and reads, 2,941
+// synapses: 6,221 us as launches per step, 2,359 us so (2,741 with each synapse's own expf and reads, 2,941
 // with words and traces in registers for all ten synapses' paths: spills).
 constexpr int kLearnChunk = 10;
 constexpr int kLearnVars = 6;   // learning variables a persistent thread keeps in shared memory
@@ -1557,9 +1557,9 @@ __global__ void __launch_bounds__(kCta) v1_step_kernel(V1Params P, const long lo
 //     wait.
 // Bound by the latency of one warp's instruction stream (two warps per scheduler).  Measured per
 // call, against general CTAs with a full grid barrier per step and LGN words per synapse: one block
-// 800 steps 5,715 -> 3,380 us, 4 blocks with noise and failures 301 steps 3,151 -> 1,990, 8 blocks
-// with far synapses 203 steps 2,261 -> 1,636, the 32-block patch with its movie 800 steps 13,400 ->
-// 10,320; 12 trials of 4 blocks in one sweep 29,755 -> 16,170.
+// 800 steps 5,698 -> 3,492 us, 4 blocks with noise and failures 301 steps 3,128 -> 2,025, 8 blocks
+// with far synapses 203 steps 2,260 -> 1,689, the 32-block patch with its movie 800 steps 13,039 ->
+// 10,737; 12 trials of 4 blocks in one sweep 29,617 -> 16,424.
 constexpr unsigned kBarrierAbort = 0x80000000u;
 constexpr int kPushU = 2;       // far items a lane fetches together
 constexpr int kMaxBitWords = 2048;   // LGN spike bits kept in shared memory (two rows of up to 65,536 cells)
